@@ -138,8 +138,11 @@ size_t state_device_bytes(const State& s)
                     &s.preToBfs, &s.childOffsets, &s.internalToLeaf, &s.levelRange, &s.leafToInternal, &s.jlist,
                     &s.activeA, &s.activeB, &s.allLeaves, &s.nodeValsTmp, &s.leafNext, &s.nbl, &s.nblCount,
                     &s.rowItems, &s.jlistPrev, &s.walked, &s.walkScratch, &s.coverFlag, &s.coverLeaves, &s.extraCnt,
-                    &s.extraBucket, &s.nblJ})
+                    &s.extraBucket, &s.nblJ, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1],
+                    &s.nearSum[0], &s.nearSum[1], &s.nearCover, &s.nearOver})
         add(*d);
+    add(s.nearNode);
+    add(s.nearLoop);
     add(s.items);
     add(s.extras);
     add(s.extraOff);
@@ -166,8 +169,11 @@ void release_state(State& s)
                     &s.preToBfs, &s.childOffsets, &s.internalToLeaf, &s.levelRange, &s.leafToInternal, &s.jlist,
                     &s.activeA, &s.activeB, &s.allLeaves, &s.nodeValsTmp, &s.leafNext, &s.nbl, &s.nblCount,
                     &s.rowItems, &s.jlistPrev, &s.walked, &s.walkScratch, &s.coverFlag, &s.coverLeaves, &s.extraCnt,
-                    &s.extraBucket, &s.nblJ})
+                    &s.extraBucket, &s.nblJ, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1],
+                    &s.nearSum[0], &s.nearSum[1], &s.nearCover, &s.nearOver})
         b->release(s.st);
+    s.nearNode.release(s.st);
+    s.nearLoop.release(s.st);
     s.items.release(s.st);
     s.extras.release(s.st);
     s.extraOff.release(s.st);
@@ -183,6 +189,12 @@ void release_state(State& s)
     s.loopGraphDef = nullptr;
     s.loopGraphKey.clear();
     s.loopKeyPending.clear();
+    if (s.nearGraphExec) COSMO_CUDA(cudaGraphExecDestroy(s.nearGraphExec));
+    if (s.nearGraphDef) COSMO_CUDA(cudaGraphDestroy(s.nearGraphDef));
+    s.nearGraphExec = nullptr;
+    s.nearGraphDef = nullptr;
+    s.nearGraphKey.clear();
+    s.nearKeyPending.clear();
     for (auto& e : s.evPool) COSMO_CUDA(cudaEventDestroy(e));
     s.evPool.clear();
     if (s.hscal)

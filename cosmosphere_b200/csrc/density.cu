@@ -9,8 +9,10 @@
  * still holds an unconverged particle appends the leaf to the next iteration's list.
  */
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 
+#include "near.cuh"
 #include "newton_kernels.cuh"
 
 namespace cosmo {
@@ -37,11 +39,40 @@ __device__ inline double xi_limiter(const double g[9])
 // The sums of the post-convergence sweep for one particle (src/density_base.cu:529-714),
 // added pair by pair in ascending j, and the finish: rho, gradh at the converged h, div v,
 // the xi limiter and d(div v)/dt.
+constexpr int kGradTerms = 27;   // 21 terms added, then the 6 of the R matrix subtracted
+
+// The terms of one pair, put(k, value) in the order of the sums: W, -q dW/dq - 3W, div v, the
+// velocity and the acceleration gradient, the R matrix.  Separation (dx, dy, dz) at the
+// nearest image, r^2 and q^2 = r^2 / h_i^2.
+template<class Put>
+__device__ __forceinline__ void grad_terms(double dx, double dy, double dz, double r2, double q2, const double4& vi,
+                                           const double4& ai, const double4& vj, const double4& aj, double pm, Put&& put)
+{
+    const double q = sqrt(q2);
+    double wk, dwk;
+    sph_kernel(q2, q, wk, dwk);
+    put(0, wk);
+    put(1, -q * dwk - 3.0 * wk);
+    const double rij = sqrt(r2);
+    const double rij1 = 1.0 / (rij + 2.220446049250313e-16);
+    const double rg = rij1 * dwk;
+    const double rx = dx * rg * pm, ry = dy * rg * pm, rz = dz * rg * pm;
+    const double dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
+    put(2, dvx * rx + dvy * ry + dvz * rz);
+    put(3, dvx * rx); put(4, dvx * ry); put(5, dvx * rz);
+    put(6, dvy * rx); put(7, dvy * ry); put(8, dvy * rz);
+    put(9, dvz * rx); put(10, dvz * ry); put(11, dvz * rz);
+    const double dax = ai.x - aj.x, day = ai.y - aj.y, daz = ai.z - aj.z;
+    put(12, dax * rx); put(13, dax * ry); put(14, dax * rz);
+    put(15, day * rx); put(16, day * ry); put(17, day * rz);
+    put(18, daz * rx); put(19, daz * ry); put(20, daz * rz);
+    put(21, dx * rx); put(22, dx * ry); put(23, dx * rz);
+    put(24, dy * ry); put(25, dy * rz); put(26, dz * rz);
+}
+
 struct GradSums
 {
-    double rhoi = 0.0, gradhi = 0.0, divs = 0.0;
-    double dv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, da[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    double rxx = 0, rxy = 0, rxz = 0, ryy = 0, ryz = 0, rzz = 0;
+    double s[kGradTerms] = {};
     unsigned int gp = 0;
 
     // One pair: separation (dx, dy, dz) at the nearest image, r^2 and q^2 = r^2 / h_i^2.
@@ -49,37 +80,23 @@ struct GradSums
                                         const double4& ai, const double4& vj, const double4& aj, double pm)
     {
         ++gp;
-        const double q = sqrt(q2);
-        double wk, dwk;
-        sph_kernel(q2, q, wk, dwk);
-        rhoi += wk;
-        gradhi += -q * dwk - 3.0 * wk;
-        const double rij = sqrt(r2);
-        const double rij1 = 1.0 / (rij + 2.220446049250313e-16);
-        const double rg = rij1 * dwk;
-        const double rx = dx * rg * pm, ry = dy * rg * pm, rz = dz * rg * pm;
-        const double dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
-        divs += dvx * rx + dvy * ry + dvz * rz;
-        dv[0] += dvx * rx; dv[1] += dvx * ry; dv[2] += dvx * rz;
-        dv[3] += dvy * rx; dv[4] += dvy * ry; dv[5] += dvy * rz;
-        dv[6] += dvz * rx; dv[7] += dvz * ry; dv[8] += dvz * rz;
-        const double dax = ai.x - aj.x, day = ai.y - aj.y, daz = ai.z - aj.z;
-        da[0] += dax * rx; da[1] += dax * ry; da[2] += dax * rz;
-        da[3] += day * rx; da[4] += day * ry; da[5] += day * rz;
-        da[6] += daz * rx; da[7] += daz * ry; da[8] += daz * rz;
-        rxx -= dx * rx; rxy -= dx * ry; rxz -= dx * rz;
-        ryy -= dy * ry; ryz -= dy * rz; rzz -= dz * rz;
+        grad_terms(dx, dy, dz, r2, q2, vi, ai, vj, aj, pm, [&](int k, double v) {
+            if (k < 21) s[k] += v;
+            else s[k] -= v;
+        });
     }
 
     __device__ __forceinline__ void finish(uint32_t i, double hi, double pm, double* __restrict__ rho,
                                            double* __restrict__ gradh, double* __restrict__ divv,
                                            double* __restrict__ xiOut, double* __restrict__ ddivvdt) const
     {
+        const double *dv = s + 3, *da = s + 12;
+        const double rxx = s[21], rxy = s[22], rxz = s[23], ryy = s[24], ryz = s[25], rzz = s[26];
         const double hi1 = 1.0 / hi;
         const double hi31 = hi1 * hi1 * hi1;
         const double hi41 = hi31 * hi1;
-        const double rho_i = rhoi * kCnormk * pm * hi31;
-        const double grad_i = gradhi * kCnormk * pm * hi41;
+        const double rho_i = s[0] * kCnormk * pm * hi31;
+        const double grad_i = s[1] * kCnormk * pm * hi41;
         rho[i] = rho_i;
         gradh[i] = grad_i;
         if (!(rho_i > 0.0))
@@ -98,7 +115,7 @@ struct GradSums
         const double rm3 = rzz * rxx - rxz * rxz;
         const double rm4 = rxy * rxz - rxx * ryz;
         const double rm5 = rxx * ryy - rxy * rxy;
-        divv[i] = -divs * term;
+        divv[i] = -s[2] * term;
         double gm[9], div_a;
         if (fabs(denom) > 2.2250738585072014e-308)
         {
@@ -145,8 +162,10 @@ gradient_row_kernel(int nAlive, const int* __restrict__ nbl, const int* __restri
                     const double4* __restrict__ xyzh, const double4* __restrict__ vel4,
                     const double4* __restrict__ acc4, double* __restrict__ rho, double* __restrict__ gradh,
                     double* __restrict__ divv, double* __restrict__ xiOut, double* __restrict__ ddivvdt,
-                    double pmass, const DevBox* __restrict__ box, DevScalars* __restrict__ ds)
+                    double pmass, const DevBox* __restrict__ box, DevScalars* __restrict__ ds,
+                    const int* __restrict__ active)
 {
+    if (active != nullptr && *active > 0) return;   // the Newton loop did not converge
     double lx = 0, ly = 0, lz = 0;
     if (Periodic) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
     unsigned long long pairs = 0;
@@ -177,6 +196,120 @@ gradient_row_kernel(int nAlive, const int* __restrict__ nbl, const int* __restri
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(&ds->pairs[1], pairs);
+}
+
+// Post-convergence sweep of the particles without a row (the block-tree solve's over list):
+// one warp searches for one particle, evaluates 32 of its pairs at a time, one per lane, and
+// adds their terms in ascending j with one sum per lane.
+template<bool Periodic>
+__global__ void __launch_bounds__(kThreads)
+gradient_over_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L, const int* __restrict__ over,
+                     const double4* __restrict__ vel4, const double4* __restrict__ acc4, double* __restrict__ rho,
+                     double* __restrict__ gradh, double* __restrict__ divv, double* __restrict__ xiOut,
+                     double* __restrict__ ddivvdt, double pmass, DevScalars* __restrict__ ds)
+{
+    __shared__ NearScratch sScr[kWarpsPerBlock];
+    __shared__ double sTerm[kWarpsPerBlock][32 * kGradTerms];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int n = L->over;
+    if (n == 0 || L->active > 0) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ds->rowOverflow = 1;
+    const int nLive = *t.nLive;
+    const NearFrame f(t.box);
+    double lx = 0, ly = 0, lz = 0;
+    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    double* term = sTerm[wib];
+    unsigned long long pairs = 0;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (gridDim.x * blockDim.x) >> 5)
+    {
+        const int i = over[w];
+        const double4 pi = t.xyzh[i], vi = vel4[i], ai = acc4[i];
+        const double hinv2 = 1.0 / (pi.w * pi.w);
+        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
+        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
+        double sum = 0.0;   // lane k: sum k
+        unsigned int gp = 0;
+        near_blocks<Periodic, false>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+            near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
+                double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+                const double r2 = pair_r2(dx, dy, dz);
+                const double q2 = r2 * hinv2;
+                const bool acc = valid && q2 < kRadK2;
+                const uint32_t m = __ballot_sync(0xffffffffu, acc);
+                if (acc)
+                {
+                    double* mine = term + __popc(m & ((1u << lane) - 1u)) * kGradTerms;
+                    grad_terms(dx, dy, dz, r2, q2, vi, ai, ldg4(vel4 + j), ldg4(acc4 + j), pmass,
+                               [&](int k, double v) { mine[k] = v; });
+                }
+                __syncwarp();
+                const int c = __popc(m);
+                gp += c;
+                if (lane < 21)
+                    for (int k = 0; k < c; ++k) sum += term[k * kGradTerms + lane];
+                else if (lane < kGradTerms)
+                    for (int k = 0; k < c; ++k) sum -= term[k * kGradTerms + lane];
+                __syncwarp();
+                return true;
+            });
+            return r;
+        });
+        GradSums g;
+#pragma unroll
+        for (int k = 0; k < kGradTerms; ++k) g.s[k] = __shfl_sync(0xffffffffu, sum, k);
+        if (lane == 0)
+        {
+            pairs += gp;
+            g.finish(uint32_t(i), pi.w, pmass, rho, gradh, divv, xiOut, ddivvdt);
+        }
+    }
+    if (lane == 0 && pairs) atomicAdd(&ds->pairs[1], pairs);
+}
+
+// The pairs the particles without a row add to others' rows: every j within a support of
+// theirs that lies beyond what j's own row covers (the test sym_from_rows_kernel makes for
+// the pairs of a row).
+template<bool Periodic>
+__global__ void __launch_bounds__(kThreads)
+over_extras_kernel(const __grid_constant__ NearTree t, const NearLoop* __restrict__ L, const int* __restrict__ over,
+                   const double* __restrict__ hs, const double* __restrict__ rowH,
+                   unsigned long long* __restrict__ extras, int extraCap, DevScalars* __restrict__ ds)
+{
+    __shared__ NearScratch sScr[kWarpsPerBlock];
+    const int wib = threadIdx.x >> 5;
+    const int n = L->over;
+    if (n == 0) return;
+    const int nLive = *t.nLive;
+    const NearFrame f(t.box);
+    double lx = 0, ly = 0, lz = 0;
+    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (gridDim.x * blockDim.x) >> 5)
+    {
+        const int i = over[w];
+        const double4 pi = t.xyzh[i];
+        const double bi = kRadK2 * (pi.w * pi.w) * (1.0 + 1e-10);
+        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
+        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
+        near_blocks<Periodic, false>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+            near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
+                double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+                const double dr2 = pair_r2(dx, dy, dz);
+                if (valid && dr2 < bi)
+                {
+                    const double hj = hs[j], ch = rowH[j];
+                    if (!(dr2 < kRadK2 * (hj * hj)) && !(dr2 < kRadK2 * (ch * ch) * (1.0 - 1e-9)))
+                    {
+                        const int k = atomicAdd(&ds->extraCount, 1);
+                        if (k < extraCap) extras[k] = (static_cast<unsigned long long>(j) << 32) | uint32_t(i);
+                    }
+                }
+                return true;
+            });
+            return r;
+        });
+    }
 }
 
 // Post-convergence sweep over the group path (src/density_base.cu:529-714) for the
@@ -337,6 +470,7 @@ sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restr
     {
         extraCnt[i] = 0;
         const int cnt = nblCount[i];
+        if (unsigned(cnt) > unsigned(kNbl)) continue;   // no row (its passes search for it)
         const double hi = hs[i];
         const double bi = kRadK2 * (hi * hi) * (1.0 + 1e-10);
         const int4* inJ = reinterpret_cast<const int4*>(row_flat(rowsJ, uint32_t(i)));
@@ -427,18 +561,30 @@ __global__ void extras_place_kernel(const unsigned long long* __restrict__ extra
 
 // Each row owner merges its extras into its row: sorted, those the row already holds
 // dropped, the rest merged in from the back so the row stays ascending.  A row that would
-// exceed kNbl sets mergeOverflow (the symmetric rows are then built instead).
+// exceed kNbl joins the over list when there is one (its passes then search for it), else
+// sets mergeOverflow (the symmetric rows are then built instead).  A particle without a row
+// takes none.
 __global__ void extras_merge_kernel(int nA, const uint32_t* __restrict__ off, int* __restrict__ bucket,
-                                    int* __restrict__ nbl, int* __restrict__ nblCount, DevScalars* __restrict__ ds)
+                                    int* __restrict__ nbl, int* __restrict__ nblCount, DevScalars* __restrict__ ds,
+                                    int* __restrict__ over, int* __restrict__ overCount)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nA) return;
     const uint32_t b0 = off[t], e = off[t + 1] - b0;
     if (e == 0) return;
     const int cnt = nblCount[t];
+    if (unsigned(cnt) > unsigned(kNbl)) return;
+    auto full = [&]() {
+        if (over != nullptr)
+        {
+            nblCount[t] = kNbl + 1;
+            over[atomicAdd(overCount, 1)] = t;
+        }
+        else ds->mergeOverflow = 1;
+    };
     if (cnt + int(e) > 2 * kNbl)
     {
-        ds->mergeOverflow = 1;
+        full();
         return;
     }
     int* ex = bucket + b0;
@@ -467,7 +613,7 @@ __global__ void extras_merge_kernel(int nA, const uint32_t* __restrict__ off, in
     if (u == 0) return;
     if (cnt + int(u) > kNbl)
     {
-        ds->mergeOverflow = 1;
+        full();
         return;
     }
     int r = cnt - 1, x = int(u) - 1, w = cnt + int(u) - 1;
@@ -909,7 +1055,7 @@ static bool cover_rows(State& s, int itemCap, FixedSplit cut, int spreadG)
 // pairs other particles' supports add, merged into their rows -- all on the device, the
 // extras' number read there.  Whether they all fitted is known from extraCount (at most
 // extraCap) and mergeOverflow once the stream has been read.
-static void sym_rows_from_newton(State& s, int extraCap)
+static void sym_rows_from_newton(State& s, int extraCap, bool near)
 {
     DevScalars* ds = s.dscal.get();
     const int nA = s.nAlive;
@@ -934,6 +1080,13 @@ static void sym_rows_from_newton(State& s, int extraCap)
     }
     else compact(sym_from_rows_kernel<double, false>, s.nblR2.get());
     COSMO_LAUNCHED();
+    if (near)
+    {
+        auto ov = s.periodic ? over_extras_kernel<true> : over_extras_kernel<false>;
+        ov<<<2 * s.numSMs, kThreads, 0, s.st>>>(near_tree(s), s.nearLoop.get(), s.nearOver.get(), s.hs.get(),
+                                                s.nblH.get(), s.extras.get(), extraCap, ds);
+        COSMO_LAUNCHED();
+    }
     extras_count_kernel<<<iceil(extraCap, 256), 256, 0, s.st>>>(s.extras.get(), extraCap, ds, s.extraCnt.get());
     COSMO_LAUNCHED();
     scan_exclusive(s, reinterpret_cast<const uint32_t*>(s.extraCnt.get()), s.extraOff.get(), nA, false);
@@ -941,8 +1094,19 @@ static void sym_rows_from_newton(State& s, int extraCap)
                                                                s.extraCnt.get(), s.extraBucket.get());
     COSMO_LAUNCHED();
     extras_merge_kernel<<<iceil(nA, 256), 256, 0, s.st>>>(nA, s.extraOff.get(), s.extraBucket.get(), s.nbl.get(),
-                                                         s.nblCount.get(), ds);
+                                                         s.nblCount.get(), ds, near ? s.nearOver.get() : nullptr,
+                                                         near ? &s.nearLoop.get()->over : nullptr);
     COSMO_LAUNCHED();
+}
+
+// Whether a solve's Newton loop runs over the block tree (near.cu): the plain form with the
+// gradient sweep.  The mixed form keeps the group engine (its rounding is defined by the
+// groups), a solve without gradients the lists it must leave behind, and so does one asked
+// for a variant of the list-based loop.
+static bool near_solve(const State& s, bool withGradients)
+{
+    return withGradients && s.precision == 0 && s.staging == 0 && s.splitStream == 0 && s.splitWork == 0 &&
+           s.spreadGroups == 0 && s.graphListStorePct == 0;
 }
 
 DensResult solve_density(State& s, int n, double pmass, const double* periodicBox, double tolh, double hfact,
@@ -966,7 +1130,9 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     // next few solves do not write them.
     const bool tryRows = s.symRowsSkip == 0;
     if (s.symRowsSkip > 0) --s.symRowsSkip;
-    const bool writeJ = withGradients && s.symFromRows && s.frozenFor != n && tryRows;
+    const bool near = near_solve(s, withGradients);
+    const bool writeJ = near ? s.symFromRows != 0
+                             : withGradients && s.symFromRows && s.frozenFor != n && tryRows;
 
     // the tree; its particle gather also zeroes rho, gradh, the convergence flags, the
     // Newton rows' h (0: no row this solve) and the pair counters
@@ -977,8 +1143,11 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     s.activeB.resize(nL, s.st);
     s.leafNext.resize(nL, s.st);
     const int itemCap = std::max(s.nAlive, 1);
-    s.items.resize(itemCap, s.st);
-    s.rowItems.resize(itemCap, s.st);
+    if (!near)
+    {
+        s.items.resize(itemCap, s.st);
+        s.rowItems.resize(itemCap, s.st);
+    }
     s.nblR2.resize(size_t(itemCap) * kNbl, s.st);
     s.nblCount.resize(itemCap, s.st);
     s.nblH.resize(itemCap, s.st);
@@ -994,14 +1163,17 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     s.rowsFromNewton = false;
     s.hmaxNodeDone = true;
     s.listsLoose = false;
+    s.nearOverCount = 0;
+    if (near) s.listsSym = false;
 
     // the host loop swaps the two active-leaf buffers every iteration: put them back in
     // one order, so that a graph captured with them serves the next solve too
     if (s.activeA.get() > s.activeB.get()) std::swap(s.activeA, s.activeB);
-    COSMO_CUDA(cudaMemcpyAsync(s.activeA.get(), s.allLeaves.get(), size_t(nL) * 4, cudaMemcpyDeviceToDevice, s.st));
+    if (!near)
+        COSMO_CUDA(cudaMemcpyAsync(s.activeA.get(), s.allLeaves.get(), size_t(nL) * 4, cudaMemcpyDeviceToDevice, s.st));
     int nActiveLeaves = nL;
     long long nActiveParticles = s.nAlive;
-    if (s.frozenFor == n && s.nAlive > 0)
+    if (!near && s.frozenFor == n && s.nAlive > 0)
     {
         // the caller's fixed particles start converged: neighbours only
         COSMO_CUDA(cudaMemsetAsync(&ds->frozenAlive, 0, sizeof(int), s.st));
@@ -1025,7 +1197,9 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     bool listsValid = false, listsWidened = false, rowsReady = false;
     long long settlingPrev = 0;
     bool graphRan = false;
-    if (allowGraph && s.newtonGraph && maxIter <= kLoopIters && nActiveParticles > 0)
+    cudaEvent_t n0 = ev(s);
+    if (near) near_newton(s, pmass, tolh, hfact, maxIter, allowGraph, writeJ ? rowsJ : nullptr);
+    else if (allowGraph && s.newtonGraph && maxIter <= kLoopIters && nActiveParticles > 0)
     {
         const LoopGraph lg =
             newton_loop_graph(s, pmass, tolh, hfact, maxIter, cut, spreadG, nActiveParticles, rowsJ);
@@ -1042,9 +1216,9 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             return solve_density(s, n, pmass, periodicBox, tolh, hfact, maxIter, withGradients, false);
         }
     }
-    s.lastLoopGraph = graphRan ? 1 : 0;
+    if (!near) s.lastLoopGraph = graphRan ? 1 : 0;
     cudaEvent_t e3 = ev(s);
-    for (int iter = 0; iter < maxIter && !graphRan; ++iter)
+    for (int iter = 0; iter < maxIter && !graphRan && !near; ++iter)
     {
         cudaEvent_t j0 = ev(s);
         hmax_leaves(s, s.activeA.get(), nActiveLeaves);
@@ -1123,7 +1297,6 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         std::swap(s.activeA, s.activeB);
         if (nActiveParticles == 0) break;
     }
-    (void)e3;
     if (listsWidened && !withGradients)
     {
         cudaEvent_t j0 = ev(s);
@@ -1132,16 +1305,19 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         COSMO_CUDA(cudaEventSynchronize(j1));
         s.t.jbuild += elapsed_s(j0, j1);
     }
-    check_dev_err(s, "solveDensH", listsWidened && !withGradients);
-    tree_timings(s);
-    res.itersRun = s.itersRun;
-    res.unconverged = int(nActiveParticles);
-    if (nActiveParticles > 0)
+    if (!near)
     {
-        res.status = 1;
-        return res;
+        check_dev_err(s, "solveDensH", listsWidened && !withGradients);
+        tree_timings(s);
+        res.itersRun = s.itersRun;
+        res.unconverged = int(nActiveParticles);
+        if (nActiveParticles > 0)
+        {
+            res.status = 1;
+            return res;
+        }
     }
-    if (s.periodic && s.nAlive > 0)
+    if (!near && s.periodic && s.nAlive > 0)
     {
         const int nb = std::min(iceil(s.nAlive, 256), 2 * s.numSMs);
         s.redTmp.resize(std::max<size_t>(s.redTmp.n, nb), s.st, false);
@@ -1170,10 +1346,19 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         cudaEvent_t g0 = ev(s);
         hmax_leaves(s, s.allLeaves.get(), nL);
         const bool rowsBuilt = graphRan ? s.lastLoopRowBuilds > 0 : rowsReady;
-        fromRows = writeJ && s.nAlive > 0 && rowsBuilt && cover_rows(s, itemCap, cut, spreadG);
-        const int extraCap = s.symExtraCap > 0 ? std::min(s.symExtraCap, itemCap) : itemCap;
+        // the block-tree loop's rows cover every particle but those it lists (over)
+        if (near && writeJ && s.nAlive > 0)
+        {
+            near_cover(s, rowsJ);
+            fromRows = true;
+        }
+        else
+            fromRows = writeJ && s.nAlive > 0 && rowsBuilt && cover_rows(s, itemCap, cut, spreadG);
+        // pairs other particles' supports add: about ten a particle where h scatters
+        const int extraCap = s.symExtraCap > 0 ? std::min(s.symExtraCap, itemCap) : near ? int(std::min(16ll * itemCap, 1ll << 30)) : itemCap;
+        const int* active = near ? &s.nearLoop.get()->active : nullptr;
         if (fromRows)
-            sym_rows_from_newton(s, extraCap);
+            sym_rows_from_newton(s, extraCap, near);
         else
         {
             build_symmetric(s);
@@ -1188,15 +1373,23 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             auto gr = s.periodic ? gradient_row_kernel<true> : gradient_row_kernel<false>;
             gr<<<std::max(1, std::min(iceil(s.nAlive, kThreads), 8 * s.numSMs)), kThreads, 0, s.st>>>(
                 s.nAlive, s.nbl.get(), s.nblCount.get(), s.xyzh.get(), s.vel4.get(), s.acc4.get(), s.rho.get(),
-                s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), ds);
+                s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), ds, active);
             COSMO_LAUNCHED();
+            if (near && fromRows)
+            {
+                auto go = s.periodic ? gradient_over_kernel<true> : gradient_over_kernel<false>;
+                go<<<2 * s.numSMs, kThreads, 0, s.st>>>(near_tree(s), s.nearLoop.get(), s.nearOver.get(), s.vel4.get(),
+                                                        s.acc4.get(), s.rho.get(), s.gradh.get(), s.divv.get(),
+                                                        s.xi.get(), s.ddivvdt.get(), pmass, ds);
+                COSMO_LAUNCHED();
+            }
             // the group sweep of the rows that overflowed (none: it returns at once)
             auto gk = s.periodic ? gradient_kernel<true> : gradient_kernel<false>;
-            gk<<<grid, kThreads, 0, s.st>>>(nL, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),
+            if (!(near && fromRows)) gk<<<grid, kThreads, 0, s.st>>>(nL, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),
                                             s.xyzh.get(), s.vel4.get(), s.acc4.get(), s.rho.get(), s.gradh.get(),
                                             s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(),
                                             s.nblCount.get(), ds);
-            COSMO_LAUNCHED();
+            if (!(near && fromRows)) COSMO_LAUNCHED();
         }
         if (n > s.nAlive)
         {
@@ -1205,10 +1398,41 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             COSMO_LAUNCHED();
         }
         cudaEvent_t g2 = ev(s);
+        NearLoop nl;
+        if (near)
+            COSMO_CUDA(cudaMemcpyAsync(&nl, s.nearLoop.get(), sizeof(NearLoop), cudaMemcpyDeviceToHost, s.st));
         read_scalars(s);
+        if (near)
+        {
+            check_dev_err(s, "solveDensH", false);
+            tree_timings(s);
+            nActiveParticles = near_results(s, nl);
+            s.nearOverCount = nl.over;
+            s.t.nrkern += elapsed_s(n0, e3);
+            res.itersRun = s.itersRun;
+            res.unconverged = int(nActiveParticles);
+            s.hscal->unconverged = res.unconverged;
+            if (nActiveParticles > 0)
+            {
+                res.status = 1;
+                return res;
+            }
+            if (s.periodic && s.nAlive > 0)
+            {
+                double hm;
+                std::memcpy(&hm, &s.hscal->hmaxConv, sizeof hm);
+                const double lmin = std::min({periodicBox[1] - periodicBox[0], periodicBox[3] - periodicBox[2],
+                                              periodicBox[5] - periodicBox[4]});
+                if (kRadKernel * hm >= 0.5 * lmin)
+                {
+                    res.status = 2;
+                    return res;
+                }
+            }
+        }
         // the rows serve the force pass if every extra was kept and merged
         if (fromRows) s.rowsFromNewton = s.hscal->extraCount <= extraCap && s.hscal->mergeOverflow == 0;
-        if (writeJ && !s.rowsFromNewton) s.symRowsSkip = kSymRowsSkip;
+        if (writeJ && !near && !s.rowsFromNewton) s.symRowsSkip = kSymRowsSkip;
         s.t.gjbuild += elapsed_s(g0, g1);
         s.t.gradkern += elapsed_s(g1, g2);
     }
@@ -1222,7 +1446,8 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         s.hmaxNodeDone = false;
     }
     // the lists held are the Newton loop's widened gather lists
-    s.listsLoose = withGradients && !symBuilt && listsWidened;
+    // (the block-tree loop makes none: what is held belongs to an earlier tree)
+    s.listsLoose = withGradients && !symBuilt && (listsWidened || near);
     return res;
 }
 

@@ -7,6 +7,7 @@
  */
 #include <algorithm>
 
+#include "near.cuh"
 #include "pairstream.cuh"
 #include "rows.cuh"
 #include "state.hpp"
@@ -54,6 +55,12 @@ __global__ void force_prep_kernel(const double4* __restrict__ xyzh, const double
     vel4[i].w = grkfac;
 }
 
+// The terms of one pair's force, put in the sums' own order: the i-side pressure (added), the
+// j-side pressure (subtracted), the four energy terms (pdV, shock, the two conductions, added
+// one after the other to one sum), div v, and the signal velocity (a maximum).
+constexpr int kForceTerms = 12;
+enum : int { kFix = 0, kFiy, kFiz, kFjx, kFjy, kFjz, kFpdv, kFdiss, kFcondi, kFcondj, kFdiv, kFvs };
+
 // The i-side quantities of one particle and its force sums.
 struct ForceAcc
 {
@@ -70,20 +77,22 @@ struct ForceAcc
     }
 
     // One pair with j (src/force.cu:232-383): the exact tests dr^2 > 0 and
-    // dr^2 < R^2 max(h_i^2, h_j^2)(1 + 1e-10), then the i-side and j-side terms.  The j
-    // side is four 32-byte records (xyzh, prepA, vel4 with grkfac, thermo4).
-    template<bool Periodic, bool Disc>
-    __device__ __forceinline__ void add(const double4& pj, int j, const double4* __restrict__ vel4,
-                                        const double4* __restrict__ thermo4, const double4* __restrict__ prepA,
-                                        double lx, double ly, double lz, double pm, double alphau, double beta,
-                                        int pdv, int shock)
+    // dr^2 < R^2 max(h_i^2, h_j^2)(1 + 1e-10), then the i-side and j-side terms, handed to
+    // put(k, value) in the order of the sums (a side outside its support hands none).  The j
+    // side is four 32-byte records (xyzh, prepA, vel4 with grkfac, thermo4).  Returns whether
+    // either side took it.
+    template<bool Periodic, bool Disc, class Put>
+    __device__ __forceinline__ bool terms(const double4& pj, int j, const double4* __restrict__ vel4,
+                                          const double4* __restrict__ thermo4, const double4* __restrict__ prepA,
+                                          double lx, double ly, double lz, double pm, double alphau, double beta,
+                                          int pdv, int shock, Put&& put) const
     {
         double dx = p.x - pj.x, dy = p.y - pj.y, dz = p.z - pj.z;
         nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
         const double dr2 = pair_r2(dx, dy, dz);
-        if (!(dr2 > 0.0)) return;
+        if (!(dr2 > 0.0)) return false;
         const double hi = p.w, hj = pj.w;
-        if (dr2 >= kRadK2 * fmax(hi * hi, hj * hj) * (1.0 + 1e-10)) return;
+        if (dr2 >= kRadK2 * fmax(hi * hi, hj * hj) * (1.0 + 1e-10)) return false;
         const double pro2i = t.x, vwavei = t.y, alphai = t.z, eni = t.w;
         const double hsqinvi = a.x, hinvi = a.y, rhoi = a.z, rho1i = a.w;
         const double grkfaci = b.x, pri = b.y, autermi = b.z;
@@ -133,34 +142,59 @@ struct ForceAcc
         if (qi2 < kRadK2)
         {
             took = true;
-            vsm = fmax(vsm, pvs);
+            put(kFvs, pvs);
             double wk, dwk;
             const double q = dr * hinvi;
             sph_kernel(qi2, q, wk, dwk);
-            divs += pm * dwk * projv;
+            put(kFdiv, pm * dwk * projv);
             const double gki = dwk * grkfaci;
             const double gpi = pm * (pro2i + qr2i) * gki;
-            itx += -gpi * rx; ity += -gpi * ry; itz += -gpi * rz;
+            put(kFix, -gpi * rx); put(kFiy, -gpi * ry); put(kFiz, -gpi * rz);
             const double pdvi = pm * pro2i * projv * gki;
             const double dissi = Disc ? -0.5 * pm * rho1i * alphai * vwavei * (hi * rij1) * projv * projv * gki
                                       : pm * qr2i * projv * gki;
             const double condi = vsigu * denij * autermi * gki;
-            if (pdv) f4s += pdvi;
-            if (shock) f4s += dissi;
-            f4s += condi;
+            if (pdv) put(kFpdv, pdvi);
+            if (shock) put(kFdiss, dissi);
+            put(kFcondi, condi);
         }
         if (qj2 < kRadK2)
         {
             took = true;
-            vsm = fmax(vsm, pvs);
+            put(kFvs, pvs);
             double wk, dwk;
             const double q = dr * aj.y;
             sph_kernel(qj2, q, wk, dwk);
             const double gkj = dwk * vj.w;
             const double gpj = pm * (pro2j + qr2j) * gkj;
-            jtx -= gpj * rx; jty -= gpj * ry; jtz -= gpj * rz;
-            f4s += vsigu * denij * autermj * gkj;
+            put(kFjx, gpj * rx); put(kFjy, gpj * ry); put(kFjz, gpj * rz);
+            put(kFcondj, vsigu * denij * autermj * gkj);
         }
+        return took;
+    }
+
+    // The pair's terms added to the sums.
+    template<bool Periodic, bool Disc>
+    __device__ __forceinline__ void add(const double4& pj, int j, const double4* __restrict__ vel4,
+                                        const double4* __restrict__ thermo4, const double4* __restrict__ prepA,
+                                        double lx, double ly, double lz, double pm, double alphau, double beta,
+                                        int pdv, int shock)
+    {
+        const bool took = terms<Periodic, Disc>(pj, j, vel4, thermo4, prepA, lx, ly, lz, pm, alphau, beta, pdv, shock,
+                                                [&](int k, double x) {
+            switch (k)
+            {
+                case kFix: itx += x; break;
+                case kFiy: ity += x; break;
+                case kFiz: itz += x; break;
+                case kFjx: jtx -= x; break;
+                case kFjy: jty -= x; break;
+                case kFjz: jtz -= x; break;
+                case kFdiv: divs += x; break;
+                case kFvs: vsm = fmax(vsm, x); break;
+                default: f4s += x;
+            }
+        });
         if (took) ++gp;
     }
 
@@ -346,6 +380,83 @@ force_row_kernel(int nAlive, const int* __restrict__ nbl, const int* __restrict_
     if ((threadIdx.x & 31) == 0) atomicAdd(&ds->pairs[2], pairs);
 }
 
+// Force pass of the particles without a row (the block-tree solve's over list): one warp
+// searches for one particle -- its own support and every block's -- evaluates 32 pairs at a
+// time, one per lane, and adds their terms in ascending j with one sum per lane (a term a
+// pair does not have is zero, which leaves its sum as it is).
+template<bool Periodic, bool Disc>
+__global__ void __launch_bounds__(kThreads)
+force_over_kernel(const __grid_constant__ NearTree t, int n, const int* __restrict__ over,
+                  const double4* __restrict__ vel4, const double4* __restrict__ thermo4,
+                  const double4* __restrict__ prepA, const double4* __restrict__ prepB, double* __restrict__ fx,
+                  double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ f4,
+                  double* __restrict__ vsigmax, double* __restrict__ divvF, double pmass, double alphau, double beta,
+                  int pdv, int shock, DevScalars* __restrict__ ds)
+{
+    __shared__ NearScratch sScr[kWarpsPerBlock];
+    __shared__ double sTerm[kWarpsPerBlock][32 * (kForceTerms + 1)];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    constexpr int kStride = kForceTerms + 1;
+    const int nLive = *t.nLive;
+    const NearFrame f(t.box);
+    double lx = 0, ly = 0, lz = 0;
+    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    double* term = sTerm[wib];
+    unsigned long long pairs = 0;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (gridDim.x * blockDim.x) >> 5)
+    {
+        const int i = over[w];
+        ForceAcc A;
+        A.load(uint32_t(i), t.xyzh, vel4, thermo4, prepA, prepB);
+        const float x = float(A.p.x - f.cx), y = float(A.p.y - f.cy), z = float(A.p.z - f.cz);
+        const float slack = f.slack(x, y, z);
+        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * A.p.w) + slack;
+        double sum = 0.0;   // lanes 0-5: the pressure sums, 6: the energy, 7: div v, 8: vsig
+        near_blocks<Periodic, true>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
+            near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
+                double* mine = term + lane * kStride;
+                for (int k = 0; k < kForceTerms; ++k) mine[k] = 0.0;
+                const bool took = valid && A.terms<Periodic, Disc>(pj, j, vel4, thermo4, prepA, lx, ly, lz, pmass,
+                                                                   alphau, beta, pdv, shock,
+                                                                   [&](int k, double v) { mine[k] = v; });
+                uint32_t m = __ballot_sync(0xffffffffu, took);
+                A.gp += __popc(m);
+                __syncwarp();
+                for (; m; m &= m - 1)
+                {
+                    const double* q = term + (__ffs(m) - 1) * kStride;
+                    if (lane < 3) sum += q[lane];
+                    else if (lane < 6) sum -= q[lane];
+                    else if (lane == 6)
+                    {
+                        sum += q[kFpdv];
+                        sum += q[kFdiss];
+                        sum += q[kFcondi];
+                        sum += q[kFcondj];
+                    }
+                    else if (lane == 7) sum += q[kFdiv];
+                    else if (lane == 8) sum = fmax(sum, q[kFvs]);
+                }
+                __syncwarp();
+                return true;
+            });
+            return r;
+        });
+        A.itx = __shfl_sync(0xffffffffu, sum, 0); A.ity = __shfl_sync(0xffffffffu, sum, 1);
+        A.itz = __shfl_sync(0xffffffffu, sum, 2); A.jtx = __shfl_sync(0xffffffffu, sum, 3);
+        A.jty = __shfl_sync(0xffffffffu, sum, 4); A.jtz = __shfl_sync(0xffffffffu, sum, 5);
+        A.f4s = __shfl_sync(0xffffffffu, sum, 6);
+        A.divs = __shfl_sync(0xffffffffu, sum, 7);
+        A.vsm = __shfl_sync(0xffffffffu, sum, 8);
+        if (lane == 0)
+        {
+            pairs += A.gp;
+            A.store(uint32_t(i), fx, fy, fz, f4, vsigmax, divvF);
+        }
+    }
+    if (lane == 0 && pairs) atomicAdd(&ds->pairs[2], pairs);
+}
+
 // Dead particles: no force (src/force.cu:191-200).
 __global__ void force_dead_kernel(int nAlive, int n, double* fx, double* fy, double* fz, double* f4,
                                   double* vsigmax, double* divvF)
@@ -434,10 +545,24 @@ void compute_forces(State& s, double pmass, double beta, double alphau, bool dis
         COSMO_LAUNCHED();
         if (!s.rowsFromNewton)
         {
-            // the group pass of the rows that overflowed (none: it returns at once); rows
-            // from the Newton rows never overflow
+            // the group pass of the rows that overflowed (none: it returns at once)
             if (s.periodic) { if (disc) launch(force_kernel<true, true>); else launch(force_kernel<true, false>); }
             else { if (disc) launch(force_kernel<false, true>); else launch(force_kernel<false, false>); }
+            COSMO_LAUNCHED();
+        }
+        else if (s.nearOverCount > 0)
+        {
+            // the particles whose rows would not hold their pairs.  A node's h are those its
+            // boxes were made with, at the solve's start: remade at the converged h first
+            near_build(s);
+            auto go = [&](auto kern) {
+                kern<<<std::min(iceil(s.nearOverCount, kWarpsPerBlock), 8 * s.numSMs), kThreads, 0, s.st>>>(
+                    near_tree(s), s.nearOverCount, s.nearOver.get(), s.vel4.get(), s.thermo4.get(), s.prepA.get(),
+                    s.prepB.get(), s.fx.get(), s.fy.get(), s.fz.get(), s.f4.get(), s.vsigmax.get(), s.divvF.get(),
+                    pmass, alphau, beta, pdv ? 1 : 0, shock ? 1 : 0, ds);
+            };
+            if (s.periodic) { if (disc) go(force_over_kernel<true, true>); else go(force_over_kernel<true, false>); }
+            else { if (disc) go(force_over_kernel<false, true>); else go(force_over_kernel<false, false>); }
             COSMO_LAUNCHED();
         }
     }

@@ -1,0 +1,912 @@
+/*
+ * near.cu -- the plain FP64 density solve over neighbour rows found by the block-tree search
+ * (near.cuh): the reference's src/density_base.cu:237-334 and 804-886 for one particle set.
+ *
+ * Every active particle is in one of three lists.  Those without a row that is complete for
+ * their h are searched (near_rows_kernel: r^2 and j of every neighbour within kNearMargin of
+ * their support, at most kNbl); those with one take their Newton step from it, one lane
+ * each; those with more neighbours than a row holds are summed straight from a search, one
+ * warp each.  A step that leaves h inside the row's reach keeps the row, one that outgrows
+ * it puts the particle back on the search list.  Lists, counts and decisions stay on the
+ * device: the loop is one graph launch (a while node), or the same kernels from the host.
+ *
+ * The pairs a particle accepts, and their order, are those of any complete candidate
+ * stream in ascending j, so h, rho and gradh agree with the oracle bit for bit.
+ */
+#include <algorithm>
+
+#include "near.cuh"
+#include "newton_step.cuh"
+#include "state.hpp"
+
+namespace cosmo {
+
+namespace {
+
+constexpr int kThreads = 32 * kNearWarps;
+
+// Rows reach kNearMargin of the support at the h they are made for, so that they serve
+// while h grows by up to that.
+#ifndef MARG
+#define MARG 1.04
+#endif
+constexpr double kNearMargin = MARG;
+constexpr float kNearWide = 1.5f;   // a member this much wider than its warp's mean searches alone
+constexpr double kCoverMargin = 1.0 + 1e-8;   // rows made for a converged h: just beyond the force test's slack
+constexpr double kCoverSlack = 1.0 + 1e-9;    // a row serves the gradient and force passes at h kCoverSlack <= rowH
+
+// ---------------------------------------------------------------- the block tree
+__device__ __forceinline__ NearNode node_of(float lx, float ly, float lz, float hx, float hy, float hz, float hm)
+{
+    NearNode n;
+    if (!(lx <= hx && ly <= hy && lz <= hz))
+    {
+        n.cx = n.cy = n.cz = 0.0f;
+        n.ex = n.ey = n.ez = -INFINITY;
+        n.hmax = 0.0f;
+        n.pad = 0.0f;
+        return n;
+    }
+    n.cx = 0.5f * lx + 0.5f * hx; n.ex = fmaxf(__fsub_ru(hx, n.cx), __fsub_ru(n.cx, lx));
+    n.cy = 0.5f * ly + 0.5f * hy; n.ey = fmaxf(__fsub_ru(hy, n.cy), __fsub_ru(n.cy, ly));
+    n.cz = 0.5f * lz + 0.5f * hz; n.ez = fmaxf(__fsub_ru(hz, n.cz), __fsub_ru(n.cz, lz));
+    n.hmax = hm;
+    n.pad = 0.0f;
+    return n;
+}
+
+// A parent of up to eight nodes, combined from the given ones by a loop (count >= 1).
+template<class Get>
+__device__ __forceinline__ NearNode node_parent(int count, Get&& get)
+{
+    float lx = INFINITY, ly = INFINITY, lz = INFINITY, hx = -INFINITY, hy = -INFINITY, hz = -INFINITY, hm = 0.0f;
+    for (int k = 0; k < count; ++k)
+    {
+        const NearNode c = get(k);
+        lx = fminf(lx, __fsub_rd(c.cx, c.ex)); hx = fmaxf(hx, __fadd_ru(c.cx, c.ex));
+        ly = fminf(ly, __fsub_rd(c.cy, c.ey)); hy = fmaxf(hy, __fadd_ru(c.cy, c.ey));
+        lz = fminf(lz, __fsub_rd(c.cz, c.ez)); hz = fmaxf(hz, __fadd_ru(c.cz, c.ez));
+        hm = fmaxf(hm, c.hmax);
+    }
+    return node_of(lx, ly, lz, hx, hy, hz, hm);
+}
+
+// Levels 0 to 2: 512 particles a block, one per thread; each level's boxes are reduced in
+// shared memory and written once (one 32-byte read per particle: DRAM bound, 11 us at 1.4 M).
+__global__ void __launch_bounds__(512)
+near_leaf_levels_kernel(const __grid_constant__ NearTree t, NearNode* __restrict__ out)
+{
+    __shared__ NearNode s0[64], s1[8];
+    const int n = *t.nLive;
+    const NearFrame f(t.box);
+    for (int b = blockIdx.x; b * 512 < n; b += gridDim.x)
+    {
+        const int i = b * 512 + int(threadIdx.x);
+        float lx = INFINITY, ly = INFINITY, lz = INFINITY, hx = -INFINITY, hy = -INFINITY, hz = -INFINITY, hm = 0.0f;
+        if (i < n)
+        {
+            const double4 p = t.xyzh[i];
+            const double x = p.x - f.cx, y = p.y - f.cy, z = p.z - f.cz;
+            lx = __double2float_rd(x); hx = __double2float_ru(x);
+            ly = __double2float_rd(y); hy = __double2float_ru(y);
+            lz = __double2float_rd(z); hz = __double2float_ru(z);
+            hm = __double2float_ru(p.w);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+        {
+            lx = fminf(lx, __shfl_xor_sync(0xffffffffu, lx, o)); hx = fmaxf(hx, __shfl_xor_sync(0xffffffffu, hx, o));
+            ly = fminf(ly, __shfl_xor_sync(0xffffffffu, ly, o)); hy = fmaxf(hy, __shfl_xor_sync(0xffffffffu, hy, o));
+            lz = fminf(lz, __shfl_xor_sync(0xffffffffu, lz, o)); hz = fmaxf(hz, __shfl_xor_sync(0xffffffffu, hz, o));
+            hm = fmaxf(hm, __shfl_xor_sync(0xffffffffu, hm, o));
+        }
+        if ((threadIdx.x & 7) == 0)
+        {
+            const NearNode nd = node_of(lx, ly, lz, hx, hy, hz, hm);
+            s0[threadIdx.x >> 3] = nd;
+            if (i < n) out[t.off[0] + (i >> 3)] = nd;
+        }
+        __syncthreads();
+        if (threadIdx.x < 8)
+        {
+            const NearNode nd = node_parent(8, [&](int k) { return s0[threadIdx.x * 8 + k]; });
+            s1[threadIdx.x] = nd;
+            const int q = b * 8 + int(threadIdx.x);
+            if (q * 64 < n) out[t.off[1] + q] = nd;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) out[t.off[2] + b] = node_parent(8, [&](int k) { return s1[k]; });
+        __syncthreads();
+    }
+}
+
+// The levels above, up to the first of at most 32 nodes: one block, level by level.
+__global__ void __launch_bounds__(1024)
+near_upper_levels_kernel(const __grid_constant__ NearTree t, NearNode* out)
+{
+    const int n = *t.nLive;
+    for (int l = 3; l < kNearLevels && near_count(n, l - 1) > 32; ++l)
+    {
+        const int below = near_count(n, l - 1), here = near_count(n, l);
+        for (int q = threadIdx.x; q < here; q += blockDim.x)
+            out[t.off[l] + q] = node_parent(min(8, below - 8 * q), [&](int k) { return out[t.off[l - 1] + 8 * q + k]; });
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------- lists
+// Append v to a list for the lanes that want to, one atomic per warp.
+__device__ __forceinline__ void warp_append(bool want, int v, int* __restrict__ list, int* __restrict__ count)
+{
+    const uint32_t m = __ballot_sync(0xffffffffu, want);
+    if (m == 0u) return;
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(count, __popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (want) list[base + __popc(m & ((1u << lane) - 1u))] = v;
+}
+
+// The same for a whole block of kThreads and three lists (to: 0, 1, 2, or -1 for none; every
+// thread calls it): one atomic per block and list, so that particles next to each other in
+// the sorted order stay together and the counters -- single addresses for the whole grid --
+// take a quarter of the atomics.  sh: 3 (kNearWarps + 1) ints.
+__device__ __forceinline__ void block_append(int to, int v, int* l0, int* c0, int* l1, int* c1, int* l2, int* c2,
+                                             int* sh)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t m0 = __ballot_sync(0xffffffffu, to == 0), m1 = __ballot_sync(0xffffffffu, to == 1);
+    const uint32_t m2 = __ballot_sync(0xffffffffu, to == 2);
+    if (lane < 3) sh[lane * (kNearWarps + 1) + w] = __popc(lane == 0 ? m0 : (lane == 1 ? m1 : m2));
+    __syncthreads();
+    if (threadIdx.x < 3)
+    {
+        int* c = sh + threadIdx.x * (kNearWarps + 1);
+        int* count = threadIdx.x == 0 ? c0 : (threadIdx.x == 1 ? c1 : c2);
+        int run = 0;
+        for (int k = 0; k < kNearWarps; ++k) { const int x = c[k]; c[k] = run; run += x; }
+        c[kNearWarps] = run > 0 ? atomicAdd(count, run) : 0;
+    }
+    __syncthreads();
+    if (to >= 0)
+    {
+        const int* c = sh + to * (kNearWarps + 1);
+        const uint32_t m = to == 0 ? m0 : (to == 1 ? m1 : m2);
+        int* list = to == 0 ? l0 : (to == 1 ? l1 : l2);
+        list[c[kNearWarps] + c[w] + __popc(m & lt)] = v;
+    }
+    __syncthreads();
+}
+
+// Largest h used and largest converged h of a block's particles (as bit patterns, which
+// order as the non-negative doubles they are), one atomic each per block.
+__device__ __forceinline__ void note_h(unsigned long long seen, unsigned long long conv, DevScalars* ds,
+                                       unsigned long long* sh)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        const unsigned long long a = __shfl_xor_sync(0xffffffffu, seen, o), b = __shfl_xor_sync(0xffffffffu, conv, o);
+        seen = a > seen ? a : seen;
+        conv = b > conv ? b : conv;
+    }
+    if (threadIdx.x == 0) sh[0] = sh[1] = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0)
+    {
+        atomicMax(&sh[0], seen);
+        atomicMax(&sh[1], conv);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        if (sh[0]) atomicMax(&ds->hmaxSeen, sh[0]);
+        if (sh[1]) atomicMax(&ds->hmaxConv, sh[1]);
+    }
+}
+
+// All live particles are searched first (the identity list); the counters of the row passes
+// after the loop start from zero too.
+__global__ void near_init_kernel(NearLoop* L, DevScalars* ds, int maxIter, int frozen)
+{
+    const int n = ds->nAlive;
+    L->iter = 0;
+    L->maxIter = maxIter;
+    L->active = n;
+    L->all = frozen ? 0 : 1;
+    L->cover = L->over = 0;
+    L->cnt[0] = NearCounts{0, frozen ? 0 : n, 0, 0};
+    L->cnt[1] = NearCounts{0, 0, 0, 0};
+    L->ticket[0] = L->ticket[1] = L->ticket[2] = L->ticket[3] = 0;
+    ds->extraCount = 0;
+    ds->mergeOverflow = 0;
+    ds->rowOverflow = 0;
+    ds->hmaxConv = 0;
+}
+
+// The initial search list with fixed particles (the caller's mask through the sort order;
+// they are neighbours only and count as converged): the others.
+__global__ void __launch_bounds__(kThreads)
+near_frozen_kernel(NearLoop* L, const int* __restrict__ order, const int* __restrict__ frozen,
+                   const int* __restrict__ nLive, const double4* __restrict__ xyzh, int* __restrict__ converged,
+                   double* __restrict__ hs, NearLists lists, DevScalars* __restrict__ ds)
+{
+    __shared__ int sh[3 * (kNearWarps + 1)];
+    __shared__ unsigned long long shH[2];
+    const int n = *nLive;
+    unsigned long long hconv = 0;
+    for (int b = blockIdx.x * kThreads; b < n; b += gridDim.x * kThreads)
+    {
+        const int k = b + int(threadIdx.x);
+        const bool f = k < n && frozen[order[k]] != 0;
+        if (k < n)
+        {
+            converged[k] = f ? 1 : 0;
+            if (f)
+            {
+                const double h = xyzh[k].w;
+                hs[k] = h;
+                const unsigned long long b = (unsigned long long)__double_as_longlong(h);
+                hconv = b > hconv ? b : hconv;
+            }
+        }
+        // a fixed particle has no row yet: one is made at its h with the others' at the end
+        block_append(k < n ? (f ? 2 : 1) : -1, k, nullptr, nullptr, lists.build[0], &L->cnt[0].build, lists.cover,
+                     &L->cover, sh);
+    }
+    note_h(0, hconv, ds, shH);
+}
+
+__global__ void near_frozen_count_kernel(NearLoop* L) { L->active = L->cnt[0].build; }
+
+// ---------------------------------------------------------------- rows
+// Rows of the listed particles (all live ones when the list is the identity): the members of
+// a warp are up to 32 consecutive entries -- fewer where the list is short, so that it still
+// spreads over the chip -- in runs that search together (near_runs).  Each member takes the
+// blocks its own sphere reaches and tests 32 candidates per step with the exact FP64 test;
+// what passes is written at once, consecutive entries by consecutive lanes.  A row that
+// would exceed kNbl is given up (its count is kNbl + 1) and stops its member's search.
+// Bound by issue: on a lattice about 6 steps of 28 instructions and 80 for the blocks per
+// particle.
+//   cover = 0: rows for the next Newton iteration; complete rows go to the row list, the
+//              others to the list of direct sums.
+//   cover = 1: rows at the converged h of particles left without; the others are listed
+//              (over) and marked as covering everything (rowH infinite: no pair of theirs
+//              is looked for from the other side).
+#ifndef NB
+#define NB 6
+#endif
+template<bool Periodic>
+__global__ void __launch_bounds__(kThreads, NB)
+near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
+                 const __grid_constant__ NearLists lists, double* __restrict__ rowsR2,
+                 int* __restrict__ rowsJ, int* __restrict__ nblCount, double* __restrict__ rowH, int cover)
+{
+    __shared__ NearScratch sScr[kNearWarps];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    NearScratch& scr = sScr[wib];
+    const int cur = L->iter & 1;
+    const int n = cover ? L->cover : L->cnt[cur].build;
+    if (n == 0) return;
+    const int* list = cover ? lists.cover : (L->all ? nullptr : lists.build[cur]);
+    int* ticket = &L->ticket[cover ? 2 : 0];
+    const double margin = cover ? kCoverMargin : kNearMargin;
+    const double wide2 = kRadK2 * (margin * margin);
+    const int nLive = *t.nLive;
+    const NearFrame f(t.box);
+    double lx = 0, ly = 0, lz = 0;
+    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    int g = 32;
+    while (g > 1 && n < g * int(gridDim.x) * kNearWarps) g >>= 1;
+    for (;;)
+    {
+        int w = 0;
+        if (lane == 0) w = atomicAdd(ticket, 1);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (long(w) * g >= n) break;
+        const int at = w * g + lane;
+        const bool mine = lane < g && at < n;
+        const int i = mine ? (list ? list[at] : at) : 0;
+        const double4 pi = t.xyzh[i];
+        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
+        const float slack = f.slack(x, y, z);
+        const float r = mine ? __double2float_ru(kRadKernel * margin * (1.0 + 1e-6) * pi.w) + slack : -1.0f;
+        scr.P[lane] = make_double4(pi.x, pi.y, pi.z, 1.0 / (pi.w * pi.w));
+        scr.Q[lane] = make_float4(x, y, z, r * r * 1.000001f);
+        // a member much wider than the others (a scattered h) searches by itself, after them
+        const uint32_t all = __ballot_sync(0xffffffffu, mine);
+        float mean = mine ? r : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mean += __shfl_xor_sync(0xffffffffu, mean, o);
+        const uint32_t wide = __ballot_sync(0xffffffffu, mine && r * float(__popc(all)) > kNearWide * mean);
+        const NearRun run = near_runs(x, y, z, (wide >> lane) & 1u ? -1.0f : r);
+        int rowLen = 0;
+        uint32_t todo = all;
+        __syncwarp();
+        for (int a = 0; todo; a += run.w)
+        {
+            uint32_t members;
+            float bx, by, bz, ex, ey, ez, reach;
+            if (a < 32)
+            {
+                members = todo & ~wide & ((run.w == 32 ? 0xffffffffu : ((1u << run.w) - 1u)) << a);
+                if (members == 0u) continue;
+                bx = __shfl_sync(0xffffffffu, run.cx, a); ex = __shfl_sync(0xffffffffu, run.ex, a);
+                by = __shfl_sync(0xffffffffu, run.cy, a); ey = __shfl_sync(0xffffffffu, run.ey, a);
+                bz = __shfl_sync(0xffffffffu, run.cz, a); ez = __shfl_sync(0xffffffffu, run.ez, a);
+                reach = __shfl_sync(0xffffffffu, run.reach, a);
+            }
+            else
+            {
+                const int p = __ffs(todo) - 1;
+                members = 1u << p;
+                bx = __shfl_sync(0xffffffffu, x, p);
+                by = __shfl_sync(0xffffffffu, y, p);
+                bz = __shfl_sync(0xffffffffu, z, p);
+                reach = __shfl_sync(0xffffffffu, r, p);
+                ex = ey = ez = 0.0f;
+            }
+            near_blocks<Periodic, false>(t, f, nLive, scr, bx, by, bz, ex, ey, ez, reach, 0.0f, [&](int nb) -> float {
+                // the blocks of this batch, kNearBlocks / 32 per lane
+                constexpr int kU = kNearBlocks / 32;
+                NearNode nd[kU];
+                int id[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u)
+                {
+                    const int k = 32 * u + lane;
+                    id[u] = k < nb ? scr.blk[k] : -1;
+                    if (32 * u < nb) nd[u] = ld_node(t.node + t.off[0] + max(id[u], 0));
+                }
+                bool dropped = false;
+                for (uint32_t rest = todo & members; rest; rest &= rest - 1)
+                {
+                    const int p = __ffs(rest) - 1;
+                    const float4 q = scr.Q[p];
+                    int ns = 0;
+#pragma unroll
+                    for (int u = 0; u < kU; ++u)
+                    {
+                        if (32 * u >= nb) break;
+                        const bool hit = id[u] >= 0 &&
+                                         near_gap2<Periodic>(q.x, q.y, q.z, 0.0f, 0.0f, 0.0f, nd[u], f) <= q.w;
+                        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+                        if (hit) scr.sel[ns + __popc(m & lt)] = id[u];
+                        ns += __popc(m);
+                    }
+                    if (ns == 0) continue;
+                    __syncwarp();
+                    const double4 gp = scr.P[p];
+                    const size_t row = size_t(__shfl_sync(0xffffffffu, i, p)) * kNbl;
+                    int len = __shfl_sync(0xffffffffu, rowLen, p);
+                    near_candidates(scr.sel, ns, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
+                        double dx = gp.x - pj.x, dy = gp.y - pj.y, dz = gp.z - pj.z;
+                        nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+                        const double r2 = pair_r2(dx, dy, dz);
+                        const bool acc = valid && r2 * gp.w < wide2;
+                        const uint32_t m = __ballot_sync(0xffffffffu, acc);
+                        const int k = len + __popc(m & lt);
+                        if (acc && k < kNbl)
+                        {
+                            rowsR2[row + k] = r2;
+                            if (rowsJ) rowsJ[row + k] = j;
+                        }
+                        len += __popc(m);
+                        return len <= kNbl;
+                    });
+                    if (lane == p) rowLen = len;
+                    if (len > kNbl)
+                    {
+                        todo &= ~(1u << p);
+                        dropped = true;
+                    }
+                    __syncwarp();
+                }
+                if (!dropped) return reach;
+                // the members still searching may need less
+                return warp_max_f(((todo & members) >> lane) & 1u ? r : -1.0f);
+            });
+            todo &= ~members;
+            __syncwarp();
+        }
+        const bool full = mine && rowLen > kNbl;
+        if (mine)
+        {
+            nblCount[i] = full ? kNbl + 1 : rowLen;
+            rowH[i] = full ? (cover ? double(INFINITY) : 0.0) : margin * pi.w * (1.0 - 1e-12);
+        }
+        if (cover)
+            warp_append(full, i, lists.over, &L->over);
+        else
+        {
+            warp_append(mine && !full, i, lists.row[cur], &L->cnt[cur].row);
+            warp_append(full, i, lists.sum[cur], &L->cnt[cur].sum);
+        }
+        __syncwarp();
+    }
+}
+
+// Where a particle goes after its Newton step (the lists of block_append).  Converged: to the
+// cover list when its row does not cover its h for the gradient and force passes, else
+// nowhere.  Otherwise its next iteration is from its row while h stays inside the row's
+// reach, from a new one beyond.
+__device__ __forceinline__ int next_of(bool conv, double ho, double rowHi)
+{
+    if (conv) return ho * kCoverSlack <= rowHi ? -1 : 2;
+    return ho <= rowHi ? 0 : 1;
+}
+
+// One Newton iteration from the rows: one lane per particle streams its own row (8 bytes an
+// entry), tests every entry with the exact test and adds in the row's order.
+__global__ void __launch_bounds__(kThreads)
+near_step_kernel(NearLoop* __restrict__ L, const __grid_constant__ NearLists lists, const double* __restrict__ rowsR2,
+                 const int* __restrict__ nblCount, const double* __restrict__ rowH, double4* __restrict__ xyzh,
+                 double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
+                 double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
+{
+    __shared__ int sh[3 * (kNearWarps + 1)];
+    __shared__ unsigned long long shH[2];
+    const int cur = L->iter & 1, nxt = cur ^ 1;
+    const int n = L->cnt[cur].row;
+    if (n == 0) return;
+    const int* list = lists.row[cur];
+    unsigned long long pairs = 0, seen = 0, hconv = 0;
+    for (int b = blockIdx.x * kThreads; b < n; b += gridDim.x * kThreads)
+    {
+        const int at = b + int(threadIdx.x);
+        int to = -1;
+        int i = 0;
+        if (at < n)
+        {
+            i = list[at];
+            const double hi = xyzh[i].w;
+            const double hinv2 = 1.0 / (hi * hi);
+            const double rh = rowH[i];
+            double sr = 0.0, sg = 0.0;
+            unsigned int gp = 0;
+            for_flat_row(row_flat(rowsR2, uint32_t(i)), nblCount[i], [&](double r2) {
+                const double q2 = r2 * hinv2;
+                if (!(q2 < kRadK2)) return;
+                ++gp;
+                const double q = sqrt(q2);
+                double wk, dwk;
+                sph_kernel(q2, q, wk, dwk);
+                sr += wk;
+                sg += -q * dwk - 3.0 * wk;
+            });
+            pairs += gp;
+            double ro, go, ho;
+            int conv;
+            newton_step(sr, sg, hi, pmass, hfact, tolh, ro, go, ho, conv);
+            rho[i] = ro;
+            gradh[i] = go;
+            reinterpret_cast<double*>(xyzh + i)[3] = ho;
+            const unsigned long long hb = (unsigned long long)__double_as_longlong(hi);
+            const unsigned long long ob = (unsigned long long)__double_as_longlong(ho);
+            seen = hb > seen ? hb : seen;
+            if (conv)
+            {
+                converged[i] = 1;
+                hs[i] = ho;
+                hconv = ob > hconv ? ob : hconv;
+            }
+            to = next_of(conv != 0, ho, rh);
+        }
+        block_append(to, i, lists.row[nxt], &L->cnt[nxt].row, lists.build[nxt], &L->cnt[nxt].build, lists.cover,
+                     &L->cover, sh);
+    }
+    note_h(seen, hconv, ds, shH);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
+}
+
+// ---------------------------------------------------------------- direct sums
+constexpr int kNearRec = 256;   // records of one ordered sum
+
+// Add v[0 .. 256) to s in order, as 256 successive rounded additions would: with s in one
+// binade throughout, each addition rounds v to a multiple u of that binade's last place and
+// adds it exactly, so the rounded terms may be summed in any order.  t = (v + C) - C with
+// C = 1.5 * 2^e is that rounding (to nearest even); a term exactly halfway (|v - t| = u/2)
+// rounds by the parity of the running sum instead, and a sum that could leave the binade
+// changes u, so either sends the 256 to the plain loop.  One lane adds 8 terms; two sums
+// of a multi-thousand-pair particle take about 200 instructions per 256 pairs in place of
+// 256 dependent additions each.
+__device__ __forceinline__ bool ordered_fast(const double* v, double& s)
+{
+    const int lane = threadIdx.x & 31;
+    const double a = fabs(s);
+    const long long bits = __double_as_longlong(a);
+    const int e = int(bits >> 52);
+    if (e < 64 || e > 2000) return false;   // zero, tiny, huge, infinite or NaN: the plain loop
+    const double lo = __longlong_as_double((long long)e << 52);       // 2^e <= |s| < 2^(e+1)
+    const double C = 1.5 * lo, half = 0.5 * lo, u = lo * 2.220446049250313e-16;
+    const double sign = s < 0.0 ? -1.0 : 1.0;
+    double P = 0.0, N = 0.0;
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < kNearRec / 32; ++k)
+    {
+        const double w = sign * v[32 * k + lane];
+        const double t = (w + C) - C;
+        ok = ok && fabs(w) < half && fabs(w - t) != 0.5 * u;
+        P += fmax(t, 0.0);
+        N += fmax(-t, 0.0);
+    }
+    // P and N are multiples of u; while they stay under the binade's width their sums are exact
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        P += __shfl_xor_sync(0xffffffffu, P, o);
+        N += __shfl_xor_sync(0xffffffffu, N, o);
+    }
+    ok = ok && P < lo && N < lo && a + P + 512.0 * u < 2.0 * lo && a - N - 512.0 * u >= lo;
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    s = sign * ((a + P) - N);
+    return true;
+}
+
+__device__ __forceinline__ void ordered_sum(const double* v, int m, double& s)
+{
+    if (m == kNearRec && ordered_fast(v, s)) return;
+    for (int k = 0; k < m; ++k) s += v[k];
+}
+
+// m records of q^2 in recW evaluated, one per lane, and added to the sums in order.
+__device__ __noinline__ double2 near_add_records(double* recW, double* recG, int m, double2 s)
+{
+    __syncwarp();
+    for (int k = threadIdx.x & 31; k < m; k += 32)
+    {
+        const double q2 = recW[k];
+        const double q = sqrt(q2);
+        double wk, dwk;
+        sph_kernel(q2, q, wk, dwk);
+        recW[k] = wk;
+        recG[k] = -q * dwk - 3.0 * wk;
+    }
+    __syncwarp();
+    ordered_sum(recW, m, s.x);
+    ordered_sum(recG, m, s.y);
+    __syncwarp();
+    return s;
+}
+
+// One Newton iteration of the particles whose neighbours do not fit a row: a warp searches
+// for one particle (its own sphere's blocks), packs the accepted q^2 into a record buffer in
+// ascending j, evaluates the records with one per lane and adds them in order.
+template<bool Periodic>
+__global__ void __launch_bounds__(kThreads)
+near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
+                const __grid_constant__ NearLists lists, double4* __restrict__ xyzh,
+                double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
+                double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
+{
+    __shared__ NearScratch sScr[kNearWarps];
+    __shared__ double sW[kNearWarps][kNearRec], sG[kNearWarps][kNearRec];
+    __shared__ unsigned long long shH[2];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    NearScratch& scr = sScr[wib];
+    double* recW = sW[wib];
+    double* recG = sG[wib];
+    const int cur = L->iter & 1, nxt = cur ^ 1;
+    const int n = L->cnt[cur].sum;
+    if (n == 0) return;
+    const int nLive = *t.nLive;
+    const NearFrame f(t.box);
+    double lx = 0, ly = 0, lz = 0;
+    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    unsigned long long pairs = 0, seen = 0, hconv = 0;
+    for (;;)
+    {
+        int w = 0;
+        if (lane == 0) w = atomicAdd(&L->ticket[1], 1);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (w >= n) break;
+        const int i = lists.sum[cur][w];
+        const double4 pi = xyzh[i];
+        const double hi = pi.w, hinv2 = 1.0 / (hi * hi);
+        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
+        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * hi) + f.slack(x, y, z);
+        double2 sums = make_double2(0.0, 0.0);
+        int nrec = 0;
+        unsigned int got = 0;
+        near_blocks<Periodic, false>(t, f, nLive, scr, x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+            near_candidates(scr.blk, nb, nLive, t.xyzh, [&](const double4& pj, int, bool valid) {
+                double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+                const double q2 = pair_r2(dx, dy, dz) * hinv2;
+                const bool acc = valid && q2 < kRadK2;
+                const uint32_t m = __ballot_sync(0xffffffffu, acc);
+                const int k = nrec + __popc(m & lt);
+                if (acc && k < kNearRec) recW[k] = q2;
+                nrec += __popc(m);
+                if (nrec >= kNearRec)
+                {
+                    sums = near_add_records(recW, recG, kNearRec, sums);
+                    got += kNearRec;
+                    nrec -= kNearRec;   // those beyond the buffer start the next one
+                    if (acc && k >= kNearRec) recW[k - kNearRec] = q2;
+                    __syncwarp();
+                }
+                return true;
+            });
+            return r;
+        });
+        sums = near_add_records(recW, recG, nrec, sums);
+        got += nrec;
+        double ro, go, ho;
+        int conv;
+        newton_step(sums.x, sums.y, hi, pmass, hfact, tolh, ro, go, ho, conv);
+        if (lane == 0)
+        {
+            pairs += got;
+            rho[i] = ro;
+            gradh[i] = go;
+            reinterpret_cast<double*>(xyzh + i)[3] = ho;
+            const unsigned long long hb = (unsigned long long)__double_as_longlong(hi);
+            const unsigned long long ob = (unsigned long long)__double_as_longlong(ho);
+            seen = hb > seen ? hb : seen;
+            if (conv)
+            {
+                converged[i] = 1;
+                hs[i] = ho;
+                hconv = ob > hconv ? ob : hconv;
+                lists.cover[atomicAdd(&L->cover, 1)] = i;
+            }
+            else
+            {
+                // about got * (kNearMargin ho / hi)^3 entries in a row made now
+                const double grow = kNearMargin * ho / hi;
+                const bool fits = double(got) * grow * grow * grow < 0.95 * kNbl;
+                if (fits) lists.build[nxt][atomicAdd(&L->cnt[nxt].build, 1)] = i;
+                else lists.sum[nxt][atomicAdd(&L->cnt[nxt].sum, 1)] = i;
+            }
+        }
+        __syncwarp();
+    }
+    note_h(seen, hconv, ds, shH);
+    if (lane == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
+}
+
+// End of an iteration: what it left active, the next one's lists in place, and whether it
+// runs (the graph's while condition when run as a graph).
+__global__ void near_epilogue_kernel(NearLoop* L, cudaGraphConditionalHandle more, int setCondition)
+{
+    const int it = L->iter, cur = it & 1, nxt = cur ^ 1;
+    if (it < kLoopIters) L->activePerIter[it] = L->active;
+    L->cnt[cur] = NearCounts{};
+    L->ticket[0] = L->ticket[1] = 0;
+    L->all = 0;
+    L->active = L->cnt[nxt].row + L->cnt[nxt].build + L->cnt[nxt].sum;
+    L->iter = it + 1;
+    if (setCondition) cudaGraphSetConditional(more, L->active > 0 && it + 1 < L->maxIter ? 1u : 0u);
+}
+
+} // namespace
+
+// ---------------------------------------------------------------- host side
+NearTree near_tree(State& s)
+{
+    NearTree t;
+    t.node = reinterpret_cast<const NearNode*>(s.nearNode.get());
+    t.xyzh = s.xyzh.get();
+    t.box = s.box.get();
+    t.nLive = &s.dscal.get()->nAlive;
+    int off = 0;
+    for (int l = 0; l < kNearLevels; ++l)
+    {
+        t.off[l] = off;
+        off += near_count(s.ngas, l);
+    }
+    return t;
+}
+
+// The block tree of the sorted particles (their positions stay while a solve's h change;
+// the boxes' h are those of the last call).
+void near_build(State& s)
+{
+    const int n = std::max(s.ngas, 1);
+    size_t nodes = 0;
+    for (int l = 0; l < kNearLevels; ++l) nodes += size_t(near_count(n, l));
+    s.nearNode.resize(nodes * (sizeof(NearNode) / sizeof(float4)), s.st);
+    const NearTree t = near_tree(s);
+    NearNode* out = reinterpret_cast<NearNode*>(s.nearNode.get());
+    near_leaf_levels_kernel<<<std::min(iceil(n, 512), 8 * s.numSMs), 512, 0, s.st>>>(t, out);
+    COSMO_LAUNCHED();
+    if (n > 512 * 32)
+    {
+        near_upper_levels_kernel<<<1, 1024, 0, s.st>>>(t, out);
+        COSMO_LAUNCHED();
+    }
+}
+
+static NearLists near_lists(State& s)
+{
+    NearLists l;
+    for (int k = 0; k < 2; ++k)
+    {
+        l.row[k] = s.nearRow[k].get();
+        l.build[k] = s.nearBuild[k].get();
+        l.sum[k] = s.nearSum[k].get();
+    }
+    l.cover = s.nearCover.get();
+    l.over = s.nearOver.get();
+    return l;
+}
+
+// One iteration's kernels, in the stream's order.
+static void near_iteration(State& s, double pmass, double tolh, double hfact, int* rowsJ, int n,
+                           cudaGraphConditionalHandle more, int setCondition)
+{
+    const NearTree t = near_tree(s);
+    const NearLists lists = near_lists(s);
+    NearLoop* L = s.nearLoop.get();
+    DevScalars* ds = s.dscal.get();
+    auto rows = s.periodic ? near_rows_kernel<true> : near_rows_kernel<false>;
+    rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(t, L, lists, s.nblR2.get(), rowsJ,
+                                                                      s.nblCount.get(), s.nblH.get(), 0);
+    COSMO_LAUNCHED();
+    near_step_kernel<<<std::max(1, std::min(iceil(n, kThreads), 16 * s.numSMs)), kThreads, 0, s.st>>>(
+        L, lists, s.nblR2.get(), s.nblCount.get(), s.nblH.get(), s.xyzh.get(), s.rho.get(), s.gradh.get(),
+        s.converged.get(), s.hs.get(), pmass, tolh, hfact, ds);
+    COSMO_LAUNCHED();
+    auto sum = s.periodic ? near_sum_kernel<true> : near_sum_kernel<false>;
+    sum<<<persistent_blocks(s, sum, kThreads), kThreads, 0, s.st>>>(t, L, lists, s.xyzh.get(), s.rho.get(),
+                                                                    s.gradh.get(), s.converged.get(), s.hs.get(), pmass,
+                                                                    tolh, hfact, ds);
+    COSMO_LAUNCHED();
+    near_epilogue_kernel<<<1, 1, 0, s.st>>>(L, more, setCondition);
+    COSMO_LAUNCHED();
+}
+
+// The loop as a graph: a while node over near_iteration.  It depends on the buffers, the
+// solve's scalars and the particle count only; built for parameters met a second time in a
+// row (a stepping caller's), as the list-based loop's is.  False: not run (build or use the
+// host loop).
+static bool near_graph(State& s, double pmass, double tolh, double hfact, int maxIter, int* rowsJ, int n)
+{
+    std::vector<unsigned char> key;
+    auto add = [&](const auto& v) {
+        const unsigned char* p = reinterpret_cast<const unsigned char*>(&v);
+        key.insert(key.end(), p, p + sizeof(v));
+    };
+    for (const void* q : {(const void*)s.nearLoop.get(), (const void*)s.dscal.get(), (const void*)s.nearNode.get(),
+                          (const void*)s.xyzh.get(), (const void*)s.box.get(), (const void*)s.nblR2.get(),
+                          (const void*)rowsJ, (const void*)s.nblCount.get(), (const void*)s.nblH.get(),
+                          (const void*)s.rho.get(), (const void*)s.gradh.get(), (const void*)s.converged.get(),
+                          (const void*)s.hs.get(), (const void*)s.nearRow[0].get(), (const void*)s.nearRow[1].get(),
+                          (const void*)s.nearBuild[0].get(), (const void*)s.nearBuild[1].get(),
+                          (const void*)s.nearSum[0].get(), (const void*)s.nearSum[1].get(),
+                          (const void*)s.nearCover.get(), (const void*)s.nearOver.get()})
+        add(q);
+    for (int v : {n, s.ngas, s.periodic, s.numSMs, maxIter}) add(v);
+    for (double v : {pmass, tolh, hfact}) add(v);
+    s.loopKeyLast = key;
+    if (!s.nearGraphExec || key != s.nearGraphKey)
+    {
+        if (key != s.nearKeyPending)
+        {
+            s.nearKeyPending = key;
+            return false;
+        }
+        if (s.nearGraphExec) COSMO_CUDA(cudaGraphExecDestroy(s.nearGraphExec));
+        if (s.nearGraphDef) COSMO_CUDA(cudaGraphDestroy(s.nearGraphDef));
+        s.nearGraphExec = nullptr;
+        s.nearGraphDef = nullptr;
+        s.nearGraphKey.clear();
+        const unsigned long long launches0 = g_launches.load();
+        cudaGraph_t g = nullptr;
+        cudaGraphExec_t ex = nullptr;
+        bool built = false;
+        do
+        {
+            if (cudaGraphCreate(&g, 0) != cudaSuccess) break;
+            cudaGraphConditionalHandle more;
+            if (cudaGraphConditionalHandleCreate(&more, g, 1, cudaGraphCondAssignDefault) != cudaSuccess) break;
+            cudaGraphNodeParams wp = {};
+            wp.type = cudaGraphNodeTypeConditional;
+            wp.conditional.handle = more;
+            wp.conditional.type = cudaGraphCondTypeWhile;
+            wp.conditional.size = 1;
+            cudaGraphNode_t wnode;
+            if (cudaGraphAddNode(&wnode, g, nullptr, 0, &wp) != cudaSuccess) break;
+            cudaGraph_t body = wp.conditional.phGraph_out[0];
+            if (cudaStreamBeginCaptureToGraph(s.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) !=
+                cudaSuccess)
+                break;
+            near_iteration(s, pmass, tolh, hfact, rowsJ, n, more, 1);
+            if (cudaStreamEndCapture(s.st, &body) != cudaSuccess) break;
+            if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) break;
+            built = true;
+        } while (false);
+        // what was captured did not run: the launches counted are those the graph executes
+        s.nearKernels = g_launches.load() - launches0;
+        g_launches -= s.nearKernels;
+        if (!built)
+        {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(s.st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
+            {
+                cudaGraph_t junk = nullptr;
+                cudaStreamEndCapture(s.st, &junk);
+                if (junk) cudaGraphDestroy(junk);
+            }
+            if (ex) cudaGraphExecDestroy(ex);
+            if (g) cudaGraphDestroy(g);
+            (void)cudaGetLastError();
+            return false;
+        }
+        s.nearGraphDef = g;
+        s.nearGraphExec = ex;
+        s.nearGraphKey = key;
+        ++s.loopGraphBuilds;
+    }
+    COSMO_CUDA(cudaGraphLaunch(s.nearGraphExec, s.st));
+    return true;
+}
+
+// The Newton loop of one plain solve over the block tree, every live (and not fixed)
+// particle active.  Issued on the stream; near_results reads what it did.  rowsJ: the rows'
+// j, for the gradient and force passes (may be null).
+void near_newton(State& s, double pmass, double tolh, double hfact, int maxIter, bool allowGraph, int* rowsJ)
+{
+    const int n = std::max(s.nAlive, 1);
+    DevScalars* ds = s.dscal.get();
+    for (auto* b : {&s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1], &s.nearSum[0], &s.nearSum[1],
+                    &s.nearCover, &s.nearOver})
+        b->resize(n, s.st);
+    s.hs.resize(n, s.st);
+    s.nearLoop.resize(1, s.st);
+    near_build(s);
+    const bool frozen = s.frozenFor == s.ngas && s.nAlive > 0;
+    near_init_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get(), ds, maxIter, frozen ? 1 : 0);
+    COSMO_LAUNCHED();
+    if (frozen)
+    {
+        near_frozen_kernel<<<std::min(iceil(n, kThreads), 8 * s.numSMs), kThreads, 0, s.st>>>(
+            s.nearLoop.get(), s.orderA.get(), s.frozen.get(), &ds->nAlive, s.xyzh.get(), s.converged.get(), s.hs.get(),
+            near_lists(s), ds);
+        COSMO_LAUNCHED();
+        near_frozen_count_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get());
+        COSMO_LAUNCHED();
+    }
+    s.lastLoopGraph = 0;
+    if (allowGraph && s.newtonGraph && maxIter <= kLoopIters && s.nAlive > 0 &&
+        near_graph(s, pmass, tolh, hfact, maxIter, rowsJ, n))
+    {
+        s.lastLoopGraph = 1;
+        return;
+    }
+    for (int it = 0; it < maxIter; ++it)
+    {
+        near_iteration(s, pmass, tolh, hfact, rowsJ, n, cudaGraphConditionalHandle(0), 0);
+        COSMO_CUDA(cudaMemcpyAsync(s.hsmall, s.nearLoop.get(), 4 * sizeof(int), cudaMemcpyDeviceToHost, s.st));
+        COSMO_CUDA(cudaStreamSynchronize(s.st));
+        if (s.hsmall[2] == 0) break;
+    }
+}
+
+// After the loop: rows at the converged h of the particles whose rows do not cover it.
+void near_cover(State& s, int* rowsJ)
+{
+    auto rows = s.periodic ? near_rows_kernel<true> : near_rows_kernel<false>;
+    rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(near_tree(s), s.nearLoop.get(), near_lists(s),
+                                                                      s.nblR2.get(), rowsJ, s.nblCount.get(),
+                                                                      s.nblH.get(), 1);
+    COSMO_LAUNCHED();
+}
+
+// What the loop did, once the stream has been read (h: its state on the host).
+long long near_results(State& s, const NearLoop& h)
+{
+    if (s.lastLoopGraph) g_launches += (unsigned long long)h.iter * s.nearKernels;
+    s.itersRun = h.iter;
+    s.activePerIter.assign(h.activePerIter, h.activePerIter + std::min(h.iter, kLoopIters));
+    return h.active;
+}
+
+} // namespace cosmo

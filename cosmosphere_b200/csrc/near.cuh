@@ -1,0 +1,272 @@
+/*
+ * near.cuh -- neighbour search over the sorted particles themselves: an implicit 8-ary
+ * tree of bounding boxes (8 consecutive particles of the Hilbert order make a block, 8
+ * blocks a node of the next level, and so on up) and the warp search that walks it.
+ *
+ * Why beside the octree: a leaf's list is made for the widest particle of the leaf and
+ * streamed by every group of it, so a group tests several times the pairs it accepts, and
+ * where h varies (a scattered start, the edge of a concentrated set) one warp streams whole
+ * lists for a few particles while the chip idles.  Here a group finds the 8-particle blocks
+ * its members' spheres reach, and each member then takes only the blocks its OWN sphere
+ * touches: on a lattice (58 neighbours) about 180 candidates per particle instead of 440,
+ * and no list, no work items and no per-leaf bookkeeping between iterations.
+ *
+ * Boxes are FP32 relative to the root box's centre, rounded outward, and every radius
+ * carries a slack above the rounding of the tests, so a block is never left out that
+ * holds a pair the exact FP64 test accepts.  Blocks come out in ascending order and the
+ * lanes of a step hold 32 consecutive candidates of one particle, so what is accepted is
+ * in ascending j, the order of every sum.
+ */
+#pragma once
+
+#include <algorithm>
+#include <type_traits>
+
+#include "common.cuh"
+#include "rows.cuh"
+#include "state.hpp"
+
+namespace cosmo {
+
+constexpr int kNearLevels = 9;     // level 0: blocks of 8 particles; 32 * 8^9 particles at most
+#ifndef NBLK
+#define NBLK 128
+#endif
+constexpr int kNearBlocks = NBLK;   // blocks a warp holds at once
+constexpr int kNearWarps  = 4;     // warps per block of the search kernels
+
+// A node's box: centre, half extents (empty: negative infinity) and its largest h.
+struct alignas(32) NearNode
+{
+    float cx, cy, cz, hmax, ex, ey, ez, pad;
+};
+
+// The nodes of level l start at node[off[l]] (laid out for the capacity of the arrays); the
+// live particle count is read on the device, so one set of arguments serves every solve.
+struct NearTree
+{
+    const NearNode* __restrict__ node;
+    const double4* __restrict__ xyzh;
+    const DevBox* __restrict__ box;
+    const int* nLive;
+    int off[kNearLevels];
+};
+
+__host__ __device__ inline int near_count(int n, int level) { return (n + (8 << (3 * level)) - 1) >> (3 * level + 3); }
+
+// Per-warp shared scratch of a search.
+struct NearScratch
+{
+    double4 P[32];                 // the members: position and one test value
+    float4 Q[32];                  // position relative to the box centre, squared reach
+    int front[kNearLevels][32];    // accepted nodes of each level, not yet expanded
+    int blk[kNearBlocks];          // accepted blocks, ascending
+    int sel[kNearBlocks];          // those one member reaches
+};
+
+__device__ __forceinline__ NearNode ld_node(const NearNode* p)
+{
+    NearNode n;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(n.cx), "=f"(n.cy), "=f"(n.cz), "=f"(n.hmax), "=f"(n.ex), "=f"(n.ey), "=f"(n.ez), "=f"(n.pad)
+        : "l"(p));
+    return n;
+}
+
+// The search frame: box centre and periods, and the slack of a radius.  A relative
+// coordinate a is rounded by at most 2^-24 |a|, and a gap's two subtractions (and the fold
+// at the period) by as much again of terms no larger than the box, so the gap of a point
+// errs by less than 2^-22 (len + |a|) per axis; 4e-7 (len + |a|_1) covers three axes.
+struct NearFrame
+{
+    double cx, cy, cz;
+    float lx, ly, lz, len;
+
+    __device__ __forceinline__ explicit NearFrame(const DevBox* b)
+    {
+        cx = b->lo[0] + 0.5 * b->len[0];
+        cy = b->lo[1] + 0.5 * b->len[1];
+        cz = b->lo[2] + 0.5 * b->len[2];
+        lx = float(b->len[0]);
+        ly = float(b->len[1]);
+        lz = float(b->len[2]);
+        len = fmaxf(lx, fmaxf(ly, lz));
+    }
+    __device__ __forceinline__ float slack(float x, float y, float z) const
+    {
+        return 4e-7f * (len + fabsf(x) + fabsf(y) + fabsf(z));
+    }
+};
+
+// Squared gap between the box (c, e) and a node's box, at the nearest image.
+template<bool Periodic>
+__device__ __forceinline__ float near_gap2(float x, float y, float z, float ex, float ey, float ez, const NearNode& n,
+                                           const NearFrame& f)
+{
+    float dx = fabsf(x - n.cx), dy = fabsf(y - n.cy), dz = fabsf(z - n.cz);
+    if (Periodic)
+    {
+        dx = fminf(dx, f.lx - dx);
+        dy = fminf(dy, f.ly - dy);
+        dz = fminf(dz, f.lz - dz);
+    }
+    dx = fmaxf(dx - (ex + n.ex), 0.0f);
+    dy = fmaxf(dy - (ey + n.ey), 0.0f);
+    dz = fmaxf(dz - (ez + n.ez), 0.0f);
+    return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+}
+
+// What a node's own h adds to a symmetric search's reach.
+__device__ __forceinline__ float near_sym_reach(float hmax, float slack)
+{
+    return fmaf(hmax, float(kRadKernel) * 1.000001f, slack);
+}
+
+// The blocks within reach of the box (c, e) -- or, Sym, within a block's own support of it
+// -- in ascending order, kNearBlocks at a time: flush(count) uses scr.blk and returns the
+// reach to go on with (the members still searching may be narrower), negative to stop.
+// The top level (at most 32 nodes) is tested first; then always the first four nodes of the
+// deepest level that holds any are expanded, one child per lane, so each level holds at
+// most 32 nodes and the blocks come out in order.
+template<bool Periodic, bool Sym, class Flush>
+__device__ __forceinline__ void near_blocks(const NearTree& t, const NearFrame& f, int nLive, NearScratch& scr, float x,
+                                            float y, float z, float ex, float ey, float ez, float reach, float slack,
+                                            Flush&& flush)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    int top = 0;
+    while (near_count(nLive, top) > 32) ++top;
+    int nb = 0;
+    int left = 0, pos = 0;   // lane l: nodes of level l not yet expanded, and the first of them
+    auto test = [&](int level, int idx) {
+        const NearNode n = ld_node(t.node + t.off[level] + idx);
+        const float r = Sym ? fmaxf(reach, near_sym_reach(n.hmax, slack)) : reach;
+        return near_gap2<Periodic>(x, y, z, ex, ey, ez, n, f) <= r * r;
+    };
+    // children of up to four nodes, or the top level: accepted ones of level into the next list
+    auto accept = [&](int level, int idx, bool valid) {
+        const bool ok = valid && test(level, idx);
+        const uint32_t m = __ballot_sync(0xffffffffu, ok);
+        const int c = __popc(m);
+        if (level == 0)
+        {
+            if (ok) scr.blk[nb + __popc(m & lt)] = idx;
+            nb += c;
+        }
+        else
+        {
+            if (ok) scr.front[level][__popc(m & lt)] = idx;
+            if (lane == level) { left = c; pos = 0; }
+        }
+        __syncwarp();
+    };
+    accept(top, lane, lane < near_count(nLive, top));
+    int lev = top;
+    for (;;)
+    {
+        int have = 0;
+        while (lev > 0 && lev <= top && (have = __shfl_sync(0xffffffffu, left, lev)) == 0) ++lev;
+        const bool end = lev == 0 || lev > top;
+        if (end || (lev == 1 && nb + 32 > kNearBlocks))
+        {
+            if (nb > 0) reach = flush(nb);
+            if (end || reach < 0.0f) return;
+            __syncwarp();
+            nb = 0;
+        }
+        const int first = __shfl_sync(0xffffffffu, pos, lev);
+        const int m = min(have, 4);
+        const int node = scr.front[lev][first + min(lane >> 3, m - 1)];
+        const int child = node * 8 + (lane & 7);
+        if (lane == lev) { left -= m; pos += m; }
+        accept(lev - 1, child, (lane >> 3) < m && child < near_count(nLive, lev - 1));
+        if (lev > 1) --lev;
+    }
+}
+
+__device__ __forceinline__ float warp_max_f(float v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// Members of a warp's search in equal runs of consecutive lanes: as many lanes per run (a
+// power of two) as keep every run's bounding box within kNearSpread of its largest reach,
+// so that sparse members (an active list late in the loop, the edge of a set) do not share
+// one search over everything between them.  x, y, z, r: the lane's member (r < 0: none);
+// on return the run's box (centre, half) and reach on every lane of it.
+constexpr float kNearSpread = 1.5f;
+struct NearRun
+{
+    int w;
+    float cx, cy, cz, ex, ey, ez, reach;
+};
+
+__device__ __forceinline__ NearRun near_runs(float x, float y, float z, float r)
+{
+    const bool on = r >= 0.0f;
+    float lx = on ? x : INFINITY, hx = on ? x : -INFINITY;
+    float ly = on ? y : INFINITY, hy = on ? y : -INFINITY;
+    float lz = on ? z : INFINITY, hz = on ? z : -INFINITY;
+    NearRun u;
+    u.w = 1;
+    u.reach = r;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const float ax = fminf(lx, __shfl_xor_sync(0xffffffffu, lx, o)), bx = fmaxf(hx, __shfl_xor_sync(0xffffffffu, hx, o));
+        const float ay = fminf(ly, __shfl_xor_sync(0xffffffffu, ly, o)), by = fmaxf(hy, __shfl_xor_sync(0xffffffffu, hy, o));
+        const float az = fminf(lz, __shfl_xor_sync(0xffffffffu, lz, o)), bz = fmaxf(hz, __shfl_xor_sync(0xffffffffu, hz, o));
+        const float rr = fmaxf(u.reach, __shfl_xor_sync(0xffffffffu, u.reach, o));
+        const float ext = fmaxf(bx - ax, fmaxf(by - ay, bz - az));
+        if (u.w != o || !__all_sync(0xffffffffu, !(ext > kNearSpread * rr))) continue;
+        lx = ax; hx = bx; ly = ay; hy = by; lz = az; hz = bz;
+        u.reach = rr;
+        u.w = 2 * o;
+    }
+    // box sides rounded by at most 2^-23 of the coordinates: inside the slack
+    u.cx = 0.5f * (lx + hx); u.ex = fmaxf(hx - u.cx, u.cx - lx);
+    u.cy = 0.5f * (ly + hy); u.ey = fmaxf(hy - u.cy, u.cy - ly);
+    u.cz = 0.5f * (lz + hz); u.ez = fmaxf(hz - u.cz, u.cz - lz);
+    return u;
+}
+
+NearTree near_tree(State& s);   // the arguments of a search of s's live particles
+
+// As many blocks of a kernel as the device holds at once.
+template<class K>
+inline int persistent_blocks(const State& s, K kernel, int threads)
+{
+    int perSM = 0;
+    COSMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel, threads, 0));
+    return std::max(1, perSM) * s.numSMs;
+}
+
+// Candidates of the blocks ids[0 .. ns) (ns >= 1): use(pj, j, valid) for 32 consecutive
+// candidates per step (lane: its own), the next step's loads in flight meanwhile.  use
+// returns false, on every lane, to stop.
+template<class Use>
+__device__ __forceinline__ void near_candidates(const int* ids, int ns, int nLive, const double4* __restrict__ xyzh,
+                                                Use&& use)
+{
+    const int lane = threadIdx.x & 31;
+    const int sub = lane >> 3, off = lane & 7;
+    int j = ids[min(sub, ns - 1)] * 8 + off;
+    bool valid = sub < ns && j < nLive;
+    double4 p = ldg4(xyzh + (valid ? j : 0));
+    for (int k = 0; k < ns; k += 4)
+    {
+        const int kn = k + 4 + sub;
+        const int jn = ids[min(kn, ns - 1)] * 8 + off;
+        const bool vn = kn < ns && jn < nLive;
+        const double4 pn = ldg4(xyzh + (vn ? jn : 0));
+        if (!use(p, j, valid)) return;
+        j = jn;
+        valid = vn;
+        p = pn;
+    }
+}
+
+} // namespace cosmo

@@ -107,6 +107,7 @@ struct DevScalars
     int rowsJOn;                 // the Newton row builder writes the index rows (nonzero)
     int leafStart;               // leaves of the grid the leaf tree's refinement starts from
     int leafDone;                // that grid is the leaf tree (no node of it holds more than kBucket)
+    unsigned long long hmaxConv; // bits of the largest converged h (the block-tree loop)
 };
 
 // The single-set Newton loop run as a graph: what the host loop kept in host variables
@@ -121,6 +122,30 @@ struct NewtonLoop
     long long settling0;
     long long activePerIter[kLoopIters];
     unsigned int listEntries[kLoopIters];   // gather-list entries each iteration ran on
+};
+
+// The Newton loop over the block tree (near.cu): the lists an iteration works on and fills
+// (double-buffered by the iteration's parity) and its state on the device.
+struct NearCounts
+{
+    int row, build, sum, pad;    // particles with a row, without one, with more neighbours than one holds
+};
+struct NearLoop
+{
+    int iter, maxIter, active;   // active: particles the next iteration updates
+    int all;                     // the search list is every live particle
+    int cover, over;             // rows still to be made at the converged h; those that do not fit one
+    int ticket[4];               // work tickets: row search, direct sums, cover search, over passes
+    NearCounts cnt[2];
+    long long activePerIter[kLoopIters];
+};
+struct NearLists
+{
+    int* row[2];
+    int* build[2];
+    int* sum[2];
+    int* cover;
+    int* over;
 };
 
 struct Timings
@@ -204,6 +229,12 @@ struct State
     std::vector<unsigned char> loopGraphKey;
     std::vector<unsigned char> loopKeyPending;   // parameters met once, not yet built for
     std::vector<unsigned char> loopKeyLast;      // the last solve's parameters (a diagnostic)
+    // the same for the block-tree loop
+    cudaGraph_t nearGraphDef = nullptr;
+    cudaGraphExec_t nearGraphExec = nullptr;
+    std::vector<unsigned char> nearGraphKey, nearKeyPending;
+    unsigned long long nearKernels = 0;              // kernels of one iteration
+    int nearOverCount = 0;                           // particles the last solve left without a row
     unsigned long long loopKernels[3] = {0, 0, 0};   // kernels of the body, the list branch, the rows branch
     int loopGraphBuilds = 0, loopGraphUpdates = 0;
     int lastLoopRebuilds = 0, lastLoopRowBuilds = 0;   // its list rebuilds and row builds
@@ -258,6 +289,9 @@ struct State
     DBuf<int> extraBucket;                      // the extras' j, grouped by owner
     DBuf<int> leafNext;                         // leaf already queued for the next iteration
     DBuf<int> activeA, activeB, allLeaves;
+    DBuf<float4> nearNode;                      // the block tree (near.cuh), two float4 a node
+    DBuf<int> nearRow[2], nearBuild[2], nearSum[2], nearCover, nearOver;   // the block-tree loop's lists
+    DBuf<NearLoop> nearLoop;                    // its state
 
     // scratch
     DBuf<uint32_t> scanTmp, sortHist, sortBase, sortLookback;
@@ -304,6 +338,12 @@ uint32_t scan_exclusive(State& s, const uint32_t* in, uint32_t* out, int n, bool
 // The same with the element count on the device (*nPtr <= nCap); the total goes to out[*nPtr].
 void scan_exclusive_dev(State& s, const uint32_t* in, uint32_t* out, int nCap, const int* nPtr);
 void scan_reserve(State& s, int nCap);   // size the scan scratch for up to nCap elements
+
+// near.cu: the plain solve's Newton loop over the block tree
+void near_build(State& s);
+void near_newton(State& s, double pmass, double tolh, double hfact, int maxIter, bool allowGraph, int* rowsJ);
+void near_cover(State& s, int* rowsJ);
+long long near_results(State& s, const NearLoop& h);   // particles left unconverged
 
 // density.cu
 struct DensResult { int itersRun; int unconverged; int status; };
