@@ -531,12 +531,15 @@ int grid_for(const State& s, int work)
 
 } // namespace
 
+// The row passes launch a thread per particle: with a grid of eight blocks a multiprocessor,
+// striding over the particles, the last, partly filled stride of nine left a third of the
+// chip idle (lattice 100: gradient 1.08 -> 0.80 ms, force 1.17 -> 0.92 ms).
 void launch_gradient_mixed(State& s, double pmass)
 {
     const int nL = s.nLeaves;
     const int grid = grid_for(s, nL);
     auto rows = [&](auto kern) {
-        kern<<<std::max(1, std::min(iceil(s.nAlive, kThreads), 8 * s.numSMs)), kThreads, 0, s.st>>>(
+        kern<<<std::max(1, iceil(s.nAlive, kThreads)), kThreads, 0, s.st>>>(
             s.nAlive, s.nbl.get(), s.nblCount.get(), s.xyzh.get(), s.vel4.get(), s.acc4.get(), s.rho.get(),
             s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), s.dscal.get());
     };
@@ -563,7 +566,7 @@ void launch_force_mixed(State& s, double pmass, double beta, bool disc, bool pdv
     COSMO_LAUNCHED();
     const int grid = grid_for(s, nL);
     auto rows = [&](auto kern) {
-        kern<<<std::max(1, std::min(iceil(s.nAlive, kThreads), 8 * s.numSMs)), kThreads, 0, s.st>>>(
+        kern<<<std::max(1, iceil(s.nAlive, kThreads)), kThreads, 0, s.st>>>(
             s.nAlive, s.nbl.get(), s.nblCount.get(), s.xyzh.get(), s.vel4.get(), s.thermof.get(), s.prepAf.get(),
             s.prepBf.get(), s.fx.get(), s.fy.get(), s.fz.get(), s.f4.get(), s.vsigmax.get(), s.divvF.get(), pmass,
             beta, pdv ? 1 : 0, shock ? 1 : 0, s.box.get(), s.dscal.get());
