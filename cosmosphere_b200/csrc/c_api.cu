@@ -139,7 +139,7 @@ size_t state_device_bytes(const State& s)
                     &s.activeA, &s.activeB, &s.allLeaves, &s.nodeValsTmp, &s.leafNext, &s.nbl, &s.nblCount,
                     &s.rowItems, &s.jlistPrev, &s.walked, &s.walkScratch, &s.coverFlag, &s.coverLeaves, &s.extraCnt,
                     &s.extraBucket, &s.nblJ, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1],
-                    &s.nearSum[0], &s.nearSum[1], &s.nearCover, &s.nearOver})
+                    &s.nearSum[0], &s.nearSum[1], &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
         add(*d);
     add(s.nearNode);
     add(s.nearLoop);
@@ -170,7 +170,7 @@ void release_state(State& s)
                     &s.activeA, &s.activeB, &s.allLeaves, &s.nodeValsTmp, &s.leafNext, &s.nbl, &s.nblCount,
                     &s.rowItems, &s.jlistPrev, &s.walked, &s.walkScratch, &s.coverFlag, &s.coverLeaves, &s.extraCnt,
                     &s.extraBucket, &s.nblJ, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1],
-                    &s.nearSum[0], &s.nearSum[1], &s.nearCover, &s.nearOver})
+                    &s.nearSum[0], &s.nearSum[1], &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
         b->release(s.st);
     s.nearNode.release(s.st);
     s.nearLoop.release(s.st);

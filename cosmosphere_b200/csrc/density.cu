@@ -229,7 +229,7 @@ gradient_over_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ 
         const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
         double sum = 0.0;   // lane k: sum k
         unsigned int gp = 0;
-        near_blocks<Periodic, false>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+        near_blocks<0, Periodic, false>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
             near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
                 double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                 nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
@@ -291,7 +291,7 @@ over_extras_kernel(const __grid_constant__ NearTree t, const NearLoop* __restric
         const double bi = kRadK2 * (pi.w * pi.w) * (1.0 + 1e-10);
         const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
         const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
-        near_blocks<Periodic, false>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+        near_blocks<0, Periodic, false>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
             near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
                 double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                 nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
@@ -1371,7 +1371,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         else
         {
             auto gr = s.periodic ? gradient_row_kernel<true> : gradient_row_kernel<false>;
-            gr<<<std::max(1, std::min(iceil(s.nAlive, kThreads), 8 * s.numSMs)), kThreads, 0, s.st>>>(
+            gr<<<std::max(1, iceil(s.nAlive, kThreads)), kThreads, 0, s.st>>>(
                 s.nAlive, s.nbl.get(), s.nblCount.get(), s.xyzh.get(), s.vel4.get(), s.acc4.get(), s.rho.get(),
                 s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), ds, active);
             COSMO_LAUNCHED();

@@ -412,7 +412,7 @@ force_over_kernel(const __grid_constant__ NearTree t, int n, const int* __restri
         const float slack = f.slack(x, y, z);
         const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * A.p.w) + slack;
         double sum = 0.0;   // lanes 0-5: the pressure sums, 6: the energy, 7: div v, 8: vsig
-        near_blocks<Periodic, true>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
+        near_blocks<0, Periodic, true>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
             near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
                 double* mine = term + lane * kStride;
                 for (int k = 0; k < kForceTerms; ++k) mine[k] = 0.0;
@@ -529,7 +529,7 @@ void compute_forces(State& s, double pmass, double beta, double alphau, bool dis
                                           shock ? 1 : 0, s.box.get(), s.nblCount.get(), ds);
     };
     auto launchRows = [&](auto kern) {
-        kern<<<std::max(1, std::min(iceil(s.nAlive, kThreads), 8 * s.numSMs)), kThreads, 0, s.st>>>(
+        kern<<<std::max(1, iceil(s.nAlive, kThreads)), kThreads, 0, s.st>>>(
             s.nAlive, s.nbl.get(), s.nblCount.get(), s.xyzh.get(), s.vel4.get(), s.thermo4.get(), s.prepA.get(),
             s.prepB.get(), s.fx.get(), s.fy.get(), s.fz.get(), s.f4.get(), s.vsigmax.get(), s.divvF.get(), pmass,
             alphau, beta, pdv ? 1 : 0, shock ? 1 : 0, s.box.get(), ds);

@@ -26,11 +26,10 @@ namespace {
 constexpr int kThreads = 32 * kNearWarps;
 
 // Rows reach kNearMargin of the support at the h they are made for, so that they serve
-// while h grows by up to that.
-#ifndef MARG
-#define MARG 1.04
-#endif
-constexpr double kNearMargin = MARG;
+// while h grows by up to that.  Measured on the lattice-100 loop (cold start / mid-run): 1.02
+// 3.14 / 2.77 ms (particles outgrow their rows), 1.04 3.26 / 2.46, 1.10 3.68 / 2.55 (longer
+// rows in every iteration).
+constexpr double kNearMargin = 1.04;
 constexpr float kNearWide = 1.5f;   // a member this much wider than its warp's mean searches alone
 constexpr double kCoverMargin = 1.0 + 1e-8;   // rows made for a converged h: just beyond the force test's slack
 constexpr double kCoverSlack = 1.0 + 1e-9;    // a row serves the gradient and force passes at h kCoverSlack <= rowH
@@ -274,11 +273,8 @@ __global__ void near_frozen_count_kernel(NearLoop* L) { L->active = L->cnt[0].bu
 //   cover = 1: rows at the converged h of particles left without; the others are listed
 //              (over) and marked as covering everything (rowH infinite: no pair of theirs
 //              is looked for from the other side).
-#ifndef NB
-#define NB 6
-#endif
 template<bool Periodic>
-__global__ void __launch_bounds__(kThreads, NB)
+__global__ void __launch_bounds__(kThreads, 6)
 near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                  const __grid_constant__ NearLists lists, double* __restrict__ rowsR2,
                  int* __restrict__ rowsJ, int* __restrict__ nblCount, double* __restrict__ rowH, int cover)
@@ -348,7 +344,7 @@ near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                 reach = __shfl_sync(0xffffffffu, r, p);
                 ex = ey = ez = 0.0f;
             }
-            near_blocks<Periodic, false>(t, f, nLive, scr, bx, by, bz, ex, ey, ez, reach, 0.0f, [&](int nb) -> float {
+            near_blocks<0, Periodic, false>(t, f, nLive, scr, bx, by, bz, ex, ey, ez, reach, 0.0f, [&](int nb) -> float {
                 // the blocks of this batch, kNearBlocks / 32 per lane
                 constexpr int kU = kNearBlocks / 32;
                 NearNode nd[kU];
@@ -504,94 +500,169 @@ near_step_kernel(NearLoop* __restrict__ L, const __grid_constant__ NearLists lis
 }
 
 // ---------------------------------------------------------------- direct sums
-constexpr int kNearRec = 256;   // records of one ordered sum
+// A particle whose neighbours do not fit a row is summed straight from its search: accepted
+// q^2 are packed into a record buffer in ascending j, evaluated one per lane, and W and
+// -q dW/dq - 3W added in order.
+constexpr int kNearRec = 256;        // records of one ordered sum
+constexpr int kHugeWarps = 8;        // warps that share a particle of very many neighbours
+constexpr unsigned int kHuge = 4096; // as many neighbours and more
 
-// Add v[0 .. 256) to s in order, as 256 successive rounded additions would: with s in one
-// binade throughout, each addition rounds v to a multiple u of that binade's last place and
-// adds it exactly, so the rounded terms may be summed in any order.  t = (v + C) - C with
-// C = 1.5 * 2^e is that rounding (to nearest even); a term exactly halfway (|v - t| = u/2)
-// rounds by the parity of the running sum instead, and a sum that could leave the binade
-// changes u, so either sends the 256 to the plain loop.  One lane adds 8 terms; two sums
-// of a multi-thousand-pair particle take about 200 instructions per 256 pairs in place of
-// 256 dependent additions each.
-__device__ __forceinline__ bool ordered_fast(const double* v, double& s)
+// Successive rounded additions of v[0 .. m) to s, in parallel.  While the running sum stays
+// in one binade, each addition rounds its term to a multiple u of that binade's last place
+// and adds it exactly, so the rounded terms may be added in any order.  t = (w + C) - C with
+// C = 1.5 * 2^e is that rounding (to nearest even).  A term exactly halfway (|w - t| = u/2)
+// rounds by the parity of the running sum instead, and a sum that might leave the binade
+// changes u: then ok is false and the terms must be added one by one.  up and down: the sums
+// of the positive and the negative rounded terms (multiples of u, exact while below 2^e).
+struct OrderedPart
+{
+    double up, down;
+    bool ok;
+};
+
+struct Binade
+{
+    double a, lo, u, sign;   // |s|, 2^e <= |s| < 2^(e+1), 2^(e-52), the sign of s
+    bool ok;
+    __device__ __forceinline__ explicit Binade(double s)
+    {
+        a = fabs(s);
+        sign = s < 0.0 ? -1.0 : 1.0;
+        const int e = int(__double_as_longlong(a) >> 52);
+        ok = e >= 64 && e <= 2000;   // not zero, tiny, huge, infinite or NaN
+        lo = __longlong_as_double((long long)(ok ? e : 1023) << 52);
+        u = lo * 2.220446049250313e-16;
+    }
+    // whether terms of these sums keep every partial sum inside the binade
+    __device__ __forceinline__ bool holds(double up, double down) const
+    {
+        return up < lo && down < lo && a + up + 512.0 * u < 2.0 * lo && a - down - 512.0 * u >= lo;
+    }
+};
+
+// Component c of the records, by one warp.
+__device__ __forceinline__ OrderedPart ordered_part(const double2* rec, int c, int m, const Binade& b)
 {
     const int lane = threadIdx.x & 31;
-    const double a = fabs(s);
-    const long long bits = __double_as_longlong(a);
-    const int e = int(bits >> 52);
-    if (e < 64 || e > 2000) return false;   // zero, tiny, huge, infinite or NaN: the plain loop
-    const double lo = __longlong_as_double((long long)e << 52);       // 2^e <= |s| < 2^(e+1)
-    const double C = 1.5 * lo, half = 0.5 * lo, u = lo * 2.220446049250313e-16;
-    const double sign = s < 0.0 ? -1.0 : 1.0;
-    double P = 0.0, N = 0.0;
-    bool ok = true;
+    const double C = 1.5 * b.lo, half = 0.5 * b.lo, tie = 0.5 * b.u;
+    OrderedPart r{0.0, 0.0, b.ok};
 #pragma unroll
     for (int k = 0; k < kNearRec / 32; ++k)
     {
-        const double w = sign * v[32 * k + lane];
+        const int at = 32 * k + lane;
+        const double w = at < m ? b.sign * (c ? rec[at].y : rec[at].x) : 0.0;
         const double t = (w + C) - C;
-        ok = ok && fabs(w) < half && fabs(w - t) != 0.5 * u;
-        P += fmax(t, 0.0);
-        N += fmax(-t, 0.0);
+        r.ok = r.ok && fabs(w) < half && fabs(w - t) != tie;
+        r.up += fmax(t, 0.0);
+        r.down += fmax(-t, 0.0);
     }
-    // P and N are multiples of u; while they stay under the binade's width their sums are exact
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
     {
-        P += __shfl_xor_sync(0xffffffffu, P, o);
-        N += __shfl_xor_sync(0xffffffffu, N, o);
+        r.up += __shfl_xor_sync(0xffffffffu, r.up, o);
+        r.down += __shfl_xor_sync(0xffffffffu, r.down, o);
     }
-    ok = ok && P < lo && N < lo && a + P + 512.0 * u < 2.0 * lo && a - N - 512.0 * u >= lo;
-    if (!__all_sync(0xffffffffu, ok)) return false;
-    s = sign * ((a + P) - N);
-    return true;
+    r.ok = __all_sync(0xffffffffu, r.ok);
+    return r;
 }
 
-__device__ __forceinline__ void ordered_sum(const double* v, int m, double& s)
+// The records' two components added to the two sums in order, by one warp: in parallel where
+// a full buffer allows it, else one by one (even lanes one sum, odd lanes the other).
+__device__ __forceinline__ double2 ordered_add(const double2* rec, int m, double2 s)
 {
-    if (m == kNearRec && ordered_fast(v, s)) return;
-    for (int k = 0; k < m; ++k) s += v[k];
+    bool doneW = false, doneG = false;
+    if (m == kNearRec)
+    {
+        const Binade bw(s.x), bg(s.y);
+        const OrderedPart w = ordered_part(rec, 0, m, bw), g = ordered_part(rec, 1, m, bg);
+        if (w.ok && bw.holds(w.up, w.down)) { s.x = bw.sign * ((bw.a + w.up) - w.down); doneW = true; }
+        if (g.ok && bg.holds(g.up, g.down)) { s.y = bg.sign * ((bg.a + g.up) - g.down); doneG = true; }
+        if (doneW && doneG) return s;
+    }
+    const bool odd = threadIdx.x & 1;
+    const double* v = reinterpret_cast<const double*>(rec) + (odd ? 1 : 0);
+    double t = odd ? s.y : s.x;
+#pragma unroll 8
+    for (int k = 0; k < m; ++k) t += v[2 * k];
+    const double tw = __shfl_sync(0xffffffffu, t, 0), tg = __shfl_sync(0xffffffffu, t, 1);
+    if (!doneW) s.x = tw;
+    if (!doneG) s.y = tg;
+    return s;
 }
 
-// m records of q^2 in recW evaluated, one per lane, and added to the sums in order.
-__device__ __noinline__ double2 near_add_records(double* recW, double* recG, int m, double2 s)
+__device__ __forceinline__ void eval_records(double2* rec, int m)
 {
-    __syncwarp();
     for (int k = threadIdx.x & 31; k < m; k += 32)
     {
-        const double q2 = recW[k];
+        const double q2 = rec[k].x;
         const double q = sqrt(q2);
         double wk, dwk;
         sph_kernel(q2, q, wk, dwk);
-        recW[k] = wk;
-        recG[k] = -q * dwk - 3.0 * wk;
+        rec[k] = make_double2(wk, -q * dwk - 3.0 * wk);
     }
+}
+
+// m records of q^2 evaluated and added to the sums in order.
+__device__ __noinline__ double2 near_add_records(double2* rec, int m, double2 s)
+{
     __syncwarp();
-    ordered_sum(recW, m, s.x);
-    ordered_sum(recG, m, s.y);
+    eval_records(rec, m);
+    __syncwarp();
+    s = ordered_add(rec, m, s);
     __syncwarp();
     return s;
 }
 
-// One Newton iteration of the particles whose neighbours do not fit a row: a warp searches
-// for one particle (its own sphere's blocks), packs the accepted q^2 into a record buffer in
-// ascending j, evaluates the records with one per lane and adds them in order.
+// The Newton step of a directly summed particle, by one thread: stored, and the particle put
+// on its next list by how many neighbours it had (got): enough room in a row once made,
+// one warp's work, or a block's.
+__device__ __forceinline__ void sum_finish(int i, double hi, double2 sums, unsigned int got, NearLoop* L,
+                                           const NearLists& lists, int nxt, double4* xyzh, double* rho, double* gradh,
+                                           int* converged, double* hs, double pmass, double tolh, double hfact,
+                                           unsigned long long& seen, unsigned long long& hconv)
+{
+    double ro, go, ho;
+    int conv;
+    newton_step(sums.x, sums.y, hi, pmass, hfact, tolh, ro, go, ho, conv);
+    rho[i] = ro;
+    gradh[i] = go;
+    reinterpret_cast<double*>(xyzh + i)[3] = ho;
+    const unsigned long long hb = (unsigned long long)__double_as_longlong(hi);
+    const unsigned long long ob = (unsigned long long)__double_as_longlong(ho);
+    seen = hb > seen ? hb : seen;
+    if (conv)
+    {
+        converged[i] = 1;
+        hs[i] = ho;
+        hconv = ob > hconv ? ob : hconv;
+        lists.cover[atomicAdd(&L->cover, 1)] = i;
+        return;
+    }
+    const double ratio = ho / hi, expect = double(got) * ratio * ratio * ratio;
+    if (expect * (kNearMargin * kNearMargin * kNearMargin) < 0.95 * kNbl)
+        lists.build[nxt][atomicAdd(&L->cnt[nxt].build, 1)] = i;
+    else if (expect < double(kHuge))
+        lists.sum[nxt][atomicAdd(&L->cnt[nxt].sum, 1)] = i;
+    else
+        lists.huge[nxt][atomicAdd(&L->cnt[nxt].huge, 1)] = i;
+}
+
+// One Newton iteration of the particles whose neighbours do not fit a row, one warp each.
+// One that turns out to have kHuge of them is left to the block kernel.
 template<bool Periodic>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 5)
 near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                 const __grid_constant__ NearLists lists, double4* __restrict__ xyzh,
                 double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
                 double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
 {
     __shared__ NearScratch sScr[kNearWarps];
-    __shared__ double sW[kNearWarps][kNearRec], sG[kNearWarps][kNearRec];
+    __shared__ double2 sRec[kNearWarps][kNearRec];
     __shared__ unsigned long long shH[2];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     NearScratch& scr = sScr[wib];
-    double* recW = sW[wib];
-    double* recG = sG[wib];
+    double2* rec = sRec[wib];
     const int cur = L->iter & 1, nxt = cur ^ 1;
     const int n = L->cnt[cur].sum;
     if (n == 0) return;
@@ -614,7 +685,7 @@ near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
         double2 sums = make_double2(0.0, 0.0);
         int nrec = 0;
         unsigned int got = 0;
-        near_blocks<Periodic, false>(t, f, nLive, scr, x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+        near_blocks<0, Periodic, false>(t, f, nLive, scr, x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
             near_candidates(scr.blk, nb, nLive, t.xyzh, [&](const double4& pj, int, bool valid) {
                 double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                 nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
@@ -622,54 +693,176 @@ near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                 const bool acc = valid && q2 < kRadK2;
                 const uint32_t m = __ballot_sync(0xffffffffu, acc);
                 const int k = nrec + __popc(m & lt);
-                if (acc && k < kNearRec) recW[k] = q2;
+                if (acc && k < kNearRec) rec[k].x = q2;
                 nrec += __popc(m);
                 if (nrec >= kNearRec)
                 {
-                    sums = near_add_records(recW, recG, kNearRec, sums);
+                    sums = near_add_records(rec, kNearRec, sums);
                     got += kNearRec;
                     nrec -= kNearRec;   // those beyond the buffer start the next one
-                    if (acc && k >= kNearRec) recW[k - kNearRec] = q2;
+                    if (acc && k >= kNearRec) rec[k - kNearRec].x = q2;
                     __syncwarp();
                 }
-                return true;
+                return got < kHuge;
             });
-            return r;
+            return got < kHuge ? r : -1.0f;
         });
-        sums = near_add_records(recW, recG, nrec, sums);
+        if (got >= kHuge)
+        {
+            if (lane == 0) lists.huge[cur][atomicAdd(&L->cnt[cur].huge, 1)] = i;
+            __syncwarp();
+            continue;
+        }
+        sums = near_add_records(rec, nrec, sums);
         got += nrec;
-        double ro, go, ho;
-        int conv;
-        newton_step(sums.x, sums.y, hi, pmass, hfact, tolh, ro, go, ho, conv);
         if (lane == 0)
         {
             pairs += got;
-            rho[i] = ro;
-            gradh[i] = go;
-            reinterpret_cast<double*>(xyzh + i)[3] = ho;
-            const unsigned long long hb = (unsigned long long)__double_as_longlong(hi);
-            const unsigned long long ob = (unsigned long long)__double_as_longlong(ho);
-            seen = hb > seen ? hb : seen;
-            if (conv)
-            {
-                converged[i] = 1;
-                hs[i] = ho;
-                hconv = ob > hconv ? ob : hconv;
-                lists.cover[atomicAdd(&L->cover, 1)] = i;
-            }
-            else
-            {
-                // about got * (kNearMargin ho / hi)^3 entries in a row made now
-                const double grow = kNearMargin * ho / hi;
-                const bool fits = double(got) * grow * grow * grow < 0.95 * kNbl;
-                if (fits) lists.build[nxt][atomicAdd(&L->cnt[nxt].build, 1)] = i;
-                else lists.sum[nxt][atomicAdd(&L->cnt[nxt].sum, 1)] = i;
-            }
+            sum_finish(i, hi, sums, got, L, lists, nxt, xyzh, rho, gradh, converged, hs, pmass, tolh, hfact, seen,
+                       hconv);
         }
         __syncwarp();
     }
     note_h(seen, hconv, ds, shH);
     if (lane == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
+}
+
+// The same for a particle of very many neighbours (the widest supports of a scattered start
+// reach whole sets), one block each: the first warp walks the tree down to its 64-particle
+// nodes, every warp takes four of them at a time, and the warps' record buffers are added in
+// the warps' order -- together where all fit one binade without a tie, else one buffer after
+// the other.  Alone on one warp such a particle took 17 ns a neighbour, 2 ms for the widest
+// of 120,000 particles, which was the length of the iteration.
+template<bool Periodic>
+__global__ void __launch_bounds__(32 * kHugeWarps)
+near_huge_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
+                 const __grid_constant__ NearLists lists, double4* __restrict__ xyzh,
+                 double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
+                 double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
+{
+    __shared__ NearScratch scr;
+    __shared__ double2 sRec[kHugeWarps][kNearRec];
+    __shared__ int sSel[kHugeWarps][32];
+    __shared__ OrderedPart sPart[kHugeWarps][2];
+    __shared__ int sCount[kHugeWarps];
+    __shared__ int sItem, sNodes;
+    __shared__ double2 sSums;
+    __shared__ unsigned long long shH[2];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const int cur = L->iter & 1, nxt = cur ^ 1;
+    const int n = L->cnt[cur].huge;
+    if (n == 0) return;
+    const int nLive = *t.nLive;
+    const NearFrame f(t.box);
+    double lx = 0, ly = 0, lz = 0;
+    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    double2* rec = sRec[wib];
+    unsigned long long pairs = 0, seen = 0, hconv = 0;
+    for (;;)
+    {
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            sItem = atomicAdd(&L->ticket[3], 1);
+            sSums = make_double2(0.0, 0.0);
+        }
+        __syncthreads();
+        if (sItem >= n) break;
+        const int i = lists.huge[cur][sItem];
+        const double4 pi = xyzh[i];
+        const double hi = pi.w, hinv2 = 1.0 / (hi * hi);
+        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
+        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * hi) + f.slack(x, y, z);
+        const float r2max = r * r * 1.000001f;
+        unsigned int got = 0;   // of this warp
+        // the whole block over the 64-particle nodes scr.blk[0 .. cnt)
+        auto work = [&](int cnt) {
+            for (int c0 = 0; c0 < cnt; c0 += 4 * kHugeWarps)
+            {
+                const int at = c0 + 4 * wib + (lane >> 3);
+                const int id = at < cnt ? scr.blk[at] * 8 + (lane & 7) : -1;
+                bool hit = id >= 0 && id < near_count(nLive, 0);
+                if (hit)
+                    hit = near_gap2<Periodic>(x, y, z, 0.0f, 0.0f, 0.0f, ld_node(t.node + t.off[0] + id), f) <= r2max;
+                const uint32_t hm = __ballot_sync(0xffffffffu, hit);
+                if (hit) sSel[wib][__popc(hm & lt)] = id;
+                __syncwarp();
+                int m = 0;
+                if (hm)
+                    near_candidates(sSel[wib], __popc(hm), nLive, t.xyzh, [&](const double4& pj, int, bool valid) {
+                        double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                        nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+                        const double q2 = pair_r2(dx, dy, dz) * hinv2;
+                        const bool acc = valid && q2 < kRadK2;
+                        const uint32_t am = __ballot_sync(0xffffffffu, acc);
+                        if (acc) rec[m + __popc(am & lt)].x = q2;   // at most 32 blocks of 8: kNearRec
+                        m += __popc(am);
+                        return true;
+                    });
+                got += m;
+                __syncwarp();
+                eval_records(rec, m);
+                __syncwarp();
+                const Binade bw(sSums.x), bg(sSums.y);
+                const OrderedPart pw = ordered_part(rec, 0, m, bw), pg = ordered_part(rec, 1, m, bg);
+                if (lane == 0) { sPart[wib][0] = pw; sPart[wib][1] = pg; sCount[wib] = m; }
+                __syncthreads();
+                if (wib == 0)
+                {
+                    double2 s = sSums;
+                    bool okW = true, okG = true;
+                    double uw = 0.0, dw = 0.0, ug = 0.0, dg = 0.0;
+                    for (int k = 0; k < kHugeWarps; ++k)
+                    {
+                        okW = okW && sPart[k][0].ok; okG = okG && sPart[k][1].ok;
+                        uw += sPart[k][0].up; dw += sPart[k][0].down;
+                        ug += sPart[k][1].up; dg += sPart[k][1].down;
+                    }
+                    okW = okW && bw.holds(uw, dw);
+                    okG = okG && bg.holds(ug, dg);
+                    if (!okW || !okG)
+                        for (int k = 0; k < kHugeWarps; ++k) s = ordered_add(sRec[k], sCount[k], s);
+                    if (okW) s.x = bw.sign * ((bw.a + uw) - dw);
+                    if (okG) s.y = bg.sign * ((bg.a + ug) - dg);
+                    if (lane == 0) sSums = s;
+                }
+                __syncthreads();
+            }
+        };
+        if (wib == 0)
+        {
+            near_blocks<1, Periodic, false>(t, f, nLive, scr, x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+                if (lane == 0) sNodes = nb;
+                __syncthreads();
+                work(nb);
+                return r;
+            });
+            if (lane == 0) sNodes = 0;
+            __syncthreads();
+        }
+        else
+            for (;;)
+            {
+                __syncthreads();
+                const int cnt = sNodes;
+                if (cnt == 0) break;
+                work(cnt);
+            }
+        // the warps' counts (each lane holds its warp's)
+        if (lane == 0) sCount[wib] = int(got);
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            unsigned int all = 0;
+            for (int k = 0; k < kHugeWarps; ++k) all += unsigned(sCount[k]);
+            pairs += all;
+            sum_finish(i, hi, sSums, all, L, lists, nxt, xyzh, rho, gradh, converged, hs, pmass, tolh, hfact, seen,
+                       hconv);
+        }
+    }
+    note_h(seen, hconv, ds, shH);
+    if (threadIdx.x == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
 }
 
 // End of an iteration: what it left active, the next one's lists in place, and whether it
@@ -679,9 +872,9 @@ __global__ void near_epilogue_kernel(NearLoop* L, cudaGraphConditionalHandle mor
     const int it = L->iter, cur = it & 1, nxt = cur ^ 1;
     if (it < kLoopIters) L->activePerIter[it] = L->active;
     L->cnt[cur] = NearCounts{};
-    L->ticket[0] = L->ticket[1] = 0;
+    L->ticket[0] = L->ticket[1] = L->ticket[3] = 0;
     L->all = 0;
-    L->active = L->cnt[nxt].row + L->cnt[nxt].build + L->cnt[nxt].sum;
+    L->active = L->cnt[nxt].row + L->cnt[nxt].build + L->cnt[nxt].sum + L->cnt[nxt].huge;
     L->iter = it + 1;
     if (setCondition) cudaGraphSetConditional(more, L->active > 0 && it + 1 < L->maxIter ? 1u : 0u);
 }
@@ -732,6 +925,7 @@ static NearLists near_lists(State& s)
         l.row[k] = s.nearRow[k].get();
         l.build[k] = s.nearBuild[k].get();
         l.sum[k] = s.nearSum[k].get();
+        l.huge[k] = s.nearHuge[k].get();
     }
     l.cover = s.nearCover.get();
     l.over = s.nearOver.get();
@@ -750,7 +944,7 @@ static void near_iteration(State& s, double pmass, double tolh, double hfact, in
     rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(t, L, lists, s.nblR2.get(), rowsJ,
                                                                       s.nblCount.get(), s.nblH.get(), 0);
     COSMO_LAUNCHED();
-    near_step_kernel<<<std::max(1, std::min(iceil(n, kThreads), 16 * s.numSMs)), kThreads, 0, s.st>>>(
+    near_step_kernel<<<iceil(n, kThreads), kThreads, 0, s.st>>>(
         L, lists, s.nblR2.get(), s.nblCount.get(), s.nblH.get(), s.xyzh.get(), s.rho.get(), s.gradh.get(),
         s.converged.get(), s.hs.get(), pmass, tolh, hfact, ds);
     COSMO_LAUNCHED();
@@ -758,6 +952,11 @@ static void near_iteration(State& s, double pmass, double tolh, double hfact, in
     sum<<<persistent_blocks(s, sum, kThreads), kThreads, 0, s.st>>>(t, L, lists, s.xyzh.get(), s.rho.get(),
                                                                     s.gradh.get(), s.converged.get(), s.hs.get(), pmass,
                                                                     tolh, hfact, ds);
+    COSMO_LAUNCHED();
+    // few particles have that many neighbours, if any: a block a multiprocessor
+    auto huge = s.periodic ? near_huge_kernel<true> : near_huge_kernel<false>;
+    huge<<<s.numSMs, 32 * kHugeWarps, 0, s.st>>>(t, L, lists, s.xyzh.get(), s.rho.get(), s.gradh.get(),
+                                                 s.converged.get(), s.hs.get(), pmass, tolh, hfact, ds);
     COSMO_LAUNCHED();
     near_epilogue_kernel<<<1, 1, 0, s.st>>>(L, more, setCondition);
     COSMO_LAUNCHED();
@@ -781,6 +980,7 @@ static bool near_graph(State& s, double pmass, double tolh, double hfact, int ma
                           (const void*)s.hs.get(), (const void*)s.nearRow[0].get(), (const void*)s.nearRow[1].get(),
                           (const void*)s.nearBuild[0].get(), (const void*)s.nearBuild[1].get(),
                           (const void*)s.nearSum[0].get(), (const void*)s.nearSum[1].get(),
+                          (const void*)s.nearHuge[0].get(), (const void*)s.nearHuge[1].get(),
                           (const void*)s.nearCover.get(), (const void*)s.nearOver.get()})
         add(q);
     for (int v : {n, s.ngas, s.periodic, s.numSMs, maxIter}) add(v);
@@ -857,7 +1057,7 @@ void near_newton(State& s, double pmass, double tolh, double hfact, int maxIter,
     const int n = std::max(s.nAlive, 1);
     DevScalars* ds = s.dscal.get();
     for (auto* b : {&s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1], &s.nearSum[0], &s.nearSum[1],
-                    &s.nearCover, &s.nearOver})
+                    &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
         b->resize(n, s.st);
     s.hs.resize(n, s.st);
     s.nearLoop.resize(1, s.st);

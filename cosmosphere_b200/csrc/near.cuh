@@ -29,10 +29,7 @@
 namespace cosmo {
 
 constexpr int kNearLevels = 9;     // level 0: blocks of 8 particles; 32 * 8^9 particles at most
-#ifndef NBLK
-#define NBLK 128
-#endif
-constexpr int kNearBlocks = NBLK;   // blocks a warp holds at once
+constexpr int kNearBlocks = 128;   // blocks a warp holds at once
 constexpr int kNearWarps  = 4;     // warps per block of the search kernels
 
 // A node's box: centre, half extents (empty: negative infinity) and its largest h.
@@ -127,8 +124,9 @@ __device__ __forceinline__ float near_sym_reach(float hmax, float slack)
 // reach to go on with (the members still searching may be narrower), negative to stop.
 // The top level (at most 32 nodes) is tested first; then always the first four nodes of the
 // deepest level that holds any are expanded, one child per lane, so each level holds at
-// most 32 nodes and the blocks come out in order.
-template<bool Periodic, bool Sym, class Flush>
+// most 32 nodes and the blocks come out in order.  Stop = 1 hands out the nodes of level 1
+// instead (of more than 256 particles).
+template<int Stop, bool Periodic, bool Sym, class Flush>
 __device__ __forceinline__ void near_blocks(const NearTree& t, const NearFrame& f, int nLive, NearScratch& scr, float x,
                                             float y, float z, float ex, float ey, float ez, float reach, float slack,
                                             Flush&& flush)
@@ -149,7 +147,7 @@ __device__ __forceinline__ void near_blocks(const NearTree& t, const NearFrame& 
         const bool ok = valid && test(level, idx);
         const uint32_t m = __ballot_sync(0xffffffffu, ok);
         const int c = __popc(m);
-        if (level == 0)
+        if (level == Stop)
         {
             if (ok) scr.blk[nb + __popc(m & lt)] = idx;
             nb += c;
@@ -166,9 +164,9 @@ __device__ __forceinline__ void near_blocks(const NearTree& t, const NearFrame& 
     for (;;)
     {
         int have = 0;
-        while (lev > 0 && lev <= top && (have = __shfl_sync(0xffffffffu, left, lev)) == 0) ++lev;
-        const bool end = lev == 0 || lev > top;
-        if (end || (lev == 1 && nb + 32 > kNearBlocks))
+        while (lev > Stop && lev <= top && (have = __shfl_sync(0xffffffffu, left, lev)) == 0) ++lev;
+        const bool end = lev <= Stop || lev > top;
+        if (end || (lev == Stop + 1 && nb + 32 > kNearBlocks))
         {
             if (nb > 0) reach = flush(nb);
             if (end || reach < 0.0f) return;
@@ -181,7 +179,7 @@ __device__ __forceinline__ void near_blocks(const NearTree& t, const NearFrame& 
         const int child = node * 8 + (lane & 7);
         if (lane == lev) { left -= m; pos += m; }
         accept(lev - 1, child, (lane >> 3) < m && child < near_count(nLive, lev - 1));
-        if (lev > 1) --lev;
+        if (lev > Stop + 1) --lev;
     }
 }
 

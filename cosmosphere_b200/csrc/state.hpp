@@ -128,14 +128,14 @@ struct NewtonLoop
 // (double-buffered by the iteration's parity) and its state on the device.
 struct NearCounts
 {
-    int row, build, sum, pad;    // particles with a row, without one, with more neighbours than one holds
+    int row, build, sum, huge;   // particles with a row, without one, with more neighbours than one holds, with very many
 };
 struct NearLoop
 {
     int iter, maxIter, active;   // active: particles the next iteration updates
     int all;                     // the search list is every live particle
     int cover, over;             // rows still to be made at the converged h; those that do not fit one
-    int ticket[4];               // work tickets: row search, direct sums, cover search, over passes
+    int ticket[4];               // work tickets: row search, direct sums, cover search, direct sums by blocks
     NearCounts cnt[2];
     long long activePerIter[kLoopIters];
 };
@@ -144,6 +144,7 @@ struct NearLists
     int* row[2];
     int* build[2];
     int* sum[2];
+    int* huge[2];
     int* cover;
     int* over;
 };
@@ -290,7 +291,7 @@ struct State
     DBuf<int> leafNext;                         // leaf already queued for the next iteration
     DBuf<int> activeA, activeB, allLeaves;
     DBuf<float4> nearNode;                      // the block tree (near.cuh), two float4 a node
-    DBuf<int> nearRow[2], nearBuild[2], nearSum[2], nearCover, nearOver;   // the block-tree loop's lists
+    DBuf<int> nearRow[2], nearBuild[2], nearSum[2], nearHuge[2], nearCover, nearOver;   // the block-tree loop's lists
     DBuf<NearLoop> nearLoop;                    // its state
 
     // scratch
