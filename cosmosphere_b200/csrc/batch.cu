@@ -16,6 +16,7 @@
 #include <string>
 
 #include "densengine.cuh"
+#include "near.cuh"
 #include "pairstream.cuh"
 #include "sort.cuh"
 #include "state.hpp"
@@ -58,6 +59,7 @@ struct Batch
     uint32_t listCap = 0;
     std::vector<double> tuning;       // per set: bucket, list margin, cut stream, cut work
     bool graphUsed = false;
+    bool forestDone = false;          // the leaf forest of the last solve's sets is built
 };
 
 namespace {
@@ -696,12 +698,13 @@ __global__ void scatter_kernel_b(const int* __restrict__ order, int n, const dou
 } // namespace
 
 // ====================================================================== host side
-static void batch_build(Batch& B)
+// Every set's box, the keys, the segmented sort and the gather.
+static void batch_sort(Batch& B)
 {
     State& s = B.core;
     const int n = B.n, ns = B.nsets;
     DevScalars* ds = s.dscal.get();
-    cudaEvent_t e0 = ev(s);
+    B.forestDone = false;
     set_box_kernel_b<<<ns, 256, 0, s.st>>>(B.dOffs.get(), B.setPer.get(), B.setBox6.get(), B.ux.get(), B.uy.get(),
                                            B.uz.get(), B.boxes.get());
     COSMO_LAUNCHED();
@@ -752,7 +755,14 @@ static void batch_build(Batch& B)
     gather_kernel_b<<<iceil(n, kBlk), kBlk, 0, s.st>>>(B.orderA.get(), n, B.ux.get(), B.uy.get(), B.uz.get(),
                                                        B.uh.get(), B.xyzh.get());
     COSMO_LAUNCHED();
+}
 
+// The leaf forest of the sorted sets and its nodes: what the list-based loop walks.  The
+// block-tree loop needs none of it, and its counts are made when a caller asks for them.
+static void batch_forest(Batch& B)
+{
+    State& s = B.core;
+    const int ns = B.nsets;
     // forest leaves: one root per set, split while a node holds more than its bucket
     int L = ns;
     B.leafKey.resize(L, s.st);
@@ -820,9 +830,7 @@ static void batch_build(Batch& B)
     COSMO_LAUNCHED();
     iota_kernel_b<<<iceil(L, kBlk), kBlk, 0, s.st>>>(B.allLeaves.get(), L);
     COSMO_LAUNCHED();
-    cudaEvent_t e1 = ev(s);
-    read_scalars(s);
-    B.tBuild = elapsed_s(e0, e1);
+    B.forestDone = true;
 }
 
 // The gather lists of the given leaves (count on the device): a leaf whose kept list
@@ -943,6 +951,35 @@ static void final_rho(Batch& B)
     run_items(B, B.allLeaves.get(), &ls->nAll, true, 0.0, 0.0);
 }
 
+constexpr int kNearBatchMost = 48 << 20;   // particles
+
+// A batched solve over the sets' block trees (near.cu).
+static int batch_solve_near(Batch& B, double tolh, double hfact, int maxIter, int flags, cudaEvent_t t0)
+{
+    State& s = B.core;
+    const NearForest f{B.n, B.nsets, B.dOffs.get(), B.nAliveSet.get(), B.setOf.get(), B.boxes.get(), B.pmass.get(),
+                       B.xyzh.get(), B.rho.get(), B.gradh.get(), B.converged.get()};
+    cudaEvent_t t1 = ev(s);
+    near_forest_newton(s, f, tolh, hfact, maxIter, (flags & COSMO_BATCH_GRAPH) != 0);
+    B.graphUsed = s.lastLoopGraph != 0;
+    cudaEvent_t t2 = ev(s);
+    if (flags & COSMO_BATCH_FINAL_RHO) near_forest_eval(s, f);
+    cudaEvent_t t3 = ev(s);
+    NearLoop h;
+    COSMO_CUDA(cudaMemcpyAsync(&h, s.nearLoop.get(), sizeof(NearLoop), cudaMemcpyDeviceToHost, s.st));
+    read_scalars(s);
+    check_dev_err(s, "cosmo_batch_density", false);
+    B.unconverged = int(near_results(s, h));
+    B.itersRun = s.itersRun;
+    B.activePerIter = s.activePerIter;
+    B.tBuild = elapsed_s(t0, t1);
+    B.tNR = elapsed_s(t1, t2);
+    B.tList = 0.0;
+    B.tTotal = elapsed_s(t0, t3);
+    B.pairs = s.hscal->pairs[0];
+    return B.unconverged > 0 ? 1 : 0;
+}
+
 static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int flags, int attempt = 0)
 {
     State& s = B.core;
@@ -955,7 +992,12 @@ static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int fla
     COSMO_CUDA(cudaMemsetAsync(B.converged.get(), 0, size_t(B.n) * 4, s.st));
     COSMO_CUDA(cudaMemsetAsync(&ds->pairs[0], 0, sizeof(ds->pairs), s.st));
     cudaEvent_t t0 = ev(s);
-    batch_build(B);
+    batch_sort(B);
+    // The plain form runs over the sets' block trees (the mixed form's rounding is defined by
+    // the group engine's groups; the staged feed is a variant of that engine).  Its rows take
+    // 1 KB a particle: very large batches keep the lists, which take less.
+    if (s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost) return batch_solve_near(B, tolh, hfact, maxIter, flags, t0);
+    batch_forest(B);
     const int L = B.nLeaves;
     long long nAliveTotal = 0;
     {
@@ -1072,6 +1114,7 @@ int cosmo_batch_init(int nsets, const int* offsets)
     if (n < 1) return -1;
     B.nsets = nsets;
     B.n = n;
+    B.itersRun = 0;   // nothing solved yet
     B.offs.assign(offsets, offsets + nsets + 1);
     for (auto* b : {&B.dOffs, &B.setLeafStart, &B.setNodeStart}) b->resize(size_t(nsets) + 1, s.st);
     for (auto* b : {&B.nAliveSet, &B.bucket, &B.setPer}) b->resize(nsets, s.st);
@@ -1214,6 +1257,11 @@ double cosmo_batch_scalar(const char* name)
 {
     Batch& B = batch();
     const std::string k(name);
+    if ((k == "nLeaves" || k == "numNodes") && B.itersRun > 0 && !B.forestDone)
+    {
+        batch_forest(B);
+        COSMO_CUDA(cudaStreamSynchronize(B.core.st));
+    }
     if (k == "nLeaves") return B.nLeaves;
     if (k == "numNodes") return B.numNodes;
     if (k == "itersRun") return B.itersRun;

@@ -214,8 +214,8 @@ gradient_over_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ 
     const int n = L->over;
     if (n == 0 || L->active > 0) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) ds->rowOverflow = 1;
-    const int nLive = *t.nLive;
     const NearFrame f(t.box);
+    const NearView v = near_view(t, f);
     double lx = 0, ly = 0, lz = 0;
     if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
     double* term = sTerm[wib];
@@ -229,8 +229,8 @@ gradient_over_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ 
         const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
         double sum = 0.0;   // lane k: sum k
         unsigned int gp = 0;
-        near_blocks<0, Periodic, false>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
-            near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
+        near_blocks<0, Periodic, false>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+            near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, [&](const double4& pj, int j, bool valid) {
                 double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                 nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
                 const double r2 = pair_r2(dx, dy, dz);
@@ -241,7 +241,7 @@ gradient_over_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ 
                 {
                     double* mine = term + __popc(m & ((1u << lane) - 1u)) * kGradTerms;
                     grad_terms(dx, dy, dz, r2, q2, vi, ai, ldg4(vel4 + j), ldg4(acc4 + j), pmass,
-                               [&](int k, double v) { mine[k] = v; });
+                               [&](int k, double x) { mine[k] = x; });
                 }
                 __syncwarp();
                 const int c = __popc(m);
@@ -280,8 +280,8 @@ over_extras_kernel(const __grid_constant__ NearTree t, const NearLoop* __restric
     const int wib = threadIdx.x >> 5;
     const int n = L->over;
     if (n == 0) return;
-    const int nLive = *t.nLive;
     const NearFrame f(t.box);
+    const NearView v = near_view(t, f);
     double lx = 0, ly = 0, lz = 0;
     if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
     for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (gridDim.x * blockDim.x) >> 5)
@@ -291,8 +291,8 @@ over_extras_kernel(const __grid_constant__ NearTree t, const NearLoop* __restric
         const double bi = kRadK2 * (pi.w * pi.w) * (1.0 + 1e-10);
         const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
         const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
-        near_blocks<0, Periodic, false>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
-            near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
+        near_blocks<0, Periodic, false>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+            near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, [&](const double4& pj, int j, bool valid) {
                 double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                 nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
                 const double dr2 = pair_r2(dx, dy, dz);
@@ -1354,8 +1354,9 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         }
         else
             fromRows = writeJ && s.nAlive > 0 && rowsBuilt && cover_rows(s, itemCap, cut, spreadG);
-        // pairs other particles' supports add: about ten a particle where h scatters
-        const int extraCap = s.symExtraCap > 0 ? std::min(s.symExtraCap, itemCap) : near ? int(std::min(16ll * itemCap, 1ll << 30)) : itemCap;
+        // pairs other particles' supports add: about ten a particle where h scatters (a set so
+        // large that their buffer matters goes back to the lists when they are that many)
+        const int extraCap = s.symExtraCap > 0 ? std::min(s.symExtraCap, itemCap) : near && itemCap <= 1 << 24 ? 16 * itemCap : itemCap;
         const int* active = near ? &s.nearLoop.get()->active : nullptr;
         if (fromRows)
             sym_rows_from_newton(s, extraCap, near);

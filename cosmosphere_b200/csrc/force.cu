@@ -397,8 +397,8 @@ force_over_kernel(const __grid_constant__ NearTree t, int n, const int* __restri
     __shared__ double sTerm[kWarpsPerBlock][32 * (kForceTerms + 1)];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     constexpr int kStride = kForceTerms + 1;
-    const int nLive = *t.nLive;
     const NearFrame f(t.box);
+    const NearView v = near_view(t, f);
     double lx = 0, ly = 0, lz = 0;
     if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
     double* term = sTerm[wib];
@@ -412,13 +412,13 @@ force_over_kernel(const __grid_constant__ NearTree t, int n, const int* __restri
         const float slack = f.slack(x, y, z);
         const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * A.p.w) + slack;
         double sum = 0.0;   // lanes 0-5: the pressure sums, 6: the energy, 7: div v, 8: vsig
-        near_blocks<0, Periodic, true>(t, f, nLive, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
-            near_candidates(sScr[wib].blk, nb, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
+        near_blocks<0, Periodic, true>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
+            near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, [&](const double4& pj, int j, bool valid) {
                 double* mine = term + lane * kStride;
                 for (int k = 0; k < kForceTerms; ++k) mine[k] = 0.0;
                 const bool took = valid && A.terms<Periodic, Disc>(pj, j, vel4, thermo4, prepA, lx, ly, lz, pmass,
                                                                    alphau, beta, pdv, shock,
-                                                                   [&](int k, double v) { mine[k] = v; });
+                                                                   [&](int k, double x) { mine[k] = x; });
                 uint32_t m = __ballot_sync(0xffffffffu, took);
                 A.gp += __popc(m);
                 __syncwarp();

@@ -72,19 +72,37 @@ __device__ __forceinline__ NearNode node_parent(int count, Get&& get)
 
 // Levels 0 to 2: 512 particles a block, one per thread; each level's boxes are reduced in
 // shared memory and written once (one 32-byte read per particle: DRAM bound, 11 us at 1.4 M).
+// A batch's blocks are its level-2 slots, each looked up to find its set.
+template<bool Forest>
 __global__ void __launch_bounds__(512)
-near_leaf_levels_kernel(const __grid_constant__ NearTree t, NearNode* __restrict__ out)
+near_leaf_levels_kernel(const __grid_constant__ NearTree t, NearNode* __restrict__ out,
+                        const NearSet* __restrict__ sets, int nsets, int slots)
 {
     __shared__ NearNode s0[64], s1[8];
-    const int n = *t.nLive;
-    const NearFrame f(t.box);
-    for (int b = blockIdx.x; b * 512 < n; b += gridDim.x)
+    NearFrame f(t.box);
+    NearView v = Forest ? NearView{0, 0, 0, 0.0f, 0.0f, 0.0f} : near_view(t, f);
+    for (int q = blockIdx.x; q < slots; q += gridDim.x)
     {
+        int b = q;
+        if constexpr (Forest)
+        {
+            int lo = 0, hi = nsets;   // the last set whose slots start at or before q
+            while (hi - lo > 1)
+            {
+                const int mid = (lo + hi) >> 1;
+                if ((sets[mid].p0 >> 9) + mid <= q) lo = mid;
+                else hi = mid;
+            }
+            f = NearFrame(sets[lo]);
+            v = NearView{sets[lo].p0, lo, sets[lo].n, 0.0f, 0.0f, 0.0f};
+            b = q - ((v.p0 >> 9) + lo);
+        }
+        if (b * 512 >= v.n) continue;
         const int i = b * 512 + int(threadIdx.x);
         float lx = INFINITY, ly = INFINITY, lz = INFINITY, hx = -INFINITY, hy = -INFINITY, hz = -INFINITY, hm = 0.0f;
-        if (i < n)
+        if (i < v.n)
         {
-            const double4 p = t.xyzh[i];
+            const double4 p = t.xyzh[v.p0 + i];
             const double x = p.x - f.cx, y = p.y - f.cy, z = p.z - f.cz;
             lx = __double2float_rd(x); hx = __double2float_ru(x);
             ly = __double2float_rd(y); hy = __double2float_ru(y);
@@ -99,38 +117,60 @@ near_leaf_levels_kernel(const __grid_constant__ NearTree t, NearNode* __restrict
             lz = fminf(lz, __shfl_xor_sync(0xffffffffu, lz, o)); hz = fmaxf(hz, __shfl_xor_sync(0xffffffffu, hz, o));
             hm = fmaxf(hm, __shfl_xor_sync(0xffffffffu, hm, o));
         }
+        auto put = [&](int level, int idx, const NearNode& nd) { out[near_node(t, v, level, idx) - t.node] = nd; };
         if ((threadIdx.x & 7) == 0)
         {
             const NearNode nd = node_of(lx, ly, lz, hx, hy, hz, hm);
             s0[threadIdx.x >> 3] = nd;
-            if (i < n) out[t.off[0] + (i >> 3)] = nd;
+            if (i < v.n) put(0, i >> 3, nd);
         }
         __syncthreads();
         if (threadIdx.x < 8)
         {
             const NearNode nd = node_parent(8, [&](int k) { return s0[threadIdx.x * 8 + k]; });
             s1[threadIdx.x] = nd;
-            const int q = b * 8 + int(threadIdx.x);
-            if (q * 64 < n) out[t.off[1] + q] = nd;
+            const int p = b * 8 + int(threadIdx.x);
+            if (p * 64 < v.n) put(1, p, nd);
         }
         __syncthreads();
-        if (threadIdx.x == 0) out[t.off[2] + b] = node_parent(8, [&](int k) { return s1[k]; });
+        if (threadIdx.x == 0) put(2, b, node_parent(8, [&](int k) { return s1[k]; }));
         __syncthreads();
     }
 }
 
-// The levels above, up to the first of at most 32 nodes: one block, level by level.
+// The levels above, up to the first of at most 32 nodes: one block a set, level by level.
+template<bool Forest>
 __global__ void __launch_bounds__(1024)
-near_upper_levels_kernel(const __grid_constant__ NearTree t, NearNode* out)
+near_upper_levels_kernel(const __grid_constant__ NearTree t, NearNode* out, const NearSet* __restrict__ sets)
 {
-    const int n = *t.nLive;
-    for (int l = 3; l < kNearLevels && near_count(n, l - 1) > 32; ++l)
+    const NearFrame f(t.box);
+    const NearView v = Forest ? NearView{sets[blockIdx.x].p0, int(blockIdx.x), sets[blockIdx.x].n, 0.0f, 0.0f, 0.0f}
+                              : near_view(t, f);
+    for (int l = 3; l < kNearLevels && near_count(v.n, l - 1) > 32; ++l)
     {
-        const int below = near_count(n, l - 1), here = near_count(n, l);
+        const int below = near_count(v.n, l - 1), here = near_count(v.n, l);
         for (int q = threadIdx.x; q < here; q += blockDim.x)
-            out[t.off[l] + q] = node_parent(min(8, below - 8 * q), [&](int k) { return out[t.off[l - 1] + 8 * q + k]; });
+            out[near_node(t, v, l, q) - t.node] =
+                node_parent(min(8, below - 8 * q), [&](int k) { return out[near_node(t, v, l - 1, 8 * q + k) - t.node]; });
         __syncthreads();
     }
+}
+
+// The sets of a batch as the searches read them (boxes and live counts are those of the
+// batch's key sort).
+__global__ void near_sets_kernel(int nsets, const int* __restrict__ offs, const int* __restrict__ nAlive,
+                                 const DevBox* __restrict__ boxes, const double* __restrict__ pmass,
+                                 NearSet* __restrict__ sets)
+{
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nsets) return;
+    const DevBox b = boxes[s];
+    const NearFrame f(&b);
+    const bool per = b.periodic != 0;
+    const float inf = INFINITY;
+    const double dinf = double(inf);
+    sets[s] = NearSet{offs[s], nAlive[s], per ? f.lx : inf, per ? f.ly : inf, per ? f.lz : inf, f.len, f.cx, f.cy, f.cz,
+                      per ? b.len[0] : dinf, per ? b.len[1] : dinf, per ? b.len[2] : dinf, pmass[s]};
 }
 
 // ---------------------------------------------------------------- lists
@@ -257,7 +297,38 @@ near_frozen_kernel(NearLoop* L, const int* __restrict__ order, const int* __rest
     note_h(0, hconv, ds, shH);
 }
 
-__global__ void near_frozen_count_kernel(NearLoop* L) { L->active = L->cnt[0].build; }
+__global__ void near_active_kernel(NearLoop* L) { L->active = L->cnt[0].build; }
+
+// A batch starts with the live particles of all its sets (each set's come first in its part
+// of the sorted order) on the search list.
+__global__ void near_forest_zero_kernel(NearLoop* L, int maxIter)
+{
+    L->iter = 0;
+    L->maxIter = maxIter;
+    L->active = 0;
+    L->all = 0;
+    L->cover = L->over = 0;
+    L->cnt[0] = L->cnt[1] = NearCounts{0, 0, 0, 0};
+    L->ticket[0] = L->ticket[1] = L->ticket[2] = L->ticket[3] = 0;
+}
+
+__global__ void __launch_bounds__(kThreads)
+near_forest_init_kernel(NearLoop* L, int n, const NearSet* __restrict__ sets, const int* __restrict__ setOf,
+                        const __grid_constant__ NearLists lists)
+{
+    __shared__ int sh[3 * (kNearWarps + 1)];
+    for (int b = blockIdx.x * kThreads; b < n; b += gridDim.x * kThreads)
+    {
+        const int k = b + int(threadIdx.x);
+        bool live = false;
+        if (k < n)
+        {
+            const NearSet& s = sets[setOf[k]];
+            live = k - s.p0 < s.n;
+        }
+        block_append(live ? 0 : -1, k, lists.build[0], &L->cnt[0].build, nullptr, nullptr, nullptr, nullptr, sh);
+    }
+}
 
 // ---------------------------------------------------------------- rows
 // Rows of the listed particles (all live ones when the list is the identity): the members of
@@ -273,10 +344,10 @@ __global__ void near_frozen_count_kernel(NearLoop* L) { L->active = L->cnt[0].bu
 //   cover = 1: rows at the converged h of particles left without; the others are listed
 //              (over) and marked as covering everything (rowH infinite: no pair of theirs
 //              is looked for from the other side).
-template<bool Periodic>
+template<bool Forest, bool Periodic>
 __global__ void __launch_bounds__(kThreads, 6)
-near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
-                 const __grid_constant__ NearLists lists, double* __restrict__ rowsR2,
+near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__ sets, const int* __restrict__ setOf,
+                 NearLoop* __restrict__ L, const __grid_constant__ NearLists lists, double* __restrict__ rowsR2,
                  int* __restrict__ rowsJ, int* __restrict__ nblCount, double* __restrict__ rowH, int cover)
 {
     __shared__ NearScratch sScr[kNearWarps];
@@ -290,10 +361,10 @@ near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
     int* ticket = &L->ticket[cover ? 2 : 0];
     const double margin = cover ? kCoverMargin : kNearMargin;
     const double wide2 = kRadK2 * (margin * margin);
-    const int nLive = *t.nLive;
     const NearFrame f(t.box);
+    NearView v = Forest ? NearView{0, 0, 0, 0.0f, 0.0f, 0.0f} : near_view(t, f);
     double lx = 0, ly = 0, lz = 0;
-    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    if (Periodic && !Forest) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
     int g = 32;
     while (g > 1 && n < g * int(gridDim.x) * kNearWarps) g >>= 1;
     for (;;)
@@ -305,9 +376,20 @@ near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
         const int at = w * g + lane;
         const bool mine = lane < g && at < n;
         const int i = mine ? (list ? list[at] : at) : 0;
+        const int set = Forest ? setOf[i] : 0;
         const double4 pi = t.xyzh[i];
-        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
-        const float slack = f.slack(x, y, z);
+        float x, y, z, slack;
+        if constexpr (Forest)
+        {
+            const NearFrame fs(sets[set]);
+            x = float(pi.x - fs.cx); y = float(pi.y - fs.cy); z = float(pi.z - fs.cz);
+            slack = fs.slack(x, y, z);
+        }
+        else
+        {
+            x = float(pi.x - f.cx); y = float(pi.y - f.cy); z = float(pi.z - f.cz);
+            slack = f.slack(x, y, z);
+        }
         const float r = mine ? __double2float_ru(kRadKernel * margin * (1.0 + 1e-6) * pi.w) + slack : -1.0f;
         scr.P[lane] = make_double4(pi.x, pi.y, pi.z, 1.0 / (pi.w * pi.w));
         scr.Q[lane] = make_float4(x, y, z, r * r * 1.000001f);
@@ -317,7 +399,7 @@ near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mean += __shfl_xor_sync(0xffffffffu, mean, o);
         const uint32_t wide = __ballot_sync(0xffffffffu, mine && r * float(__popc(all)) > kNearWide * mean);
-        const NearRun run = near_runs(x, y, z, (wide >> lane) & 1u ? -1.0f : r);
+        const NearRun run = near_runs<Forest>(x, y, z, (wide >> lane) & 1u ? -1.0f : r, set);
         int rowLen = 0;
         uint32_t todo = all;
         __syncwarp();
@@ -344,7 +426,15 @@ near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                 reach = __shfl_sync(0xffffffffu, r, p);
                 ex = ey = ez = 0.0f;
             }
-            near_blocks<0, Periodic, false>(t, f, nLive, scr, bx, by, bz, ex, ey, ez, reach, 0.0f, [&](int nb) -> float {
+            if constexpr (Forest)
+            {
+                const int sid = __shfl_sync(0xffffffffu, set, __ffs(members) - 1);
+                const NearSet& st = sets[sid];
+                v = NearView{st.p0, sid, st.n, st.lx, st.ly, st.lz};
+                lx = st.dlx; ly = st.dly; lz = st.dlz;
+            }
+            const double4* at0 = t.xyzh + v.p0;
+            near_blocks<0, Periodic, false>(t, v, scr, bx, by, bz, ex, ey, ez, reach, 0.0f, [&](int nb) -> float {
                 // the blocks of this batch, kNearBlocks / 32 per lane
                 constexpr int kU = kNearBlocks / 32;
                 NearNode nd[kU];
@@ -354,7 +444,7 @@ near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                 {
                     const int k = 32 * u + lane;
                     id[u] = k < nb ? scr.blk[k] : -1;
-                    if (32 * u < nb) nd[u] = ld_node(t.node + t.off[0] + max(id[u], 0));
+                    if (32 * u < nb) nd[u] = ld_node(near_node(t, v, 0, max(id[u], 0)));
                 }
                 bool dropped = false;
                 for (uint32_t rest = todo & members; rest; rest &= rest - 1)
@@ -367,7 +457,7 @@ near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                     {
                         if (32 * u >= nb) break;
                         const bool hit = id[u] >= 0 &&
-                                         near_gap2<Periodic>(q.x, q.y, q.z, 0.0f, 0.0f, 0.0f, nd[u], f) <= q.w;
+                                         near_gap2<Periodic>(q.x, q.y, q.z, 0.0f, 0.0f, 0.0f, nd[u], v) <= q.w;
                         const uint32_t m = __ballot_sync(0xffffffffu, hit);
                         if (hit) scr.sel[ns + __popc(m & lt)] = id[u];
                         ns += __popc(m);
@@ -377,7 +467,7 @@ near_rows_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                     const double4 gp = scr.P[p];
                     const size_t row = size_t(__shfl_sync(0xffffffffu, i, p)) * kNbl;
                     int len = __shfl_sync(0xffffffffu, rowLen, p);
-                    near_candidates(scr.sel, ns, nLive, t.xyzh, [&](const double4& pj, int j, bool valid) {
+                    near_candidates(scr.sel, ns, v.n, at0, [&](const double4& pj, int j, bool valid) {
                         double dx = gp.x - pj.x, dy = gp.y - pj.y, dz = gp.z - pj.z;
                         nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
                         const double r2 = pair_r2(dx, dy, dz);
@@ -436,8 +526,9 @@ __device__ __forceinline__ int next_of(bool conv, double ho, double rowHi)
 
 // One Newton iteration from the rows: one lane per particle streams its own row (8 bytes an
 // entry), tests every entry with the exact test and adds in the row's order.
+template<bool Forest>
 __global__ void __launch_bounds__(kThreads)
-near_step_kernel(NearLoop* __restrict__ L, const __grid_constant__ NearLists lists, const double* __restrict__ rowsR2,
+near_step_kernel(const NearSet* __restrict__ sets, const int* __restrict__ setOf, NearLoop* __restrict__ L, const __grid_constant__ NearLists lists, const double* __restrict__ rowsR2,
                  const int* __restrict__ nblCount, const double* __restrict__ rowH, double4* __restrict__ xyzh,
                  double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
                  double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
@@ -475,7 +566,7 @@ near_step_kernel(NearLoop* __restrict__ L, const __grid_constant__ NearLists lis
             pairs += gp;
             double ro, go, ho;
             int conv;
-            newton_step(sr, sg, hi, pmass, hfact, tolh, ro, go, ho, conv);
+            newton_step(sr, sg, hi, Forest ? sets[setOf[i]].pmass : pmass, hfact, tolh, ro, go, ho, conv);
             rho[i] = ro;
             gradh[i] = go;
             reinterpret_cast<double*>(xyzh + i)[3] = ho;
@@ -494,6 +585,51 @@ near_step_kernel(NearLoop* __restrict__ L, const __grid_constant__ NearLists lis
                      &L->cover, sh);
     }
     note_h(seen, hconv, ds, shH);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
+}
+
+// rho and d(rho)/dh at h from the un-normalised sums (src/density_base.cu:635-643).
+__device__ __forceinline__ void eval_store(int i, double hi, double sr, double sg, double pmass,
+                                           double* __restrict__ rho, double* __restrict__ gradh)
+{
+    const double hi1 = 1.0 / hi;
+    const double hi31 = hi1 * hi1 * hi1;
+    rho[i] = sr * kCnormk * pmass * hi31;
+    gradh[i] = sg * kCnormk * pmass * (hi31 * hi1);
+}
+
+// The same for every live particle of a batch with a row, at its final h.
+__global__ void __launch_bounds__(kThreads)
+near_eval_kernel(int n, const NearSet* __restrict__ sets, const int* __restrict__ setOf,
+                 const double* __restrict__ rowsR2, const int* __restrict__ nblCount, const double4* __restrict__ xyzh,
+                 double* __restrict__ rho, double* __restrict__ gradh, DevScalars* __restrict__ ds)
+{
+    unsigned int gp = 0;
+    const int i = blockIdx.x * kThreads + int(threadIdx.x);
+    if (i < n)
+    {
+        const NearSet& s = sets[setOf[i]];
+        if (i - s.p0 < s.n && unsigned(nblCount[i]) <= unsigned(kNbl))
+        {
+            const double hi = xyzh[i].w;
+            const double hinv2 = 1.0 / (hi * hi);
+            double sr = 0.0, sg = 0.0;
+            for_flat_row(row_flat(rowsR2, uint32_t(i)), nblCount[i], [&](double r2) {
+                const double q2 = r2 * hinv2;
+                if (!(q2 < kRadK2)) return;
+                ++gp;
+                const double q = sqrt(q2);
+                double wk, dwk;
+                sph_kernel(q2, q, wk, dwk);
+                sr += wk;
+                sg += -q * dwk - 3.0 * wk;
+            });
+            eval_store(i, hi, sr, sg, s.pmass, rho, gradh);
+        }
+    }
+    unsigned long long pairs = gp;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
     if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
@@ -648,10 +784,12 @@ __device__ __forceinline__ void sum_finish(int i, double hi, double2 sums, unsig
 }
 
 // One Newton iteration of the particles whose neighbours do not fit a row, one warp each.
-// One that turns out to have kHuge of them is left to the block kernel.
-template<bool Periodic>
+// One that turns out to have kHuge of them is left to the block kernel.  Eval: rho and
+// d(rho)/dh of the particles without a row (over list) at their h instead.
+template<bool Forest, bool Periodic, bool Eval>
 __global__ void __launch_bounds__(kThreads, 5)
-near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
+near_sum_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__ sets,
+                const int* __restrict__ setOf, NearLoop* __restrict__ L,
                 const __grid_constant__ NearLists lists, double4* __restrict__ xyzh,
                 double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
                 double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
@@ -664,12 +802,14 @@ near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
     NearScratch& scr = sScr[wib];
     double2* rec = sRec[wib];
     const int cur = L->iter & 1, nxt = cur ^ 1;
-    const int n = L->cnt[cur].sum;
+    const int n = Eval ? L->over : L->cnt[cur].sum;
     if (n == 0) return;
-    const int nLive = *t.nLive;
-    const NearFrame f(t.box);
+    const int* list = Eval ? lists.over : lists.sum[cur];
+    const unsigned int most = Eval ? 0xffffffffu : kHuge;
+    NearFrame f(t.box);
+    NearView v = Forest ? NearView{0, 0, 0, 0.0f, 0.0f, 0.0f} : near_view(t, f);
     double lx = 0, ly = 0, lz = 0;
-    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    if (Periodic && !Forest) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
     unsigned long long pairs = 0, seen = 0, hconv = 0;
     for (;;)
     {
@@ -677,16 +817,26 @@ near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
         if (lane == 0) w = atomicAdd(&L->ticket[1], 1);
         w = __shfl_sync(0xffffffffu, w, 0);
         if (w >= n) break;
-        const int i = lists.sum[cur][w];
+        const int i = list[w];
         const double4 pi = xyzh[i];
+        if constexpr (Forest)
+        {
+            const int sid = setOf[i];
+            const NearSet& st = sets[sid];
+            f = NearFrame(st);
+            v = NearView{st.p0, sid, st.n, st.lx, st.ly, st.lz};
+            lx = st.dlx; ly = st.dly; lz = st.dlz;
+            pmass = st.pmass;
+        }
+        const double4* at0 = t.xyzh + v.p0;
         const double hi = pi.w, hinv2 = 1.0 / (hi * hi);
         const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
         const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * hi) + f.slack(x, y, z);
         double2 sums = make_double2(0.0, 0.0);
         int nrec = 0;
         unsigned int got = 0;
-        near_blocks<0, Periodic, false>(t, f, nLive, scr, x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
-            near_candidates(scr.blk, nb, nLive, t.xyzh, [&](const double4& pj, int, bool valid) {
+        near_blocks<0, Periodic, false>(t, v, scr, x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+            near_candidates(scr.blk, nb, v.n, at0, [&](const double4& pj, int, bool valid) {
                 double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                 nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
                 const double q2 = pair_r2(dx, dy, dz) * hinv2;
@@ -703,11 +853,11 @@ near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
                     if (acc && k >= kNearRec) rec[k - kNearRec].x = q2;
                     __syncwarp();
                 }
-                return got < kHuge;
+                return got < most;
             });
-            return got < kHuge ? r : -1.0f;
+            return got < most ? r : -1.0f;
         });
-        if (got >= kHuge)
+        if (got >= most)
         {
             if (lane == 0) lists.huge[cur][atomicAdd(&L->cnt[cur].huge, 1)] = i;
             __syncwarp();
@@ -718,12 +868,14 @@ near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
         if (lane == 0)
         {
             pairs += got;
-            sum_finish(i, hi, sums, got, L, lists, nxt, xyzh, rho, gradh, converged, hs, pmass, tolh, hfact, seen,
-                       hconv);
+            if constexpr (Eval) eval_store(i, hi, sums.x, sums.y, pmass, rho, gradh);
+            else
+                sum_finish(i, hi, sums, got, L, lists, nxt, xyzh, rho, gradh, converged, hs, pmass, tolh, hfact, seen,
+                           hconv);
         }
         __syncwarp();
     }
-    note_h(seen, hconv, ds, shH);
+    if constexpr (!Eval) note_h(seen, hconv, ds, shH);
     if (lane == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
 }
 
@@ -733,9 +885,10 @@ near_sum_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
 // the warps' order -- together where all fit one binade without a tie, else one buffer after
 // the other.  Alone on one warp such a particle took 17 ns a neighbour, 2 ms for the widest
 // of 120,000 particles, which was the length of the iteration.
-template<bool Periodic>
+template<bool Forest, bool Periodic>
 __global__ void __launch_bounds__(32 * kHugeWarps)
-near_huge_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
+near_huge_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__ sets,
+                const int* __restrict__ setOf, NearLoop* __restrict__ L,
                  const __grid_constant__ NearLists lists, double4* __restrict__ xyzh,
                  double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
                  double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
@@ -753,10 +906,10 @@ near_huge_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
     const int cur = L->iter & 1, nxt = cur ^ 1;
     const int n = L->cnt[cur].huge;
     if (n == 0) return;
-    const int nLive = *t.nLive;
-    const NearFrame f(t.box);
+    NearFrame f(t.box);
+    NearView v = Forest ? NearView{0, 0, 0, 0.0f, 0.0f, 0.0f} : near_view(t, f);
     double lx = 0, ly = 0, lz = 0;
-    if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
+    if (Periodic && !Forest) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
     double2* rec = sRec[wib];
     unsigned long long pairs = 0, seen = 0, hconv = 0;
     for (;;)
@@ -771,6 +924,16 @@ near_huge_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
         if (sItem >= n) break;
         const int i = lists.huge[cur][sItem];
         const double4 pi = xyzh[i];
+        if constexpr (Forest)
+        {
+            const int sid = setOf[i];
+            const NearSet& st = sets[sid];
+            f = NearFrame(st);
+            v = NearView{st.p0, sid, st.n, st.lx, st.ly, st.lz};
+            lx = st.dlx; ly = st.dly; lz = st.dlz;
+            pmass = st.pmass;
+        }
+        const double4* at0 = t.xyzh + v.p0;
         const double hi = pi.w, hinv2 = 1.0 / (hi * hi);
         const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
         const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * hi) + f.slack(x, y, z);
@@ -782,15 +945,15 @@ near_huge_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
             {
                 const int at = c0 + 4 * wib + (lane >> 3);
                 const int id = at < cnt ? scr.blk[at] * 8 + (lane & 7) : -1;
-                bool hit = id >= 0 && id < near_count(nLive, 0);
+                bool hit = id >= 0 && id < near_count(v.n, 0);
                 if (hit)
-                    hit = near_gap2<Periodic>(x, y, z, 0.0f, 0.0f, 0.0f, ld_node(t.node + t.off[0] + id), f) <= r2max;
+                    hit = near_gap2<Periodic>(x, y, z, 0.0f, 0.0f, 0.0f, ld_node(near_node(t, v, 0, id)), v) <= r2max;
                 const uint32_t hm = __ballot_sync(0xffffffffu, hit);
                 if (hit) sSel[wib][__popc(hm & lt)] = id;
                 __syncwarp();
                 int m = 0;
                 if (hm)
-                    near_candidates(sSel[wib], __popc(hm), nLive, t.xyzh, [&](const double4& pj, int, bool valid) {
+                    near_candidates(sSel[wib], __popc(hm), v.n, at0, [&](const double4& pj, int, bool valid) {
                         double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                         nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
                         const double q2 = pair_r2(dx, dy, dz) * hinv2;
@@ -832,7 +995,7 @@ near_huge_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L,
         };
         if (wib == 0)
         {
-            near_blocks<1, Periodic, false>(t, f, nLive, scr, x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+            near_blocks<1, Periodic, false>(t, v, scr, x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
                 if (lane == 0) sNodes = nb;
                 __syncthreads();
                 work(nb);
@@ -882,19 +1045,26 @@ __global__ void near_epilogue_kernel(NearLoop* L, cudaGraphConditionalHandle mor
 } // namespace
 
 // ---------------------------------------------------------------- host side
+// The block trees of n particles in nsets sets: where each level starts, and the nodes in all.
+static size_t near_layout(int n, int nsets, NearTree& t)
+{
+    size_t off = 0;
+    for (int l = 0; l < kNearLevels; ++l)
+    {
+        t.off[l] = int(off);
+        off += size_t(n >> (3 * l + 3)) + nsets + 1;
+    }
+    return off;
+}
+
 NearTree near_tree(State& s)
 {
     NearTree t;
+    near_layout(s.ngas, 1, t);
     t.node = reinterpret_cast<const NearNode*>(s.nearNode.get());
     t.xyzh = s.xyzh.get();
     t.box = s.box.get();
     t.nLive = &s.dscal.get()->nAlive;
-    int off = 0;
-    for (int l = 0; l < kNearLevels; ++l)
-    {
-        t.off[l] = off;
-        off += near_count(s.ngas, l);
-    }
     return t;
 }
 
@@ -903,16 +1073,16 @@ NearTree near_tree(State& s)
 void near_build(State& s)
 {
     const int n = std::max(s.ngas, 1);
-    size_t nodes = 0;
-    for (int l = 0; l < kNearLevels; ++l) nodes += size_t(near_count(n, l));
-    s.nearNode.resize(nodes * (sizeof(NearNode) / sizeof(float4)), s.st);
-    const NearTree t = near_tree(s);
+    NearTree t;
+    s.nearNode.resize(near_layout(n, 1, t) * (sizeof(NearNode) / sizeof(float4)), s.st);
+    t = near_tree(s);
     NearNode* out = reinterpret_cast<NearNode*>(s.nearNode.get());
-    near_leaf_levels_kernel<<<std::min(iceil(n, 512), 8 * s.numSMs), 512, 0, s.st>>>(t, out);
+    const int slots = iceil(n, 512);
+    near_leaf_levels_kernel<false><<<std::min(slots, 8 * s.numSMs), 512, 0, s.st>>>(t, out, nullptr, 1, slots);
     COSMO_LAUNCHED();
     if (n > 512 * 32)
     {
-        near_upper_levels_kernel<<<1, 1024, 0, s.st>>>(t, out);
+        near_upper_levels_kernel<false><<<1, 1024, 0, s.st>>>(t, out, nullptr);
         COSMO_LAUNCHED();
     }
 }
@@ -932,41 +1102,56 @@ static NearLists near_lists(State& s)
     return l;
 }
 
-// One iteration's kernels, in the stream's order.
-static void near_iteration(State& s, double pmass, double tolh, double hfact, int* rowsJ, int n,
-                           cudaGraphConditionalHandle more, int setCondition)
+// The buffers a loop over n particles needs beside the particles' own.
+static void near_buffers(State& s, int n)
 {
-    const NearTree t = near_tree(s);
+    for (auto* b : {&s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1], &s.nearSum[0], &s.nearSum[1],
+                    &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
+        b->resize(n, s.st);
+    s.hs.resize(n, s.st);
+    s.nearLoop.resize(1, s.st);
+}
+
+// The instance of a kernel a job needs: one set, open or periodic, or the sets of a batch.
+#define NEAR_PICK(kern, job, ...) \
+    ((job).sets != nullptr ? kern<true, true __VA_ARGS__> \
+                           : ((job).periodic ? kern<false, true __VA_ARGS__> : kern<false, false __VA_ARGS__>))
+#define NEAR_COMMA ,
+
+// One iteration's kernels, in the stream's order.
+static void near_iteration(State& s, const NearJob& j, cudaGraphConditionalHandle more, int setCondition)
+{
     const NearLists lists = near_lists(s);
     NearLoop* L = s.nearLoop.get();
     DevScalars* ds = s.dscal.get();
-    auto rows = s.periodic ? near_rows_kernel<true> : near_rows_kernel<false>;
-    rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(t, L, lists, s.nblR2.get(), rowsJ,
-                                                                      s.nblCount.get(), s.nblH.get(), 0);
+    auto rows = NEAR_PICK(near_rows_kernel, j);
+    rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(j.tree, j.sets, j.setOf, L, lists, s.nblR2.get(),
+                                                                      j.rowsJ, s.nblCount.get(), s.nblH.get(), 0);
     COSMO_LAUNCHED();
-    near_step_kernel<<<iceil(n, kThreads), kThreads, 0, s.st>>>(
-        L, lists, s.nblR2.get(), s.nblCount.get(), s.nblH.get(), s.xyzh.get(), s.rho.get(), s.gradh.get(),
-        s.converged.get(), s.hs.get(), pmass, tolh, hfact, ds);
+    auto step = j.sets ? near_step_kernel<true> : near_step_kernel<false>;
+    step<<<iceil(j.n, kThreads), kThreads, 0, s.st>>>(j.sets, j.setOf, L, lists, s.nblR2.get(), s.nblCount.get(),
+                                                      s.nblH.get(), j.xyzh, j.rho, j.gradh, j.converged, s.hs.get(),
+                                                      j.pmass, j.tolh, j.hfact, ds);
     COSMO_LAUNCHED();
-    auto sum = s.periodic ? near_sum_kernel<true> : near_sum_kernel<false>;
-    sum<<<persistent_blocks(s, sum, kThreads), kThreads, 0, s.st>>>(t, L, lists, s.xyzh.get(), s.rho.get(),
-                                                                    s.gradh.get(), s.converged.get(), s.hs.get(), pmass,
-                                                                    tolh, hfact, ds);
+    auto sum = NEAR_PICK(near_sum_kernel, j, NEAR_COMMA false);
+    sum<<<persistent_blocks(s, sum, kThreads), kThreads, 0, s.st>>>(j.tree, j.sets, j.setOf, L, lists, j.xyzh, j.rho,
+                                                                    j.gradh, j.converged, s.hs.get(), j.pmass, j.tolh,
+                                                                    j.hfact, ds);
     COSMO_LAUNCHED();
     // few particles have that many neighbours, if any: a block a multiprocessor
-    auto huge = s.periodic ? near_huge_kernel<true> : near_huge_kernel<false>;
-    huge<<<s.numSMs, 32 * kHugeWarps, 0, s.st>>>(t, L, lists, s.xyzh.get(), s.rho.get(), s.gradh.get(),
-                                                 s.converged.get(), s.hs.get(), pmass, tolh, hfact, ds);
+    auto huge = NEAR_PICK(near_huge_kernel, j);
+    huge<<<s.numSMs, 32 * kHugeWarps, 0, s.st>>>(j.tree, j.sets, j.setOf, L, lists, j.xyzh, j.rho, j.gradh, j.converged,
+                                                 s.hs.get(), j.pmass, j.tolh, j.hfact, ds);
     COSMO_LAUNCHED();
     near_epilogue_kernel<<<1, 1, 0, s.st>>>(L, more, setCondition);
     COSMO_LAUNCHED();
 }
 
 // The loop as a graph: a while node over near_iteration.  It depends on the buffers, the
-// solve's scalars and the particle count only; built for parameters met a second time in a
-// row (a stepping caller's), as the list-based loop's is.  False: not run (build or use the
-// host loop).
-static bool near_graph(State& s, double pmass, double tolh, double hfact, int maxIter, int* rowsJ, int n)
+// solve's scalars and the particle count only.  defer: built for parameters met a second time
+// in a row (a stepping caller's), as the list-based loop's is.  False: not run (the host loop
+// is to be used).
+static bool near_graph(State& s, const NearJob& j, int maxIter, bool defer)
 {
     std::vector<unsigned char> key;
     auto add = [&](const auto& v) {
@@ -974,21 +1159,22 @@ static bool near_graph(State& s, double pmass, double tolh, double hfact, int ma
         key.insert(key.end(), p, p + sizeof(v));
     };
     for (const void* q : {(const void*)s.nearLoop.get(), (const void*)s.dscal.get(), (const void*)s.nearNode.get(),
-                          (const void*)s.xyzh.get(), (const void*)s.box.get(), (const void*)s.nblR2.get(),
-                          (const void*)rowsJ, (const void*)s.nblCount.get(), (const void*)s.nblH.get(),
-                          (const void*)s.rho.get(), (const void*)s.gradh.get(), (const void*)s.converged.get(),
+                          (const void*)j.tree.xyzh, (const void*)j.tree.box, (const void*)j.sets, (const void*)j.setOf,
+                          (const void*)s.nblR2.get(), (const void*)j.rowsJ, (const void*)s.nblCount.get(),
+                          (const void*)s.nblH.get(), (const void*)j.rho, (const void*)j.gradh, (const void*)j.converged,
                           (const void*)s.hs.get(), (const void*)s.nearRow[0].get(), (const void*)s.nearRow[1].get(),
                           (const void*)s.nearBuild[0].get(), (const void*)s.nearBuild[1].get(),
                           (const void*)s.nearSum[0].get(), (const void*)s.nearSum[1].get(),
                           (const void*)s.nearHuge[0].get(), (const void*)s.nearHuge[1].get(),
                           (const void*)s.nearCover.get(), (const void*)s.nearOver.get()})
         add(q);
-    for (int v : {n, s.ngas, s.periodic, s.numSMs, maxIter}) add(v);
-    for (double v : {pmass, tolh, hfact}) add(v);
+    for (int v : j.tree.off) add(v);
+    for (int v : {j.n, j.periodic, s.numSMs, maxIter}) add(v);
+    for (double v : {j.pmass, j.tolh, j.hfact}) add(v);
     s.loopKeyLast = key;
     if (!s.nearGraphExec || key != s.nearGraphKey)
     {
-        if (key != s.nearKeyPending)
+        if (defer && key != s.nearKeyPending)
         {
             s.nearKeyPending = key;
             return false;
@@ -1018,7 +1204,7 @@ static bool near_graph(State& s, double pmass, double tolh, double hfact, int ma
             if (cudaStreamBeginCaptureToGraph(s.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) !=
                 cudaSuccess)
                 break;
-            near_iteration(s, pmass, tolh, hfact, rowsJ, n, more, 1);
+            near_iteration(s, j, more, 1);
             if (cudaStreamEndCapture(s.st, &body) != cudaSuccess) break;
             if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) break;
             built = true;
@@ -1049,6 +1235,24 @@ static bool near_graph(State& s, double pmass, double tolh, double hfact, int ma
     return true;
 }
 
+// The loop's iterations, as a graph or from the host.
+static void near_run(State& s, const NearJob& j, int maxIter, bool graph, bool defer)
+{
+    s.lastLoopGraph = 0;
+    if (graph && maxIter <= kLoopIters && near_graph(s, j, maxIter, defer))
+    {
+        s.lastLoopGraph = 1;
+        return;
+    }
+    for (int it = 0; it < maxIter; ++it)
+    {
+        near_iteration(s, j, cudaGraphConditionalHandle(0), 0);
+        COSMO_CUDA(cudaMemcpyAsync(s.hsmall, s.nearLoop.get(), 4 * sizeof(int), cudaMemcpyDeviceToHost, s.st));
+        COSMO_CUDA(cudaStreamSynchronize(s.st));
+        if (s.hsmall[2] == 0) break;
+    }
+}
+
 // The Newton loop of one plain solve over the block tree, every live (and not fixed)
 // particle active.  Issued on the stream; near_results reads what it did.  rowsJ: the rows'
 // j, for the gradient and force passes (may be null).
@@ -1056,11 +1260,7 @@ void near_newton(State& s, double pmass, double tolh, double hfact, int maxIter,
 {
     const int n = std::max(s.nAlive, 1);
     DevScalars* ds = s.dscal.get();
-    for (auto* b : {&s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1], &s.nearSum[0], &s.nearSum[1],
-                    &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
-        b->resize(n, s.st);
-    s.hs.resize(n, s.st);
-    s.nearLoop.resize(1, s.st);
+    near_buffers(s, n);
     near_build(s);
     const bool frozen = s.frozenFor == s.ngas && s.nAlive > 0;
     near_init_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get(), ds, maxIter, frozen ? 1 : 0);
@@ -1071,32 +1271,21 @@ void near_newton(State& s, double pmass, double tolh, double hfact, int maxIter,
             s.nearLoop.get(), s.orderA.get(), s.frozen.get(), &ds->nAlive, s.xyzh.get(), s.converged.get(), s.hs.get(),
             near_lists(s), ds);
         COSMO_LAUNCHED();
-        near_frozen_count_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get());
+        near_active_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get());
         COSMO_LAUNCHED();
     }
-    s.lastLoopGraph = 0;
-    if (allowGraph && s.newtonGraph && maxIter <= kLoopIters && s.nAlive > 0 &&
-        near_graph(s, pmass, tolh, hfact, maxIter, rowsJ, n))
-    {
-        s.lastLoopGraph = 1;
-        return;
-    }
-    for (int it = 0; it < maxIter; ++it)
-    {
-        near_iteration(s, pmass, tolh, hfact, rowsJ, n, cudaGraphConditionalHandle(0), 0);
-        COSMO_CUDA(cudaMemcpyAsync(s.hsmall, s.nearLoop.get(), 4 * sizeof(int), cudaMemcpyDeviceToHost, s.st));
-        COSMO_CUDA(cudaStreamSynchronize(s.st));
-        if (s.hsmall[2] == 0) break;
-    }
+    const NearJob j{near_tree(s), nullptr, nullptr, s.xyzh.get(), s.rho.get(), s.gradh.get(), s.converged.get(), rowsJ,
+                    n, s.periodic, pmass, tolh, hfact};
+    near_run(s, j, maxIter, allowGraph && s.newtonGraph && s.nAlive > 0, true);
 }
 
 // After the loop: rows at the converged h of the particles whose rows do not cover it.
 void near_cover(State& s, int* rowsJ)
 {
-    auto rows = s.periodic ? near_rows_kernel<true> : near_rows_kernel<false>;
-    rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(near_tree(s), s.nearLoop.get(), near_lists(s),
-                                                                      s.nblR2.get(), rowsJ, s.nblCount.get(),
-                                                                      s.nblH.get(), 1);
+    auto rows = s.periodic ? near_rows_kernel<false, true> : near_rows_kernel<false, false>;
+    rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(near_tree(s), nullptr, nullptr, s.nearLoop.get(),
+                                                                      near_lists(s), s.nblR2.get(), rowsJ,
+                                                                      s.nblCount.get(), s.nblH.get(), 1);
     COSMO_LAUNCHED();
 }
 
@@ -1107,6 +1296,71 @@ long long near_results(State& s, const NearLoop& h)
     s.itersRun = h.iter;
     s.activePerIter.assign(h.activePerIter, h.activePerIter + std::min(h.iter, kLoopIters));
     return h.active;
+}
+
+// The Newton loop of a plain batch over its sets' block trees (the batch's arrays in b, its
+// scratch in s), every live particle of every set active.  Issued on the stream.
+void near_forest_newton(State& s, const NearForest& b, double tolh, double hfact, int maxIter, bool graph)
+{
+    NearTree t;
+    const size_t nodes = near_layout(b.n, b.nsets, t);
+    s.nearNode.resize(nodes * (sizeof(NearNode) / sizeof(float4)), s.st);
+    s.nearSets.resize(b.nsets, s.st);
+    near_buffers(s, b.n);
+    s.nblR2.resize(size_t(b.n) * kNbl, s.st);
+    s.nblCount.resize(b.n, s.st);
+    s.nblH.resize(b.n, s.st);
+    t.node = reinterpret_cast<const NearNode*>(s.nearNode.get());
+    t.xyzh = b.xyzh;
+    t.box = b.boxes;
+    t.nLive = &s.dscal.get()->nAlive;
+    NearNode* out = reinterpret_cast<NearNode*>(s.nearNode.get());
+    near_sets_kernel<<<iceil(b.nsets, 256), 256, 0, s.st>>>(b.nsets, b.offs, b.nAlive, b.boxes, b.pmass,
+                                                            s.nearSets.get());
+    COSMO_LAUNCHED();
+    const int slots = (b.n >> 9) + b.nsets + 1;
+    near_leaf_levels_kernel<true><<<std::min(slots, 8 * s.numSMs), 512, 0, s.st>>>(t, out, s.nearSets.get(), b.nsets,
+                                                                                  slots);
+    COSMO_LAUNCHED();
+    near_upper_levels_kernel<true><<<b.nsets, 1024, 0, s.st>>>(t, out, s.nearSets.get());
+    COSMO_LAUNCHED();
+    near_forest_zero_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get(), maxIter);
+    COSMO_LAUNCHED();
+    near_forest_init_kernel<<<std::min(iceil(b.n, kThreads), 16 * s.numSMs), kThreads, 0, s.st>>>(
+        s.nearLoop.get(), b.n, s.nearSets.get(), b.setOf, near_lists(s));
+    COSMO_LAUNCHED();
+    near_active_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get());
+    COSMO_LAUNCHED();
+    const NearJob j{t, s.nearSets.get(), b.setOf, b.xyzh, b.rho, b.gradh, b.converged, nullptr, b.n, 1, 0.0, tolh,
+                    hfact};
+    near_run(s, j, maxIter, graph, false);
+}
+
+// rho and d(rho)/dh of every live particle of the batch at its final h.
+void near_forest_eval(State& s, const NearForest& b)
+{
+    NearTree t;
+    near_layout(b.n, b.nsets, t);
+    t.node = reinterpret_cast<const NearNode*>(s.nearNode.get());
+    t.xyzh = b.xyzh;
+    t.box = b.boxes;
+    t.nLive = &s.dscal.get()->nAlive;
+    const NearLists lists = near_lists(s);
+    NearLoop* L = s.nearLoop.get();
+    auto rows = near_rows_kernel<true, true>;
+    rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(t, s.nearSets.get(), b.setOf, L, lists,
+                                                                      s.nblR2.get(), nullptr, s.nblCount.get(),
+                                                                      s.nblH.get(), 1);
+    COSMO_LAUNCHED();
+    near_eval_kernel<<<iceil(b.n, kThreads), kThreads, 0, s.st>>>(b.n, s.nearSets.get(), b.setOf, s.nblR2.get(),
+                                                                  s.nblCount.get(), b.xyzh, b.rho, b.gradh,
+                                                                  s.dscal.get());
+    COSMO_LAUNCHED();
+    auto sum = near_sum_kernel<true, true, true>;
+    sum<<<persistent_blocks(s, sum, kThreads), kThreads, 0, s.st>>>(t, s.nearSets.get(), b.setOf, L, lists, b.xyzh,
+                                                                    b.rho, b.gradh, b.converged, s.hs.get(), 0.0, 0.0,
+                                                                    0.0, s.dscal.get());
+    COSMO_LAUNCHED();
 }
 
 } // namespace cosmo

@@ -38,8 +38,11 @@ struct alignas(32) NearNode
     float cx, cy, cz, hmax, ex, ey, ez, pad;
 };
 
-// The nodes of level l start at node[off[l]] (laid out for the capacity of the arrays); the
-// live particle count is read on the device, so one set of arguments serves every solve.
+// The block trees of one particle set, or of the sets of a batch one after the other in the
+// sorted order (set s from its first particle p0 on).  Level l of set s starts at
+// node[off[l] + (p0 >> (3 l + 3)) + s]: a set's nodes of a level never reach the next set's
+// start, so no table is needed.  The live particle count (of the one set) is read on the
+// device, so one set of arguments serves every solve.
 struct NearTree
 {
     const NearNode* __restrict__ node;
@@ -47,6 +50,24 @@ struct NearTree
     const DevBox* __restrict__ box;
     const int* nLive;
     int off[kNearLevels];
+};
+
+// One set of a batch, as the search kernels read it.  An open set's periods are infinite, so
+// that one periodic instance of a kernel serves both (no separation is folded).
+struct NearSet
+{
+    int p0, n;                 // first particle of the sorted order, live particles
+    float lx, ly, lz, len;     // periods, largest side
+    double cx, cy, cz;         // box centre
+    double dlx, dly, dlz;      // periods
+    double pmass;
+};
+
+// What a search knows of its set: the one set of a solve, or one of a batch.
+struct NearView
+{
+    int p0, s, n;
+    float lx, ly, lz;
 };
 
 __host__ __device__ inline int near_count(int n, int level) { return (n + (8 << (3 * level)) - 1) >> (3 * level + 3); }
@@ -89,16 +110,30 @@ struct NearFrame
         lz = float(b->len[2]);
         len = fmaxf(lx, fmaxf(ly, lz));
     }
+    __device__ __forceinline__ explicit NearFrame(const NearSet& s)
+        : cx(s.cx), cy(s.cy), cz(s.cz), lx(s.lx), ly(s.ly), lz(s.lz), len(s.len)
+    {
+    }
     __device__ __forceinline__ float slack(float x, float y, float z) const
     {
         return 4e-7f * (len + fabsf(x) + fabsf(y) + fabsf(z));
     }
 };
 
+__device__ __forceinline__ NearView near_view(const NearTree& t, const NearFrame& f)
+{
+    return NearView{0, 0, *t.nLive, f.lx, f.ly, f.lz};
+}
+
+__device__ __forceinline__ const NearNode* near_node(const NearTree& t, const NearView& v, int level, int idx)
+{
+    return t.node + (t.off[level] + (v.p0 >> (3 * level + 3)) + v.s + idx);
+}
+
 // Squared gap between the box (c, e) and a node's box, at the nearest image.
 template<bool Periodic>
 __device__ __forceinline__ float near_gap2(float x, float y, float z, float ex, float ey, float ez, const NearNode& n,
-                                           const NearFrame& f)
+                                           const NearView& f)
 {
     float dx = fabsf(x - n.cx), dy = fabsf(y - n.cy), dz = fabsf(z - n.cz);
     if (Periodic)
@@ -127,20 +162,20 @@ __device__ __forceinline__ float near_sym_reach(float hmax, float slack)
 // most 32 nodes and the blocks come out in order.  Stop = 1 hands out the nodes of level 1
 // instead (of more than 256 particles).
 template<int Stop, bool Periodic, bool Sym, class Flush>
-__device__ __forceinline__ void near_blocks(const NearTree& t, const NearFrame& f, int nLive, NearScratch& scr, float x,
-                                            float y, float z, float ex, float ey, float ez, float reach, float slack,
+__device__ __forceinline__ void near_blocks(const NearTree& t, const NearView& v, NearScratch& scr, float x, float y,
+                                            float z, float ex, float ey, float ez, float reach, float slack,
                                             Flush&& flush)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
     int top = 0;
-    while (near_count(nLive, top) > 32) ++top;
+    while (near_count(v.n, top) > 32) ++top;
     int nb = 0;
     int left = 0, pos = 0;   // lane l: nodes of level l not yet expanded, and the first of them
     auto test = [&](int level, int idx) {
-        const NearNode n = ld_node(t.node + t.off[level] + idx);
+        const NearNode n = ld_node(near_node(t, v, level, idx));
         const float r = Sym ? fmaxf(reach, near_sym_reach(n.hmax, slack)) : reach;
-        return near_gap2<Periodic>(x, y, z, ex, ey, ez, n, f) <= r * r;
+        return near_gap2<Periodic>(x, y, z, ex, ey, ez, n, v) <= r * r;
     };
     // children of up to four nodes, or the top level: accepted ones of level into the next list
     auto accept = [&](int level, int idx, bool valid) {
@@ -159,7 +194,7 @@ __device__ __forceinline__ void near_blocks(const NearTree& t, const NearFrame& 
         }
         __syncwarp();
     };
-    accept(top, lane, lane < near_count(nLive, top));
+    accept(top, lane, lane < near_count(v.n, top));
     int lev = top;
     for (;;)
     {
@@ -178,7 +213,7 @@ __device__ __forceinline__ void near_blocks(const NearTree& t, const NearFrame& 
         const int node = scr.front[lev][first + min(lane >> 3, m - 1)];
         const int child = node * 8 + (lane & 7);
         if (lane == lev) { left -= m; pos += m; }
-        accept(lev - 1, child, (lane >> 3) < m && child < near_count(nLive, lev - 1));
+        accept(lev - 1, child, (lane >> 3) < m && child < near_count(v.n, lev - 1));
         if (lev > Stop + 1) --lev;
     }
 }
@@ -193,8 +228,9 @@ __device__ __forceinline__ float warp_max_f(float v)
 // Members of a warp's search in equal runs of consecutive lanes: as many lanes per run (a
 // power of two) as keep every run's bounding box within kNearSpread of its largest reach,
 // so that sparse members (an active list late in the loop, the edge of a set) do not share
-// one search over everything between them.  x, y, z, r: the lane's member (r < 0: none);
-// on return the run's box (centre, half) and reach on every lane of it.
+// one search over everything between them, and all of a run in one set.  x, y, z, r, set:
+// the lane's member (r < 0: none); on return the run's box (centre, half) and reach on every
+// lane of it.
 constexpr float kNearSpread = 1.5f;
 struct NearRun
 {
@@ -202,12 +238,14 @@ struct NearRun
     float cx, cy, cz, ex, ey, ez, reach;
 };
 
-__device__ __forceinline__ NearRun near_runs(float x, float y, float z, float r)
+template<bool Forest>
+__device__ __forceinline__ NearRun near_runs(float x, float y, float z, float r, int set)
 {
     const bool on = r >= 0.0f;
     float lx = on ? x : INFINITY, hx = on ? x : -INFINITY;
     float ly = on ? y : INFINITY, hy = on ? y : -INFINITY;
     float lz = on ? z : INFINITY, hz = on ? z : -INFINITY;
+    int s0 = on ? set : 0x7fffffff, s1 = on ? set : -1;   // the run's sets
     NearRun u;
     u.w = 1;
     u.reach = r;
@@ -219,7 +257,10 @@ __device__ __forceinline__ NearRun near_runs(float x, float y, float z, float r)
         const float az = fminf(lz, __shfl_xor_sync(0xffffffffu, lz, o)), bz = fmaxf(hz, __shfl_xor_sync(0xffffffffu, hz, o));
         const float rr = fmaxf(u.reach, __shfl_xor_sync(0xffffffffu, u.reach, o));
         const float ext = fmaxf(bx - ax, fmaxf(by - ay, bz - az));
-        if (u.w != o || !__all_sync(0xffffffffu, !(ext > kNearSpread * rr))) continue;
+        const int a0 = Forest ? min(s0, __shfl_xor_sync(0xffffffffu, s0, o)) : 0;
+        const int a1 = Forest ? max(s1, __shfl_xor_sync(0xffffffffu, s1, o)) : 0;
+        if (u.w != o || !__all_sync(0xffffffffu, !(ext > kNearSpread * rr) && (!Forest || a1 <= a0))) continue;
+        if (Forest) { s0 = a0; s1 = a1; }
         lx = ax; hx = bx; ly = ay; hy = by; lz = az; hz = bz;
         u.reach = rr;
         u.w = 2 * o;
@@ -232,6 +273,34 @@ __device__ __forceinline__ NearRun near_runs(float x, float y, float z, float r)
 }
 
 NearTree near_tree(State& s);   // the arguments of a search of s's live particles
+
+// One loop: its trees, the sets and the particles' set (a batch; null for one set), the
+// particle arrays, the rows' j (or null), the particles its launches cover, and its scalars.
+struct NearJob
+{
+    NearTree tree;
+    const NearSet* sets;
+    const int* setOf;
+    double4* xyzh;
+    double *rho, *gradh;
+    int *converged, *rowsJ;
+    int n, periodic;
+    double pmass, tolh, hfact;
+};
+
+// A batch as its loop reads it: set s holds [offs[s], offs[s] + nAlive[s]) of the sorted order.
+struct NearForest
+{
+    int n, nsets;
+    const int *offs, *nAlive, *setOf;
+    const DevBox* boxes;
+    const double* pmass;
+    double4* xyzh;
+    double *rho, *gradh;
+    int* converged;
+};
+void near_forest_newton(State& s, const NearForest& b, double tolh, double hfact, int maxIter, bool graph);
+void near_forest_eval(State& s, const NearForest& b);
 
 // As many blocks of a kernel as the device holds at once.
 template<class K>

@@ -155,6 +155,8 @@ struct Timings
            gradkern = 0, upsweep = 0, fjbuild = 0, prep = 0, fkern = 0;
 };
 
+struct NearSet;   // near.cuh
+
 struct State
 {
     cudaStream_t st = nullptr;
@@ -293,6 +295,7 @@ struct State
     DBuf<float4> nearNode;                      // the block tree (near.cuh), two float4 a node
     DBuf<int> nearRow[2], nearBuild[2], nearSum[2], nearHuge[2], nearCover, nearOver;   // the block-tree loop's lists
     DBuf<NearLoop> nearLoop;                    // its state
+    DBuf<NearSet> nearSets;                     // the sets of a batch, as its searches read them
 
     // scratch
     DBuf<uint32_t> scanTmp, sortHist, sortBase, sortLookback;
