@@ -267,14 +267,26 @@ gradient_over_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ 
     if (lane == 0 && pairs) atomicAdd(&ds->pairs[1], pairs);
 }
 
+// Extras: the pairs a row must gain from another particle's support, kExtra places a
+// particle.  (Once appended to one list through one counter, then counted, scanned and placed:
+// where h scatters there are ten a particle, and the counter's atomics took 5 ms of a
+// 2-million-particle step.)  extraCnt counts them all, so a particle with more than fit shows.
+constexpr int kExtra = kQuintic ? 64 : 32;   // of 2 M quintic Plummer particles 1% gain more than 32
+
+__device__ __forceinline__ void add_extra(int* __restrict__ extras, int* __restrict__ extraCnt, int j, int i)
+{
+    const int k = atomicAdd(extraCnt + j, 1);
+    if (k < kExtra) extras[size_t(j) * kExtra + k] = i;
+}
+
 // The pairs the particles without a row add to others' rows: every j within a support of
 // theirs that lies beyond what j's own row covers (the test sym_from_rows_kernel makes for
 // the pairs of a row).
 template<bool Periodic>
 __global__ void __launch_bounds__(kThreads)
 over_extras_kernel(const __grid_constant__ NearTree t, const NearLoop* __restrict__ L, const int* __restrict__ over,
-                   const double* __restrict__ hs, const double* __restrict__ rowH,
-                   unsigned long long* __restrict__ extras, int extraCap, DevScalars* __restrict__ ds)
+                   const double* __restrict__ hs, const double* __restrict__ rowH, int* __restrict__ extras,
+                   int* __restrict__ extraCnt, DevScalars* __restrict__ ds)
 {
     __shared__ NearScratch sScr[kWarpsPerBlock];
     const int wib = threadIdx.x >> 5;
@@ -301,8 +313,8 @@ over_extras_kernel(const __grid_constant__ NearTree t, const NearLoop* __restric
                     const double hj = hs[j], ch = rowH[j];
                     if (!(dr2 < kRadK2 * (hj * hj)) && !(dr2 < kRadK2 * (ch * ch) * (1.0 - 1e-9)))
                     {
-                        const int k = atomicAdd(&ds->extraCount, 1);
-                        if (k < extraCap) extras[k] = (static_cast<unsigned long long>(j) << 32) | uint32_t(i);
+                        add_extra(extras, extraCnt, j, i);
+                        atomicAdd(&ds->extraCount, 1);   // a few particles' pairs
                     }
                 }
                 return true;
@@ -450,8 +462,7 @@ __global__ void row_cover_kernel(int nL, const uint32_t* __restrict__ layout, co
 // sorted order, 8 bytes a particle).  A pair the force pass takes because of this
 // particle's support (dr^2 < R^2 h_i^2 (1 + 1e-10)) is in j's Newton row too unless dr^2
 // reaches the radius j's row covers (R rowH, with 1e-9 to spare; only a pair beyond j's
-// own support can); such a pair is appended as (j << 32 | i), for i to be merged into
-// j's row.  The mixed form's rows hold that double rounded to float (within 2^-24 of
+// own support can); such a pair puts i among j's extras, to be merged into j's row.  The mixed form's rows hold that double rounded to float (within 2^-24 of
 // it): where it lies within 1e-6 of a bound the test uses, dr^2 is taken again from the
 // positions, so every test decides as on the double and the rows are the same.
 template<class T, bool Periodic>
@@ -459,16 +470,15 @@ __global__ void __launch_bounds__(kThreads)
 sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restrict__ rowsR2,
                      int* __restrict__ nblCount, const double* __restrict__ hs, const double* __restrict__ rowH,
                      const double4* __restrict__ xyzh, const DevBox* __restrict__ box, int* __restrict__ nbl,
-                     unsigned long long* __restrict__ extras, int extraCap, int* __restrict__ extraCnt,
-                     DevScalars* __restrict__ ds)
+                     int* __restrict__ extras, int* __restrict__ extraCnt, DevScalars* __restrict__ ds)
 {
     constexpr bool kExact = std::is_same<T, double>::value;
     using R4 = typename std::conditional<kExact, double4, float4>::type;
     double lx = 0, ly = 0, lz = 0;
     if (Periodic && !kExact) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
+    int added = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nAlive; i += gridDim.x * blockDim.x)
     {
-        extraCnt[i] = 0;
         const int cnt = nblCount[i];
         if (unsigned(cnt) > unsigned(kNbl)) continue;   // no row (its passes search for it)
         const double hi = hs[i];
@@ -499,8 +509,8 @@ sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restr
                 if (!exact && near(cover)) retake();
                 if (!(dr2 < cover))
                 {
-                    const int k = atomicAdd(&ds->extraCount, 1);
-                    if (k < extraCap) extras[k] = (static_cast<unsigned long long>(j) << 32) | uint32_t(i);
+                    add_extra(extras, extraCnt, j, i);
+                    ++added;
                 }
             }
         };
@@ -538,25 +548,8 @@ sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restr
         }
         nblCount[i] = w;
     }
-}
-
-// The extras of each row owner (their number read on the device, at most cap of them):
-// counted, then placed at the owner's offset.
-__global__ void extras_count_kernel(const unsigned long long* __restrict__ extras, int cap,
-                                    const DevScalars* __restrict__ ds, int* __restrict__ cnt)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < min(ds->extraCount, cap)) atomicAdd(&cnt[int(extras[k] >> 32)], 1);
-}
-
-__global__ void extras_place_kernel(const unsigned long long* __restrict__ extras, int cap,
-                                    const DevScalars* __restrict__ ds, const uint32_t* __restrict__ off,
-                                    int* __restrict__ cnt, int* __restrict__ bucket)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= min(ds->extraCount, cap)) return;
-    const int t = int(extras[k] >> 32);
-    bucket[off[t] + uint32_t(atomicSub(&cnt[t], 1) - 1)] = int(uint32_t(extras[k]));
+    added = __reduce_add_sync(0xffffffffu, added);
+    if ((threadIdx.x & 31) == 0 && added) atomicAdd(&ds->extraCount, added);
 }
 
 // Each row owner merges its extras into its row: sorted, those the row already holds
@@ -564,13 +557,13 @@ __global__ void extras_place_kernel(const unsigned long long* __restrict__ extra
 // exceed kNbl joins the over list when there is one (its passes then search for it), else
 // sets mergeOverflow (the symmetric rows are then built instead).  A particle without a row
 // takes none.
-__global__ void extras_merge_kernel(int nA, const uint32_t* __restrict__ off, int* __restrict__ bucket,
+__global__ void extras_merge_kernel(int nA, const int* __restrict__ extraCnt, int* __restrict__ extras,
                                     int* __restrict__ nbl, int* __restrict__ nblCount, DevScalars* __restrict__ ds,
                                     int* __restrict__ over, int* __restrict__ overCount)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nA) return;
-    const uint32_t b0 = off[t], e = off[t + 1] - b0;
+    const uint32_t e = uint32_t(extraCnt[t]);
     if (e == 0) return;
     const int cnt = nblCount[t];
     if (unsigned(cnt) > unsigned(kNbl)) return;
@@ -582,12 +575,12 @@ __global__ void extras_merge_kernel(int nA, const uint32_t* __restrict__ off, in
         }
         else ds->mergeOverflow = 1;
     };
-    if (cnt + int(e) > 2 * kNbl)
+    if (e > uint32_t(kExtra))
     {
         full();
         return;
     }
-    int* ex = bucket + b0;
+    int* ex = extras + size_t(t) * kExtra;
     for (uint32_t a = 1; a < e; ++a)
     {
         const int v = ex[a];
@@ -786,7 +779,7 @@ static LoopGraph newton_loop_graph(State& s, double pmass, double tolh, double h
     lc = std::min<size_t>({lc, s.jOffset.cap - 1, s.jOffsetPrev.cap - 1, s.layout.cap - 1});
     const int leafCap = int(std::min<size_t>(lc, size_t(1) << 30));
     const size_t ic = std::min<size_t>({s.items.cap, s.rowItems.cap, s.nblCount.cap, s.nblH.cap,
-                                        s.nblR2.cap / size_t(kNbl)});
+                                        s.nblR2.cap * (mx ? 2 : 1) / size_t(kNbl)});
     const int itemCap = int(std::min<size_t>(ic, size_t(1) << 30));
     scan_reserve(s, leafCap);
 
@@ -1052,24 +1045,21 @@ static bool cover_rows(State& s, int itemCap, FixedSplit cut, int spreadG)
 }
 
 // The symmetric rows from the covering Newton rows (sym_from_rows_kernel), then the
-// pairs other particles' supports add, merged into their rows -- all on the device, the
-// extras' number read there.  Whether they all fitted is known from extraCount (at most
-// extraCap) and mergeOverflow once the stream has been read.
-static void sym_rows_from_newton(State& s, int extraCap, bool near)
+// pairs other particles' supports add, merged into their rows -- all on the device.  Whether
+// they all fitted is known from mergeOverflow once the stream has been read.
+static void sym_rows_from_newton(State& s, bool near)
 {
     DevScalars* ds = s.dscal.get();
     const int nA = s.nAlive;
-    s.extras.resize(extraCap, s.st);
+    s.extras.resize(size_t(nA) * kExtra, s.st);
     s.extraCnt.resize(nA, s.st);
-    s.extraOff.resize(size_t(nA) + 1, s.st);
-    s.extraBucket.resize(extraCap, s.st);
-    // extraCount, mergeOverflow and rowOverflow were zeroed by the coverage check; each
-    // particle's extras count by the compaction
-    const int grid = std::max(1, std::min(iceil(nA, kThreads), 16 * s.numSMs));
+    COSMO_CUDA(cudaMemsetAsync(s.extraCnt.get(), 0, size_t(nA) * sizeof(int), s.st));
+    // extraCount, mergeOverflow and rowOverflow were zeroed by the coverage check (or the
+    // block-tree loop's start)
+    const int grid = std::max(1, iceil(nA, kThreads));
     auto compact = [&](auto kern, const auto* rows) {
         kern<<<grid, kThreads, 0, s.st>>>(nA, s.nblJ.get(), rows, s.nblCount.get(), s.hs.get(), s.nblH.get(),
-                                          s.xyzh.get(), s.box.get(), s.nbl.get(), s.extras.get(), extraCap,
-                                          s.extraCnt.get(), ds);
+                                          s.xyzh.get(), s.box.get(), s.nbl.get(), s.extras.get(), s.extraCnt.get(), ds);
     };
     // the mixed form's Newton rows hold FP32 r^2 in the same buffer
     const float* rowsF = reinterpret_cast<const float*>(s.nblR2.get());
@@ -1084,16 +1074,10 @@ static void sym_rows_from_newton(State& s, int extraCap, bool near)
     {
         auto ov = s.periodic ? over_extras_kernel<true> : over_extras_kernel<false>;
         ov<<<2 * s.numSMs, kThreads, 0, s.st>>>(near_tree(s), s.nearLoop.get(), s.nearOver.get(), s.hs.get(),
-                                                s.nblH.get(), s.extras.get(), extraCap, ds);
+                                                s.nblH.get(), s.extras.get(), s.extraCnt.get(), ds);
         COSMO_LAUNCHED();
     }
-    extras_count_kernel<<<iceil(extraCap, 256), 256, 0, s.st>>>(s.extras.get(), extraCap, ds, s.extraCnt.get());
-    COSMO_LAUNCHED();
-    scan_exclusive(s, reinterpret_cast<const uint32_t*>(s.extraCnt.get()), s.extraOff.get(), nA, false);
-    extras_place_kernel<<<iceil(extraCap, 256), 256, 0, s.st>>>(s.extras.get(), extraCap, ds, s.extraOff.get(),
-                                                               s.extraCnt.get(), s.extraBucket.get());
-    COSMO_LAUNCHED();
-    extras_merge_kernel<<<iceil(nA, 256), 256, 0, s.st>>>(nA, s.extraOff.get(), s.extraBucket.get(), s.nbl.get(),
+    extras_merge_kernel<<<iceil(nA, 256), 256, 0, s.st>>>(nA, s.extraCnt.get(), s.extras.get(), s.nbl.get(),
                                                          s.nblCount.get(), ds, near ? s.nearOver.get() : nullptr,
                                                          near ? &s.nearLoop.get()->over : nullptr);
     COSMO_LAUNCHED();
@@ -1148,7 +1132,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         s.items.resize(itemCap, s.st);
         s.rowItems.resize(itemCap, s.st);
     }
-    s.nblR2.resize(size_t(itemCap) * kNbl, s.st);
+    s.nblR2.resize(size_t(itemCap) * kNbl / (s.precision == 1 ? 2 : 1), s.st);   // FP32 rows in the mixed form
     s.nblCount.resize(itemCap, s.st);
     s.nblH.resize(itemCap, s.st);
     // the index rows' buffer is passed whenever the form has one (the Newton-loop graph
@@ -1198,7 +1182,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     long long settlingPrev = 0;
     bool graphRan = false;
     cudaEvent_t n0 = ev(s);
-    if (near) near_newton(s, pmass, tolh, hfact, maxIter, allowGraph, writeJ ? rowsJ : nullptr);
+    if (near) near_newton(s, pmass, tolh, hfact, maxIter, allowGraph, rowsJ);
     else if (allowGraph && s.newtonGraph && maxIter <= kLoopIters && nActiveParticles > 0)
     {
         const LoopGraph lg =
@@ -1354,12 +1338,9 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         }
         else
             fromRows = writeJ && s.nAlive > 0 && rowsBuilt && cover_rows(s, itemCap, cut, spreadG);
-        // pairs other particles' supports add: about ten a particle where h scatters (a set so
-        // large that their buffer matters goes back to the lists when they are that many)
-        const int extraCap = s.symExtraCap > 0 ? std::min(s.symExtraCap, itemCap) : near && itemCap <= 1 << 24 ? 16 * itemCap : itemCap;
         const int* active = near ? &s.nearLoop.get()->active : nullptr;
         if (fromRows)
-            sym_rows_from_newton(s, extraCap, near);
+            sym_rows_from_newton(s, near);
         else
         {
             build_symmetric(s);
@@ -1432,7 +1413,9 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             }
         }
         // the rows serve the force pass if every extra was kept and merged
-        if (fromRows) s.rowsFromNewton = s.hscal->extraCount <= extraCap && s.hscal->mergeOverflow == 0;
+        if (fromRows)
+            s.rowsFromNewton = (s.symExtraCap == 0 || s.hscal->extraCount <= s.symExtraCap) &&
+                               s.hscal->mergeOverflow == 0;
         if (writeJ && !near && !s.rowsFromNewton) s.symRowsSkip = kSymRowsSkip;
         s.t.gjbuild += elapsed_s(g0, g1);
         s.t.gradkern += elapsed_s(g1, g2);

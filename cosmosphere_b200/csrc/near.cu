@@ -31,6 +31,12 @@ constexpr int kThreads = 32 * kNearWarps;
 // rows in every iteration).
 constexpr double kNearMargin = 1.04;
 constexpr float kNearWide = 1.5f;   // a member this much wider than its warp's mean searches alone
+// Batches of blocks after which members that reach less than kNearShare of them search one by
+// one: about what a search alone costs, so giving up late never costs more than twice the
+// better choice (a 120,000-particle Plummer sphere's loop: 4.4 ms without, 3.05 at 6 batches,
+// 3.25 at 4; lattices and boxes never get there).
+constexpr int kNearPatience = 6;
+constexpr float kNearShare = 0.1f;
 constexpr double kCoverMargin = 1.0 + 1e-8;   // rows made for a converged h: just beyond the force test's slack
 constexpr double kCoverSlack = 1.0 + 1e-9;    // a row serves the gradient and force passes at h kCoverSlack <= rowH
 
@@ -249,6 +255,8 @@ __device__ __forceinline__ void note_h(unsigned long long seen, unsigned long lo
 // after the loop start from zero too.
 __global__ void near_init_kernel(NearLoop* L, DevScalars* ds, int maxIter, int frozen)
 {
+    L->queue[threadIdx.x] = 0;
+    if (threadIdx.x != 0) return;
     const int n = ds->nAlive;
     L->iter = 0;
     L->maxIter = maxIter;
@@ -303,6 +311,8 @@ __global__ void near_active_kernel(NearLoop* L) { L->active = L->cnt[0].build; }
 // of the sorted order) on the search list.
 __global__ void near_forest_zero_kernel(NearLoop* L, int maxIter)
 {
+    L->queue[threadIdx.x] = 0;
+    if (threadIdx.x != 0) return;
     L->iter = 0;
     L->maxIter = maxIter;
     L->active = 0;
@@ -330,6 +340,41 @@ near_forest_init_kernel(NearLoop* L, int n, const NearSet* __restrict__ sets, co
     }
 }
 
+// Work in nq queues of consecutive items, one a multiprocessor: the warps of a multiprocessor
+// take items from its own queue, so at any time they search next to one another and find
+// each other's blocks in its L1 cache; one whose queue is empty goes on with the first that
+// is not.  own: the warp's queue.  The item, or -1 when none is left.
+__device__ __forceinline__ int queue_pop(int* queue, int nq, int items, int& own)
+{
+    const int lane = lane_id();
+    for (;;)
+    {
+        const int a = int((long long)items * own / nq), b = int((long long)items * (own + 1) / nq);
+        int k = 0;
+        if (lane == 0) k = a < b ? atomicAdd(queue + own, 1) : 0;
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (a + k < b) return a + k;
+        int next = -1;
+        for (int q0 = 0; q0 < nq && next < 0; q0 += 32)
+        {
+            const int q = q0 + lane < nq ? (own + 1 + q0 + lane) % nq : own;
+            const int left = int((long long)items * (q + 1) / nq) - int((long long)items * q / nq);
+            const uint32_t m = __ballot_sync(0xffffffffu,
+                                             q != own && *reinterpret_cast<volatile int*>(queue + q) < left);
+            if (m) next = __shfl_sync(0xffffffffu, q, __ffs(m) - 1);
+        }
+        if (next < 0) return -1;
+        own = next;
+    }
+}
+
+__device__ __forceinline__ int sm_id()
+{
+    int s;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(s));
+    return s;
+}
+
 // ---------------------------------------------------------------- rows
 // Rows of the listed particles (all live ones when the list is the identity): the members of
 // a warp are up to 32 consecutive entries -- fewer where the list is short, so that it still
@@ -345,20 +390,19 @@ near_forest_init_kernel(NearLoop* L, int n, const NearSet* __restrict__ sets, co
 //              (over) and marked as covering everything (rowH infinite: no pair of theirs
 //              is looked for from the other side).
 template<bool Forest, bool Periodic>
-__global__ void __launch_bounds__(kThreads, 6)
+__global__ void __launch_bounds__(kThreads, 7)
 near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__ sets, const int* __restrict__ setOf,
                  NearLoop* __restrict__ L, const __grid_constant__ NearLists lists, double* __restrict__ rowsR2,
-                 int* __restrict__ rowsJ, int* __restrict__ nblCount, double* __restrict__ rowH, int cover)
+                 int* __restrict__ rowsJ, int* __restrict__ nblCount, double* __restrict__ rowH, int cover, int nq)
 {
     __shared__ NearScratch sScr[kNearWarps];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int lane = lane_id(), wib = threadIdx.x >> 5, sub = lane >> 3, off = lane & 7;
     const uint32_t lt = (1u << lane) - 1u;
     NearScratch& scr = sScr[wib];
     const int cur = L->iter & 1;
     const int n = cover ? L->cover : L->cnt[cur].build;
     if (n == 0) return;
     const int* list = cover ? lists.cover : (L->all ? nullptr : lists.build[cur]);
-    int* ticket = &L->ticket[cover ? 2 : 0];
     const double margin = cover ? kCoverMargin : kNearMargin;
     const double wide2 = kRadK2 * (margin * margin);
     const NearFrame f(t.box);
@@ -367,12 +411,11 @@ near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
     if (Periodic && !Forest) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
     int g = 32;
     while (g > 1 && n < g * int(gridDim.x) * kNearWarps) g >>= 1;
+    int own = sm_id() % nq;
     for (;;)
     {
-        int w = 0;
-        if (lane == 0) w = atomicAdd(ticket, 1);
-        w = __shfl_sync(0xffffffffu, w, 0);
-        if (long(w) * g >= n) break;
+        const int w = queue_pop(L->queue, nq, (n + g - 1) / g, own);
+        if (w < 0) break;
         const int at = w * g + lane;
         const bool mine = lane < g && at < n;
         const int i = mine ? (list ? list[at] : at) : 0;
@@ -398,7 +441,7 @@ near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
         float mean = mine ? r : 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mean += __shfl_xor_sync(0xffffffffu, mean, o);
-        const uint32_t wide = __ballot_sync(0xffffffffu, mine && r * float(__popc(all)) > kNearWide * mean);
+        uint32_t wide = __ballot_sync(0xffffffffu, mine && r * float(__popc(all)) > kNearWide * mean);
         const NearRun run = near_runs<Forest>(x, y, z, (wide >> lane) & 1u ? -1.0f : r, set);
         int rowLen = 0;
         uint32_t todo = all;
@@ -434,6 +477,9 @@ near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
                 lx = st.dlx; ly = st.dly; lz = st.dlz;
             }
             const double4* at0 = t.xyzh + v.p0;
+            bool apart = false;
+            int batches = 0, hits = 0;
+            float shared = 0.0f;
             near_blocks<0, Periodic, false>(t, v, scr, bx, by, bz, ex, ey, ez, reach, 0.0f, [&](int nb) -> float {
                 // the blocks of this batch, kNearBlocks / 32 per lane
                 constexpr int kU = kNearBlocks / 32;
@@ -447,6 +493,7 @@ near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
                     if (32 * u < nb) nd[u] = ld_node(near_node(t, v, 0, max(id[u], 0)));
                 }
                 bool dropped = false;
+                const int searching = __popc(todo & members);
                 for (uint32_t rest = todo & members; rest; rest &= rest - 1)
                 {
                     const int p = __ffs(rest) - 1;
@@ -459,29 +506,47 @@ near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
                         const bool hit = id[u] >= 0 &&
                                          near_gap2<Periodic>(q.x, q.y, q.z, 0.0f, 0.0f, 0.0f, nd[u], v) <= q.w;
                         const uint32_t m = __ballot_sync(0xffffffffu, hit);
-                        if (hit) scr.sel[ns + __popc(m & lt)] = id[u];
+                        st_shared_if(hit, scr.sel + ns + __popc(m & lt), id[u]);
                         ns += __popc(m);
                     }
                     if (ns == 0) continue;
+                    hits += ns;
+                    st_shared_if(lane < 8, scr.sel + ns + lane, kNearNone);
                     __syncwarp();
                     const double4 gp = scr.P[p];
                     const size_t row = size_t(__shfl_sync(0xffffffffu, i, p)) * kNbl;
+                    double* outR = rowsR2 + row;
+                    int* outJ = Forest ? nullptr : rowsJ + row;
                     int len = __shfl_sync(0xffffffffu, rowLen, p);
-                    near_candidates(scr.sel, ns, v.n, at0, [&](const double4& pj, int j, bool valid) {
+                    auto fetch = [&](int k, double4& pj, int& j) {
+                        j = scr.sel[k + sub] * 8 + off;
+                        pj = ldg4(at0 + min(j, v.n - 1));
+                    };
+                    // an entry beyond the row's room lands on its last one: the row is given up
+                    auto take = [&](const double4& pj, int j) {
                         double dx = gp.x - pj.x, dy = gp.y - pj.y, dz = gp.z - pj.z;
                         nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
                         const double r2 = pair_r2(dx, dy, dz);
-                        const bool acc = valid && r2 * gp.w < wide2;
+                        const bool acc = j < v.n && r2 * gp.w < wide2;
                         const uint32_t m = __ballot_sync(0xffffffffu, acc);
-                        const int k = len + __popc(m & lt);
-                        if (acc && k < kNbl)
-                        {
-                            rowsR2[row + k] = r2;
-                            if (rowsJ) rowsJ[row + k] = j;
-                        }
+                        const int k = min(len + __popc(m & lt), kNbl - 1);
                         len += __popc(m);
-                        return len <= kNbl;
-                    });
+                        st_if(acc, outR + k, r2);
+                        if (!Forest) st_if(acc, outJ + k, j);
+                    };
+                    // two sets of registers in turn: a step's loads are in flight while the one
+                    // before it is tested
+                    double4 pa, pb;
+                    int ja, jb;
+                    fetch(0, pa, ja);
+                    for (int k = 0; k < ns; k += 8)
+                    {
+                        fetch(k + 4, pb, jb);
+                        take(pa, ja);
+                        if (k + 4 >= ns) break;
+                        fetch(k + 8, pa, ja);
+                        take(pb, jb);
+                    }
                     if (lane == p) rowLen = len;
                     if (len > kNbl)
                     {
@@ -490,11 +555,22 @@ near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
                     }
                     __syncwarp();
                 }
+                // members that reach little of batch after batch: what lies between them (the flank
+                // of a concentrated set) is tested by all of them, so they go on one by one,
+                // from the start
+                shared += float(searching) * float(nb);
+                if (++batches == kNearPatience && searching > 1 && float(hits) < kNearShare * shared)
+                {
+                    if (((todo & members) >> lane) & 1u) rowLen = 0;
+                    wide |= todo & members;
+                    apart = true;
+                    return -1.0f;
+                }
                 if (!dropped) return reach;
                 // the members still searching may need less
                 return warp_max_f(((todo & members) >> lane) & 1u ? r : -1.0f);
             });
-            todo &= ~members;
+            if (!apart) todo &= ~members;
             __syncwarp();
         }
         const bool full = mine && rowLen > kNbl;
@@ -1032,6 +1108,8 @@ near_huge_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
 // runs (the graph's while condition when run as a graph).
 __global__ void near_epilogue_kernel(NearLoop* L, cudaGraphConditionalHandle more, int setCondition)
 {
+    L->queue[threadIdx.x] = 0;
+    if (threadIdx.x != 0) return;
     const int it = L->iter, cur = it & 1, nxt = cur ^ 1;
     if (it < kLoopIters) L->activePerIter[it] = L->active;
     L->cnt[cur] = NearCounts{};
@@ -1126,7 +1204,8 @@ static void near_iteration(State& s, const NearJob& j, cudaGraphConditionalHandl
     DevScalars* ds = s.dscal.get();
     auto rows = NEAR_PICK(near_rows_kernel, j);
     rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(j.tree, j.sets, j.setOf, L, lists, s.nblR2.get(),
-                                                                      j.rowsJ, s.nblCount.get(), s.nblH.get(), 0);
+                                                                      j.rowsJ, s.nblCount.get(), s.nblH.get(), 0,
+                                                                      std::min(s.numSMs, kNearQueues));
     COSMO_LAUNCHED();
     auto step = j.sets ? near_step_kernel<true> : near_step_kernel<false>;
     step<<<iceil(j.n, kThreads), kThreads, 0, s.st>>>(j.sets, j.setOf, L, lists, s.nblR2.get(), s.nblCount.get(),
@@ -1143,7 +1222,7 @@ static void near_iteration(State& s, const NearJob& j, cudaGraphConditionalHandl
     huge<<<s.numSMs, 32 * kHugeWarps, 0, s.st>>>(j.tree, j.sets, j.setOf, L, lists, j.xyzh, j.rho, j.gradh, j.converged,
                                                  s.hs.get(), j.pmass, j.tolh, j.hfact, ds);
     COSMO_LAUNCHED();
-    near_epilogue_kernel<<<1, 1, 0, s.st>>>(L, more, setCondition);
+    near_epilogue_kernel<<<1, kNearQueues, 0, s.st>>>(L, more, setCondition);
     COSMO_LAUNCHED();
 }
 
@@ -1263,7 +1342,7 @@ void near_newton(State& s, double pmass, double tolh, double hfact, int maxIter,
     near_buffers(s, n);
     near_build(s);
     const bool frozen = s.frozenFor == s.ngas && s.nAlive > 0;
-    near_init_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get(), ds, maxIter, frozen ? 1 : 0);
+    near_init_kernel<<<1, kNearQueues, 0, s.st>>>(s.nearLoop.get(), ds, maxIter, frozen ? 1 : 0);
     COSMO_LAUNCHED();
     if (frozen)
     {
@@ -1285,7 +1364,7 @@ void near_cover(State& s, int* rowsJ)
     auto rows = s.periodic ? near_rows_kernel<false, true> : near_rows_kernel<false, false>;
     rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(near_tree(s), nullptr, nullptr, s.nearLoop.get(),
                                                                       near_lists(s), s.nblR2.get(), rowsJ,
-                                                                      s.nblCount.get(), s.nblH.get(), 1);
+                                                                      s.nblCount.get(), s.nblH.get(), 1, std::min(s.numSMs, kNearQueues));
     COSMO_LAUNCHED();
 }
 
@@ -1324,7 +1403,7 @@ void near_forest_newton(State& s, const NearForest& b, double tolh, double hfact
     COSMO_LAUNCHED();
     near_upper_levels_kernel<true><<<b.nsets, 1024, 0, s.st>>>(t, out, s.nearSets.get());
     COSMO_LAUNCHED();
-    near_forest_zero_kernel<<<1, 1, 0, s.st>>>(s.nearLoop.get(), maxIter);
+    near_forest_zero_kernel<<<1, kNearQueues, 0, s.st>>>(s.nearLoop.get(), maxIter);
     COSMO_LAUNCHED();
     near_forest_init_kernel<<<std::min(iceil(b.n, kThreads), 16 * s.numSMs), kThreads, 0, s.st>>>(
         s.nearLoop.get(), b.n, s.nearSets.get(), b.setOf, near_lists(s));
@@ -1350,7 +1429,7 @@ void near_forest_eval(State& s, const NearForest& b)
     auto rows = near_rows_kernel<true, true>;
     rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(t, s.nearSets.get(), b.setOf, L, lists,
                                                                       s.nblR2.get(), nullptr, s.nblCount.get(),
-                                                                      s.nblH.get(), 1);
+                                                                      s.nblH.get(), 1, std::min(s.numSMs, kNearQueues));
     COSMO_LAUNCHED();
     near_eval_kernel<<<iceil(b.n, kThreads), kThreads, 0, s.st>>>(b.n, s.nearSets.get(), b.setOf, s.nblR2.get(),
                                                                   s.nblCount.get(), b.xyzh, b.rho, b.gradh,

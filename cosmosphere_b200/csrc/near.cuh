@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include "rows.cuh"
 #include "state.hpp"
+#include "tma.cuh"
 
 namespace cosmo {
 
@@ -79,8 +80,17 @@ struct NearScratch
     float4 Q[32];                  // position relative to the box centre, squared reach
     int front[kNearLevels][32];    // accepted nodes of each level, not yet expanded
     int blk[kNearBlocks];          // accepted blocks, ascending
-    int sel[kNearBlocks];          // those one member reaches
+    int sel[kNearBlocks + 8];      // those one member reaches, then kNearNone
 };
+constexpr int kNearNone = 0x0fffffff;   // a block whose particles lie beyond any set's
+
+// The lane, kept in a register (read anew it costs an instruction at every use).
+__device__ __forceinline__ int lane_id()
+{
+    int l;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
+    return l;
+}
 
 __device__ __forceinline__ NearNode ld_node(const NearNode* p)
 {
@@ -89,6 +99,24 @@ __device__ __forceinline__ NearNode ld_node(const NearNode* p)
         : "=f"(n.cx), "=f"(n.cy), "=f"(n.cz), "=f"(n.hmax), "=f"(n.ex), "=f"(n.ey), "=f"(n.ez), "=f"(n.pad)
         : "l"(p));
     return n;
+}
+
+// Stores under a predicate, without a branch around them: a warp whose lanes differ in it
+// would otherwise part and join again at every step of a search.
+__device__ __forceinline__ void st_if(bool p, double* a, double v)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %0, 0;\n\t@q st.global.f64 [%1], %2;\n\t}"
+                 :: "r"(int(p)), "l"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_if(bool p, int* a, int v)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %0, 0;\n\t@q st.global.s32 [%1], %2;\n\t}"
+                 :: "r"(int(p)), "l"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_shared_if(bool p, int* a, int v)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %0, 0;\n\t@q st.shared.s32 [%1], %2;\n\t}"
+                 :: "r"(int(p)), "r"(smem_u32(a)), "r"(v) : "memory");
 }
 
 // The search frame: box centre and periods, and the slack of a radius.  A relative
@@ -166,35 +194,38 @@ __device__ __forceinline__ void near_blocks(const NearTree& t, const NearView& v
                                             float z, float ex, float ey, float ez, float reach, float slack,
                                             Flush&& flush)
 {
-    const int lane = threadIdx.x & 31;
+    const int lane = lane_id();
     const uint32_t lt = (1u << lane) - 1u;
-    int top = 0;
-    while (near_count(v.n, top) > 32) ++top;
+    // lane l: the nodes of level l and where they start
+    const int myCount = lane < kNearLevels ? near_count(v.n, lane) : 0;
+    const int myOff = lane < kNearLevels ? t.off[lane] + (v.p0 >> (3 * lane + 3)) + v.s : 0;
+    const int top = __popc(__ballot_sync(0xffffffffu, myCount > 32));
     int nb = 0;
     int left = 0, pos = 0;   // lane l: nodes of level l not yet expanded, and the first of them
     auto test = [&](int level, int idx) {
-        const NearNode n = ld_node(near_node(t, v, level, idx));
+        const NearNode n = ld_node(t.node + (__shfl_sync(0xffffffffu, myOff, level) + idx));
         const float r = Sym ? fmaxf(reach, near_sym_reach(n.hmax, slack)) : reach;
         return near_gap2<Periodic>(x, y, z, ex, ey, ez, n, v) <= r * r;
     };
     // children of up to four nodes, or the top level: accepted ones of level into the next list
     auto accept = [&](int level, int idx, bool valid) {
-        const bool ok = valid && test(level, idx);
+        const bool ok = test(level, valid ? idx : 0) && valid;
         const uint32_t m = __ballot_sync(0xffffffffu, ok);
         const int c = __popc(m);
         if (level == Stop)
         {
-            if (ok) scr.blk[nb + __popc(m & lt)] = idx;
+            st_shared_if(ok, scr.blk + nb + __popc(m & lt), idx);
             nb += c;
         }
         else
         {
-            if (ok) scr.front[level][__popc(m & lt)] = idx;
+            st_shared_if(ok, scr.front[level] + __popc(m & lt), idx);
             if (lane == level) { left = c; pos = 0; }
         }
         __syncwarp();
     };
-    accept(top, lane, lane < near_count(v.n, top));
+    const int tops = __shfl_sync(0xffffffffu, myCount, top);
+    accept(top, lane, lane < tops);
     int lev = top;
     for (;;)
     {
@@ -212,8 +243,9 @@ __device__ __forceinline__ void near_blocks(const NearTree& t, const NearView& v
         const int m = min(have, 4);
         const int node = scr.front[lev][first + min(lane >> 3, m - 1)];
         const int child = node * 8 + (lane & 7);
+        const int below = __shfl_sync(0xffffffffu, myCount, lev - 1);
         if (lane == lev) { left -= m; pos += m; }
-        accept(lev - 1, child, (lane >> 3) < m && child < near_count(v.n, lev - 1));
+        accept(lev - 1, child, (lane >> 3) < m && child < below);
         if (lev > Stop + 1) --lev;
     }
 }
@@ -320,19 +352,26 @@ __device__ __forceinline__ void near_candidates(const int* ids, int ns, int nLiv
 {
     const int lane = threadIdx.x & 31;
     const int sub = lane >> 3, off = lane & 7;
-    int j = ids[min(sub, ns - 1)] * 8 + off;
-    bool valid = sub < ns && j < nLive;
-    double4 p = ldg4(xyzh + (valid ? j : 0));
-    for (int k = 0; k < ns; k += 4)
+    auto load = [&](int k, double4& p, int& j, bool& valid) {
+        const int at = k + sub;
+        j = ids[min(at, ns - 1)] * 8 + off;
+        valid = at < ns && j < nLive;
+        p = ldg4(xyzh + (valid ? j : 0));
+    };
+    // two sets of registers in turn: a step's loads are in flight while the one before it is
+    // tested, and nothing is copied from one to the other
+    double4 pa, pb;
+    int ja, jb;
+    bool va, vb;
+    load(0, pa, ja, va);
+    for (int k = 0;;)
     {
-        const int kn = k + 4 + sub;
-        const int jn = ids[min(kn, ns - 1)] * 8 + off;
-        const bool vn = kn < ns && jn < nLive;
-        const double4 pn = ldg4(xyzh + (vn ? jn : 0));
-        if (!use(p, j, valid)) return;
-        j = jn;
-        valid = vn;
-        p = pn;
+        load(k + 4, pb, jb, vb);
+        if (!use(pa, ja, va)) return;
+        if ((k += 4) >= ns) return;
+        load(k + 4, pa, ja, va);
+        if (!use(pb, jb, vb)) return;
+        if ((k += 4) >= ns) return;
     }
 }
 

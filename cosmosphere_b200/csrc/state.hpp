@@ -126,6 +126,7 @@ struct NewtonLoop
 
 // The Newton loop over the block tree (near.cu): the lists an iteration works on and fills
 // (double-buffered by the iteration's parity) and its state on the device.
+constexpr int kNearQueues = 256;
 struct NearCounts
 {
     int row, build, sum, huge;   // particles with a row, without one, with more neighbours than one holds, with very many
@@ -138,6 +139,7 @@ struct NearLoop
     int ticket[4];               // work tickets: row search, direct sums, cover search, direct sums by blocks
     NearCounts cnt[2];
     long long activePerIter[kLoopIters];
+    int queue[kNearQueues];      // the row search's work, one queue a multiprocessor
 };
 struct NearLists
 {
@@ -204,9 +206,9 @@ struct State
     // "sym_from_rows", COSMO_SYM_FROM_ROWS).  The results are the same either way.
     int symFromRows = 1;
     int symRowsSkip = 0;   // solves left that do not try it (after one that could not)
-    // pairs the other side's supports may add that the rows' merge holds (0: one per live
-    // particle); a smaller figure sends the force pass back to the list-built rows when
-    // more are found (cosmo_x_set_option "sym_extra_cap", a test of that fallback)
+    // pairs the other side's supports may add in all (0: as many as the particles' places
+    // hold); a figure sends the force pass back to the list-built rows when more are found
+    // (cosmo_x_set_option "sym_extra_cap", a test of that fallback)
     int symExtraCap = 0;
     // list storage of the graph loop's rebuilds as a percentage of the first lists' total
     // (0: the built-in, twice the total plus 65536 entries); a figure under 100 makes a
@@ -286,10 +288,8 @@ struct State
     DBuf<int> nblJ;                             // the Newton rows' j (flat, beside nblR2)
     DBuf<double> hs;                            // h in the sorted order (rows from the Newton rows)
     DBuf<int> coverFlag, coverLeaves;           // rows to complete after a solve: particle flags, leaves
-    DBuf<unsigned long long> extras;            // (row owner << 32 | j) a row must gain
-    DBuf<int> extraCnt;                         // extras per particle
-    DBuf<uint32_t> extraOff;                    // their offsets (exclusive scan)
-    DBuf<int> extraBucket;                      // the extras' j, grouped by owner
+    DBuf<int> extras;                           // the j a row must gain, kExtra places a particle
+    DBuf<int> extraCnt;                         // how many
     DBuf<int> leafNext;                         // leaf already queued for the next iteration
     DBuf<int> activeA, activeB, allLeaves;
     DBuf<float4> nearNode;                      // the block tree (near.cuh), two float4 a node
