@@ -198,22 +198,26 @@ gradient_row_kernel(int nAlive, const int* __restrict__ nbl, const int* __restri
     if ((threadIdx.x & 31) == 0) atomicAdd(&ds->pairs[1], pairs);
 }
 
-// Post-convergence sweep of the particles without a row (the block-tree solve's over list):
-// one warp searches for one particle, evaluates 32 of its pairs at a time, one per lane, and
-// adds their terms in ascending j with one sum per lane.
-template<bool Periodic>
+// Post-convergence sweep with one warp per particle: 32 of its pairs at a time are evaluated,
+// one per lane, and their terms added in ascending j with one sum per lane.  Rows: all live
+// particles of a small set over their rows -- there one lane per particle leaves most of the
+// chip idle and takes as long as the longest row.  Otherwise the particles without a row (the
+// block-tree solve's over list), each over its own search.
+template<bool Periodic, bool Rows>
 __global__ void __launch_bounds__(kThreads)
-gradient_over_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ L, const int* __restrict__ over,
+gradient_warp_kernel(const __grid_constant__ NearTree t, const NearLoop* __restrict__ L, int nAlive,
+                     const int* __restrict__ over, const int* __restrict__ nbl, const int* __restrict__ nblCount,
                      const double4* __restrict__ vel4, const double4* __restrict__ acc4, double* __restrict__ rho,
                      double* __restrict__ gradh, double* __restrict__ divv, double* __restrict__ xiOut,
                      double* __restrict__ ddivvdt, double pmass, DevScalars* __restrict__ ds)
 {
-    __shared__ NearScratch sScr[kWarpsPerBlock];
+    __shared__ NearScratch sScr[Rows ? 1 : kWarpsPerBlock];
     __shared__ double sTerm[kWarpsPerBlock][32 * kGradTerms];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int n = L->over;
-    if (n == 0 || L->active > 0) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ds->rowOverflow = 1;
+    if (L != nullptr && L->active > 0) return;   // the Newton loop did not converge
+    const int n = Rows ? nAlive : L->over;
+    if (n == 0) return;
+    if (!Rows && blockIdx.x == 0 && threadIdx.x == 0) ds->rowOverflow = 1;
     const NearFrame f(t.box);
     const NearView v = near_view(t, f);
     double lx = 0, ly = 0, lz = 0;
@@ -222,39 +226,58 @@ gradient_over_kernel(const __grid_constant__ NearTree t, NearLoop* __restrict__ 
     unsigned long long pairs = 0;
     for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (gridDim.x * blockDim.x) >> 5)
     {
-        const int i = over[w];
+        const int i = Rows ? w : over[w];
+        const int cnt = Rows ? nblCount[i] : 0;
+        if (Rows && unsigned(cnt) > unsigned(kNbl)) continue;
         const double4 pi = t.xyzh[i], vi = vel4[i], ai = acc4[i];
         const double hinv2 = 1.0 / (pi.w * pi.w);
-        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
-        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
         double sum = 0.0;   // lane k: sum k
         unsigned int gp = 0;
-        near_blocks<0, Periodic, false>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
-            near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, [&](const double4& pj, int j, bool valid) {
-                double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
-                const double r2 = pair_r2(dx, dy, dz);
-                const double q2 = r2 * hinv2;
-                const bool acc = valid && q2 < kRadK2;
-                const uint32_t m = __ballot_sync(0xffffffffu, acc);
-                if (acc)
-                {
-                    double* mine = term + __popc(m & ((1u << lane) - 1u)) * kGradTerms;
-                    grad_terms(dx, dy, dz, r2, q2, vi, ai, ldg4(vel4 + j), ldg4(acc4 + j), pmass,
-                               [&](int k, double x) { mine[k] = x; });
-                }
-                __syncwarp();
-                const int c = __popc(m);
-                gp += c;
-                if (lane < 21)
-                    for (int k = 0; k < c; ++k) sum += term[k * kGradTerms + lane];
-                else if (lane < kGradTerms)
-                    for (int k = 0; k < c; ++k) sum -= term[k * kGradTerms + lane];
-                __syncwarp();
-                return true;
+        auto pair = [&](const double4& pj, int j, bool valid) {
+            double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+            nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+            const double r2 = pair_r2(dx, dy, dz);
+            const double q2 = r2 * hinv2;
+            const bool acc = valid && q2 < kRadK2;
+            const uint32_t m = __ballot_sync(0xffffffffu, acc);
+            if (acc)
+            {
+                double* mine = term + __popc(m & ((1u << lane) - 1u)) * kGradTerms;
+                grad_terms(dx, dy, dz, r2, q2, vi, ai, ldg4(vel4 + j), ldg4(acc4 + j), pmass,
+                           [&](int k, double x) { mine[k] = x; });
+            }
+            __syncwarp();
+            const int c = __popc(m);
+            gp += c;
+            const double* my = term + min(lane, kGradTerms - 1);
+            if (lane < 21)
+#pragma unroll 8
+                for (int k = 0; k < c; ++k) sum += my[k * kGradTerms];
+            else
+#pragma unroll 8
+                for (int k = 0; k < c; ++k) sum -= my[k * kGradTerms];
+            __syncwarp();
+            return true;
+        };
+        if constexpr (Rows)
+        {
+            const int* row = row_of(nbl, uint32_t(i));
+            for (int k0 = 0; k0 < cnt; k0 += 32)
+            {
+                const bool valid = k0 + lane < cnt;
+                const int j = valid ? row[size_t(k0 + lane) * kRowStride] : i;
+                pair(ldg4(t.xyzh + j), j, valid);
+            }
+        }
+        else
+        {
+            const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
+            const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
+            near_blocks<0, Periodic, false>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
+                near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, pair);
+                return r;
             });
-            return r;
-        });
+        }
         GradSums g;
 #pragma unroll
         for (int k = 0; k < kGradTerms; ++k) g.s[k] = __shfl_sync(0xffffffffu, sum, k);
@@ -454,6 +477,35 @@ __global__ void row_cover_kernel(int nL, const uint32_t* __restrict__ layout, co
     }
 }
 
+// The tests of one entry of a Newton row (dr2: the pair's squared distance) on its way into
+// the symmetric rows: keep, whether the force pass takes the pair; extra, whether j's own row
+// may lack it (cover(): the h that row covers).  Not kExact: dr2 is the double rounded to
+// float, and retake() gives the double where it lies within 1e-6 of a bound.
+struct SymTest
+{
+    double bi, bj, own;
+    __device__ __forceinline__ SymTest(double boundI, double hj)
+        : bi(boundI), bj(kRadK2 * (hj * hj) * (1.0 + 1e-10)), own(kRadK2 * (hj * hj))
+    {
+    }
+    template<bool kExact, class Retake, class Cover>
+    __device__ __forceinline__ void test(double dr2, bool& keep, bool& extra, Retake&& retake, Cover&& cover) const
+    {
+        bool exact = kExact;
+        auto near = [&](double bound) { return fabs(dr2 - bound) <= 1e-6 * bound; };
+        if (!exact && (near(fmax(bi, bj)) || near(bi) || near(own))) { dr2 = retake(); exact = true; }
+        keep = !(dr2 >= fmax(bi, bj));
+        extra = false;
+        if (dr2 < bi && !(dr2 < own))
+        {
+            const double ch = cover();
+            const double c2 = kRadK2 * (ch * ch) * (1.0 - 1e-9);
+            if (!exact && near(c2)) dr2 = retake();
+            extra = !(dr2 < c2);
+        }
+    }
+};
+
 // The symmetric rows from the Newton rows, for every live particle whose row covers its
 // converged h: the j of its Newton row (flat, ascending, r^2 beside each -- the same
 // double as the force pass's dr^2) that the force pass takes,
@@ -488,30 +540,18 @@ sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restr
         int* out = row_of(nbl, uint32_t(i));
         int w = 0;
         auto entry = [&](int j, double dr2, double hj) {
-            bool exact = kExact;
-            auto near = [&](double bound) { return fabs(dr2 - bound) <= 1e-6 * bound; };
-            auto retake = [&]() {
-                if (exact) return;
+            bool keep, extra;
+            SymTest(bi, hj).template test<kExact>(dr2, keep, extra, [&]() {
                 const double4 pa = xyzh[i], pb = ldg4(xyzh + j);
                 double dx = pa.x - pb.x, dy = pa.y - pb.y, dz = pa.z - pb.z;
                 nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
-                dr2 = pair_r2(dx, dy, dz);
-                exact = true;
-            };
-            const double bj = kRadK2 * (hj * hj) * (1.0 + 1e-10);
-            const double own = kRadK2 * (hj * hj);
-            if (!exact && (near(fmax(bi, bj)) || near(bi) || near(own))) retake();
-            if (!(dr2 >= fmax(bi, bj))) out[size_t(w++) * kRowStride] = j;
-            if (dr2 < bi && !(dr2 < own))
+                return pair_r2(dx, dy, dz);
+            }, [&]() { return __ldg(rowH + j); });
+            if (keep) out[size_t(w++) * kRowStride] = j;
+            if (extra)
             {
-                const double ch = __ldg(rowH + j);
-                const double cover = kRadK2 * (ch * ch) * (1.0 - 1e-9);
-                if (!exact && near(cover)) retake();
-                if (!(dr2 < cover))
-                {
-                    add_extra(extras, extraCnt, j, i);
-                    ++added;
-                }
+                add_extra(extras, extraCnt, j, i);
+                ++added;
             }
         };
         // groups of four entries in a two-stage pipeline: while a group is tested, the next
@@ -552,70 +592,142 @@ sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restr
     if ((threadIdx.x & 31) == 0 && added) atomicAdd(&ds->extraCount, added);
 }
 
-// Each row owner merges its extras into its row: sorted, those the row already holds
-// dropped, the rest merged in from the back so the row stays ascending.  A row that would
-// exceed kNbl joins the over list when there is one (its passes then search for it), else
-// sets mergeOverflow (the symmetric rows are then built instead).  A particle without a row
-// takes none.
-__global__ void extras_merge_kernel(int nA, const int* __restrict__ extraCnt, int* __restrict__ extras,
-                                    int* __restrict__ nbl, int* __restrict__ nblCount, DevScalars* __restrict__ ds,
-                                    int* __restrict__ over, int* __restrict__ overCount)
+// sym_from_rows_kernel for a small set: one warp per particle, one entry per lane.
+template<class T, bool Periodic>
+__global__ void __launch_bounds__(kThreads)
+sym_from_rows_warp_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restrict__ rowsR2,
+                          int* __restrict__ nblCount, const double* __restrict__ hs, const double* __restrict__ rowH,
+                          const double4* __restrict__ xyzh, const DevBox* __restrict__ box, int* __restrict__ nbl,
+                          int* __restrict__ extras, int* __restrict__ extraCnt, DevScalars* __restrict__ ds)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nA) return;
-    const uint32_t e = uint32_t(extraCnt[t]);
-    if (e == 0) return;
-    const int cnt = nblCount[t];
-    if (unsigned(cnt) > unsigned(kNbl)) return;
-    auto full = [&]() {
-        if (over != nullptr)
+    constexpr bool kExact = std::is_same<T, double>::value;
+    double lx = 0, ly = 0, lz = 0;
+    if (Periodic && !kExact) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
+    const int lane = threadIdx.x & 31;
+    int added = 0;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nAlive; i += (gridDim.x * blockDim.x) >> 5)
+    {
+        const int cnt = nblCount[i];
+        if (unsigned(cnt) > unsigned(kNbl)) continue;
+        const double hi = hs[i];
+        const double bi = kRadK2 * (hi * hi) * (1.0 + 1e-10);
+        const int* inJ = row_flat(rowsJ, uint32_t(i));
+        const T* inR = row_flat(rowsR2, uint32_t(i));
+        int* out = row_of(nbl, uint32_t(i));
+        int w = 0;
+        for (int k0 = 0; k0 < cnt; k0 += 32)
         {
-            nblCount[t] = kNbl + 1;
-            over[atomicAdd(overCount, 1)] = t;
+            const bool valid = k0 + lane < cnt;
+            const int j = valid ? inJ[k0 + lane] : i;
+            double dr2 = valid ? double(inR[k0 + lane]) : 0.0;
+            const SymTest s(bi, hs[j]);
+            bool keep = false, extra = false;
+            if (valid) s.template test<kExact>(dr2, keep, extra, [&]() {
+                const double4 pa = xyzh[i], pb = ldg4(xyzh + j);
+                double dx = pa.x - pb.x, dy = pa.y - pb.y, dz = pa.z - pb.z;
+                nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+                return pair_r2(dx, dy, dz);
+            }, [&]() { return __ldg(rowH + j); });
+            if (extra)
+            {
+                add_extra(extras, extraCnt, j, i);
+                ++added;
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, keep);
+            if (keep) out[size_t(w + __popc(m & ((1u << lane) - 1u))) * kRowStride] = j;
+            w += __popc(m);
         }
-        else ds->mergeOverflow = 1;
-    };
-    if (e > uint32_t(kExtra))
-    {
-        full();
-        return;
+        __syncwarp();
+        if (lane == 0) nblCount[i] = w;
     }
-    int* ex = extras + size_t(t) * kExtra;
-    for (uint32_t a = 1; a < e; ++a)
+    added = __reduce_add_sync(0xffffffffu, added);
+    if (lane == 0 && added) atomicAdd(&ds->extraCount, added);
+}
+
+// Each row owner's extras merged into its row, in order, those the row already holds dropped
+// (no two extras are the same: a particle appends another at most once).  A warp takes 32
+// owners and, together, those with extras: a lane per extra finds its place in the row by
+// bisection and its rank among the extras, every entry moves up by the extras before it.
+// (One thread per owner, sorting and merging in place, took 1.7 ms for 2 M Plummer particles
+// with ten extras each.)  A row that would exceed kNbl joins the over list when there is one
+// (its passes then search for it), else sets mergeOverflow (the symmetric rows are then built
+// instead).  A particle without a row takes none.
+__global__ void __launch_bounds__(256)
+extras_merge_kernel(int nA, const int* __restrict__ extraCnt, const int* __restrict__ extras, int* __restrict__ nbl,
+                    int* __restrict__ nblCount, DevScalars* __restrict__ ds, int* __restrict__ over,
+                    int* __restrict__ overCount)
+{
+    constexpr int kPer = kExtra / 32, kRowPer = kNbl / 32;
+    const int lane = threadIdx.x & 31;
+    const int t0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
+    const int mineE = t0 + lane < nA ? extraCnt[t0 + lane] : 0;
+    const int mineCnt = mineE > 0 ? nblCount[t0 + lane] : 0;
+    for (uint32_t rest = __ballot_sync(0xffffffffu, mineE > 0 && unsigned(mineCnt) <= unsigned(kNbl)); rest;
+         rest &= rest - 1)
     {
-        const int v = ex[a];
-        uint32_t k = a;
-        for (; k > 0 && ex[k - 1] > v; --k) ex[k] = ex[k - 1];
-        ex[k] = v;
-    }
-    int* row = row_of(nbl, uint32_t(t));
-    auto at = [&](int k) -> int& { return row[size_t(k) * kRowStride]; };
-    uint32_t u = 0;
-    for (uint32_t a = 0; a < e; ++a)
-    {
-        const int v = ex[a];
-        int lo = 0, hi = cnt;
-        while (lo < hi)
+        const int p = __ffs(rest) - 1, t = t0 + p;
+        const int e = __shfl_sync(0xffffffffu, mineE, p), cnt = __shfl_sync(0xffffffffu, mineCnt, p);
+        int* row = row_of(nbl, uint32_t(t));
+        auto at = [&](int k) -> int& { return row[size_t(k) * kRowStride]; };
+        int x[kPer], lo[kPer], rank[kPer], u = 0;
+        bool keep[kPer];
+#pragma unroll
+        for (int c = 0; c < kPer; ++c)
         {
-            const int mid = (lo + hi) >> 1;
-            if (at(mid) < v) lo = mid + 1;
-            else hi = mid;
+            x[c] = 32 * c + lane < min(e, kExtra) ? extras[size_t(t) * kExtra + 32 * c + lane] : 0x7fffffff;
+            int a = 0, b = cnt;
+            while (a < b)
+            {
+                const int mid = (a + b) >> 1;
+                if (at(mid) < x[c]) a = mid + 1;
+                else b = mid;
+            }
+            lo[c] = a;
+            rank[c] = 0;
+            keep[c] = 32 * c + lane < min(e, kExtra) && !(a < cnt && at(a) == x[c]);
+            u += __popc(__ballot_sync(0xffffffffu, keep[c]));
         }
-        if (!(lo < cnt && at(lo) == v)) ex[u++] = v;
+        if (u == 0 && e <= kExtra) continue;
+        if (e > kExtra || cnt + u > kNbl)
+        {
+            if (lane == 0)
+            {
+                if (over != nullptr)
+                {
+                    nblCount[t] = kNbl + 1;
+                    over[atomicAdd(overCount, 1)] = t;
+                }
+                else ds->mergeOverflow = 1;
+            }
+            continue;
+        }
+        int val[kRowPer], up[kRowPer];
+#pragma unroll
+        for (int c = 0; c < kRowPer; ++c)
+        {
+            val[c] = 32 * c + lane < cnt ? at(32 * c + lane) : 0;
+            up[c] = 0;
+        }
+#pragma unroll
+        for (int d = 0; d < kPer; ++d)
+            for (uint32_t k = __ballot_sync(0xffffffffu, keep[d]); k; k &= k - 1)
+            {
+                const int src = __ffs(k) - 1;
+                const int xs = __shfl_sync(0xffffffffu, x[d], src), ls = __shfl_sync(0xffffffffu, lo[d], src);
+#pragma unroll
+                for (int c = 0; c < kPer; ++c) rank[c] += xs < x[c];
+#pragma unroll
+                for (int c = 0; c < kRowPer; ++c) up[c] += ls <= 32 * c + lane;
+            }
+        __syncwarp();   // every entry has been read
+#pragma unroll
+        for (int c = 0; c < kRowPer; ++c)
+            if (32 * c + lane < cnt && up[c] > 0) at(32 * c + lane + up[c]) = val[c];
+#pragma unroll
+        for (int c = 0; c < kPer; ++c)
+            if (keep[c]) at(lo[c] + rank[c]) = x[c];
+        if (lane == 0) nblCount[t] = cnt + u;
     }
-    if (u == 0) return;
-    if (cnt + int(u) > kNbl)
-    {
-        full();
-        return;
-    }
-    int r = cnt - 1, x = int(u) - 1, w = cnt + int(u) - 1;
-    while (x >= 0)
-    {
-        if (r >= 0 && at(r) > ex[x]) at(w--) = at(r--);
-        else at(w--) = ex[x--];
-    }
-    nblCount[t] = cnt + int(u);
 }
 
 __global__ void hmax_live_kernel(const double4* __restrict__ xyzh, int nAlive, double* __restrict__ part)
@@ -1056,7 +1168,8 @@ static void sym_rows_from_newton(State& s, bool near)
     COSMO_CUDA(cudaMemsetAsync(s.extraCnt.get(), 0, size_t(nA) * sizeof(int), s.st));
     // extraCount, mergeOverflow and rowOverflow were zeroed by the coverage check (or the
     // block-tree loop's start)
-    const int grid = std::max(1, iceil(nA, kThreads));
+    const bool warp = nA <= kWarpPerParticle;
+    const int grid = std::max(1, iceil(nA, warp ? kWarpsPerBlock : kThreads));
     auto compact = [&](auto kern, const auto* rows) {
         kern<<<grid, kThreads, 0, s.st>>>(nA, s.nblJ.get(), rows, s.nblCount.get(), s.hs.get(), s.nblH.get(),
                                           s.xyzh.get(), s.box.get(), s.nbl.get(), s.extras.get(), s.extraCnt.get(), ds);
@@ -1065,10 +1178,11 @@ static void sym_rows_from_newton(State& s, bool near)
     const float* rowsF = reinterpret_cast<const float*>(s.nblR2.get());
     if (s.precision == 1)
     {
-        if (s.periodic) compact(sym_from_rows_kernel<float, true>, rowsF);
-        else compact(sym_from_rows_kernel<float, false>, rowsF);
+        if (s.periodic) compact(warp ? sym_from_rows_warp_kernel<float, true> : sym_from_rows_kernel<float, true>, rowsF);
+        else compact(warp ? sym_from_rows_warp_kernel<float, false> : sym_from_rows_kernel<float, false>, rowsF);
     }
-    else compact(sym_from_rows_kernel<double, false>, s.nblR2.get());
+    else
+        compact(warp ? sym_from_rows_warp_kernel<double, false> : sym_from_rows_kernel<double, false>, s.nblR2.get());
     COSMO_LAUNCHED();
     if (near)
     {
@@ -1352,19 +1466,26 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             launch_gradient_mixed(s, pmass);
         else
         {
-            auto gr = s.periodic ? gradient_row_kernel<true> : gradient_row_kernel<false>;
-            gr<<<std::max(1, iceil(s.nAlive, kThreads)), kThreads, 0, s.st>>>(
-                s.nAlive, s.nbl.get(), s.nblCount.get(), s.xyzh.get(), s.vel4.get(), s.acc4.get(), s.rho.get(),
-                s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), ds, active);
-            COSMO_LAUNCHED();
-            if (near && fromRows)
+            auto warps = [&](auto kern, int blocks) {
+                kern<<<blocks, kThreads, 0, s.st>>>(near_tree(s), near ? s.nearLoop.get() : nullptr, s.nAlive,
+                                                    s.nearOver.get(), s.nbl.get(), s.nblCount.get(), s.vel4.get(),
+                                                    s.acc4.get(), s.rho.get(), s.gradh.get(), s.divv.get(), s.xi.get(),
+                                                    s.ddivvdt.get(), pmass, ds);
+                COSMO_LAUNCHED();
+            };
+            if (s.nAlive <= kWarpPerParticle)
+                warps(s.periodic ? gradient_warp_kernel<true, true> : gradient_warp_kernel<false, true>,
+                      std::max(1, iceil(s.nAlive, kWarpsPerBlock)));
+            else
             {
-                auto go = s.periodic ? gradient_over_kernel<true> : gradient_over_kernel<false>;
-                go<<<2 * s.numSMs, kThreads, 0, s.st>>>(near_tree(s), s.nearLoop.get(), s.nearOver.get(), s.vel4.get(),
-                                                        s.acc4.get(), s.rho.get(), s.gradh.get(), s.divv.get(),
-                                                        s.xi.get(), s.ddivvdt.get(), pmass, ds);
+                auto gr = s.periodic ? gradient_row_kernel<true> : gradient_row_kernel<false>;
+                gr<<<iceil(s.nAlive, kThreads), kThreads, 0, s.st>>>(
+                    s.nAlive, s.nbl.get(), s.nblCount.get(), s.xyzh.get(), s.vel4.get(), s.acc4.get(), s.rho.get(),
+                    s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), ds, active);
                 COSMO_LAUNCHED();
             }
+            if (near && fromRows)
+                warps(s.periodic ? gradient_warp_kernel<true, false> : gradient_warp_kernel<false, false>, 2 * s.numSMs);
             // the group sweep of the rows that overflowed (none: it returns at once)
             auto gk = s.periodic ? gradient_kernel<true> : gradient_kernel<false>;
             if (!(near && fromRows)) gk<<<grid, kThreads, 0, s.st>>>(nL, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),

@@ -380,20 +380,22 @@ force_row_kernel(int nAlive, const int* __restrict__ nbl, const int* __restrict_
     if ((threadIdx.x & 31) == 0) atomicAdd(&ds->pairs[2], pairs);
 }
 
-// Force pass of the particles without a row (the block-tree solve's over list): one warp
-// searches for one particle -- its own support and every block's -- evaluates 32 pairs at a
-// time, one per lane, and adds their terms in ascending j with one sum per lane (a term a
-// pair does not have is zero, which leaves its sum as it is).
-template<bool Periodic, bool Disc>
+// Force pass with one warp per particle: 32 of its pairs at a time are evaluated, one per lane,
+// and their terms added in ascending j with one sum per lane (a term a pair does not have is
+// zero, which leaves its sum as it is).  Rows: all live particles of a small set over their
+// rows.  Otherwise the particles without a row (the block-tree solve's over list), each over a
+// search of its own support and every block's.
+template<bool Periodic, bool Disc, bool Rows>
 __global__ void __launch_bounds__(kThreads)
-force_over_kernel(const __grid_constant__ NearTree t, int n, const int* __restrict__ over,
-                  const double4* __restrict__ vel4, const double4* __restrict__ thermo4,
-                  const double4* __restrict__ prepA, const double4* __restrict__ prepB, double* __restrict__ fx,
-                  double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ f4,
-                  double* __restrict__ vsigmax, double* __restrict__ divvF, double pmass, double alphau, double beta,
-                  int pdv, int shock, DevScalars* __restrict__ ds)
+force_warp_kernel(const __grid_constant__ NearTree t, int n, const int* __restrict__ over, const int* __restrict__ nbl,
+                  const int* __restrict__ nblCount, const double4* __restrict__ vel4,
+                  const double4* __restrict__ thermo4, const double4* __restrict__ prepA,
+                  const double4* __restrict__ prepB, double* __restrict__ fx, double* __restrict__ fy,
+                  double* __restrict__ fz, double* __restrict__ f4, double* __restrict__ vsigmax,
+                  double* __restrict__ divvF, double pmass, double alphau, double beta, int pdv, int shock,
+                  DevScalars* __restrict__ ds)
 {
-    __shared__ NearScratch sScr[kWarpsPerBlock];
+    __shared__ NearScratch sScr[Rows ? 1 : kWarpsPerBlock];
     __shared__ double sTerm[kWarpsPerBlock][32 * (kForceTerms + 1)];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     constexpr int kStride = kForceTerms + 1;
@@ -402,46 +404,65 @@ force_over_kernel(const __grid_constant__ NearTree t, int n, const int* __restri
     double lx = 0, ly = 0, lz = 0;
     if (Periodic) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
     double* term = sTerm[wib];
+    const bool energy = lane == 6, largest = lane == 8;
+    const int first = lane < 6 ? kFix + lane : (lane == 6 ? kFpdv : (lane == 7 ? kFdiv : kFvs));
     unsigned long long pairs = 0;
     for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (gridDim.x * blockDim.x) >> 5)
     {
-        const int i = over[w];
+        const int i = Rows ? w : over[w];
+        const int cnt = Rows ? nblCount[i] : 0;
+        if (Rows && unsigned(cnt) > unsigned(kNbl)) continue;
         ForceAcc A;
         A.load(uint32_t(i), t.xyzh, vel4, thermo4, prepA, prepB);
-        const float x = float(A.p.x - f.cx), y = float(A.p.y - f.cy), z = float(A.p.z - f.cz);
-        const float slack = f.slack(x, y, z);
-        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * A.p.w) + slack;
-        double sum = 0.0;   // lanes 0-5: the pressure sums, 6: the energy, 7: div v, 8: vsig
-        near_blocks<0, Periodic, true>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
-            near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, [&](const double4& pj, int j, bool valid) {
-                double* mine = term + lane * kStride;
-                for (int k = 0; k < kForceTerms; ++k) mine[k] = 0.0;
-                const bool took = valid && A.terms<Periodic, Disc>(pj, j, vel4, thermo4, prepA, lx, ly, lz, pmass,
-                                                                   alphau, beta, pdv, shock,
-                                                                   [&](int k, double x) { mine[k] = x; });
-                uint32_t m = __ballot_sync(0xffffffffu, took);
-                A.gp += __popc(m);
-                __syncwarp();
-                for (; m; m &= m - 1)
-                {
-                    const double* q = term + (__ffs(m) - 1) * kStride;
-                    if (lane < 3) sum += q[lane];
-                    else if (lane < 6) sum -= q[lane];
-                    else if (lane == 6)
-                    {
-                        sum += q[kFpdv];
-                        sum += q[kFdiss];
-                        sum += q[kFcondi];
-                        sum += q[kFcondj];
-                    }
-                    else if (lane == 7) sum += q[kFdiv];
-                    else if (lane == 8) sum = fmax(sum, q[kFvs]);
-                }
-                __syncwarp();
-                return true;
+        // lanes 0-5: the pressure sums (the j side's terms stored negated), 6: the energy, 7:
+        // div v, 8: vsig.  Every lane runs the energy's four additions, zeros for the others
+        double sum = 0.0;
+        auto pair = [&](const double4& pj, int j, bool valid) {
+            double* mine = term + lane * kStride;
+#pragma unroll
+            for (int k = 0; k < kForceTerms; ++k) mine[k] = 0.0;
+            const bool took = valid && A.terms<Periodic, Disc>(pj, j, vel4, thermo4, prepA, lx, ly, lz, pmass, alphau,
+                                                               beta, pdv, shock,
+                                                               [&](int k, double x) {
+                                                                   mine[k] = k >= kFjx && k <= kFjz ? -x : x;
+                                                               });
+            A.gp += __popc(__ballot_sync(0xffffffffu, took));
+            __syncwarp();
+            const int c = 32 - __clz(__ballot_sync(0xffffffffu, valid));
+#pragma unroll 4
+            for (int k = 0; k < c; ++k)
+            {
+                const double* q = term + k * kStride;
+                const double x0 = q[first], x1 = energy ? q[kFdiss] : 0.0;
+                const double x2 = energy ? q[kFcondi] : 0.0, x3 = energy ? q[kFcondj] : 0.0;
+                sum = largest ? fmax(sum, x0) : sum + x0;
+                sum += x1;
+                sum += x2;
+                sum += x3;
+            }
+            __syncwarp();
+            return true;
+        };
+        if constexpr (Rows)
+        {
+            const int* row = row_of(nbl, uint32_t(i));
+            for (int k0 = 0; k0 < cnt; k0 += 32)
+            {
+                const bool valid = k0 + lane < cnt;
+                const int j = valid ? row[size_t(k0 + lane) * kRowStride] : i;
+                pair(ldg4(t.xyzh + j), j, valid);
+            }
+        }
+        else
+        {
+            const float x = float(A.p.x - f.cx), y = float(A.p.y - f.cy), z = float(A.p.z - f.cz);
+            const float slack = f.slack(x, y, z);
+            const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * A.p.w) + slack;
+            near_blocks<0, Periodic, true>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
+                near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, pair);
+                return r;
             });
-            return r;
-        });
+        }
         A.itx = __shfl_sync(0xffffffffu, sum, 0); A.ity = __shfl_sync(0xffffffffu, sum, 1);
         A.itz = __shfl_sync(0xffffffffu, sum, 2); A.jtx = __shfl_sync(0xffffffffu, sum, 3);
         A.jty = __shfl_sync(0xffffffffu, sum, 4); A.jtz = __shfl_sync(0xffffffffu, sum, 5);
@@ -540,9 +561,25 @@ void compute_forces(State& s, double pmass, double beta, double alphau, bool dis
         launch_force_mixed(s, pmass, beta, disc, pdv, shock);
     else if (nL > 0)
     {
-        if (s.periodic) { if (disc) launchRows(force_row_kernel<true, true>); else launchRows(force_row_kernel<true, false>); }
-        else { if (disc) launchRows(force_row_kernel<false, true>); else launchRows(force_row_kernel<false, false>); }
-        COSMO_LAUNCHED();
+        auto warps = [&](auto kern, int n, int blocks) {
+            kern<<<blocks, kThreads, 0, s.st>>>(
+                near_tree(s), n, s.nearOver.get(), s.nbl.get(), s.nblCount.get(), s.vel4.get(), s.thermo4.get(),
+                s.prepA.get(), s.prepB.get(), s.fx.get(), s.fy.get(), s.fz.get(), s.f4.get(), s.vsigmax.get(),
+                s.divvF.get(), pmass, alphau, beta, pdv ? 1 : 0, shock ? 1 : 0, ds);
+            COSMO_LAUNCHED();
+        };
+        if (s.nAlive <= kWarpPerParticleForce)
+        {
+            const int blocks = std::max(1, iceil(s.nAlive, kWarpsPerBlock));
+            if (s.periodic) { if (disc) warps(force_warp_kernel<true, true, true>, s.nAlive, blocks); else warps(force_warp_kernel<true, false, true>, s.nAlive, blocks); }
+            else { if (disc) warps(force_warp_kernel<false, true, true>, s.nAlive, blocks); else warps(force_warp_kernel<false, false, true>, s.nAlive, blocks); }
+        }
+        else
+        {
+            if (s.periodic) { if (disc) launchRows(force_row_kernel<true, true>); else launchRows(force_row_kernel<true, false>); }
+            else { if (disc) launchRows(force_row_kernel<false, true>); else launchRows(force_row_kernel<false, false>); }
+            COSMO_LAUNCHED();
+        }
         if (!s.rowsFromNewton)
         {
             // the group pass of the rows that overflowed (none: it returns at once)
@@ -555,15 +592,9 @@ void compute_forces(State& s, double pmass, double beta, double alphau, bool dis
             // the particles whose rows would not hold their pairs.  A node's h are those its
             // boxes were made with, at the solve's start: remade at the converged h first
             near_build(s);
-            auto go = [&](auto kern) {
-                kern<<<std::min(iceil(s.nearOverCount, kWarpsPerBlock), 8 * s.numSMs), kThreads, 0, s.st>>>(
-                    near_tree(s), s.nearOverCount, s.nearOver.get(), s.vel4.get(), s.thermo4.get(), s.prepA.get(),
-                    s.prepB.get(), s.fx.get(), s.fy.get(), s.fz.get(), s.f4.get(), s.vsigmax.get(), s.divvF.get(),
-                    pmass, alphau, beta, pdv ? 1 : 0, shock ? 1 : 0, ds);
-            };
-            if (s.periodic) { if (disc) go(force_over_kernel<true, true>); else go(force_over_kernel<true, false>); }
-            else { if (disc) go(force_over_kernel<false, true>); else go(force_over_kernel<false, false>); }
-            COSMO_LAUNCHED();
+            const int m = s.nearOverCount, blocks = std::min(iceil(m, kWarpsPerBlock), 8 * s.numSMs);
+            if (s.periodic) { if (disc) warps(force_warp_kernel<true, true, false>, m, blocks); else warps(force_warp_kernel<true, false, false>, m, blocks); }
+            else { if (disc) warps(force_warp_kernel<false, true, false>, m, blocks); else warps(force_warp_kernel<false, false, false>, m, blocks); }
         }
     }
     if (n > s.nAlive)

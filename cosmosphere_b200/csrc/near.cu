@@ -600,25 +600,56 @@ __device__ __forceinline__ int next_of(bool conv, double ho, double rowHi)
     return ho <= rowHi ? 0 : 1;
 }
 
-// One Newton iteration from the rows: one lane per particle streams its own row (8 bytes an
-// entry), tests every entry with the exact test and adds in the row's order.
-template<bool Forest>
+// W and -q dW/dq - 3W of m records of q^2, one per lane.
+__device__ __forceinline__ void eval_records(double2* rec, int m)
+{
+    for (int k = threadIdx.x & 31; k < m; k += 32)
+    {
+        const double q2 = rec[k].x;
+        const double q = sqrt(q2);
+        double wk, dwk;
+        sph_kernel(q2, q, wk, dwk);
+        rec[k] = make_double2(wk, -q * dwk - 3.0 * wk);
+    }
+}
+
+// The records' two components added to the two sums one by one (even lanes one sum, odd lanes
+// the other).
+__device__ __forceinline__ double2 serial_add(const double2* rec, int m, double2 s)
+{
+    const bool odd = threadIdx.x & 1;
+    const double* v = reinterpret_cast<const double*>(rec) + (odd ? 1 : 0);
+    double t = odd ? s.y : s.x;
+#pragma unroll 8
+    for (int k = 0; k < m; ++k) t += v[2 * k];
+    return make_double2(__shfl_sync(0xffffffffu, t, 0), __shfl_sync(0xffffffffu, t, 1));
+}
+
+// One Newton iteration from the rows.  Warp = false: one lane per particle streams its own row
+// (8 bytes an entry), tests every entry with the exact test and adds in the row's order.
+// Warp: one warp per particle (a small set), an entry per lane, the accepted values packed in
+// order and then added one by one.
+template<bool Forest, bool Warp>
 __global__ void __launch_bounds__(kThreads)
-near_step_kernel(const NearSet* __restrict__ sets, const int* __restrict__ setOf, NearLoop* __restrict__ L, const __grid_constant__ NearLists lists, const double* __restrict__ rowsR2,
+near_step_kernel(const NearSet* __restrict__ sets, const int* __restrict__ setOf, NearLoop* __restrict__ L,
+                 const __grid_constant__ NearLists lists, const double* __restrict__ rowsR2,
                  const int* __restrict__ nblCount, const double* __restrict__ rowH, double4* __restrict__ xyzh,
                  double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
                  double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
 {
     __shared__ int sh[3 * (kNearWarps + 1)];
     __shared__ unsigned long long shH[2];
+    __shared__ double2 sRec[Warp ? kNearWarps : 1][Warp ? kNbl : 1];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int cur = L->iter & 1, nxt = cur ^ 1;
     const int n = L->cnt[cur].row;
     if (n == 0) return;
     const int* list = lists.row[cur];
     unsigned long long pairs = 0, seen = 0, hconv = 0;
-    for (int b = blockIdx.x * kThreads; b < n; b += gridDim.x * kThreads)
+    const int perBlock = Warp ? kNearWarps : kThreads;
+    for (int b = blockIdx.x * perBlock; b < n; b += gridDim.x * perBlock)
     {
-        const int at = b + int(threadIdx.x);
+        const int at = b + (Warp ? wib : int(threadIdx.x));
         int to = -1;
         int i = 0;
         if (at < n)
@@ -629,33 +660,59 @@ near_step_kernel(const NearSet* __restrict__ sets, const int* __restrict__ setOf
             const double rh = rowH[i];
             double sr = 0.0, sg = 0.0;
             unsigned int gp = 0;
-            for_flat_row(row_flat(rowsR2, uint32_t(i)), nblCount[i], [&](double r2) {
-                const double q2 = r2 * hinv2;
-                if (!(q2 < kRadK2)) return;
-                ++gp;
-                const double q = sqrt(q2);
-                double wk, dwk;
-                sph_kernel(q2, q, wk, dwk);
-                sr += wk;
-                sg += -q * dwk - 3.0 * wk;
-            });
-            pairs += gp;
+            const double* row = row_flat(rowsR2, uint32_t(i));
+            const int cnt = nblCount[i];
+            if constexpr (Warp)
+            {
+                double2* rec = sRec[wib];
+                for (int k0 = 0; k0 < cnt; k0 += 32)
+                {
+                    const bool valid = k0 + lane < cnt;
+                    const double q2 = (valid ? row[k0 + lane] : 0.0) * hinv2;
+                    const bool acc = valid && q2 < kRadK2;
+                    const uint32_t m = __ballot_sync(0xffffffffu, acc);
+                    if (acc) rec[gp + __popc(m & ((1u << lane) - 1u))].x = q2;
+                    gp += __popc(m);
+                }
+                __syncwarp();
+                eval_records(rec, int(gp));
+                __syncwarp();
+                const double2 s = serial_add(rec, int(gp), make_double2(0.0, 0.0));
+                sr = s.x;
+                sg = s.y;
+            }
+            else
+                for_flat_row(row, cnt, [&](double r2) {
+                    const double q2 = r2 * hinv2;
+                    if (!(q2 < kRadK2)) return;
+                    ++gp;
+                    const double q = sqrt(q2);
+                    double wk, dwk;
+                    sph_kernel(q2, q, wk, dwk);
+                    sr += wk;
+                    sg += -q * dwk - 3.0 * wk;
+                });
             double ro, go, ho;
             int conv;
             newton_step(sr, sg, hi, Forest ? sets[setOf[i]].pmass : pmass, hfact, tolh, ro, go, ho, conv);
-            rho[i] = ro;
-            gradh[i] = go;
-            reinterpret_cast<double*>(xyzh + i)[3] = ho;
-            const unsigned long long hb = (unsigned long long)__double_as_longlong(hi);
-            const unsigned long long ob = (unsigned long long)__double_as_longlong(ho);
-            seen = hb > seen ? hb : seen;
-            if (conv)
+            if (!Warp || lane == 0)
             {
-                converged[i] = 1;
-                hs[i] = ho;
-                hconv = ob > hconv ? ob : hconv;
+                pairs += gp;
+                rho[i] = ro;
+                gradh[i] = go;
+                reinterpret_cast<double*>(xyzh + i)[3] = ho;
+                const unsigned long long hb = (unsigned long long)__double_as_longlong(hi);
+                const unsigned long long ob = (unsigned long long)__double_as_longlong(ho);
+                seen = hb > seen ? hb : seen;
+                if (conv)
+                {
+                    converged[i] = 1;
+                    hs[i] = ho;
+                    hconv = ob > hconv ? ob : hconv;
+                }
+                to = next_of(conv != 0, ho, rh);
             }
-            to = next_of(conv != 0, ho, rh);
+            if (Warp) __syncwarp();
         }
         block_append(to, i, lists.row[nxt], &L->cnt[nxt].row, lists.build[nxt], &L->cnt[nxt].build, lists.cover,
                      &L->cover, sh);
@@ -663,7 +720,7 @@ near_step_kernel(const NearSet* __restrict__ sets, const int* __restrict__ setOf
     note_h(seen, hconv, ds, shH);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
+    if (lane == 0 && pairs) atomicAdd(&ds->pairs[0], pairs);
 }
 
 // rho and d(rho)/dh at h from the un-normalised sums (src/density_base.cu:635-643).
@@ -791,27 +848,8 @@ __device__ __forceinline__ double2 ordered_add(const double2* rec, int m, double
         if (g.ok && bg.holds(g.up, g.down)) { s.y = bg.sign * ((bg.a + g.up) - g.down); doneG = true; }
         if (doneW && doneG) return s;
     }
-    const bool odd = threadIdx.x & 1;
-    const double* v = reinterpret_cast<const double*>(rec) + (odd ? 1 : 0);
-    double t = odd ? s.y : s.x;
-#pragma unroll 8
-    for (int k = 0; k < m; ++k) t += v[2 * k];
-    const double tw = __shfl_sync(0xffffffffu, t, 0), tg = __shfl_sync(0xffffffffu, t, 1);
-    if (!doneW) s.x = tw;
-    if (!doneG) s.y = tg;
-    return s;
-}
-
-__device__ __forceinline__ void eval_records(double2* rec, int m)
-{
-    for (int k = threadIdx.x & 31; k < m; k += 32)
-    {
-        const double q2 = rec[k].x;
-        const double q = sqrt(q2);
-        double wk, dwk;
-        sph_kernel(q2, q, wk, dwk);
-        rec[k] = make_double2(wk, -q * dwk - 3.0 * wk);
-    }
+    const double2 one = serial_add(rec, m, s);
+    return make_double2(doneW ? s.x : one.x, doneG ? s.y : one.y);
 }
 
 // m records of q^2 evaluated and added to the sums in order.
@@ -1207,8 +1245,10 @@ static void near_iteration(State& s, const NearJob& j, cudaGraphConditionalHandl
                                                                       j.rowsJ, s.nblCount.get(), s.nblH.get(), 0,
                                                                       std::min(s.numSMs, kNearQueues));
     COSMO_LAUNCHED();
-    auto step = j.sets ? near_step_kernel<true> : near_step_kernel<false>;
-    step<<<iceil(j.n, kThreads), kThreads, 0, s.st>>>(j.sets, j.setOf, L, lists, s.nblR2.get(), s.nblCount.get(),
+    const bool warp = j.n <= kWarpPerParticle;
+    auto step = j.sets ? (warp ? near_step_kernel<true, true> : near_step_kernel<true, false>)
+                       : (warp ? near_step_kernel<false, true> : near_step_kernel<false, false>);
+    step<<<iceil(j.n, warp ? kNearWarps : kThreads), kThreads, 0, s.st>>>(j.sets, j.setOf, L, lists, s.nblR2.get(), s.nblCount.get(),
                                                       s.nblH.get(), j.xyzh, j.rho, j.gradh, j.converged, s.hs.get(),
                                                       j.pmass, j.tolh, j.hfact, ds);
     COSMO_LAUNCHED();

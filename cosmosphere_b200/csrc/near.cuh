@@ -33,6 +33,14 @@ constexpr int kNearLevels = 9;     // level 0: blocks of 8 particles; 32 * 8^9 p
 constexpr int kNearBlocks = 128;   // blocks a warp holds at once
 constexpr int kNearWarps  = 4;     // warps per block of the search kernels
 
+// Up to this many particles a pass over rows gives each particle a warp: one lane each would
+// leave most of the chip idle and last as long as the longest row.  648 particles: Newton step
+// 33 -> 9 us an iteration, gradient 54 -> 16, force 66 -> 17; 20,000: gradient 82 -> 65, force
+// 93 -> 115 (its energy sum is four dependent additions a pair), so its line lies lower;
+// 120,000: gradient 181 -> 337.
+constexpr int kWarpPerParticle = 32768;
+constexpr int kWarpPerParticleForce = 12288;
+
 // A node's box: centre, half extents (empty: negative infinity) and its largest h.
 struct alignas(32) NearNode
 {
