@@ -597,6 +597,7 @@ void densityiterate_gpu_c(int n, double pmass, int periodic, const double* box, 
     static const bool stats = env_on("COSMO_DENS_STATS");
     if (stats)
     {
+        ensure_tree(s);   // its leaf count is printed
         const Timings& t = s.t;
         const double gpu = 1e3 * (t.bbox + t.keysSort + t.tree + t.nodes + t.jbuild + t.nrkern + t.gjbuild + t.gradkern);
         auto ms = [](clk::time_point a, clk::time_point b) {
@@ -632,6 +633,7 @@ void force_gpu_c(int n, double pmass, double beta, double alphau, int disc_visco
     if (stats)
     {
         const double wall = std::chrono::duration<double, std::milli>(clk::now() - t0).count();
+        ensure_tree(s);
         const Timings& t = s.t;
         // upload= and download= are the transfers inside the call (src/force_c_api.cu:74-79):
         // the caller moves THERMO, VEL and FORCE_OUT with cosmo_upload_sorted / cosmo_download,
@@ -794,7 +796,9 @@ int cosmo_x_set_frozen(const int* mask, int n)
 int cosmo_x_refresh_h(void)
 {
     State& s = state();
-    if (!s.st || s.nLeaves <= 0 || s.orderFor != s.ngas) return -1;
+    if (!s.st || s.ngas <= 0 || s.orderFor != s.ngas) return -1;
+    ensure_tree(s);
+    if (s.nLeaves <= 0) return -1;
     hmax_leaves(s, s.allLeaves.get(), s.nLeaves);
     s.jlistToken = s.rowsToken = 0;
     COSMO_CUDA(cudaStreamSynchronize(s.st));
@@ -847,6 +851,7 @@ double cosmo_x_scalar(const char* name)
     State& s = state();
     const std::string k(name);
     if (k == "nAlive") return s.nAlive;
+    if (k == "nLeaves" || k == "numNodes") ensure_tree(s);
     if (k == "nLeaves") return s.nLeaves;
     if (k == "numNodes") return s.numNodes;
     if (k == "itersRun") return s.itersRun;
@@ -858,7 +863,7 @@ double cosmo_x_scalar(const char* name)
     if (k == "hmaxSeen" && s.hscal)
     {
         read_scalars(s);
-        const unsigned long long b = s.hscal->hmaxSeen;
+        const unsigned long long b = std::max(s.hscal->hmaxSeen, s.hscal->hmaxConv);
         double v;
         std::memcpy(&v, &b, sizeof v);
         return v;
@@ -917,6 +922,10 @@ long cosmo_x_array(const char* name, void* out, int* dtype)
         }
         return long(cnt);
     };
+    for (const char* t : {"particleLeaf", "csTree", "counts", "layout", "prefixes", "childOffsets", "internalToLeaf",
+                          "levelRange", "leafToInternal", "centers", "sizes", "hmax_leaf", "hmax_node", "jcount",
+                          "jOffset", "jlist"})
+        if (k == t) ensure_tree(s);
     const size_t n = size_t(s.ngas), nL = size_t(s.nLeaves), nN = size_t(s.numNodes);
     if (k == "x") return put(s.xyzh.get(), n, 8, 0, 4, 0);
     if (k == "y") return put(s.xyzh.get(), n, 8, 0, 4, 1);
@@ -1049,6 +1058,7 @@ DensTimings solveDensH(int n, double pmass, KernelMode mode, bool withGradients,
     t.download = s.downloadSeconds;
     s.downloadSeconds = 0.0;
     t.itersRun = r.itersRun;
+    ensure_tree(s);
     t.nLeavesOut = s.nLeaves;
     return t;
 }

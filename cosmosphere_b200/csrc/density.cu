@@ -166,6 +166,7 @@ gradient_row_kernel(int nAlive, const int* __restrict__ nbl, const int* __restri
                     const int* __restrict__ active)
 {
     if (active != nullptr && *active > 0) return;   // the Newton loop did not converge
+    nAlive = min(nAlive, ds->nAlive);
     double lx = 0, ly = 0, lz = 0;
     if (Periodic) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
     unsigned long long pairs = 0;
@@ -215,7 +216,7 @@ gradient_warp_kernel(const __grid_constant__ NearTree t, const NearLoop* __restr
     __shared__ double sTerm[kWarpsPerBlock][32 * kGradTerms];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (L != nullptr && L->active > 0) return;   // the Newton loop did not converge
-    const int n = Rows ? nAlive : L->over;
+    const int n = Rows ? min(nAlive, ds->nAlive) : L->over;
     if (n == 0) return;
     if (!Rows && blockIdx.x == 0 && threadIdx.x == 0) ds->rowOverflow = 1;
     const NearFrame f(t.box);
@@ -428,10 +429,10 @@ gradient_kernel(int nL, const uint32_t* __restrict__ layout, const uint32_t* __r
 }
 
 // Dead particles (h <= 0) sit after nAlive: div v = d(div v)/dt = 0, xi = 1.
-__global__ void gradient_dead_kernel(int nAlive, int n, double* __restrict__ divv, double* __restrict__ xiOut,
-                                     double* __restrict__ ddivvdt)
+__global__ void gradient_dead_kernel(int n, double* __restrict__ divv, double* __restrict__ xiOut,
+                                     double* __restrict__ ddivvdt, const DevScalars* __restrict__ ds)
 {
-    const long i = nAlive + long(blockIdx.x) * blockDim.x + threadIdx.x;
+    const long i = ds->nAlive + long(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     divv[i] = 0.0; ddivvdt[i] = 0.0; xiOut[i] = 1.0;
 }
@@ -529,6 +530,7 @@ sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restr
     double lx = 0, ly = 0, lz = 0;
     if (Periodic && !kExact) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
     int added = 0;
+    nAlive = min(nAlive, ds->nAlive);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nAlive; i += gridDim.x * blockDim.x)
     {
         const int cnt = nblCount[i];
@@ -605,6 +607,7 @@ sym_from_rows_warp_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __
     if (Periodic && !kExact) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
     const int lane = threadIdx.x & 31;
     int added = 0;
+    nAlive = min(nAlive, ds->nAlive);
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nAlive; i += (gridDim.x * blockDim.x) >> 5)
     {
         const int cnt = nblCount[i];
@@ -660,6 +663,7 @@ extras_merge_kernel(int nA, const int* __restrict__ extraCnt, const int* __restr
     constexpr int kPer = kExtra / 32, kRowPer = kNbl / 32;
     const int lane = threadIdx.x & 31;
     const int t0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
+    nA = min(nA, ds->nAlive);
     const int mineE = t0 + lane < nA ? extraCnt[t0 + lane] : 0;
     const int mineCnt = mineE > 0 ? nblCount[t0 + lane] : 0;
     for (uint32_t rest = __ballot_sync(0xffffffffu, mineE > 0 && unsigned(mineCnt) <= unsigned(kNbl)); rest;
@@ -1234,15 +1238,30 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
 
     // the tree; its particle gather also zeroes rho, gradh, the convergence flags, the
     // Newton rows' h (0: no row this solve) and the pair counters
-    build_tree(s, periodicBox, withGradients, writeJ);
+    build_order(s, periodicBox, withGradients, writeJ);
     s.orderFor = n;
-    const int nL = s.nLeaves;
-    s.activeA.resize(nL, s.st);
-    s.activeB.resize(nL, s.st);
-    s.leafNext.resize(nL, s.st);
+    if (!near) build_leaves(s);
+    const int nL = near ? 0 : s.nLeaves;
+    // The block-tree solve reads nothing back before its end when the set is small: its
+    // launches cover all n particles and its kernels read how many are live.  Above
+    // kReadAlive the count is read (12 us of a solve of milliseconds), so that the rows,
+    // 2 KB a particle, are sized by the live particles only.
+    constexpr int kReadAlive = 1 << 17;
+    if (near)
+    {
+        s.nAlive = n;
+        if (n > kReadAlive)
+        {
+            read_scalars(s);
+            s.nAlive = s.hscal->nAlive;
+        }
+    }
     const int itemCap = std::max(s.nAlive, 1);
     if (!near)
     {
+        s.activeA.resize(nL, s.st);
+        s.activeB.resize(nL, s.st);
+        s.leafNext.resize(nL, s.st);
         s.items.resize(itemCap, s.st);
         s.rowItems.resize(itemCap, s.st);
     }
@@ -1437,12 +1456,17 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     bool symBuilt = false, fromRows = false;
     if (withGradients)
     {
-        // hmax of every leaf at the converged h; then the symmetric rows of the gradient
-        // and force passes (at the converged h they hold every pair of the gather sweep
-        // too): taken from the Newton rows when every live particle's row covers its
-        // converged h, otherwise built from the symmetric lists
+        // hmax of every leaf at the converged h (the list-based loop's; the block-tree loop
+        // walks no leaves); then the symmetric rows of the gradient and force passes (at
+        // the converged h they hold every pair of the gather sweep too): taken from the
+        // Newton rows when every live particle's row covers its converged h, otherwise
+        // built from the symmetric lists
         cudaEvent_t g0 = ev(s);
-        hmax_leaves(s, s.allLeaves.get(), nL);
+        if (!near)
+        {
+            hmax_leaves(s, s.allLeaves.get(), nL);
+            s.hmaxLeafDone = true;
+        }
         const bool rowsBuilt = graphRan ? s.lastLoopRowBuilds > 0 : rowsReady;
         // the block-tree loop's rows cover every particle but those it lists (over)
         if (near && writeJ && s.nAlive > 0)
@@ -1457,11 +1481,16 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             sym_rows_from_newton(s, near);
         else
         {
+            if (near)
+            {
+                read_scalars(s);
+                s.nAlive = s.hscal->nAlive;
+            }
             build_symmetric(s);
             symBuilt = true;
         }
         cudaEvent_t g1 = ev(s);
-        const int grid = grid_for(s, nL);
+        const int grid = grid_for(s, s.treeDone ? s.nLeaves : 0);
         if (s.precision == 1)
             launch_gradient_mixed(s, pmass);
         else
@@ -1488,16 +1517,15 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
                 warps(s.periodic ? gradient_warp_kernel<true, false> : gradient_warp_kernel<false, false>, 2 * s.numSMs);
             // the group sweep of the rows that overflowed (none: it returns at once)
             auto gk = s.periodic ? gradient_kernel<true> : gradient_kernel<false>;
-            if (!(near && fromRows)) gk<<<grid, kThreads, 0, s.st>>>(nL, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),
+            if (!(near && fromRows)) gk<<<grid, kThreads, 0, s.st>>>(s.nLeaves, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),
                                             s.xyzh.get(), s.vel4.get(), s.acc4.get(), s.rho.get(), s.gradh.get(),
                                             s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(),
                                             s.nblCount.get(), ds);
             if (!(near && fromRows)) COSMO_LAUNCHED();
         }
-        if (n > s.nAlive)
+        if (near || n > s.nAlive)
         {
-            gradient_dead_kernel<<<iceil(n - s.nAlive, 256), 256, 0, s.st>>>(s.nAlive, n, s.divv.get(), s.xi.get(),
-                                                                             s.ddivvdt.get());
+            gradient_dead_kernel<<<iceil(n, 256), 256, 0, s.st>>>(n, s.divv.get(), s.xi.get(), s.ddivvdt.get(), ds);
             COSMO_LAUNCHED();
         }
         cudaEvent_t g2 = ev(s);
@@ -1509,6 +1537,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         {
             check_dev_err(s, "solveDensH", false);
             tree_timings(s);
+            s.nAlive = s.hscal->nAlive;
             nActiveParticles = near_results(s, nl);
             s.nearOverCount = nl.over;
             s.t.nrkern += elapsed_s(n0, e3);

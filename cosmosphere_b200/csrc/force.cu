@@ -492,6 +492,7 @@ __global__ void force_dead_kernel(int nAlive, int n, double* fx, double* fy, dou
 void build_symmetric(State& s)
 {
     DevScalars* ds = s.dscal.get();
+    ensure_tree(s);
     const int nL = s.nLeaves;
     hmax_upsweep(s);
     build_lists(s, true);
@@ -523,7 +524,12 @@ void compute_forces(State& s, double pmass, double beta, double alphau, bool dis
     // The symmetric lists and rows are cached per tree (src/force.cu:19-24); the density
     // solve's gradient sweep has normally built the rows already (from the Newton rows, or
     // with the symmetric lists).
-    const bool rowsReady = s.rowsToken == s.token && (s.rowsFromNewton || (s.jlistToken == s.token && s.listsSym));
+    // After a plain solve the mixed pass still goes over the leaves, and it has no walk for
+    // particles without a row: they need the lists.
+    if (s.precision == 1) ensure_tree(s);
+    const bool noRow = s.precision == 1 && s.nearOverCount > 0;
+    const bool rowsReady =
+        s.rowsToken == s.token && ((s.rowsFromNewton && !noRow) || (s.jlistToken == s.token && s.listsSym));
     if (!rowsReady)
     {
         build_symmetric(s);
@@ -540,7 +546,7 @@ void compute_forces(State& s, double pmass, double beta, double alphau, bool dis
                                                        s.vel4.get(), ds);
     COSMO_LAUNCHED();
     cudaEvent_t p1 = ev(s);
-    const int nL = s.nLeaves;
+    const int nL = s.treeDone ? s.nLeaves : 0;   // the group pass's (no tree: no such pass)
     const int grid = std::max(1, std::min(s.numSMs * 8, iceil(nL, kWarpsPerBlock)));
     auto launch = [&](auto kern) {
         kern<<<grid, kThreads, 0, s.st>>>(nL, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),
@@ -559,7 +565,7 @@ void compute_forces(State& s, double pmass, double beta, double alphau, bool dis
     // that overflowed
     if (s.precision == 1)
         launch_force_mixed(s, pmass, beta, disc, pdv, shock);
-    else if (nL > 0)
+    else if (s.nAlive > 0)
     {
         auto warps = [&](auto kern, int n, int blocks) {
             kern<<<blocks, kThreads, 0, s.st>>>(

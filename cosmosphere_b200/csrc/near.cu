@@ -269,7 +269,6 @@ __global__ void near_init_kernel(NearLoop* L, DevScalars* ds, int maxIter, int f
     ds->extraCount = 0;
     ds->mergeOverflow = 0;
     ds->rowOverflow = 0;
-    ds->hmaxConv = 0;
 }
 
 // The initial search list with fixed particles (the caller's mask through the sort order;
@@ -1358,7 +1357,7 @@ static bool near_graph(State& s, const NearJob& j, int maxIter, bool defer)
 static void near_run(State& s, const NearJob& j, int maxIter, bool graph, bool defer)
 {
     s.lastLoopGraph = 0;
-    if (graph && maxIter <= kLoopIters && near_graph(s, j, maxIter, defer))
+    if (graph && maxIter > 0 && maxIter <= kLoopIters && near_graph(s, j, maxIter, defer))
     {
         s.lastLoopGraph = 1;
         return;
@@ -1381,7 +1380,7 @@ void near_newton(State& s, double pmass, double tolh, double hfact, int maxIter,
     DevScalars* ds = s.dscal.get();
     near_buffers(s, n);
     near_build(s);
-    const bool frozen = s.frozenFor == s.ngas && s.nAlive > 0;
+    const bool frozen = s.frozenFor == s.ngas;
     near_init_kernel<<<1, kNearQueues, 0, s.st>>>(s.nearLoop.get(), ds, maxIter, frozen ? 1 : 0);
     COSMO_LAUNCHED();
     if (frozen)
@@ -1395,7 +1394,7 @@ void near_newton(State& s, double pmass, double tolh, double hfact, int maxIter,
     }
     const NearJob j{near_tree(s), nullptr, nullptr, s.xyzh.get(), s.rho.get(), s.gradh.get(), s.converged.get(), rowsJ,
                     n, s.periodic, pmass, tolh, hfact};
-    near_run(s, j, maxIter, allowGraph && s.newtonGraph && s.nAlive > 0, true);
+    near_run(s, j, maxIter, allowGraph && s.newtonGraph, true);
 }
 
 // After the loop: rows at the converged h of the particles whose rows do not cover it.

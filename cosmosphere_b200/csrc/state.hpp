@@ -175,6 +175,7 @@ struct State
     bool listsSym = false;                      // the lists held are the symmetric ones
     bool listsLoose = false;                    // the lists held are the Newton loop's widened ones
     bool forceSinceSolve = false;               // a force pass ran on the current tree
+    bool treeDone = false, hmaxLeafDone = false;   // the leaf tree and hmax of its leaves are the last solve's
     // The symmetric rows of the current tree come from the Newton rows (their j, with the
     // pairs another particle's support adds merged in): the symmetric lists and hmax per
     // node were not built, and are built only if asked for (hmaxNodeDone once done).
@@ -317,7 +318,9 @@ size_t state_device_bytes(const State& s);
 void size_particle_arrays(State& s, int n);
 
 // tree.cu
-void build_tree(State& s, const double* periodicBox, bool alsoSortVA, bool rowsJOn = false);
+void build_order(State& s, const double* periodicBox, bool alsoSortVA, bool rowsJOn = false);
+void build_leaves(State& s);
+void ensure_tree(State& s);   // the tree and hmax of its leaves, if the last solve made none
 void tree_timings(State& s);   // the last tree build's stage times, once its marks have passed
 // hmax of the leaves [0, nLeavesActive) of leaves, or of the first *countPtr of them when
 // countPtr is given (a count on the device; nLeavesActive then bounds it).

@@ -162,6 +162,7 @@ __global__ void gather_particles_kernel(const int* __restrict__ order, int n,
     {
         for (int p = 0; p < 4; ++p) r.ds->pairs[p] = 0;
         r.ds->hmaxSeen = 0;
+        r.ds->hmaxConv = 0;
         r.ds->rowsJOn = r.rowsJOn;
     }
     if (k >= n) return;
@@ -798,7 +799,7 @@ void radix_sort_u64(State& s, uint64_t* kA, uint64_t* kB, int* vA, int* vB, int 
 // ---------------------------------------------------------------------------------------
 // Hilbert keys and their stable sort with every buffer supplied by the caller (used by
 // the allocation-free entry point in noalloc.cu).  Same kernels and launch sequence as
-// build_tree's keys + radix_sort_u64; scratch is carved as laid out below.
+// build_order's keys + radix_sort_u64; scratch is carved as laid out below.
 // ---------------------------------------------------------------------------------------
 namespace {
 constexpr size_t kAlign = 256;
@@ -873,9 +874,11 @@ int keysort_raw(int n, const double* x, const double* y, const double* z, const 
     return e ? -3 : 0;
 }
 
-void build_tree(State& s, const double* periodicBox, bool alsoSortVA, bool rowsJOn)
+// The box, the keys, their sort and the gather of the particles.
+void build_order(State& s, const double* periodicBox, bool alsoSortVA, bool rowsJOn)
 {
     const int n = s.ngas;
+    s.treeDone = s.hmaxLeafDone = false;
     DevScalars* ds = s.dscal.get();
     cudaEvent_t e0 = ev(s);
 
@@ -921,7 +924,17 @@ void build_tree(State& s, const double* periodicBox, bool alsoSortVA, bool rowsJ
         SolveReset{s.rho.get(), s.gradh.get(), s.converged.get(), s.nblH.get(), ds, rowsJOn ? 1 : 0});
     COSMO_LAUNCHED();
     cudaEvent_t e2 = ev(s);
+    // the stage times are taken once the stream has been read again (tree_timings)
+    const cudaEvent_t marks[5] = {e0, e1, e2, e2, e2};
+    std::copy(marks, marks + 5, s.treeEv);
+}
 
+// The leaf tree and the linked octree of the sorted particles.
+void build_leaves(State& s)
+{
+    const int n = s.ngas;
+    DevScalars* ds = s.dscal.get();
+    cudaEvent_t e2 = ev(s);
     // cornerstone leaf tree (src/tree.cu:126-136): the refinement from the root, started at
     // the complete grid of the level above which every node splits
     s.csTree.resize((size_t(1) << (3 * kStartLevels + 3)) + 1, s.st);
@@ -1003,9 +1016,26 @@ void build_tree(State& s, const double* periodicBox, bool alsoSortVA, bool rowsJ
     iota_kernel<<<iceil(nL, kBlk), kBlk, 0, s.st>>>(s.allLeaves.get(), nL);
     COSMO_LAUNCHED();
     cudaEvent_t e4 = ev(s);
-    // the stage times are taken once the stream has been read again (tree_timings)
-    const cudaEvent_t marks[5] = {e0, e1, e2, e3, e4};
-    std::copy(marks, marks + 5, s.treeEv);
+    if (s.treeEv[4])
+    {
+        s.treeEv[2] = e2;
+        s.treeEv[3] = e3;
+        s.treeEv[4] = e4;
+    }
+    s.treeDone = true;
+}
+
+// The tree and hmax of its leaves, where the solve did not need them: the plain solve over
+// the block tree walks neither (they take 0.15 ms of a lattice-100 step, 0.4 ms and eight
+// host round trips of a 120,000-particle Plummer step), so they are made for the lists a
+// caller reads, for the fallback that walks them, and for their counts.
+void ensure_tree(State& s)
+{
+    if (s.treeDone || s.ngas <= 0 || s.orderFor != s.ngas) return;
+    build_leaves(s);
+    if (!s.hmaxLeafDone) hmax_leaves(s, s.allLeaves.get(), s.nLeaves);
+    s.hmaxLeafDone = true;
+    COSMO_CUDA(cudaStreamSynchronize(s.st));
 }
 
 void tree_timings(State& s)
