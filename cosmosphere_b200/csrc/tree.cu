@@ -766,9 +766,53 @@ static void sort_nodes_by_level(State& s, int n)
     COSMO_LAUNCHED();
 }
 
+namespace {
+// How many pairs a thread the one-kernel sort takes on n pairs (0: more than its blocks'
+// shared memory holds, 2.4 million on 148 multiprocessors; the onesweep passes sort those).
+int block_sort_ipt(int n, int numSMs)
+{
+    const int ipt = std::max(1, int((long(n) + long(numSMs) * kBsThreads - 1) / (long(numSMs) * kBsThreads)));
+    return ipt <= kBsMaxIpt ? ipt : 0;
+}
+
+size_t block_sort_words(int n, int ipt) { return size_t(iceil(n, kBsThreads * ipt)) * 256 + 16; }
+
+cudaError_t block_sort(uint64_t* kA, uint64_t* kB, int* vA, int* vB, int n, int ipt, bool iotaValues,
+                       uint32_t* table, int* err, cudaStream_t st)
+{
+    const int blocks = iceil(n, kBsThreads * ipt);
+    const size_t smem = block_sort_smem(ipt);
+    cudaError_t e = cudaMemsetAsync(table, 0, block_sort_words(n, ipt) * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    auto kern = ipt <= 4 ? block_sort_kernel<4> : ipt <= 8 ? block_sort_kernel<8> : block_sort_kernel<16>;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(block_sort_smem(ipt <= 4 ? 4 : ipt <= 8 ? 8 : kBsMaxIpt)));
+    if (e != cudaSuccess) return e;
+    unsigned int* arrived = table + size_t(blocks) * 256;
+    int iota = iotaValues ? 1 : 0;
+    long long waitNs = wait_limit_ns();
+    void* args[] = {&kA, &kB, &vA, &vB, &n, &ipt, &iota, &table, &arrived, &err, &waitNs};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kern), dim3(blocks), dim3(kBsThreads), args, smem, st);
+}
+} // namespace
+
 void radix_sort_u64(State& s, uint64_t* kA, uint64_t* kB, int* vA, int* vB, int n, bool iotaValues)
 {
     if (n <= 0) return;
+    if (const int ipt = block_sort_ipt(n, s.numSMs))
+    {
+        s.sortLookback.resize(block_sort_words(n, ipt), s.st);
+        const cudaError_t e =
+            block_sort(kA, kB, vA, vB, n, ipt, iotaValues, s.sortLookback.get(), &s.dscal.get()->err, s.st);
+        if (e == cudaSuccess)
+        {
+            COSMO_LAUNCHED();
+            return;
+        }
+        // a context that owns fewer multiprocessors than the device has: the passes sort
+        if (e != cudaErrorCooperativeLaunchTooLarge) COSMO_CUDA(e);
+        (void)cudaGetLastError();
+    }
     const int tiles = iceil(n, kSortTile);
     s.sortHist.resize(kSortPasses * 256, s.st);
     s.sortBase.resize(kSortPasses * 256, s.st);
@@ -840,10 +884,7 @@ int keysort_raw(int n, const double* x, const double* y, const double* z, const 
     int* vB = reinterpret_cast<int*>(take(size_t(n) * sizeof(int)));
 
     // The array keeps the previous call's contents: clear what must start at zero.
-    if (cudaMemsetAsync(hist, 0, kSortPasses * 256 * sizeof(uint32_t), st) != cudaSuccess) return -2;
     if (cudaMemsetAsync(tickets, 0, 16 * sizeof(unsigned int) + sizeof(int), st) != cudaSuccess) return -2;
-    if (cudaMemsetAsync(lookback, 0, size_t(kSortPasses) * tiles * 256 * sizeof(uint32_t), st) != cudaSuccess)
-        return -2;
     if (periodicBox)
         set_box_kernel<<<1, 32, 0, st>>>(periodicBox[0], periodicBox[1], periodicBox[2], periodicBox[3],
                                          periodicBox[4], periodicBox[5], box);
@@ -854,18 +895,30 @@ int keysort_raw(int n, const double* x, const double* y, const double* z, const 
         bbox_final_kernel<<<1, 32, 0, st>>>(part, nb, box);
     }
     keys_kernel<<<iceil(n, kBlk), kBlk, 0, st>>>(x, y, z, h, n, box, keysOut);
-    digit_hist_kernel<<<std::min(iceil(n, kBlk), 4 * numSMs), kBlk, 0, st>>>(keysOut, n, hist);
-    digit_base_kernel<<<kSortPasses, 256, 0, st>>>(hist, base);
-    uint64_t* ki = keysOut; uint64_t* ko = kB;
-    int* vi = nullptr; int* vo = vB;
-    for (int pass = 0; pass < kSortPasses; ++pass)
+    // the one-kernel sort's table (256 words per 1024 pairs at most) fits in the look-back
+    // words (2048 per 4096 pairs)
+    const int ipt = block_sort_ipt(n, numSMs);
+    const cudaError_t one =
+        ipt ? block_sort(keysOut, kB, orderOut, vB, n, ipt, true, lookback, err, st) : cudaErrorCooperativeLaunchTooLarge;
+    if (one == cudaErrorCooperativeLaunchTooLarge)
     {
-        onesweep_kernel<<<tiles, kSortThreads, 0, st>>>(ki, vi, ko, vo, n, 8 * pass, base + 256 * pass,
-                                                        lookback + size_t(pass) * tiles * 256, &tickets[pass], err,
-                                                        wait_limit_ns());
-        std::swap(ki, ko);
-        vi = vo;
-        vo = (vo == vB) ? orderOut : vB;
+        (void)cudaGetLastError();
+        if (cudaMemsetAsync(hist, 0, kSortPasses * 256 * sizeof(uint32_t), st) != cudaSuccess) return -2;
+        if (cudaMemsetAsync(lookback, 0, size_t(kSortPasses) * tiles * 256 * sizeof(uint32_t), st) != cudaSuccess)
+            return -2;
+        digit_hist_kernel<<<std::min(iceil(n, kBlk), 4 * numSMs), kBlk, 0, st>>>(keysOut, n, hist);
+        digit_base_kernel<<<kSortPasses, 256, 0, st>>>(hist, base);
+        uint64_t* ki = keysOut; uint64_t* ko = kB;
+        int* vi = nullptr; int* vo = vB;
+        for (int pass = 0; pass < kSortPasses; ++pass)
+        {
+            onesweep_kernel<<<tiles, kSortThreads, 0, st>>>(ki, vi, ko, vo, n, 8 * pass, base + 256 * pass,
+                                                            lookback + size_t(pass) * tiles * 256, &tickets[pass],
+                                                            err, wait_limit_ns());
+            std::swap(ki, ko);
+            vi = vo;
+            vo = (vo == vB) ? orderOut : vB;
+        }
     }
     if (cudaGetLastError() != cudaSuccess) return -2;
     int e = 0;
