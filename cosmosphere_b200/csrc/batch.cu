@@ -54,6 +54,7 @@ struct Batch
     DBuf<int4> items;                 // Newton work items (leaf, window|group|G, m0, m1)
     DBuf<int> leafNext;               // leaf already queued for the next iteration
     DBuf<uint2> leafRange;
+    DBuf<float4> leafBox;                       // the leaves' bounding boxes (leaf_box)
     DBuf<DevBox> boxes;
     DBuf<LoopState> loop;
     uint32_t listCap = 0;
@@ -358,6 +359,13 @@ __global__ void hmax_leaf_kernel_b(const double4* __restrict__ xyzh, const uint2
     hmax[l] = hm;
 }
 
+__global__ void leaf_box_kernel_b(const uint2* __restrict__ range, int L, const double4* __restrict__ xyzh,
+                                  float4* __restrict__ leafBox)
+{
+    const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l < L) leaf_box(xyzh, range[l].x, range[l].y, leafBox + 2 * size_t(l));
+}
+
 // Gather walk of one i-leaf over its own set's pre-order nodes (the single-set walk's
 // window scan, include/tree.cuh:228-389 accept test).
 template<bool Fill>
@@ -463,38 +471,28 @@ list_walk_kernel_b(const int* __restrict__ leaves, const int* __restrict__ count
             skip = preSkip[idx];
             pl = preLeaf[idx];
         }
-        const uint32_t validMask = __ballot_sync(0xffffffffu, valid);
-        const uint32_t rejMask = __ballot_sync(0xffffffffu, valid && !accept);
-        int pos = 0;
-        int next = p + 32;
-        for (;;)
+        // reached: beyond every earlier rejected node's subtree (list_walk_kernel)
+        const int end = valid && !accept ? lane + max(skip, 1) : 0;
+        const int reach = warp_prefix_max(end);
+        const int before = __shfl_up_sync(0xffffffffu, reach, 1);
+        const bool emit = accept && pl >= 0 && (lane == 0 || before <= lane);
+        const uint32_t emitMask = __ballot_sync(0xffffffffu, emit);
+        if (emit)
         {
-            const uint32_t fromPos = (pos >= 32) ? 0u : (0xffffffffu << pos);
-            const uint32_t rej = rejMask & fromPos;
-            const int r = rej ? (__ffs(rej) - 1) : 32;
-            const uint32_t runMask = validMask & fromPos & ((r >= 32) ? 0xffffffffu : ((1u << r) - 1u));
-            const uint32_t emitMask = __ballot_sync(0xffffffffu, ((runMask >> lane) & 1u) && pl >= 0);
-            if (Fill && ((emitMask >> lane) & 1u))
+            const uint32_t slot = count + __popc(emitMask & lt);
+            if (Fill)
             {
-                const uint32_t slot = count + __popc(emitMask & lt);
                 if (slot < cap) jlist[base + slot] = pl;
                 else atomicOr(err, int(kErrListCap));
             }
-            if (!Fill && ((emitMask >> lane) & 1u))
+            else
             {
                 stream += range[pl].y - range[pl].x;
-                const uint32_t slot = count + __popc(emitMask & lt);
                 if (slot < uint32_t(kWalkScratchB)) scratch[size_t(leaf) * kWalkScratchB + slot] = pl;
             }
-            count += __popc(emitMask);
-            if (r >= 32) { next = p + 32; break; }
-            int rskip = __shfl_sync(0xffffffffu, skip, r);
-            if (rskip < 1) rskip = 1;
-            const int target = p + r + rskip;
-            if (target >= p + 32 || target >= ne) { next = target; break; }
-            pos = target - p;
         }
-        p = next;
+        count += __popc(emitMask);
+        p += max(32, __shfl_sync(0xffffffffu, reach, 31));
     }
     if (!Fill)
     {
@@ -563,7 +561,7 @@ __device__ __forceinline__ bool nr_step_b(double rhoi, double gradhi, double hi,
 // set's mass, periodicity and box.  A cut item scans its set's tree for its own box
 // instead of streaming the leaf's whole list.
 template<bool Mixed, bool EvalAll, bool Staged>
-__global__ void __launch_bounds__(kThreads, 5)   // 20 warps per SM (measured best of 4, 5, 6)
+__global__ void __launch_bounds__(kThreads, Mixed ? 4 : 5)   // measured best of 4, 5, 6
 density_batch_kernel(const int4* __restrict__ items, int cap, const int* __restrict__ leafSet,
                      const uint2* __restrict__ range, const uint32_t* __restrict__ jOffset,
                      const uint32_t* __restrict__ jcount, const int* __restrict__ jlist, double4* __restrict__ xyzh,
@@ -571,7 +569,8 @@ density_batch_kernel(const int4* __restrict__ items, int cap, const int* __restr
                      const double* __restrict__ pmassSet, double tolh, double hfact, const DevBox* __restrict__ boxes,
                      int* __restrict__ leafNext, int* __restrict__ nextLeaves, PreorderTree tree,
                      const int* __restrict__ setNodeStart, const int* __restrict__ leafPre,
-                     const double* __restrict__ hmaxLeaf, DevScalars* __restrict__ ds, long long waitNs)
+                     const double* __restrict__ hmaxLeaf, const float4* __restrict__ leafBox,
+                     DevScalars* __restrict__ ds, long long waitNs)
 {
     __shared__ __align__(16) unsigned char sScr[kWarpsPerBlock][DensScratch<Mixed>::kBytes];
     __shared__ __align__(128) WarpStage sStage[Staged ? kWarpsPerBlock : 1];
@@ -620,7 +619,7 @@ density_batch_kernel(const int4* __restrict__ items, int cap, const int* __restr
         // the code the warps of a mixed ensemble would otherwise share the instruction
         // cache with
         density_group<true, Mixed, Staged, false>(sScr[wib], mine, d.ng, pi, per ? bxs.len[0] : 0.0, per ? bxs.len[1] : 0.0,
-                                   per ? bxs.len[2] : 0.0, src, rhoi, gradhi, gp, gc);
+                                   per ? bxs.len[2] : 0.0, src, leafBox, rhoi, gradhi, gp, gc);
         if (EvalAll)
         {
             // rho and d(rho)/dh at the converged h (src/density_base.cu:635-643)
@@ -790,6 +789,9 @@ static void batch_forest(Batch& B)
         L = total;
     }
     B.nLeaves = L;
+    B.leafBox.resize(2 * size_t(L), s.st);
+    leaf_box_kernel_b<<<iceil(L, 128), 128, 0, s.st>>>(B.leafRange.get(), L, B.xyzh.get(), B.leafBox.get());
+    COSMO_LAUNCHED();
     B.setLeafStart.resize(size_t(ns) + 1, s.st);
     set_leaf_start_kernel<<<iceil(L + 1, kBlk), kBlk, 0, s.st>>>(B.leafSet.get(), L, ns, B.setLeafStart.get());
     COSMO_LAUNCHED();
@@ -887,8 +889,8 @@ static void run_items(Batch& B, const int* leaves, const int* countPtr, bool eva
         kern<<<persistent_grid(s, kern, kThreads), kThreads, 0, s.st>>>(
             B.items.get(), cap, B.leafSet.get(), B.leafRange.get(), B.jOffset.get(), B.jcount.get(), B.jlist.get(),
             B.xyzh.get(), B.rho.get(), B.gradh.get(), B.converged.get(), B.pmass.get(), tolh, hfact, B.boxes.get(),
-            B.leafNext.get(), B.activeB.get(), tree, B.setNodeStart.get(), B.leafPre.get(), B.hmaxLeaf.get(), ds,
-            wait_limit_ns());
+            B.leafNext.get(), B.activeB.get(), tree, B.setNodeStart.get(), B.leafPre.get(), B.hmaxLeaf.get(),
+            B.leafBox.get(), ds, wait_limit_ns());
     };
     const bool mx = s.precision == 1, st = s.staging != 0;
     if (evalAll)

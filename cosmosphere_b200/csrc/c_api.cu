@@ -141,6 +141,7 @@ size_t state_device_bytes(const State& s)
                     &s.extras, &s.nblJ, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1],
                     &s.nearSum[0], &s.nearSum[1], &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
         add(*d);
+    add(s.leafBox);
     add(s.nearNode);
     add(s.nearLoop);
     add(s.items);
@@ -170,6 +171,7 @@ void release_state(State& s)
                     &s.extras, &s.nblJ, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1],
                     &s.nearSum[0], &s.nearSum[1], &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
         b->release(s.st);
+    s.leafBox.release(s.st);
     s.nearNode.release(s.st);
     s.nearLoop.release(s.st);
     s.items.release(s.st);

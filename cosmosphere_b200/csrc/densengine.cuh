@@ -2,24 +2,32 @@
  * densengine.cuh -- the density sums of one warp group over its leaf's gather list, shared
  * by the single-set Newton kernel and the batched forest kernel, plain FP64 or mixed.
  *
- * Candidates pass the group box filter into the warp's ring (stream_ranges).  Each batch
- * of up to 32 is then tested with j on the lanes: for each group particle in turn, every
- * lane tests its candidate, and the accepted pairs are appended, particle-major, to the
- * warp's record buffer -- so each particle's records are contiguous and in ascending j.
- * The records are evaluated with one pair per lane (W and -q dW/dq - 3W), and each
- * particle's owner lane adds its own records in order.  All lanes work in every phase
- * whatever the group's size or spatial spread.
+ * The leaf's list is culled by the leaves' own boxes (near_ranges), and the candidates that
+ * pass the group's region go into the warp's ring (GroupSource).
  *
- *   plain  the exact FP64 test q^2 = r^2 / h_i^2 < R^2 (src/density_base.cu:270-283) and
- *          FP64 sums in ascending j: bit for bit the oracle's.
+ *   plain  each batch of up to 32 is tested with j on the lanes: for each group particle in
+ *          turn, every lane tests its candidate, and the accepted pairs are appended,
+ *          particle-major, to the warp's record buffer -- so each particle's records are
+ *          contiguous and in ascending j.  The records are evaluated with one pair per lane
+ *          (W and -q dW/dq - 3W), and each particle's owner lane adds its own records in
+ *          order.  The exact FP64 test q^2 = r^2 / h_i^2 < R^2 (src/density_base.cu:270-283)
+ *          and FP64 sums in ascending j: bit for bit the oracle's.
  * The periodic form with zero periods behaves, bit for bit, as the open form (the batched
  * kernel runs open and periodic sets through the one periodic instance).
  *
  *   mixed  coordinates relative to the group box centre (at the nearest periodic image
  *          of that centre when the box is small enough for it to be every pair's nearest
- *          image), the test and W, dW in FP32, two group particles per packed f32x2
- *          instruction; the owner's sums are FP32 with Kahan compensation, combined in
- *          FP64.
+ *          image), the test and W, dW in FP32, sums in FP32 with Kahan compensation,
+ *          combined in FP64.  Each particle's lane tests the candidates, two in a packed
+ *          f32x2 instruction, and keeps the q^2 of those it accepts in a column of its own
+ *          in shared memory; the columns are evaluated and added when one is nearly full.
+ *          With the records of the plain form the owners' serial additions ran over a
+ *          batch's longest list while most lanes had none: they were two fifths of the
+ *          kernel's instructions, the FP64 filter over whole lists most of the rest
+ *          (a solve of 40 sets of 10,000 to 300,000: 51.8 -> 34.1 ms in this kernel; first
+ *          iteration of a 300,000-particle box 663 -> 550 us, 1670 -> 1200 instructions a
+ *          particle).  The batch code is the kernel's largest loop and stays there once:
+ *          four copies of it stalled two issues in three on the instruction cache.
  */
 #pragma once
 
@@ -29,27 +37,38 @@ namespace cosmo {
 
 constexpr int kRec = 256;   // pair records per warp
 
-// Per-warp shared scratch of density_group: the ring, the group's particles, the pair
-// records, and at kBoxAt the group's rounded box (read by the filter from shared memory
+// Per-warp shared scratch of density_group: the ring, the group's particles and the pair
+// records (mixed: the ring and the columns), and at kBoxAt the group's rounded box (read by the filter from shared memory
 // rather than held in registers through the stream).
+constexpr int kTest = 8;     // mixed: candidates a lane tests in one turn of its loop
+constexpr int kColumn = 64;   // mixed: accepted pairs a lane keeps before they are evaluated
+
 template<bool Mixed>
 struct DensScratch
 {
-    static constexpr int kBoxAt = Mixed ? (kRing * 16 + 4 * 32 * 4 + 2 * kRec * 4)
+    static constexpr int kBoxAt = Mixed ? (3 * kRing * 4 + kColumn * 32 * 4)
                                         : (kRing * 32 + 32 * 32 + 2 * kRec * 8);
     static constexpr int kBytes = kBoxAt + 64;
 };
 
-// q = sqrt(q2) in FP32 (q2 >= 0); exact 0 for the self pair.
-__device__ __forceinline__ float sqrt_q(float q2) { return q2 > 0.0f ? q2 * rsqrtf(q2) : 0.0f; }
+// q = sqrt(q2) in FP32 (q2 >= 0); exact 0 for the self pair.  A subnormal q2 counts as 0
+// too (W and -q dW/dq - 3W round to the same for any q below 1e-18), which leaves out the
+// scaling that rsqrtf does for such values.
+__device__ __forceinline__ float sqrt_q(float q2)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q2));
+    return q2 >= 1.17549435e-38f ? q2 * r : 0.0f;
+}
 
 // Sums over the gather list of one group: the lanes [0, ng) own the group's particles
 // (pi, with mine set); rhoi and gradhi receive the un-normalised sums (W and
 // -q dW/dq - 3W over accepted j), gp the accepted pairs and gc the candidates offered.
 template<bool Periodic, bool Mixed, bool Staged = false, bool Round = true, class Ranges>
 __device__ __forceinline__ void density_group(unsigned char* scr, bool mine, int ng, const double4& pi, double lx,
-                                              double ly, double lz, const GroupSource<Ranges>& src, double& rhoi,
-                                              double& gradhi, unsigned int& gp, unsigned int& gc)
+                                              double ly, double lz, const GroupSource<Ranges>& list,
+                                              const float4* __restrict__ leafBox, double& rhoi, double& gradhi,
+                                              unsigned int& gp, unsigned int& gc)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -58,22 +77,29 @@ __device__ __forceinline__ void density_group(unsigned char* scr, bool mine, int
     const double rs = kRadKernel * hi;
     const double rmax = warp_max(mine ? rs : 0.0);
     const GroupBox bx = group_box(mine, pi.x, pi.y, pi.z, rs, rmax);
-    // Round: candidates, and the cells of a cut group's tree scan, are taken within the
-    // largest support of the members' own bounding box (a rounded box: a single particle's
-    // is its sphere), with the box's slack (1e-9 of the support, 1e-13 of |c|) on the
-    // radius, far above the rounding of the exact test, so no accepted pair is lost.
-    // Otherwise within the box of the search spheres (the batched kernel: its sets' h do
-    // not scatter, and its registers are tighter).
+    // Candidates, and the cells of a cut group's tree scan, are taken within the largest
+    // support of the members' own bounding box (a rounded box: a single particle's is its
+    // sphere), with the box's slack (1e-9 of the support, 1e-13 of |c|) on the radius, far
+    // above the rounding of the exact test, so no accepted pair is lost.  Not Round: within
+    // the box of the search spheres (the batched plain kernel: its sets' h do not scatter,
+    // and its registers are tighter).  The mixed form of several particles filters by the
+    // rounded box in FP32.  A single particle's partial sums, one a lane, depend on the
+    // candidates' places in the ring: it keeps the FP64 filter.
+    const GroupBox pb = group_box(mine, pi.x, pi.y, pi.z, 0.0, rmax);
     RoundBox* rbp = Round ? reinterpret_cast<RoundBox*>(scr + DensScratch<Mixed>::kBoxAt) : nullptr;
+    const double rr = rmax + 1e-9 * rmax + 1e-13 * (fabs(pb.cx) + fabs(pb.cy) + fabs(pb.cz)) + 1e-300;
     if constexpr (Round)
     {
-        const GroupBox pb = group_box(mine, pi.x, pi.y, pi.z, 0.0, rmax);
-        if (lane == 0)
-            *rbp = RoundBox{pb.cx, pb.cy, pb.cz, pb.ex, pb.ey, pb.ez,
-                            rmax + 1e-9 * rmax + 1e-13 * (fabs(pb.cx) + fabs(pb.cy) + fabs(pb.cz)) + 1e-300};
+        if (lane == 0) *rbp = RoundBox{pb.cx, pb.cy, pb.cz, pb.ex, pb.ey, pb.ez, rr};
         __syncwarp();
     }
+    const bool cube = !Round && (!Mixed || ng == 1);
+    const GroupRegion region = group_region<Periodic>(cube ? bx : pb, cube ? 0.0 : rr, lx, ly, lz);
+    GroupSource<NearRanges<Periodic, Ranges>> src{list.jlist, list.jb, list.nj,
+                                                  near_ranges<Periodic>(list.ranges, leafBox, region), list.xyzh,
+                                                  list.walk, list.tree, list.rc, list.re, list.stage};
     auto gather = [&](const double4& pj) {
+        if (Mixed && ng > 1) return in_region<Periodic>(pj, region);
         if constexpr (Round) return in_round_box<Periodic>(pj, *rbp, lx, ly, lz);
         else return in_gather_box<Periodic>(pj, bx, lx, ly, lz);
     };
@@ -186,128 +212,130 @@ __device__ __forceinline__ void density_group(unsigned char* scr, bool mine, int
     }
     else
     {
-        float4* ringf = reinterpret_cast<float4*>(scr);
-        float* gx = reinterpret_cast<float*>(ringf + kRing);
-        float* gy = gx + 32;
-        float* gz = gy + 32;
-        float* gh = gz + 32;
-        float* recQ = gh + 32;
-        float* recG = recQ + kRec;
+        float* rx = reinterpret_cast<float*>(scr);   // the candidates' -x, -y, -z, kRing each
+        float* column = rx + 3 * kRing + lane;       // q^2 of accepted pair t at column[32 t]
         // relative coordinates at the centre's nearest image are every accepted pair's
         // nearest image when the box (search spheres included) spans under half a period
         const bool shifted = !Periodic || lx == 0.0 || (bx.ex < 0.5 * lx && bx.ey < 0.5 * ly && bx.ez < 0.5 * lz);
         const double sx = shifted && Periodic ? lx : 0.0, sy = shifted && Periodic ? ly : 0.0;
         const double sz = shifted && Periodic ? lz : 0.0;
-        gx[lane] = mine ? float(pi.x - bx.cx) : 0.0f;
-        gy[lane] = mine ? float(pi.y - bx.cy) : 0.0f;
-        gz[lane] = mine ? float(pi.z - bx.cz) : 0.0f;
-        gh[lane] = mine ? float(hinv2) : 0.0f;
-        __syncwarp();
+        // a lane without a particle is infinitely far from everything
+        const float inf = __int_as_float(0x7f800000);
+        const float gx = mine ? float(pi.x - bx.cx) : inf, gy = mine ? float(pi.y - bx.cy) : inf;
+        const float gz = mine ? float(pi.z - bx.cz) : inf, gh = mine ? float(hinv2) : 1.0f;
+        const float2 gx2 = make_float2(gx, gx), gy2 = make_float2(gy, gy), gz2 = make_float2(gz, gz);
+        const float2 gh2 = make_float2(gh, gh);
         const float Lx = float(lx), Ly = float(ly), Lz = float(lz);
-        KahanF kr, kg, lr, lg;
+        KahanF lr, lg;
+        KahanF2 sums;
+        int kept = 0;
+        auto evaluate = [&]() {
+#pragma unroll 2
+            for (int t = 0; t < kept; ++t)
+            {
+                const float q2 = column[32 * t];
+                const float q = sqrt_q(q2);
+                float wk, dwk;
+                sph_kernel_f(q2, q, wk, dwk);
+                sums.add(wk, fmaf(-q, dwk, -3.0f * wk));
+            }
+            gp += kept;
+            kept = 0;
+            __syncwarp();
+        };
         src.template stream<false, true, false, Periodic, Staged>(
-            nullptr, ringf, nullptr, bx, sx, sy, sz, lx, ly, lz, gather,
-            [&](const double4*, const float4* rf, const int*, int head, int count) {
+            nullptr, reinterpret_cast<float4*>(rx), nullptr, bx, sx, sy, sz, lx, ly, lz, gather,
+            [&](const double4*, const float4*, const int*, int head, int count) {
                 gc += count;
-                const float4 pf = rf[(head + (lane < count ? lane : 0)) & (kRing - 1)];
                 if (ng == 1)
                 {
                     // a single particle (a cut group): every lane keeps its own compensated
                     // partial sums, combined in FP64 after the stream
-                    float dx = gx[0] - pf.x, dy = gy[0] - pf.y, dz = gz[0] - pf.z;
+                    const int at = (head + (lane < count ? lane : 0)) & (kRing - 1);
+                    const float fx = rx[at], fy = rx[kRing + at], fz = rx[2 * kRing + at];
+                    const float x0 = __shfl_sync(0xffffffffu, gx, 0), y0 = __shfl_sync(0xffffffffu, gy, 0);
+                    const float z0 = __shfl_sync(0xffffffffu, gz, 0), h0 = __shfl_sync(0xffffffffu, gh, 0);
+                    float dx = x0 + fx, dy = y0 + fy, dz = z0 + fz;
                     if (Periodic && !shifted)
                     {
-                        dx = axis_df<true>(gx[0], pf.x, Lx);
-                        dy = axis_df<true>(gy[0], pf.y, Ly);
-                        dz = axis_df<true>(gz[0], pf.z, Lz);
+                        dx = axis_df<true>(x0, -fx, Lx);
+                        dy = axis_df<true>(y0, -fy, Ly);
+                        dz = axis_df<true>(z0, -fz, Lz);
                     }
-                    const float q2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) * gh[0];
+                    const float q2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) * h0;
                     const bool acc = lane < count && q2 < float(kRadK2);
                     if (acc)
                     {
                         const float q = sqrt_q(q2);
                         float wk, dwk;
                         sph_kernel_f(q2, q, wk, dwk);
-                        lr.add(wk);
-                        lg.add(fmaf(-q, dwk, -3.0f * wk));
+                        lr.add_rn(wk);
+                        lg.add_rn(fmaf(-q, dwk, -3.0f * wk));
                     }
                     gp += __popc(__ballot_sync(0xffffffffu, acc));
                     return;
                 }
-                int nrec = 0, segStart = 0, segCount = 0;
-                auto flush = [&]() {
-                    __syncwarp();
-                    for (int r = lane; r < nrec; r += 32)
-                    {
-                        const float q2 = recQ[r];
-                        const float q = sqrt_q(q2);
-                        float wk, dwk;
-                        sph_kernel_f(q2, q, wk, dwk);
-                        recQ[r] = wk;
-                        recG[r] = fmaf(-q, dwk, -3.0f * wk);
-                    }
-                    __syncwarp();
-                    for (int t = 0; t < segCount; ++t)
-                    {
-                        kr.add(recQ[segStart + t]);
-                        kg.add(recG[segStart + t]);
-                    }
-                    gp += segCount;
-                    segCount = 0;
-                    nrec = 0;
-                    __syncwarp();
-                };
-                const float2 nx = make_float2(-pf.x, -pf.x), ny = make_float2(-pf.y, -pf.y);
-                const float2 nz = make_float2(-pf.z, -pf.z);
-                for (int i0 = 0; i0 < ng; i0 += 4)
+                // full batches start at a multiple of 32; a partial (last) one is filled up
+                // with candidates infinitely far the other way
+                if (lane >= count) rx[(head + lane) & (kRing - 1)] = inf;
+                __syncwarp();
+                if (__any_sync(0xffffffffu, kept > kColumn - 32)) evaluate();
+                float* put = column + 32 * kept;
+                const float* cand = rx + (head & (kRing - 1));
+#pragma unroll 1
+                for (int k0 = 0; k0 < count; k0 += kTest, cand += kTest)
                 {
-                    if (nrec + 4 * 32 > kRec) flush();
-                    float q2u[4];
-                    if (!Periodic || shifted)
-                    {
 #pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                        {
-                            const int k = i0 + 2 * h;
-                            const float2 dx = __fadd2_rn(*reinterpret_cast<const float2*>(gx + k), nx);
-                            const float2 dy = __fadd2_rn(*reinterpret_cast<const float2*>(gy + k), ny);
-                            const float2 dz = __fadd2_rn(*reinterpret_cast<const float2*>(gz + k), nz);
-                            float2 r2 = __fmul2_rn(dx, dx);
-                            r2 = __ffma2_rn(dy, dy, r2);
-                            r2 = __ffma2_rn(dz, dz, r2);
-                            const float2 q2 = __fmul2_rn(r2, *reinterpret_cast<const float2*>(gh + k));
-                            q2u[2 * h] = q2.x;
-                            q2u[2 * h + 1] = q2.y;
-                        }
-                    }
-                    else
+                    for (int k = 0; k < kTest; k += 4)
                     {
+                        const float4 X = *reinterpret_cast<const float4*>(cand + k);
+                        const float4 Y = *reinterpret_cast<const float4*>(cand + kRing + k);
+                        const float4 Z = *reinterpret_cast<const float4*>(cand + 2 * kRing + k);
+                        float q2u[4];
+                        if (!Periodic || shifted)
+                        {
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+                            {
+                                const float2 dx = __fadd2_rn(gx2, h ? make_float2(X.z, X.w) : make_float2(X.x, X.y));
+                                const float2 dy = __fadd2_rn(gy2, h ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y));
+                                const float2 dz = __fadd2_rn(gz2, h ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y));
+                                float2 r2 = __fmul2_rn(dx, dx);
+                                r2 = __ffma2_rn(dy, dy, r2);
+                                r2 = __ffma2_rn(dz, dz, r2);
+                                const float2 q2 = __fmul2_rn(r2, gh2);
+                                q2u[2 * h] = q2.x;
+                                q2u[2 * h + 1] = q2.y;
+                            }
+                        }
+                        else
+                        {
+                            const float xs[4] = {X.x, X.y, X.z, X.w}, ys[4] = {Y.x, Y.y, Y.z, Y.w};
+                            const float zs[4] = {Z.x, Z.y, Z.z, Z.w};
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+                            {
+                                const float dx = axis_df<true>(gx, -xs[u], Lx);
+                                const float dy = axis_df<true>(gy, -ys[u], Ly);
+                                const float dz = axis_df<true>(gz, -zs[u], Lz);
+                                q2u[u] = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) * gh;
+                            }
+                        }
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
-                        {
-                            const int k = i0 + u;
-                            const float dx = axis_df<true>(gx[k], pf.x, Lx);
-                            const float dy = axis_df<true>(gy[k], pf.y, Ly);
-                            const float dz = axis_df<true>(gz[k], pf.z, Lz);
-                            q2u[u] = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) * gh[k];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                    {
-                        const bool acc = lane < count && i0 + u < ng && q2u[u] < float(kRadK2);
-                        const uint32_t m = __ballot_sync(0xffffffffu, acc);
-                        const int c = __popc(m);
-                        if (acc) recQ[nrec + __popc(m & lt)] = q2u[u];
-                        if (lane == i0 + u) { segStart = nrec; segCount = c; }
-                        nrec += c;
+                            if (q2u[u] < float(kRadK2))
+                            {
+                                *put = q2u[u];
+                                put += 32;
+                            }
                     }
                 }
-                if (nrec > 0) flush();
+                kept = int(put - column) >> 5;
             },
             rbp);
-        rhoi = kr.value();
-        gradhi = kg.value();
+        evaluate();
+        rhoi = sums.first();
+        gradhi = sums.second();
         if (ng == 1)
         {
             double a = lr.value(), b = lg.value();

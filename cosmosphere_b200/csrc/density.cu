@@ -927,7 +927,7 @@ static LoopGraph newton_loop_graph(State& s, double pmass, double tolh, double h
                           (const void*)s.jOffset.get(), (const void*)s.jcount.get(), (const void*)s.jlist.get(),
                           (const void*)s.jlistPrev.get(), (const void*)s.jOffsetPrev.get(), (const void*)s.walked.get(),
                           (const void*)s.walkScratch.get(), (const void*)s.hmaxLeaf.get(), (const void*)s.hmaxPre.get(),
-                          (const void*)s.particleLeaf.get(), (const void*)s.scanTmp.get(), (const void*)nrows,
+                          (const void*)s.particleLeaf.get(), (const void*)s.scanTmp.get(), (const void*)s.leafBox.get(), (const void*)nrows,
                           (const void*)nr, (const void*)rk, (const void*)rowsJ})
         key.add(q);
     for (long long v : {(long long)leafCap, (long long)itemCap, (long long)gridRows, (long long)gridNr,
@@ -1032,8 +1032,8 @@ static LoopGraph newton_loop_graph(State& s, double pmass, double tolh, double h
             COSMO_LAUNCHED();
             nrows<<<gridRows, kThreads, 0, s.st>>>(s.items.get(), itemCap, s.layout.get(), s.jOffset.get(),
                                                    s.jcount.get(), s.jlist.get(), s.xyzh.get(), s.box.get(),
-                                                   s.listH.get(), s.nblR2.get(), s.nblCount.get(), s.nblH.get(), ds,
-                                                   rowsJ);
+                                                   s.listH.get(), s.nblR2.get(), s.nblCount.get(), s.nblH.get(),
+                                                   s.leafBox.get(), ds, rowsJ);
             COSMO_LAUNCHED();
             newton_count_kernel<<<1, 1, 0, s.st>>>(L, 1);
             COSMO_LAUNCHED();
@@ -1055,7 +1055,7 @@ static LoopGraph newton_loop_graph(State& s, double pmass, double tolh, double h
                                               s.jlist.get(), s.xyzh.get(), s.rho.get(), s.gradh.get(),
                                               s.converged.get(), pmass, tolh, hfact, s.box.get(), s.listH.get(),
                                               s.leafNext.get(), s.activeB.get(), tree, s.leafToInternal.get(),
-                                              s.centers.get(), s.sizes.get(), ds, waitNs);
+                                              s.centers.get(), s.sizes.get(), s.leafBox.get(), ds, waitNs);
             COSMO_LAUNCHED();
             rk<<<gridRow, kThreads, 0, s.st>>>(s.rowItems.get(), s.nblR2.get(), s.nblCount.get(), s.xyzh.get(),
                                               s.rho.get(), s.gradh.get(), s.converged.get(), pmass, tolh, hfact,
@@ -1154,7 +1154,8 @@ static bool cover_rows(State& s, int itemCap, FixedSplit cut, int spreadG)
                                  : (s.periodic ? newton_rows_kernel<true, false> : newton_rows_kernel<false, false>);
         nrows<<<persistent_grid(s, nrows, kThreads), kThreads, 0, s.st>>>(
             s.items.get(), itemCap, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(), s.xyzh.get(),
-            s.box.get(), s.listH.get(), s.nblR2.get(), s.nblCount.get(), s.nblH.get(), ds, s.nblJ.get());
+            s.box.get(), s.listH.get(), s.nblR2.get(), s.nblCount.get(), s.nblH.get(), s.leafBox.get(), ds,
+            s.nblJ.get());
         COSMO_LAUNCHED();
     }
     return false;
@@ -1362,8 +1363,8 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
                                          : (s.periodic ? newton_rows_kernel<true, false> : newton_rows_kernel<false, false>);
                 nrows<<<persistent_grid(s, nrows, kThreads), kThreads, 0, s.st>>>(
                     s.items.get(), itemCap, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),
-                    s.xyzh.get(), s.box.get(), s.listH.get(), s.nblR2.get(), s.nblCount.get(), s.nblH.get(), ds,
-                    rowsJ);
+                    s.xyzh.get(), s.box.get(), s.listH.get(), s.nblR2.get(), s.nblCount.get(), s.nblH.get(),
+                    s.leafBox.get(), ds, rowsJ);
                 COSMO_LAUNCHED();
                 rowsReady = true;
             }
@@ -1387,7 +1388,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
                 s.rho.get(), s.gradh.get(), s.converged.get(), pmass, tolh, hfact, s.box.get(), s.listH.get(),
                 s.leafNext.get(), s.activeB.get(),
                 PreorderTree{s.preCenter.get(), s.preHalf.get(), s.preSkip.get(), s.preLeaf.get(), 0, s.numNodes},
-                s.leafToInternal.get(), s.centers.get(), s.sizes.get(), ds, wait_limit_ns());
+                s.leafToInternal.get(), s.centers.get(), s.sizes.get(), s.leafBox.get(), ds, wait_limit_ns());
             COSMO_LAUNCHED();
             if (rowsReady)
             {

@@ -297,7 +297,8 @@ __global__ void __launch_bounds__(kThreads)
 sym_rows_kernel(const int4* __restrict__ items, int cap, const uint32_t* __restrict__ layout,
                 const uint32_t* __restrict__ jOffset, const uint32_t* __restrict__ jcount,
                 const int* __restrict__ jlist, const double4* __restrict__ xyzh, const DevBox* __restrict__ box,
-                int* __restrict__ nbl, int* __restrict__ nblCount, DevScalars* __restrict__ ds, int prefilter)
+                const float4* __restrict__ leafBox, const double* __restrict__ hmaxLeaf, int* __restrict__ nbl,
+                int* __restrict__ nblCount, DevScalars* __restrict__ ds, int prefilter)
 {
     __shared__ __align__(16) unsigned char sScr[kWarpsPerBlock][kRowsScratch];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -322,6 +323,10 @@ sym_rows_kernel(const int4* __restrict__ items, int cap, const uint32_t* __restr
         auto bound = [](double h) { return kRadK2 * (h * h) * (1.0 + 1e-10); };
         // prefilter distances: R h (1 + 1e-10) bounds sqrt(bound(h)) for either side
         auto filt = [&](const double4& pj) { return in_sym_box<Periodic>(pj, bx, rg, lx, ly, lz); };
+        // the listed leaves within the group's supports or their own
+        auto ranges = near_ranges<Periodic>(LayoutRanges{layout}, leafBox,
+                                            group_region<Periodic>(bx, rg * (1.0 + 1e-8), lx, ly, lz));
+        ranges.hmaxLeaf = hmaxLeaf;
         auto candB = [](const double4& pj) { return kRadKernel * pj.w * (1.0 + 1e-10); };
         auto exact = [&](const double4& g, const double4& pj, int j) {
             double dx = g.x - pj.x, dy = g.y - pj.y, dz = g.z - pj.z;
@@ -334,11 +339,11 @@ sym_rows_kernel(const int4* __restrict__ items, int cap, const uint32_t* __restr
         const double Bi = kRadKernel * pi.w * (1.0 + 1e-10);
         if (prefilter)
             rows_group<kRowStride, Periodic, true>(sScr[wib], mine, d.ng, gi, Bi, bx, lx, ly, lz, jOffset[d.leaf],
-                                                   jcount[d.leaf], jlist, LayoutRanges{layout}, xyzh, filt, candB,
+                                                   jcount[d.leaf], jlist, ranges, xyzh, filt, candB,
                                                    exact, myRow, rowLen);
         else
             rows_group<kRowStride, Periodic, false>(sScr[wib], mine, d.ng, gi, Bi, bx, lx, ly, lz, jOffset[d.leaf],
-                                                    jcount[d.leaf], jlist, LayoutRanges{layout}, xyzh, filt, candB,
+                                                    jcount[d.leaf], jlist, ranges, xyzh, filt, candB,
                                                     exact, myRow, rowLen);
         if (mine) nblCount[i] = rowLen;
         if (mine && rowLen > kNbl) ds->rowOverflow = 1;
@@ -511,7 +516,7 @@ void build_symmetric(State& s)
     auto rows = s.periodic ? sym_rows_kernel<true> : sym_rows_kernel<false>;
     rows<<<persistent_grid(s, rows, kThreads), kThreads, 0, s.st>>>(
         s.items.get(), nA, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(), s.xyzh.get(),
-        s.box.get(), s.nbl.get(), s.nblCount.get(), ds, s.symPrefilter);
+        s.box.get(), s.leafBox.get(), s.hmaxLeaf.get(), s.nbl.get(), s.nblCount.get(), ds, s.symPrefilter);
     COSMO_LAUNCHED();
 }
 

@@ -48,7 +48,8 @@ density_nr_kernel(const int4* __restrict__ items, int cap, const uint32_t* __res
                   double hfact, const DevBox* __restrict__ box, const double* __restrict__ listH,
                   int* __restrict__ leafNext, int* __restrict__ nextLeaves, PreorderTree tree,
                   const int* __restrict__ leafToInternal, const double* __restrict__ centers,
-                  const double* __restrict__ sizes, DevScalars* __restrict__ ds, long long waitNs)
+                  const double* __restrict__ sizes, const float4* __restrict__ leafBox, DevScalars* __restrict__ ds,
+                  long long waitNs)
 {
     __shared__ __align__(16) unsigned char sScr[kWarpsPerBlock][DensScratch<Mixed>::kBytes];
     __shared__ __align__(128) WarpStage sStage[Staged ? kWarpsPerBlock : 1];
@@ -88,7 +89,8 @@ density_nr_kernel(const int4* __restrict__ items, int cap, const uint32_t* __res
             src.rc = make_double3(centers[3 * in], centers[3 * in + 1], centers[3 * in + 2]);
             src.re = make_double3(sizes[3 * in] + ext, sizes[3 * in + 1] + ext, sizes[3 * in + 2] + ext);
         }
-        density_group<Periodic, Mixed, Staged>(sScr[wib], mine, d.ng, pi, lx, ly, lz, src, rhoi, gradhi, gp, gc);
+        density_group<Periodic, Mixed, Staged>(sScr[wib], mine, d.ng, pi, lx, ly, lz, src, leafBox, rhoi, gradhi, gp,
+                                                 gc);
         bool stillActive = false, settle = false;
         if (mine)
         {
@@ -139,7 +141,8 @@ newton_rows_kernel(const int4* __restrict__ items, int cap, const uint32_t* __re
                    const uint32_t* __restrict__ jOffset, const uint32_t* __restrict__ jcount,
                    const int* __restrict__ jlist, const double4* __restrict__ xyzh, const DevBox* __restrict__ box,
                    const double* __restrict__ listH, void* __restrict__ rowsR2, int* __restrict__ nblCount,
-                   double* __restrict__ rowH, DevScalars* __restrict__ ds, int* __restrict__ rowsJ)
+                   double* __restrict__ rowH, const float4* __restrict__ leafBox, DevScalars* __restrict__ ds,
+                   int* __restrict__ rowsJ)
 {
     using R2 = typename std::conditional<Mixed, float, double>::type;   // FP32 rows in the mixed form
     R2* nblR2 = static_cast<R2*>(rowsR2);
@@ -174,10 +177,12 @@ newton_rows_kernel(const int4* __restrict__ items, int cap, const uint32_t* __re
         const double rs = kRadKernel * kRowMargin * pi.w;
         const double rmax = warp_max(mine ? rs : 0.0);
         const GroupBox bx = group_box(mine, pi.x, pi.y, pi.z, rs, rmax);
+        const GroupRegion region =
+            group_region<Periodic>(group_box(mine, pi.x, pi.y, pi.z, 0.0, rmax), rmax * (1.0 + 1e-9), lx, ly, lz);
         int rowLen = 0;
         rows_group<1, Periodic>(sScr[wib], mine, d.ng, make_double4(pi.x, pi.y, pi.z, hinv2), rs, bx, lx, ly, lz,
-                   jOffset[d.leaf], jcount[d.leaf], jlist, LayoutRanges{layout}, xyzh,
-                   [&](const double4& pj) { return in_gather_box<Periodic>(pj, bx, lx, ly, lz); },
+                   jOffset[d.leaf], jcount[d.leaf], jlist, near_ranges<Periodic>(LayoutRanges{layout}, leafBox, region),
+                   xyzh, [&](const double4& pj) { return in_region<Periodic>(pj, region); },
                    [](const double4&) { return 0.0; },
                    [&](const double4& g, const double4& pj, int) {   // r^2 within the wide support
                        double dx = g.x - pj.x, dy = g.y - pj.y, dz = g.z - pj.z;

@@ -92,6 +92,63 @@ __device__ __forceinline__ bool in_round_box(const double4& p, const RoundBox& b
     return gx * gx + gy * gy + gz * gz <= b.r * b.r;
 }
 
+// The rounded box in FP32, for the filters that only keep a superset: the centre in FP64,
+// the distances from it in FP32 with their rounding on the radius (r2 for particles; leaves
+// are boxes in global coordinates, r2Leaf covers those too).  Lx, Ly, Lz: the periods, or
+// infinity.  A candidate costs three FP64 subtractions and a dozen FP32 instructions where
+// the FP64 test took about 45.
+struct GroupRegion
+{
+    double cx, cy, cz;
+    float ex, ey, ez, r2, r2Leaf, slackLeaf, Lx, Ly, Lz;
+};
+
+// The region of the members' bounding box b and the search radius r about them.
+template<bool Periodic>
+__device__ __forceinline__ GroupRegion group_region(const GroupBox& b, double r, double lx, double ly, double lz)
+{
+    const float inf = __int_as_float(0x7f800000);
+    GroupRegion g;
+    g.cx = b.cx; g.cy = b.cy; g.cz = b.cz;
+    g.ex = float(b.ex) * 1.0000003f; g.ey = float(b.ey) * 1.0000003f; g.ez = float(b.ez) * 1.0000003f;
+    const double slack = 1e-6 * (r + b.ex + b.ey + b.ez) + (Periodic ? 4e-7 * (lx + ly + lz) : 0.0) + 1e-300;
+    const double rr = r + slack, rl = rr + 2.5e-7 * (fabs(b.cx) + fabs(b.cy) + fabs(b.cz));
+    g.r2 = float(rr * rr * 1.000001);
+    g.r2Leaf = float(rl * rl * 1.000001);
+    g.slackLeaf = float(rl - r) * 1.00001f;
+    // an r2 below FP32's range would leave out pairs: nothing is filtered then
+    if (g.r2 < 1e-30f) g.r2 = inf;
+    if (g.r2Leaf < 1e-30f) g.r2Leaf = inf;
+    g.Lx = Periodic && lx > 0.0 ? float(lx) : inf;
+    g.Ly = Periodic && ly > 0.0 ? float(ly) : inf;
+    g.Lz = Periodic && lz > 0.0 ? float(lz) : inf;
+    return g;
+}
+
+// Squared distance of a point (its offset from the region's centre), or of a box of half
+// extents h about it, from the region's core.
+template<bool Periodic>
+__device__ __forceinline__ float region_gap2(const GroupRegion& g, float x, float y, float z, float hx = 0.0f,
+                                             float hy = 0.0f, float hz = 0.0f)
+{
+    float ax = fabsf(x), ay = fabsf(y), az = fabsf(z);
+    if (Periodic)
+    {
+        ax = fminf(ax, g.Lx - ax);
+        ay = fminf(ay, g.Ly - ay);
+        az = fminf(az, g.Lz - az);
+    }
+    const float dx = fmaxf(ax - (g.ex + hx), 0.0f), dy = fmaxf(ay - (g.ey + hy), 0.0f);
+    const float dz = fmaxf(az - (g.ez + hz), 0.0f);
+    return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+}
+
+template<bool Periodic>
+__device__ __forceinline__ bool in_region(const double4& p, const GroupRegion& g)
+{
+    return region_gap2<Periodic>(g, float(p.x - g.cx), float(p.y - g.cy), float(p.z - g.cz)) <= g.r2;
+}
+
 // Symmetric filter: within R*max(hmax_group, h_j) of the box of the group's positions.
 template<bool Periodic>
 __device__ __forceinline__ bool in_sym_box(const double4& p, const GroupBox& b, double rg, double lx, double ly,
@@ -103,6 +160,19 @@ __device__ __forceinline__ bool in_sym_box(const double4& p, const GroupBox& b, 
     const double dx = gx > 0.0 ? gx : 0.0, dy = gy > 0.0 ? gy : 0.0, dz = gz > 0.0 ? gz : 0.0;
     const double r = fmax(rg, kRadKernel * p.w) * (1.0 + 1e-9);
     return dx * dx + dy * dy + dz * dz <= r * r;
+}
+
+// The largest of the values of lanes 0 .. lane.
+__device__ __forceinline__ int warp_prefix_max(int v)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v = max(v, t);
+    }
+    return v;
 }
 
 __device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t v)
@@ -131,6 +201,68 @@ struct TableRanges
     __device__ __forceinline__ uint2 operator()(int leaf) const { return range[leaf]; }
 };
 
+// The ranges of the leaves that can hold a particle of the group's region: a leaf whose own
+// bounding box (leaf_box_kernel: centre and half extents, leaf by leaf) lies outside it has
+// an empty range.  A leaf's list covers every group of the leaf at a margin on its largest
+// h, cell by cell: of the particles a 300,000-particle box's lists stream past a group two
+// in three are in such leaves.  With sym, the region reaches each leaf's own largest
+// support too.
+template<bool Periodic, class Base>
+struct NearRanges
+{
+    Base base;
+    const float4* __restrict__ leafBox;
+    GroupRegion g;
+    float gx, gy, gz;
+    const double* __restrict__ hmaxLeaf = nullptr;   // symmetric: the leaves' largest h
+    __device__ __forceinline__ uint2 operator()(int leaf) const
+    {
+        const float4 c = __ldg(leafBox + 2 * size_t(leaf)), h = __ldg(leafBox + 2 * size_t(leaf) + 1);
+        float r2 = g.r2Leaf;
+        if (hmaxLeaf != nullptr)
+        {
+            const float hm = float(kRadKernel * hmaxLeaf[leaf]) * 1.00001f + g.slackLeaf;
+            r2 = fmaxf(r2, hm * hm * 1.000001f);
+        }
+        uint2 r = base(leaf);
+        if (region_gap2<Periodic>(g, c.x - gx, c.y - gy, c.z - gz, h.x, h.y, h.z) > r2) r.y = r.x;
+        return r;
+    }
+};
+
+template<bool Periodic, class Base>
+__device__ __forceinline__ NearRanges<Periodic, Base> near_ranges(Base base, const float4* leafBox,
+                                                                  const GroupRegion& g)
+{
+    return NearRanges<Periodic, Base>{base, leafBox, g, float(g.cx), float(g.cy), float(g.cz)};
+}
+
+// A leaf's bounding box over its particles, for near_ranges: centre and half extents, the
+// half extents widened by the rounding of both.
+__device__ __forceinline__ void leaf_box(const double4* __restrict__ xyzh, uint32_t p0, uint32_t p1,
+                                         float4* __restrict__ out)
+{
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    double lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
+    for (uint32_t j = p0; j < p1; ++j)
+    {
+        const double4 p = xyzh[j];
+        lo[0] = fmin(lo[0], p.x); hi[0] = fmax(hi[0], p.x);
+        lo[1] = fmin(lo[1], p.y); hi[1] = fmax(hi[1], p.y);
+        lo[2] = fmin(lo[2], p.z); hi[2] = fmax(hi[2], p.z);
+    }
+    float c[3], h[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+    {
+        const double m = 0.5 * (lo[d] + hi[d]);
+        c[d] = float(m);
+        h[d] = float(0.5 * (hi[d] - lo[d]) * (1.0 + 1e-6) + 2.5e-7 * fabs(m)) * 1.0000003f;
+    }
+    out[0] = make_float4(c[0], c[1], c[2], 0.0f);
+    out[1] = make_float4(h[0], h[1], h[2], 0.0f);
+}
+
 // Signed offset of x from c at the nearest periodic image (L > 0), or plain (L == 0).
 __device__ __forceinline__ double image_offset(double x, double c, double L)
 {
@@ -147,7 +279,8 @@ __device__ __forceinline__ double image_offset(double x, double c, double L)
 // it, in order, and handed to batch(ring, ringf, ringIdx, head, count) in runs of up to 32
 // on every lane.  The ring keeps what the caller asks for: the FP64 xyzh (Dbl), an FP32
 // copy relative to the group box centre at the nearest periodic image when lx, ly, lz > 0
-// (Float), and the particle index (Index).
+// (Float), and the particle index (Index).  FP32 copies alone are kept negated and by
+// component (x, y and z of kRing each), for packed arithmetic on several candidates.
 template<bool Dbl, bool Float, bool Index, bool Staged = false>
 struct CandidateRing
 {
@@ -157,6 +290,23 @@ struct CandidateRing
     double cx, cy, cz, lx, ly, lz;
     StageRef stage;
     int head = 0, cnt = 0;
+
+    __device__ __forceinline__ void put_float(int slot, const double4& pj)
+    {
+        if constexpr (Float)
+        {
+            const float x = float(image_offset(pj.x, cx, lx)), y = float(image_offset(pj.y, cy, ly));
+            const float z = float(image_offset(pj.z, cz, lz));
+            if constexpr (Dbl || Index) ringf[slot] = make_float4(x, y, z, float(pj.w));
+            else
+            {
+                float* rf = reinterpret_cast<float*>(ringf);
+                rf[slot] = -x;
+                rf[kRing + slot] = -y;
+                rf[2 * kRing + slot] = -z;
+            }
+        }
+    }
 
     template<class Batch>
     __device__ __forceinline__ void drain(int count, Batch& batch)
@@ -171,10 +321,13 @@ struct CandidateRing
     // lane order.  A warp prefix sum over the lengths flattens them, so every load batch is
     // 32 consecutive stream positions (each lane finds its particle by a 5-step binary
     // search over the prefix sums), and the next batch's loads are issued before the
-    // current batch is filtered.  filter(pj) is evaluated by the loading lane only.
+    // current batch is filtered.  filter(pj) is evaluated by the loading lane only.  After
+    // the last ranges what the ring still holds is handed on too: in the same place as the
+    // full batches, so that the batch code is in the kernel once (a copy of the mixed form's
+    // for the end, and both again for the tree scan, outgrew the instruction cache).
     template<class Filter, class Batch>
     __device__ __forceinline__ void feed(uint32_t s0, uint32_t len, int nb, const double4* __restrict__ xyzh,
-                                         Filter& filter, Batch& batch)
+                                         Filter& filter, Batch& batch, bool last)
     {
         if constexpr (Staged)
             if (stage.ws->broken == 0u)
@@ -205,7 +358,7 @@ struct CandidateRing
             j = locate(lane);
             if (uint32_t(lane) < total) pj = ldg4(xyzh + j);
         }
-        for (uint32_t p0 = 0; p0 < total; p0 += 32)
+        for (uint32_t p0 = 0; p0 < total || (last && cnt > 0); p0 += 32)
         {
             const bool valid = p0 + lane < total;
             uint32_t jn = 0;
@@ -221,14 +374,12 @@ struct CandidateRing
             {
                 const int slot = (head + cnt + __popc(m & lt)) & (kRing - 1);
                 if constexpr (Dbl) ring[slot] = pj;
-                if constexpr (Float)
-                    ringf[slot] = make_float4(float(image_offset(pj.x, cx, lx)), float(image_offset(pj.y, cy, ly)),
-                                              float(image_offset(pj.z, cz, lz)), float(pj.w));
+                put_float(slot, pj);
                 if constexpr (Index) ringIdx[slot] = int(j);
             }
             cnt += __popc(m);
             __syncwarp();
-            if (cnt >= 32) drain(32, batch);
+            if (cnt >= 32 || (last && p0 + 32 >= total && cnt > 0)) drain(min(cnt, 32), batch);
             j = jn;
             pj = pn;
         }
@@ -247,9 +398,7 @@ struct CandidateRing
         {
             const int slot = (head + cnt + __popc(m & lt)) & (kRing - 1);
             if constexpr (Dbl) ring[slot] = pj;
-            if constexpr (Float)
-                ringf[slot] = make_float4(float(image_offset(pj.x, cx, lx)), float(image_offset(pj.y, cy, ly)),
-                                          float(image_offset(pj.z, cz, lz)), float(pj.w));
+            put_float(slot, pj);
             if constexpr (Index) ringIdx[slot] = int(j);
         }
         cnt += __popc(m);
@@ -374,13 +523,13 @@ __device__ __forceinline__ void stream_ranges(double4* ring, float4* ringf, int*
             s0 = r.x;
             len = r.y - r.x;
         }
-        cr.feed(s0, len, nb, xyzh, filter, batch);
+        cr.feed(s0, len, nb, xyzh, filter, batch, lb + 32 >= nj);
     }
-    cr.finish(batch);
+    if constexpr (Staged) cr.finish(batch);
 }
 
-// The pre-order node arrays of a tree (or of one set's range [n0, n1) of a forest) for
-// stream_walk.
+// The pre-order node arrays of a tree (or of one set's range [n0, n1) of a forest), for a
+// group's own scan (GroupSource).
 struct PreorderTree
 {
     const double4* __restrict__ center;
@@ -391,98 +540,15 @@ struct PreorderTree
     const int* n1p = nullptr;   // when given, the end node n1 is read here (a captured graph)
 };
 
-// Stream the j particles of every leaf whose cell overlaps the box (c, e) -- and the
-// region (rc, re), when re.x >= 0, and the rounded box *rbp, when given -- through the
-// group filter into the ring, found by a stackless pre-order scan of the tree 32 nodes at
-// a time (the scan of list_walk_kernel): leaves come out in ascending order, so the
-// stream is in ascending j as a list's is.  Used for groups whose leaf list is far longer
-// than their own search region needs.  A group's cube can hold far more than its rounded
-// box (a large h near the edge of a centrally concentrated set: the cube of a single
-// particle reaches the dense core, its sphere does not), so cells are tested on both.
-template<bool Dbl, bool Float, bool Index, bool Periodic, bool Staged = false, class Ranges, class Filter,
-         class Batch>
-__device__ __forceinline__ void stream_walk(double4* ring, float4* ringf, int* ringIdx, double cx, double cy,
-                                            double cz, double sx, double sy, double sz, const PreorderTree& t,
-                                            double3 c, double3 e, double3 rc, double3 re, double lx, double ly,
-                                            double lz, Ranges ranges, const double4* __restrict__ xyzh,
-                                            Filter filter, Batch batch, StageRef stage = StageRef{nullptr, nullptr, 0},
-                                            const RoundBox* rbp = nullptr)
-{
-    const int lane = threadIdx.x & 31;
-    CandidateRing<Dbl, Float, Index, Staged> cr{ring, ringf, ringIdx, cx, cy, cz, sx, sy, sz, stage};
-    auto fold = [&](double d, double L) { return (Periodic && L > 0.0) ? fmin(d, L - d) : d; };
-    const int n1 = t.n1p != nullptr ? *t.n1p : t.n1;
-    int p = t.n0;
-    while (p < n1)
-    {
-        const int idx = p + lane;
-        const bool valid = idx < n1;
-        bool accept = false;
-        int skip = 1, pl = -1;
-        if (valid)
-        {
-            const double4 nc = t.center[idx];
-            const double4 nh = t.half[idx];
-            accept = fold(fabs(c.x - nc.x), lx) <= e.x + nh.x && fold(fabs(c.y - nc.y), ly) <= e.y + nh.y &&
-                     fold(fabs(c.z - nc.z), lz) <= e.z + nh.z;
-            if (re.x >= 0.0)
-                accept = accept && fold(fabs(rc.x - nc.x), lx) <= re.x + nh.x &&
-                         fold(fabs(rc.y - nc.y), ly) <= re.y + nh.y && fold(fabs(rc.z - nc.z), lz) <= re.z + nh.z;
-            if (rbp != nullptr)
-            {
-                // gap between the rounded box's core and the cell, per axis then squared
-                const RoundBox rb = *rbp;
-                const double gx = fmax(fold(fabs(rb.cx - nc.x), lx) - nh.x - rb.ex, 0.0);
-                const double gy = fmax(fold(fabs(rb.cy - nc.y), ly) - nh.y - rb.ey, 0.0);
-                const double gz = fmax(fold(fabs(rb.cz - nc.z), lz) - nh.z - rb.ez, 0.0);
-                accept = accept && gx * gx + gy * gy + gz * gz <= rb.r * rb.r;
-            }
-            skip = t.skip[idx];
-            pl = t.leaf[idx];
-        }
-        const uint32_t validMask = __ballot_sync(0xffffffffu, valid);
-        const uint32_t rejMask = __ballot_sync(0xffffffffu, valid && !accept);
-        // the reached, accepted leaves of this window, in lane (pre-) order
-        uint32_t emit = 0;
-        int pos = 0, next = p + 32;
-        for (;;)
-        {
-            const uint32_t fromPos = (pos >= 32) ? 0u : (0xffffffffu << pos);
-            const uint32_t rej = rejMask & fromPos;
-            const int r = rej ? (__ffs(rej) - 1) : 32;
-            const uint32_t runMask = validMask & fromPos & ((r >= 32) ? 0xffffffffu : ((1u << r) - 1u));
-            emit |= runMask;
-            if (r >= 32) { next = p + 32; break; }
-            int rskip = __shfl_sync(0xffffffffu, skip, r);
-            if (rskip < 1) rskip = 1;   // a subtree holds its root: the scan always advances
-            const int target = p + r + rskip;
-            if (target >= p + 32 || target >= n1) { next = target; break; }
-            pos = target - p;
-        }
-        emit &= __ballot_sync(0xffffffffu, pl >= 0);
-        if (emit)
-        {
-            // compact the emitted leaves onto the low lanes, keeping their order
-            const bool mineLeaf = (emit >> lane) & 1u;
-            const int nb = __popc(emit);
-            uint2 r = make_uint2(0, 0);
-            if (mineLeaf) r = ranges(pl);
-            // lane k takes the k-th emitted leaf's range
-            const unsigned src = __fns(emit, 0, lane + 1);
-            const int sl = src < 32u ? int(src) : 0;
-            const uint32_t rx = __shfl_sync(0xffffffffu, r.x, sl);
-            const uint32_t ry = __shfl_sync(0xffffffffu, r.y, sl);
-            const uint32_t s0 = lane < nb ? rx : 0u, len = lane < nb ? ry - rx : 0u;
-            cr.feed(s0, len, nb, xyzh, filter, batch);
-        }
-        p = next;
-    }
-    cr.finish(batch);
-}
-
 // Where a group's candidates come from: its leaf's j-leaf list (entries jb .. jb + nj of
-// jlist), or, when walk is set, a pre-order scan of the tree for the leaves overlapping
-// the group's own box, within the leaf list's region (rc, re).
+// jlist), or, when walk is set, a stackless pre-order scan of the tree 32 nodes at a time
+// (the scan of list_walk_kernel) for the leaves whose cell overlaps the group's own box --
+// and the leaf list's region (rc, re), when re.x >= 0, and the group's rounded box *rbp,
+// when given.  Leaves come out in ascending order, so the scan's stream is in ascending j
+// as a list's is.  The scan serves groups whose leaf list is far longer than their own
+// search region needs.  A group's cube can hold far more than its rounded box (a large h
+// near the edge of a centrally concentrated set: the cube of a single particle reaches the
+// dense core, its sphere does not), so cells are tested on both.
 template<class Ranges>
 struct GroupSource
 {
@@ -495,20 +561,86 @@ struct GroupSource
     double3 rc, re;
     StageRef stage;   // the warp's bulk-copy stage, or none (direct loads)
 
-    // rbp (when given): the group's rounded box, for the tree scan's cells
     template<bool Dbl, bool Float, bool Index, bool Periodic, bool Staged = false, class Filter, class Batch>
     __device__ __forceinline__ void stream(double4* ring, float4* ringf, int* ringIdx, const GroupBox& bx, double sx,
                                            double sy, double sz, double lx, double ly, double lz, Filter filter,
                                            Batch batch, const RoundBox* rbp = nullptr) const
     {
-        if (walk)
-            stream_walk<Dbl, Float, Index, Periodic, Staged>(ring, ringf, ringIdx, bx.cx, bx.cy, bx.cz, sx, sy, sz, tree,
-                                                     make_double3(bx.cx, bx.cy, bx.cz),
-                                                     make_double3(bx.ex, bx.ey, bx.ez), rc, re, lx, ly, lz, ranges,
-                                                     xyzh, filter, batch, stage, rbp);
-        else
-            stream_ranges<Dbl, Float, Index, Staged>(ring, ringf, ringIdx, bx.cx, bx.cy, bx.cz, sx, sy, sz, jb, nj,
-                                                     jlist, ranges, xyzh, filter, batch, stage);
+        const int lane = threadIdx.x & 31;
+        CandidateRing<Dbl, Float, Index, Staged> cr{ring, ringf, ringIdx, bx.cx, bx.cy, bx.cz, sx, sy, sz, stage};
+        auto fold = [&](double d, double L) { return (Periodic && L > 0.0) ? fmin(d, L - d) : d; };
+        const int n1 = !walk ? 0 : tree.n1p != nullptr ? *tree.n1p : tree.n1;
+        int p = tree.n0;
+        uint32_t lb = 0;
+        bool last = walk ? p >= n1 : nj == 0;
+        while (!last)
+        {
+            uint32_t s0 = 0, len = 0;
+            int nb;
+            if (!walk)
+            {
+                nb = int(min(32u, nj - lb));
+                if (lane < nb)
+                {
+                    const uint2 r = ranges(jlist[jb + lb + lane]);
+                    s0 = r.x;
+                    len = r.y - r.x;
+                }
+                lb += 32;
+                last = lb >= nj;
+            }
+            else
+            {
+                const int idx = p + lane;
+                const bool valid = idx < n1;
+                bool accept = false;
+                int skip = 1, pl = -1;
+                if (valid)
+                {
+                    const double4 nc = tree.center[idx];
+                    const double4 nh = tree.half[idx];
+                    accept = fold(fabs(bx.cx - nc.x), lx) <= bx.ex + nh.x &&
+                             fold(fabs(bx.cy - nc.y), ly) <= bx.ey + nh.y &&
+                             fold(fabs(bx.cz - nc.z), lz) <= bx.ez + nh.z;
+                    if (re.x >= 0.0)
+                        accept = accept && fold(fabs(rc.x - nc.x), lx) <= re.x + nh.x &&
+                                 fold(fabs(rc.y - nc.y), ly) <= re.y + nh.y &&
+                                 fold(fabs(rc.z - nc.z), lz) <= re.z + nh.z;
+                    if (rbp != nullptr)
+                    {
+                        // gap between the rounded box's core and the cell, per axis then squared
+                        const RoundBox rb = *rbp;
+                        const double gx = fmax(fold(fabs(rb.cx - nc.x), lx) - nh.x - rb.ex, 0.0);
+                        const double gy = fmax(fold(fabs(rb.cy - nc.y), ly) - nh.y - rb.ey, 0.0);
+                        const double gz = fmax(fold(fabs(rb.cz - nc.z), lz) - nh.z - rb.ez, 0.0);
+                        accept = accept && gx * gx + gy * gy + gz * gz <= rb.r * rb.r;
+                    }
+                    skip = tree.skip[idx];
+                    pl = tree.leaf[idx];
+                }
+                // the reached, accepted leaves of this window, in lane (pre-) order: those
+                // beyond every earlier rejected node's subtree
+                const int reach = warp_prefix_max(valid && !accept ? lane + max(skip, 1) : 0);
+                const int before = __shfl_up_sync(0xffffffffu, reach, 1);
+                const uint32_t emit = __ballot_sync(0xffffffffu, accept && pl >= 0 && (lane == 0 || before <= lane));
+                p += max(32, __shfl_sync(0xffffffffu, reach, 31));
+                last = p >= n1;
+                if (!emit && !last) continue;
+                // compact the emitted leaves onto the low lanes, keeping their order
+                nb = __popc(emit);
+                uint2 r = make_uint2(0, 0);
+                if ((emit >> lane) & 1u) r = ranges(pl);
+                // lane k takes the k-th emitted leaf's range
+                const unsigned src = __fns(emit, 0, lane + 1);
+                const int sl = src < 32u ? int(src) : 0;
+                const uint32_t rx = __shfl_sync(0xffffffffu, r.x, sl);
+                const uint32_t ry = __shfl_sync(0xffffffffu, r.y, sl);
+                s0 = lane < nb ? rx : 0u;
+                len = lane < nb ? ry - rx : 0u;
+            }
+            cr.feed(s0, len, nb, xyzh, filter, batch, last);
+        }
+        if constexpr (Staged) cr.finish(batch);
     }
 };
 
@@ -629,7 +761,32 @@ struct KahanF
         c = (t - s) - y;
         s = t;
     }
+    // the same where x is a product the compiler could otherwise fuse into the subtraction
+    __device__ __forceinline__ void add_rn(float x)
+    {
+        const float y = __fsub_rn(x, c);
+        const float t = __fadd_rn(s, y);
+        c = __fsub_rn(__fsub_rn(t, s), y);
+        s = t;
+    }
     __device__ __forceinline__ double value() const { return double(s) - double(c); }
+};
+
+// Two such sums in packed arithmetic: c holds what KahanF's does, negated (the same
+// roundings, which are symmetric), and t - s is formed as fma(s, -1, t).
+struct KahanF2
+{
+    float2 s = make_float2(0.0f, 0.0f), c = make_float2(0.0f, 0.0f);
+    __device__ __forceinline__ void add(float a, float b)
+    {
+        const float2 m = make_float2(-1.0f, -1.0f);
+        const float2 y = __fadd2_rn(make_float2(a, b), c);
+        const float2 t = __fadd2_rn(s, y);
+        c = __ffma2_rn(__ffma2_rn(s, m, t), m, y);
+        s = t;
+    }
+    __device__ __forceinline__ double first() const { return double(s.x) + double(c.x); }
+    __device__ __forceinline__ double second() const { return double(s.y) + double(c.y); }
 };
 
 // The SPH kernel in FP32 (same polynomials as sph_kernel).

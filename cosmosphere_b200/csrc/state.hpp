@@ -271,6 +271,7 @@ struct State
     DBuf<int> childOffsets, internalToLeaf, levelRange, leafToInternal;
     DBuf<double> centers, sizes;                // 3 per BFS node
     DBuf<double4> preCenter, preHalf;           // pre-order copies for the walk
+    DBuf<float4> leafBox;                       // the leaves' bounding boxes, centre and half extents
     DBuf<double> hmaxLeaf, hmaxNode, hmaxPre;
     DBuf<uint32_t> jcount, jOffset;
     DBuf<uint32_t> jstream;                     // particles in each leaf's gather list

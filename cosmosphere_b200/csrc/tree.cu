@@ -16,6 +16,7 @@
  */
 #include <algorithm>
 
+#include "pairstream.cuh"
 #include "sort.cuh"
 #include "state.hpp"
 
@@ -389,6 +390,13 @@ __global__ void bfs_link_kernel(const uint64_t* __restrict__ bfsPrefix, const in
     preHalf[pre] = make_double4(s[0], s[1], s[2], 0.0);
 }
 
+__global__ void leaf_box_kernel(const uint32_t* __restrict__ layout, int nL, const double4* __restrict__ xyzh,
+                                float4* __restrict__ leafBox)
+{
+    const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l < nL) leaf_box(xyzh, layout[l], layout[l + 1], leafBox + 2 * size_t(l));
+}
+
 __global__ void particle_leaf_kernel(const uint32_t* __restrict__ layout, int nL, int nAliveMax,
                                      const DevScalars* __restrict__ ds, int* __restrict__ particleLeaf)
 {
@@ -608,44 +616,33 @@ list_walk_kernel(int nL, int numNodes, const int* __restrict__ leafToInternal,
             skip = preSkip[idx];
             pl = preLeaf[idx];
         }
-        const uint32_t validMask = __ballot_sync(0xffffffffu, valid);
-        const uint32_t rejMask = __ballot_sync(0xffffffffu, valid && !accept);
-        // Walk the window: runs of reached nodes end at a rejection, after which the scan
-        // jumps over that node's subtree; a jump that lands inside the window continues.
-        int pos = 0;        // offset of the next reached node in this window
-        int next = p + 32;  // where the following window starts
-        for (;;)
+        // The window: a node is reached unless it lies in a rejected node's subtree (a
+        // rejected node that is itself not reached lies, subtree and all, in one that
+        // is), so the reached nodes are those beyond every earlier rejected subtree's
+        // end -- a prefix maximum over the lanes, where following the rejections one
+        // after the other took 25 instructions each -- and the next window starts
+        // beyond them all.
+        const int end = valid && !accept ? lane + max(skip, 1) : 0;   // a subtree holds its root
+        const int reach = warp_prefix_max(end);
+        const int before = __shfl_up_sync(0xffffffffu, reach, 1);
+        const bool emit = accept && pl >= 0 && (lane == 0 || before <= lane);
+        const uint32_t emitMask = __ballot_sync(0xffffffffu, emit);
+        if (emit)
         {
-            const uint32_t fromPos = (pos >= 32) ? 0u : (0xffffffffu << pos);
-            const uint32_t rej = rejMask & fromPos;
-            const int r = rej ? (__ffs(rej) - 1) : 32;
-            // lanes [pos, r) are reached and accepted
-            const uint32_t runMask = validMask & fromPos & ((r >= 32) ? 0xffffffffu : ((1u << r) - 1u));
-            const uint32_t emitMask = __ballot_sync(0xffffffffu, ((runMask >> lane) & 1u) && pl >= 0);
+            const uint32_t slot = count + __popc(emitMask & lt);
             if (Fill)
             {
-                if ((emitMask >> lane) & 1u)
-                {
-                    const uint32_t slot = count + __popc(emitMask & lt);
-                    if (slot < cap) jlist[base + slot] = pl;
-                    else atomicOr(err, int(kErrListCap));
-                }
+                if (slot < cap) jlist[base + slot] = pl;
+                else atomicOr(err, int(kErrListCap));
             }
-            else if ((emitMask >> lane) & 1u)
+            else
             {
                 if (jstream != nullptr) stream += layout[pl + 1] - layout[pl];
-                const uint32_t slot = count + __popc(emitMask & lt);
                 if (scratch != nullptr && slot < uint32_t(kWalkScratch)) scratch[leaf * kWalkScratch + slot] = pl;
             }
-            count += __popc(emitMask);
-            if (r >= 32) { next = p + 32; break; }
-            int rskip = __shfl_sync(0xffffffffu, skip, r);
-            if (rskip < 1) rskip = 1;   // a subtree holds its root: the scan always advances
-            const int target = p + r + rskip;
-            if (target >= p + 32 || target >= numNodes) { next = target; break; }
-            pos = target - p;
         }
-        p = next;
+        count += __popc(emitMask);
+        p += max(32, __shfl_sync(0xffffffffu, reach, 31));
         // A count walk with a stream cap stops once the list streams more than the cap:
         // such a leaf is cut into one-particle groups that scan the tree for their own
         // spheres (the cut gives one particle per group at any stream above the cut's
@@ -1057,6 +1054,9 @@ void build_leaves(State& s)
         s.centers.get(), s.sizes.get(), s.preCenter.get(), s.preHalf.get());
     COSMO_LAUNCHED();
     particle_leaf_kernel<<<iceil(n, kBlk), kBlk, 0, s.st>>>(s.layout.get(), nL, n, ds, s.particleLeaf.get());
+    COSMO_LAUNCHED();
+    s.leafBox.resize(2 * size_t(nL), s.st);
+    leaf_box_kernel<<<iceil(nL, 128), 128, 0, s.st>>>(s.layout.get(), nL, s.xyzh.get(), s.leafBox.get());
     COSMO_LAUNCHED();
     s.hmaxLeaf.resize(nL, s.st);
     s.hmaxNode.resize(numNodes, s.st);
