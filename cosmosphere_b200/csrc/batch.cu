@@ -99,11 +99,12 @@ __global__ void setof_kernel(const int* __restrict__ offs, int nsets, int n, int
 // single-set build (src/tree.cu:54-72) over this set's particles.
 __global__ void set_box_kernel_b(const int* __restrict__ offs, const int* __restrict__ per,
                                  const double* __restrict__ box6, const double* __restrict__ x,
-                                 const double* __restrict__ y, const double* __restrict__ z, DevBox* __restrict__ boxes)
+                                 const double* __restrict__ y, const double* __restrict__ z, DevBox* __restrict__ boxes, int* outside)
 {
     const int s = blockIdx.x;
     const int a = offs[s], b = offs[s + 1];
     __shared__ double sm[32][6];
+    if (s == 0 && threadIdx.x == 0) *outside = 0;
     if (per[s])
     {
         if (threadIdx.x == 0)
@@ -157,15 +158,18 @@ __global__ void set_box_kernel_b(const int* __restrict__ offs, const int* __rest
 
 __global__ void keys_kernel_b(const double* __restrict__ x, const double* __restrict__ y,
                               const double* __restrict__ z, const double* __restrict__ h, const int* __restrict__ setOf,
-                              int n, const DevBox* __restrict__ boxes, uint64_t* __restrict__ keys)
+                              int n, const DevBox* __restrict__ boxes, uint64_t* __restrict__ keys, int* outside)
 {
     const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const DevBox b = boxes[setOf[i]];
     uint64_t k = kDeadKey;
     if (h[i] > 0.0)
+    {
         k = hilbert_key(quantise(x[i], b.lo[0], b.scale[0]), quantise(y[i], b.lo[1], b.scale[1]),
                         quantise(z[i], b.lo[2], b.scale[2]));
+        if (box_left(b, x[i], y[i], z[i], h[i])) *outside = 1;
+    }
     keys[i] = k;
 }
 
@@ -705,10 +709,10 @@ static void batch_sort(Batch& B)
     DevScalars* ds = s.dscal.get();
     B.forestDone = false;
     set_box_kernel_b<<<ns, 256, 0, s.st>>>(B.dOffs.get(), B.setPer.get(), B.setBox6.get(), B.ux.get(), B.uy.get(),
-                                           B.uz.get(), B.boxes.get());
+                                           B.uz.get(), B.boxes.get(), &ds->outside);
     COSMO_LAUNCHED();
     keys_kernel_b<<<iceil(n, kBlk), kBlk, 0, s.st>>>(B.ux.get(), B.uy.get(), B.uz.get(), B.uh.get(), B.setOf.get(), n,
-                                                    B.boxes.get(), B.keysA.get());
+                                                    B.boxes.get(), B.keysA.get(), &ds->outside);
     COSMO_LAUNCHED();
     // stable key sort (8 passes), then stable set-id passes: (set, key) order
     radix_sort_u64(s, B.keysA.get(), B.keysB.get(), B.orderA.get(), B.orderB.get(), n, true);
@@ -982,7 +986,7 @@ static int batch_solve_near(Batch& B, double tolh, double hfact, int maxIter, in
     return B.unconverged > 0 ? 1 : 0;
 }
 
-static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int flags, int attempt = 0)
+static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int flags, int attempt = 0, bool lists = false)
 {
     State& s = B.core;
     if (!(hfact > 0.0)) hfact = kHfactDefault;
@@ -997,8 +1001,13 @@ static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int fla
     batch_sort(B);
     // The plain form runs over the sets' block trees (the mixed form's rounding is defined by
     // the group engine's groups; the staged feed is a variant of that engine).  Its rows take
-    // 1 KB a particle: very large batches keep the lists, which take less.
-    if (s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost) return batch_solve_near(B, tolh, hfact, maxIter, flags, t0);
+    // 1 KB a particle: very large batches keep the lists, which take less.  A batch with a
+    // particle outside its set's box is solved over the lists (solve_density).
+    if (!lists && s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost)
+    {
+        const int st = batch_solve_near(B, tolh, hfact, maxIter, flags, t0);
+        return s.hscal->outside ? batch_solve(B, tolh, hfact, maxIter, flags, 0, true) : st;
+    }
     batch_forest(B);
     const int L = B.nLeaves;
     long long nAliveTotal = 0;
@@ -1079,7 +1088,7 @@ static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int fla
     if ((s.hscal->err & kErrListFull) && attempt < 6)
     {
         COSMO_CUDA(cudaMemsetAsync(&ds->err, 0, sizeof(int), s.st));
-        return batch_solve(B, tolh, hfact, maxIter, flags, attempt + 1);
+        return batch_solve(B, tolh, hfact, maxIter, flags, attempt + 1, lists);
     }
     LoopState fin{};
     COSMO_CUDA(cudaMemcpyAsync(&fin, B.loop.get(), sizeof(LoopState), cudaMemcpyDeviceToHost, s.st));

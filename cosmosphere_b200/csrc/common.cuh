@@ -200,6 +200,17 @@ struct DevBox
     int periodic;
 };
 
+// Whether a particle lies outside the box its key is quantised in by more than a hundredth of
+// its h on some axis.  Its key is then that of an edge cell that does not hold it.  (No
+// particle of an open set with its own extents does, nor does one that has just drifted
+// over a periodic face.)
+__device__ __forceinline__ bool box_left(const DevBox& b, double x, double y, double z, double h)
+{
+    const double m = 0.01 * h;
+    return x < b.lo[0] - m || x > b.hi[0] + m || y < b.lo[1] - m || y > b.hi[1] + m || z < b.lo[2] - m ||
+           z > b.hi[2] + m;
+}
+
 __host__ __device__ inline void box_finish(DevBox& b)
 {
     for (int d = 0; d < 3; ++d)

@@ -1213,7 +1213,7 @@ static bool near_solve(const State& s, bool withGradients)
 }
 
 DensResult solve_density(State& s, int n, double pmass, const double* periodicBox, double tolh, double hfact,
-                         int maxIter, bool withGradients, bool allowGraph)
+                         int maxIter, bool withGradients, bool allowGraph, bool lists)
 {
     DensResult res{0, 0, 0};
     if (!(hfact > 0.0)) hfact = kHfactDefault;
@@ -1233,9 +1233,16 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     // next few solves do not write them.
     const bool tryRows = s.symRowsSkip == 0;
     if (s.symRowsSkip > 0) --s.symRowsSkip;
-    const bool near = near_solve(s, withGradients);
+    const bool near = !lists && near_solve(s, withGradients);
     const bool writeJ = near ? s.symFromRows != 0
                              : withGradients && s.symFromRows && s.frozenFor != n && tryRows;
+
+    // A particle outside the box lies in no cell of the leaf tree that its key puts it in, and
+    // the lists (as the reference's do) may miss its pairs, which the block tree, whose boxes
+    // are the particles' own, finds: such a solve is made over the lists.
+    auto onLists = [&]() {
+        return solve_density(s, n, pmass, periodicBox, tolh, hfact, maxIter, withGradients, allowGraph, true);
+    };
 
     // the tree; its particle gather also zeroes rho, gradh, the convergence flags, the
     // Newton rows' h (0: no row this solve) and the pair counters
@@ -1255,6 +1262,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         {
             read_scalars(s);
             s.nAlive = s.hscal->nAlive;
+            if (s.hscal->outside) return onLists();
         }
     }
     const int itemCap = std::max(s.nAlive, 1);
@@ -1537,6 +1545,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         if (near)
         {
             check_dev_err(s, "solveDensH", false);
+            if (s.hscal->outside) return onLists();
             tree_timings(s);
             s.nAlive = s.hscal->nAlive;
             nActiveParticles = near_results(s, nl);

@@ -108,6 +108,7 @@ struct DevScalars
     int leafStart;               // leaves of the grid the leaf tree's refinement starts from
     int leafDone;                // that grid is the leaf tree (no node of it holds more than kBucket)
     unsigned long long hmaxConv; // bits of the largest converged h (the block-tree loop)
+    int outside;                 // some live particle lies outside the box its key is taken in (box_left)
 };
 
 // The single-set Newton loop run as a graph: what the host loop kept in host variables
@@ -357,7 +358,7 @@ long long near_results(State& s, const NearLoop& h);   // particles left unconve
 struct DensResult { int itersRun; int unconverged; int status; };
 // allowGraph = false keeps the Newton loop on the host (the graph loop's fallback).
 DensResult solve_density(State& s, int n, double pmass, const double* periodicBox, double tolh,
-                         double hfact, int maxIter, bool withGradients, bool allowGraph = true);
+                         double hfact, int maxIter, bool withGradients, bool allowGraph = true, bool lists = false);
 
 // mixed.cu
 void launch_gradient_mixed(State& s, double pmass);

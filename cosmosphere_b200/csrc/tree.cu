@@ -67,8 +67,9 @@ __global__ void set_extent_kernel(double* part, double x0, double x1, double y0,
     part[3] = x1; part[4] = y1; part[5] = z1;
 }
 
-__global__ void bbox_final_kernel(const double* __restrict__ part, int nb, DevBox* box)
+__global__ void bbox_final_kernel(const double* __restrict__ part, int nb, DevBox* box, int* outside = nullptr)
 {
+    if (outside && threadIdx.x == 0) *outside = 0;
     // one warp: lanes stride over the block partials, then a shuffle reduction (min and
     // max are exact, so any order gives the serial result)
     const int lane = threadIdx.x & 31;
@@ -101,9 +102,11 @@ __global__ void bbox_final_kernel(const double* __restrict__ part, int nb, DevBo
     *box = b;
 }
 
-__global__ void set_box_kernel(double x0, double x1, double y0, double y1, double z0, double z1, DevBox* box)
+__global__ void set_box_kernel(double x0, double x1, double y0, double y1, double z0, double z1, DevBox* box,
+                               int* outside = nullptr)
 {
     if (threadIdx.x != 0) return;
+    if (outside) *outside = 0;
     DevBox b;
     b.lo[0] = x0; b.hi[0] = x1; b.lo[1] = y0; b.hi[1] = y1; b.lo[2] = z0; b.hi[2] = z1;
     b.periodic = 1;
@@ -113,15 +116,18 @@ __global__ void set_box_kernel(double x0, double x1, double y0, double y1, doubl
 
 __global__ void keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, const double* __restrict__ h, int n,
-                            const DevBox* __restrict__ box, uint64_t* __restrict__ keys)
+                            const DevBox* __restrict__ box, uint64_t* __restrict__ keys, int* outside = nullptr)
 {
     const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const DevBox b = *box;
     uint64_t k = kDeadKey;
     if (h[i] > 0.0)
+    {
         k = hilbert_key(quantise(x[i], b.lo[0], b.scale[0]), quantise(y[i], b.lo[1], b.scale[1]),
                         quantise(z[i], b.lo[2], b.scale[2]));
+        if (outside && box_left(b, x[i], y[i], z[i], h[i])) *outside = 1;
+    }
     keys[i] = k;
 }
 
@@ -936,7 +942,7 @@ void build_order(State& s, const double* periodicBox, bool alsoSortVA, bool rows
     if (periodicBox)
     {
         set_box_kernel<<<1, 32, 0, s.st>>>(periodicBox[0], periodicBox[1], periodicBox[2], periodicBox[3],
-                                            periodicBox[4], periodicBox[5], s.box.get());
+                                            periodicBox[4], periodicBox[5], s.box.get(), &ds->outside);
     }
     else if (s.keyExtentSet)
     {
@@ -946,7 +952,7 @@ void build_order(State& s, const double* periodicBox, bool alsoSortVA, bool rows
         const double* e = s.keyExtent;
         set_extent_kernel<<<1, 32, 0, s.st>>>(s.redTmp.get(), e[0], e[1], e[2], e[3], e[4], e[5]);
         COSMO_LAUNCHED();
-        bbox_final_kernel<<<1, 32, 0, s.st>>>(s.redTmp.get(), 1, s.box.get());
+        bbox_final_kernel<<<1, 32, 0, s.st>>>(s.redTmp.get(), 1, s.box.get(), &ds->outside);
     }
     else
     {
@@ -954,14 +960,14 @@ void build_order(State& s, const double* periodicBox, bool alsoSortVA, bool rows
         s.redTmp.resize(size_t(nb) * 6, s.st);
         bbox_partial_kernel<<<nb, kBlk, 0, s.st>>>(s.ux.get(), s.uy.get(), s.uz.get(), n, s.redTmp.get());
         COSMO_LAUNCHED();
-        bbox_final_kernel<<<1, 32, 0, s.st>>>(s.redTmp.get(), nb, s.box.get());
+        bbox_final_kernel<<<1, 32, 0, s.st>>>(s.redTmp.get(), nb, s.box.get(), &ds->outside);
     }
     COSMO_LAUNCHED();
     cudaEvent_t e1 = ev(s);
 
     // keys and sort (src/tree.cu:82-108)
     keys_kernel<<<iceil(n, kBlk), kBlk, 0, s.st>>>(s.ux.get(), s.uy.get(), s.uz.get(), s.uh.get(), n,
-                                                  s.box.get(), s.keysA.get());
+                                                  s.box.get(), s.keysA.get(), &ds->outside);
     COSMO_LAUNCHED();
     radix_sort_u64(s, s.keysA.get(), s.keysB.get(), s.orderA.get(), s.orderB.get(), n, true);
     alive_kernel<<<iceil(n, kBlk), kBlk, 0, s.st>>>(s.keysA.get(), n, ds);
