@@ -5,7 +5,9 @@
  * The sets are concatenated set-major (set s owns [off[s], off[s+1])).  Each set keeps its
  * own box, keys, leaf tree (split while a node holds more than that set's bucket size),
  * pre-order node range and j-leaf lists; a set's leaves and nodes are contiguous in the
- * forest and its walks never leave its node range.  The Newton kernel takes i-leaves
+ * forest and its walks never leave its node range.  Plain batches run over their sets' block
+ * trees instead (near.cu); the forest is then made only for its counts, when they are asked
+ * for.  The Newton kernel of the others takes i-leaves
  * from all sets through one work list; each leaf carries its set's mass, periodicity and
  * box.  Per particle, the arithmetic is the single-set form's (plain FP64 or mixed), and
  * the j order is ascending sorted index, so a set solved in a batch gives the same h and

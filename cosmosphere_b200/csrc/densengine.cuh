@@ -24,9 +24,8 @@
  *          With the records of the plain form the owners' serial additions ran over a
  *          batch's longest list while most lanes had none: they were two fifths of the
  *          kernel's instructions, the FP64 filter over whole lists most of the rest
- *          (a solve of 40 sets of 10,000 to 300,000: 51.8 -> 34.1 ms in this kernel; first
- *          iteration of a 300,000-particle box 663 -> 550 us, 1670 -> 1200 instructions a
- *          particle).  The batch code is the kernel's largest loop and stays there once:
+ *          (a solve of 40 sets of 10,000 to 300,000: 65.5 -> 46.4 ms; the Newton loop of a
+ *          300,000-particle box 3.65 -> 3.15).  The batch code is the kernel's largest loop and stays there once:
  *          four copies of it stalled two issues in three on the instruction cache.
  */
 #pragma once
@@ -41,6 +40,16 @@ constexpr int kRec = 256;   // pair records per warp
 // records (mixed: the ring and the columns), and at kBoxAt the group's rounded box (read by the filter from shared memory
 // rather than held in registers through the stream).
 constexpr int kTest = 8;     // mixed: candidates a lane tests in one turn of its loop
+// Mixed: a group of at most kFew particles (a leaf's last, or a cut group, which has
+// thousands of candidates) is tested with a candidate a lane, and its kept pairs are evaluated
+// by all lanes and only added by their owners: with a particle a lane most lanes had nothing
+// to test or evaluate (the loop of a 30,000-particle Plummer sphere 16.9 -> 12.9 ms, 9 sets of
+// 6,000 to 18,000 8.5 -> 7.1, 40 sets of 10,000 to 300,000 48.1 -> 46.4; lines at 12 and 16
+// instead measured no better).  Its columns lie one after the other, with as much room again
+// for the second term: 126 pairs of two terms for each of eight particles fit in the columns'
+// 2048 words beside the particles' own data, and 252 words a particle keep the owners'
+// accesses on different banks.
+constexpr int kFew = 8;
 constexpr int kColumn = 64;   // mixed: accepted pairs a lane keeps before they are evaluated
 
 template<bool Mixed>
@@ -213,7 +222,13 @@ __device__ __forceinline__ void density_group(unsigned char* scr, bool mine, int
     else
     {
         float* rx = reinterpret_cast<float*>(scr);   // the candidates' -x, -y, -z, kRing each
-        float* column = rx + 3 * kRing + lane;       // q^2 of accepted pair t at column[32 t]
+        // q^2 of accepted pair t at column[t * step]: interleaved by lanes, or, of a few
+        // particles, one after the other with as much room again for the second term
+        const bool few = ng <= kFew;
+        float* columns = rx + 3 * kRing;
+        const int room = few ? 126 : kColumn;
+        float* column = columns + (few ? 2 * room * lane : lane);
+        float* member = columns + kColumn * 32 - 4 * kFew;   // few: x, y, z, 1/h^2 of kFew each
         // relative coordinates at the centre's nearest image are every accepted pair's
         // nearest image when the box (search spheres included) spans under half a period
         const bool shifted = !Periodic || lx == 0.0 || (bx.ex < 0.5 * lx && bx.ey < 0.5 * ly && bx.ez < 0.5 * lz);
@@ -226,19 +241,152 @@ __device__ __forceinline__ void density_group(unsigned char* scr, bool mine, int
         const float2 gx2 = make_float2(gx, gx), gy2 = make_float2(gy, gy), gz2 = make_float2(gz, gz);
         const float2 gh2 = make_float2(gh, gh);
         const float Lx = float(lx), Ly = float(ly), Lz = float(lz);
-        KahanF lr, lg;
+        if (ng == 1)
+        {
+            // A single particle (mostly a cut group, of thousands of candidates, alone on its
+            // multiprocessor at the end of an iteration): the p-th candidate that passes the
+            // filter belongs to lane p mod 32, which keeps its own compensated partial sums,
+            // combined in FP64 at the end.  A pair is evaluated where it was loaded and its
+            // terms handed over, so four loads of 32 run side by side: one after the other
+            // (through the ring) each waits out the last one's arithmetic (six mixed sets of
+            // 6,000 to 114,000 particles: 12.9 -> 11.1 ms).
+            const float x0 = __shfl_sync(0xffffffffu, gx, 0), y0 = __shfl_sync(0xffffffffu, gy, 0);
+            const float z0 = __shfl_sync(0xffffffffu, gz, 0), h0 = __shfl_sync(0xffffffffu, gh, 0);
+            const float none = __int_as_float(0x7fc00000);
+            const uint32_t lt = (1u << lane) - 1u;
+            float2* terms = reinterpret_cast<float2*>(scr);   // [4][32], by owner
+            KahanF2 one;
+            uint32_t passed = 0;
+            src.template for_ranges<Periodic>(bx, lx, ly, lz, rbp, [&](uint32_t s0, uint32_t len, int nb, bool) {
+                const uint32_t incl = warp_incl_scan_u32(len);
+                const uint32_t excl = incl - len;
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                for (uint32_t p0 = 0; p0 < total; p0 += 128)
+                {
+                    double4 pj[4];
+                    bool pass[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                    {
+                        const uint32_t p = p0 + 32 * u + lane;
+                        int t = 0;
+#pragma unroll
+                        for (int step = 16; step > 0; step >>= 1)
+                        {
+                            const uint32_t e = __shfl_sync(0xffffffffu, excl, (t + step) & 31);
+                            if (t + step < nb && e <= p) t += step;
+                        }
+                        const uint32_t j =
+                            __shfl_sync(0xffffffffu, s0, t) + (p - __shfl_sync(0xffffffffu, excl, t));
+                        pass[u] = p < total;
+                        pj[u] = make_double4(0, 0, 0, 0);
+                        if (pass[u]) pj[u] = ldg4(src.xyzh + j);
+                    }
+                    uint32_t m[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                    {
+                        pass[u] = pass[u] && gather(pj[u]);
+                        m[u] = __ballot_sync(0xffffffffu, pass[u]);
+                    }
+                    uint32_t at[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                    {
+                        at[u] = passed;
+                        passed += __popc(m[u]);
+                        const float fx = float(image_offset(pj[u].x, bx.cx, sx));
+                        const float fy = float(image_offset(pj[u].y, bx.cy, sy));
+                        const float fz = float(image_offset(pj[u].z, bx.cz, sz));
+                        float dx = x0 - fx, dy = y0 - fy, dz = z0 - fz;
+                        if (Periodic && !shifted)
+                        {
+                            dx = axis_df<true>(x0, fx, Lx);
+                            dy = axis_df<true>(y0, fy, Ly);
+                            dz = axis_df<true>(z0, fz, Lz);
+                        }
+                        const float q2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) * h0;
+                        const bool acc = pass[u] && q2 < float(kRadK2);
+                        float2 v = make_float2(none, 0.0f);
+                        if (acc)
+                        {
+                            const float q = sqrt_q(q2);
+                            float wk, dwk;
+                            sph_kernel_f(q2, q, wk, dwk);
+                            v = make_float2(wk, fmaf(-q, dwk, -3.0f * wk));
+                        }
+                        if (pass[u]) terms[32 * u + ((at[u] + __popc(m[u] & lt)) & 31)] = v;
+                        gp += __popc(__ballot_sync(0xffffffffu, acc));
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (((lane - at[u]) & 31u) < uint32_t(__popc(m[u])))
+                        {
+                            const float2 v = terms[32 * u + lane];
+                            if (v.x == v.x) one.add(v.x, v.y);
+                        }
+                    __syncwarp();
+                }
+            });
+            gc = passed;
+            double a = one.first(), b = one.second();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                a += __shfl_xor_sync(0xffffffffu, a, o);
+                b += __shfl_xor_sync(0xffffffffu, b, o);
+            }
+            rhoi = a;
+            gradhi = b;
+            return;
+        }
+        if (few)
+        {
+            if (lane < kFew)
+            {
+                member[lane] = gx;
+                member[kFew + lane] = gy;
+                member[2 * kFew + lane] = gz;
+                member[3 * kFew + lane] = gh;
+            }
+            __syncwarp();
+        }
         KahanF2 sums;
         int kept = 0;
         auto evaluate = [&]() {
-#pragma unroll 2
-            for (int t = 0; t < kept; ++t)
+            if (few)
             {
-                const float q2 = column[32 * t];
-                const float q = sqrt_q(q2);
-                float wk, dwk;
-                sph_kernel_f(q2, q, wk, dwk);
-                sums.add(wk, fmaf(-q, dwk, -3.0f * wk));
+                // every lane evaluates, the owners add
+                __syncwarp();
+                for (int i = 0; i < ng; ++i)
+                {
+                    const int c = __shfl_sync(0xffffffffu, kept, i);
+                    float* w = columns + 2 * room * i;
+                    for (int t = lane; t < c; t += 32)
+                    {
+                        const float q2 = w[t];
+                        const float q = sqrt_q(q2);
+                        float wk, dwk;
+                        sph_kernel_f(q2, q, wk, dwk);
+                        w[t] = wk;
+                        w[room + t] = fmaf(-q, dwk, -3.0f * wk);
+                    }
+                }
+                __syncwarp();
+#pragma unroll 4
+                for (int t = 0; t < kept; ++t) sums.add(column[t], column[room + t]);
             }
+            else
+#pragma unroll 2
+                for (int t = 0; t < kept; ++t)
+                {
+                    const float q2 = column[32 * t];
+                    const float q = sqrt_q(q2);
+                    float wk, dwk;
+                    sph_kernel_f(q2, q, wk, dwk);
+                    sums.add(wk, fmaf(-q, dwk, -3.0f * wk));
+                }
             gp += kept;
             kept = 0;
             __syncwarp();
@@ -247,39 +395,56 @@ __device__ __forceinline__ void density_group(unsigned char* scr, bool mine, int
             nullptr, reinterpret_cast<float4*>(rx), nullptr, bx, sx, sy, sz, lx, ly, lz, gather,
             [&](const double4*, const float4*, const int*, int head, int count) {
                 gc += count;
-                if (ng == 1)
-                {
-                    // a single particle (a cut group): every lane keeps its own compensated
-                    // partial sums, combined in FP64 after the stream
-                    const int at = (head + (lane < count ? lane : 0)) & (kRing - 1);
-                    const float fx = rx[at], fy = rx[kRing + at], fz = rx[2 * kRing + at];
-                    const float x0 = __shfl_sync(0xffffffffu, gx, 0), y0 = __shfl_sync(0xffffffffu, gy, 0);
-                    const float z0 = __shfl_sync(0xffffffffu, gz, 0), h0 = __shfl_sync(0xffffffffu, gh, 0);
-                    float dx = x0 + fx, dy = y0 + fy, dz = z0 + fz;
-                    if (Periodic && !shifted)
-                    {
-                        dx = axis_df<true>(x0, -fx, Lx);
-                        dy = axis_df<true>(y0, -fy, Ly);
-                        dz = axis_df<true>(z0, -fz, Lz);
-                    }
-                    const float q2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) * h0;
-                    const bool acc = lane < count && q2 < float(kRadK2);
-                    if (acc)
-                    {
-                        const float q = sqrt_q(q2);
-                        float wk, dwk;
-                        sph_kernel_f(q2, q, wk, dwk);
-                        lr.add_rn(wk);
-                        lg.add_rn(fmaf(-q, dwk, -3.0f * wk));
-                    }
-                    gp += __popc(__ballot_sync(0xffffffffu, acc));
-                    return;
-                }
                 // full batches start at a multiple of 32; a partial (last) one is filled up
                 // with candidates infinitely far the other way
                 if (lane >= count) rx[(head + lane) & (kRing - 1)] = inf;
                 __syncwarp();
-                if (__any_sync(0xffffffffu, kept > kColumn - 32)) evaluate();
+                if (__any_sync(0xffffffffu, kept > room - 32)) evaluate();
+                if (few)
+                {
+                    // a candidate a lane (none beyond count: infinitely far), two particles
+                    // a packed instruction
+                    const int at = (head + lane) & (kRing - 1);
+                    const float fx = rx[at], fy = rx[kRing + at], fz = rx[2 * kRing + at];
+                    const uint32_t lt = (1u << lane) - 1u;
+                    for (int i0 = 0; i0 < ng; i0 += 2)
+                    {
+                        const float2 mx = *reinterpret_cast<const float2*>(member + i0);
+                        const float2 my = *reinterpret_cast<const float2*>(member + kFew + i0);
+                        const float2 mz = *reinterpret_cast<const float2*>(member + 2 * kFew + i0);
+                        const float2 mh = *reinterpret_cast<const float2*>(member + 3 * kFew + i0);
+                        float2 q2;
+                        if (!Periodic || shifted)
+                        {
+                            const float2 dx = __fadd2_rn(mx, make_float2(fx, fx));
+                            const float2 dy = __fadd2_rn(my, make_float2(fy, fy));
+                            const float2 dz = __fadd2_rn(mz, make_float2(fz, fz));
+                            float2 r2 = __fmul2_rn(dx, dx);
+                            r2 = __ffma2_rn(dy, dy, r2);
+                            r2 = __ffma2_rn(dz, dz, r2);
+                            q2 = __fmul2_rn(r2, mh);
+                        }
+                        else
+                        {
+                            const float ax = axis_df<true>(mx.x, -fx, Lx), bx = axis_df<true>(mx.y, -fx, Lx);
+                            const float ay = axis_df<true>(my.x, -fy, Ly), by = axis_df<true>(my.y, -fy, Ly);
+                            const float az = axis_df<true>(mz.x, -fz, Lz), bz = axis_df<true>(mz.y, -fz, Lz);
+                            q2 = make_float2(fmaf(az, az, fmaf(ay, ay, ax * ax)) * mh.x,
+                                             fmaf(bz, bz, fmaf(by, by, bx * bx)) * mh.y);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 2; ++u)
+                        {
+                            const float v = u ? q2.y : q2.x;
+                            const bool acc = v < float(kRadK2);
+                            const uint32_t m = __ballot_sync(0xffffffffu, acc);
+                            const int base = __shfl_sync(0xffffffffu, kept, i0 + u);
+                            if (acc) columns[2 * room * (i0 + u) + base + __popc(m & lt)] = v;
+                            if (lane == i0 + u) kept += __popc(m);
+                        }
+                    }
+                    return;
+                }
                 float* put = column + 32 * kept;
                 const float* cand = rx + (head & (kRing - 1));
 #pragma unroll 1
@@ -336,18 +501,6 @@ __device__ __forceinline__ void density_group(unsigned char* scr, bool mine, int
         evaluate();
         rhoi = sums.first();
         gradhi = sums.second();
-        if (ng == 1)
-        {
-            double a = lr.value(), b = lg.value();
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-            {
-                a += __shfl_xor_sync(0xffffffffu, a, o);
-                b += __shfl_xor_sync(0xffffffffu, b, o);
-            }
-            rhoi = a;
-            gradhi = b;
-        }
     }
 }
 

@@ -2,6 +2,10 @@
  * density.cu -- the Newton-Raphson smoothing-length / density solve and the
  * post-convergence gradient sweep (the reference's src/density_base.cu:237-334, 511-1015).
  *
+ * A plain solve with gradients runs its Newton loop over the block tree (near.cu); what is
+ * here of it are the passes over its rows.  The list-based loop, which the mixed form, solves
+ * without gradients and the variants' options keep:
+ *
  * One warp per i-leaf.  The leaf's unconverged particles are packed onto the lanes
  * (ballot + __fns), every lane walks the leaf's j-leaf list in ascending order, so each
  * particle's sums run over j in ascending Hilbert index -- the oracle's order -- and the

@@ -561,13 +561,13 @@ struct GroupSource
     double3 rc, re;
     StageRef stage;   // the warp's bulk-copy stage, or none (direct loads)
 
-    template<bool Dbl, bool Float, bool Index, bool Periodic, bool Staged = false, class Filter, class Batch>
-    __device__ __forceinline__ void stream(double4* ring, float4* ringf, int* ringIdx, const GroupBox& bx, double sx,
-                                           double sy, double sz, double lx, double ly, double lz, Filter filter,
-                                           Batch batch, const RoundBox* rbp = nullptr) const
+    // each(s0, len, nb, last) on up to 32 particle ranges at a time, one a lane (lanes >= nb
+    // hold none), in order.
+    template<bool Periodic, class Each>
+    __device__ __forceinline__ void for_ranges(const GroupBox& bx, double lx, double ly, double lz,
+                                               const RoundBox* rbp, Each each) const
     {
         const int lane = threadIdx.x & 31;
-        CandidateRing<Dbl, Float, Index, Staged> cr{ring, ringf, ringIdx, bx.cx, bx.cy, bx.cz, sx, sy, sz, stage};
         auto fold = [&](double d, double L) { return (Periodic && L > 0.0) ? fmin(d, L - d) : d; };
         const int n1 = !walk ? 0 : tree.n1p != nullptr ? *tree.n1p : tree.n1;
         int p = tree.n0;
@@ -638,8 +638,19 @@ struct GroupSource
                 s0 = lane < nb ? rx : 0u;
                 len = lane < nb ? ry - rx : 0u;
             }
-            cr.feed(s0, len, nb, xyzh, filter, batch, last);
+            each(s0, len, nb, last);
         }
+    }
+
+    template<bool Dbl, bool Float, bool Index, bool Periodic, bool Staged = false, class Filter, class Batch>
+    __device__ __forceinline__ void stream(double4* ring, float4* ringf, int* ringIdx, const GroupBox& bx, double sx,
+                                           double sy, double sz, double lx, double ly, double lz, Filter filter,
+                                           Batch batch, const RoundBox* rbp = nullptr) const
+    {
+        CandidateRing<Dbl, Float, Index, Staged> cr{ring, ringf, ringIdx, bx.cx, bx.cy, bx.cz, sx, sy, sz, stage};
+        for_ranges<Periodic>(bx, lx, ly, lz, rbp, [&](uint32_t s0, uint32_t len, int nb, bool last) {
+            cr.feed(s0, len, nb, xyzh, filter, batch, last);
+        });
         if constexpr (Staged) cr.finish(batch);
     }
 };

@@ -1,5 +1,5 @@
 /*
- * tree.cu -- Hilbert keys, the onesweep radix sort, the cornerstone leaf tree, the linked
+ * tree.cu -- Hilbert keys and their radix sort, the cornerstone leaf tree, the linked
  * octree with node geometry, hmax, and the j-leaf list walk.  The B200 counterpart of the
  * reference's src/tree.cu and include/tree.cuh, written without Thrust or Cornerstone.
  *

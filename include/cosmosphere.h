@@ -107,10 +107,12 @@ void cosmo_batch_set_params(const double* pmass, const int* periodic, const doub
 void cosmo_batch_set_bucket(const int* bucket_per_set);
 /* The batched Newton kernel's j-stream feed for every set of the batch: 1 staged into
  * shared memory by bulk copies, 0 (default) loaded directly.  Results do not depend on
- * it; the autotuner picks it for the whole batch. */
+ * it; the autotuner picks it for the whole batch.  (A plain batch that is not staged runs
+ * over its sets' block trees, which stream no lists.) */
 void cosmo_batch_set_staging(int on);
 
-/* Per-set launch parameters, as an autotuner picks them (NULL keeps a parameter):
+/* Per-set launch parameters of the list engine (mixed and staged batches), as an autotuner
+ * picks them (NULL keeps a parameter):
  * bucket = leaf capacity (8..1024); list_margin = widening of the gather radius the lists
  * are walked at, which lets them serve later iterations (1..2, default 1.15);
  * split_stream = gather stream (particles) above which a leaf's active particles are cut
@@ -210,7 +212,10 @@ int cosmo_x_density(int n, double pmass, int periodic, const double* box, double
 /* Wait for the library's stream. */
 void cosmo_x_sync(void);
 
-/* Select a kernel variant of the single-set solve (results do not depend on it):
+/* Select a kernel variant of the single-set solve (results do not depend on it).  A plain
+ * solve with gradients runs over the block tree unless "staging", "split_stream",
+ * "split_work", "spread_groups" or "graph_list_store" is set, which choose variants of the
+ * list-based loop:
  * "staging" 1 stages the Newton kernels' j-stream into shared memory with bulk copies
  * (cp.async.bulk completing on an mbarrier), 0 (default) loads it directly;
  * "sym_prefilter" 1 puts the symmetric row builder's tests behind the FP32 prefilter;

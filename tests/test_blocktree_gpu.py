@@ -156,6 +156,41 @@ def test_mixed_force_after_a_plain_solve(lnsigma):
         c.set_precision(False)
 
 
+@pytest.mark.parametrize("case", ["plummer_cut", "plummer_scattered", "box", "narrow", "quintic"])
+def test_mixed_groups_of_every_size(case):
+    """Leaves' last few particles, cut groups of one, of a few and of more, and a box whose
+    groups span half a period: h and rho of a mixed solve, alone and in a batch, within the
+    mixed form's 1e-5 of the plain one's."""
+    quintic, box = case == "quintic", UNIT if case in ("box", "narrow") else None
+    if case == "plummer_cut" or quintic:
+        p = inputs.plummer(20000, hfact=1.0 if quintic else 1.2, lnsigma=0.2, seed=31)
+    elif case == "plummer_scattered":
+        p = inputs.plummer(9000, hfact=1.2, lnsigma=0.7, seed=32)
+    else:
+        p = _box(300 if case == "narrow" else 8000, 33)
+    c = capi.Cosmo(quintic)
+    got = []
+    for mixed in (False, True):
+        c.set_precision(mixed)
+        try:
+            c.arrays_init(p.n)
+            c.upload(capi.POS, np.stack([p["x"], p["y"], p["z"]]))
+            c.upload(capi.HSML, p["h"])
+            assert c.density_status(p.n, p["pmass"], periodic_box=box, hfact=1.0 if quintic else 1.2) == 0
+            got.append((c.download(capi.HSML, p.n)[0], c.download(capi.DENS_OUT, p.n)[0]))
+            if not quintic:
+                b = capi.Batch([dict(p, box=box)])
+                b.upload()
+                assert b.density(tolh=1e-4, hfact=1.2, final_rho=True) == 0
+                h, rho, _ = b.download()
+                got.append((h[0], rho[0]))
+        finally:
+            c.set_precision(False)
+    for h, rho in got[1:]:
+        assert np.max(np.abs(h / got[0][0] - 1)) <= 1e-5
+        assert np.max(np.abs(rho / got[0][1] - 1)) <= 1e-5
+
+
 def _sort_sizes():
     import torch
     step = torch.cuda.get_device_properties(0).multi_processor_count * 1024 if torch.cuda.is_available() else 148 * 1024
