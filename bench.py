@@ -885,8 +885,10 @@ def run_particles(args, rank, world, local, dist, p, quintic, metric, label):
     achieved = flops / head["t_nr"] / 1e12
     peaks, src = measured_peaks()
     hbm_achieved = BYTES_PER_DENSITY_UPDATE * head["nr_upd"] / head["t_nr"] / 1e9
-    kname = ("Newton stage, per iteration: density_nr_kernel + newton_rows_kernel + density_row_kernel "
-             "+ plan_items_kernel, timed together by CUDA events")
+    kname = ("Newton stage, per iteration: "
+             + ("near_rows_kernel + near_step_kernel + near_sum_kernel" if plain is not None else
+                "density_nr_kernel + newton_rows_kernel + density_row_kernel + plan_items_kernel")
+             + ", timed together by CUDA events")
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and not quintic:
         same = args.ref_npartx == args.npartx and args.workload == "lattice100"

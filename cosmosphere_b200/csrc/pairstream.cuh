@@ -772,14 +772,6 @@ struct KahanF
         c = (t - s) - y;
         s = t;
     }
-    // the same where x is a product the compiler could otherwise fuse into the subtraction
-    __device__ __forceinline__ void add_rn(float x)
-    {
-        const float y = __fsub_rn(x, c);
-        const float t = __fadd_rn(s, y);
-        c = __fsub_rn(__fsub_rn(t, s), y);
-        s = t;
-    }
     __device__ __forceinline__ double value() const { return double(s) - double(c); }
 };
 
