@@ -339,6 +339,25 @@ near_forest_init_kernel(NearLoop* L, int n, const NearSet* __restrict__ sets, co
     }
 }
 
+// Particles the loop left on its next search and sum lists (its iterations ran out): their rows,
+// if they have one, do not reach their last h.  They join the cover list, so that an
+// evaluation at that h finds them a row or puts them on the over list, as the others.  (Those
+// on its row list keep a row that reaches it.)
+__global__ void __launch_bounds__(kThreads)
+near_pending_kernel(NearLoop* L, const __grid_constant__ NearLists lists)
+{
+    const int cur = L->iter & 1;
+    const NearCounts c = L->cnt[cur];
+    const int n = c.build + c.sum + c.huge;
+    for (int b = blockIdx.x * kThreads; b < n; b += gridDim.x * kThreads)
+    {
+        const int k = b + int(threadIdx.x);
+        const int s = k - c.build, u = s - c.sum;
+        const int v = k >= n ? 0 : (s < 0 ? lists.build[cur][k] : (u < 0 ? lists.sum[cur][s] : lists.huge[cur][u]));
+        warp_append(k < n, v, lists.cover, &L->cover);
+    }
+}
+
 // Work in nq queues of consecutive items, one a multiprocessor: the warps of a multiprocessor
 // take items from its own queue, so at any time they search next to one another and find
 // each other's blocks in its L1 cache; one whose queue is empty goes on with the first that
@@ -1454,7 +1473,7 @@ void near_forest_newton(State& s, const NearForest& b, double tolh, double hfact
     near_run(s, j, maxIter, graph, false);
 }
 
-// rho and d(rho)/dh of every live particle of the batch at its final h.
+// rho and d(rho)/dh of every live particle of the batch at its final h, converged or not.
 void near_forest_eval(State& s, const NearForest& b)
 {
     NearTree t;
@@ -1465,6 +1484,8 @@ void near_forest_eval(State& s, const NearForest& b)
     t.nLive = &s.dscal.get()->nAlive;
     const NearLists lists = near_lists(s);
     NearLoop* L = s.nearLoop.get();
+    near_pending_kernel<<<std::min(iceil(b.n, kThreads), 2 * s.numSMs), kThreads, 0, s.st>>>(L, lists);
+    COSMO_LAUNCHED();
     auto rows = near_rows_kernel<true, true>;
     rows<<<persistent_blocks(s, rows, kThreads), kThreads, 0, s.st>>>(t, s.nearSets.get(), b.setOf, L, lists,
                                                                       s.nblR2.get(), nullptr, s.nblCount.get(),

@@ -1,0 +1,77 @@
+"""The batched form where it leaves the common path: iterations running out before every h
+has converged."""
+import numpy as np
+import pytest
+
+from cosmosphere_b200 import capi, inputs
+
+pytestmark = pytest.mark.gpu
+UNIT = [0.0, 1.0, 0.0, 1.0, 0.0, 1.0]
+
+
+def _box(n, seed=1, hscale=1.2):
+    rng = np.random.default_rng(seed)
+    x, y, z = rng.random((3, n))
+    h = hscale * (1.0 / n) ** (1.0 / 3.0) * rng.uniform(0.8, 1.25, n)
+    return dict(inputs.Particles(x=x, y=y, z=z, h=h, pmass=1.0 / n), box=UNIT)
+
+
+def _plummer(n, seed=2, lnsigma=0.8, hfact=1.2):
+    return dict(inputs.plummer(n, hfact=hfact, lnsigma=lnsigma, seed=seed))
+
+
+def _batch(sets, quintic=False, staging=False, tuning=None, mixed=False, **kw):
+    capi.Cosmo(quintic).set_precision(mixed)
+    b = capi.Batch(sets, quintic=quintic)
+    b.set_staging(staging)
+    try:
+        if tuning is not None:
+            b.set_tuning(**tuning)
+        b.upload()
+        st = b.density(**kw)
+        return st, b, b.download()
+    finally:
+        b.set_staging(False)
+        capi.Cosmo(quintic).set_precision(False)
+
+
+def _kernel(q, quintic):
+    if not quintic:
+        a, b = np.maximum(2.0 - q, 0.0), np.maximum(1.0 - q, 0.0)
+        return 0.25 * (a**3 - 4.0 * b**3), 0.25 * (-3.0 * a**2 + 12.0 * b**2)
+    a, b, c = (np.maximum(k - q, 0.0) for k in (3.0, 2.0, 1.0))
+    return a**5 - 6.0 * b**5 + 15.0 * c**5, -5.0 * a**4 + 30.0 * b**4 - 75.0 * c**4
+
+
+def _direct(s, h, quintic):
+    """rho and d(rho)/dh of every particle at h by direct summation over all pairs, and the
+    sum of the second's terms' sizes, which its rounding is measured against."""
+    pos = np.stack([s["x"], s["y"], s["z"]])
+    norm = s["pmass"] * (1.0 / (120.0 * np.pi) if quintic else 1.0 / np.pi)
+    out = np.empty((3, h.size))
+    for a in range(0, h.size, 500):
+        d = pos[:, a:a + 500, None] - pos[:, None, :]
+        if s.get("box") is not None:
+            d -= np.round(d)
+        hi = h[a:a + 500, None]
+        q = np.sqrt((d * d).sum(axis=0)) / hi
+        w, dw = _kernel(q, quintic)
+        g = -q * dw - 3.0 * w
+        out[:, a:a + 500] = np.stack([w.sum(axis=1), g.sum(axis=1), np.abs(g).sum(axis=1)])
+    return out[0] * norm / h**3, out[1] * norm / h**4, out[2] * norm / h**4
+
+
+@pytest.mark.parametrize("max_iter,graph,quintic", [(1, True, False), (2, True, False), (2, False, False),
+                                                    (4, True, True)])
+def test_final_rho_of_unconverged_particles(max_iter, graph, quintic):
+    """rho and d(rho)/dh are those of the returned h for every particle, also for those whose
+    last step outgrew their row or that never had one.  Sums of up to n terms round by n
+    2^-53 of the sum of their sizes: 1e-11 is ten times that for 9000."""
+    hf = 1.0 if quintic else 1.2
+    sets = [_box(3000, 4, hf), _plummer(9000, hfact=hf), _plummer(900, seed=9, hfact=hf)]
+    st, b, (h, rho, gradh) = _batch(sets, quintic, max_iter=max_iter, graph=graph, final_rho=True, hfact=hf)
+    assert st == 1 and b.scalar("unconverged") > 1000
+    for k, s in enumerate(sets):
+        r, g, size = _direct(s, h[k], quintic)
+        assert np.max(np.abs(rho[k] / r - 1.0)) <= 1e-11, k
+        assert np.max(np.abs(gradh[k] - g) / size) <= 1e-11, k
