@@ -1466,6 +1466,30 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             return res;
         }
     }
+    // How the block-tree loop ended, once its state nl and the scalars have been read: the status
+    // the solve returns.
+    auto near_status = [&](const NearLoop& nl) {
+        check_dev_err(s, "solveDensH", false);
+        tree_timings(s);
+        s.nAlive = s.hscal->nAlive;
+        nActiveParticles = near_results(s, nl);
+        s.nearOverCount = nl.over;
+        s.t.nrkern += elapsed_s(n0, e3);
+        res.itersRun = s.itersRun;
+        res.unconverged = int(nActiveParticles);
+        s.hscal->unconverged = res.unconverged;
+        if (nActiveParticles > 0) return 1;
+        if (!s.periodic || s.nAlive == 0) return 0;
+        double hm;
+        std::memcpy(&hm, &s.hscal->hmaxConv, sizeof hm);
+        const double lmin = std::min({periodicBox[1] - periodicBox[0], periodicBox[3] - periodicBox[2],
+                                      periodicBox[5] - periodicBox[4]});
+        return kRadKernel * hm >= 0.5 * lmin ? 2 : 0;
+    };
+    auto read_near = [&](NearLoop& nl) {
+        COSMO_CUDA(cudaMemcpyAsync(&nl, s.nearLoop.get(), sizeof(NearLoop), cudaMemcpyDeviceToHost, s.st));
+        read_scalars(s);
+    };
     bool symBuilt = false, fromRows = false;
     if (withGradients)
     {
@@ -1494,10 +1518,14 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             sym_rows_from_newton(s, near);
         else
         {
+            // no lists for an h that did not converge (they could be of any length)
             if (near)
             {
-                read_scalars(s);
-                s.nAlive = s.hscal->nAlive;
+                NearLoop nl;
+                read_near(nl);
+                if (s.hscal->outside) return onLists();
+                res.status = near_status(nl);
+                if (res.status != 0) return res;
             }
             build_symmetric(s);
             symBuilt = true;
@@ -1542,40 +1570,16 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             COSMO_LAUNCHED();
         }
         cudaEvent_t g2 = ev(s);
-        NearLoop nl;
-        if (near)
-            COSMO_CUDA(cudaMemcpyAsync(&nl, s.nearLoop.get(), sizeof(NearLoop), cudaMemcpyDeviceToHost, s.st));
-        read_scalars(s);
-        if (near)
+        if (near && fromRows)
         {
-            check_dev_err(s, "solveDensH", false);
+            NearLoop nl;
+            read_near(nl);
             if (s.hscal->outside) return onLists();
-            tree_timings(s);
-            s.nAlive = s.hscal->nAlive;
-            nActiveParticles = near_results(s, nl);
-            s.nearOverCount = nl.over;
-            s.t.nrkern += elapsed_s(n0, e3);
-            res.itersRun = s.itersRun;
-            res.unconverged = int(nActiveParticles);
-            s.hscal->unconverged = res.unconverged;
-            if (nActiveParticles > 0)
-            {
-                res.status = 1;
-                return res;
-            }
-            if (s.periodic && s.nAlive > 0)
-            {
-                double hm;
-                std::memcpy(&hm, &s.hscal->hmaxConv, sizeof hm);
-                const double lmin = std::min({periodicBox[1] - periodicBox[0], periodicBox[3] - periodicBox[2],
-                                              periodicBox[5] - periodicBox[4]});
-                if (kRadKernel * hm >= 0.5 * lmin)
-                {
-                    res.status = 2;
-                    return res;
-                }
-            }
+            res.status = near_status(nl);
+            if (res.status != 0) return res;
         }
+        else
+            read_scalars(s);
         // the rows serve the force pass if every extra was kept and merged
         if (fromRows)
             s.rowsFromNewton = (s.symExtraCap == 0 || s.hscal->extraCount <= s.symExtraCap) &&

@@ -1,0 +1,52 @@
+"""The single-set solve where it leaves the common path: solves that do not end with a result,
+and what they leave behind; arrays that change under a solved set; unusual units, neighbour
+numbers and positions."""
+import numpy as np
+import pytest
+
+from cosmosphere_b200 import capi, inputs
+from test_parity_gpu import _vel_acc
+
+pytestmark = pytest.mark.gpu
+UNIT = [0.0, 1.0, 0.0, 1.0, 0.0, 1.0]
+
+
+def _box(n, seed=1, hscale=1.2):
+    rng = np.random.default_rng(seed)
+    x, y, z = rng.random((3, n))
+    h = hscale * (1.0 / n) ** (1.0 / 3.0) * rng.uniform(0.8, 1.25, n)
+    return inputs.Particles(x=x, y=y, z=z, h=h, pmass=1.0 / n)
+
+
+def _solve(p, box=None, options=(), c=None, **kw):
+    """One solve of p under the given options (restored after it); its status and library."""
+    c = c or capi.Cosmo()
+    c.set_precision(False)
+    for k, v in options:
+        assert c.set_option(k, v) == 0
+    try:
+        c.arrays_init(p.n)
+        vel, acc = _vel_acc(p)
+        for slot, data in ((capi.POS, np.stack([p["x"], p["y"], p["z"]])), (capi.HSML, p["h"]), (capi.VEL, vel),
+                           (capi.ACCEL, acc)):
+            c.upload(slot, data)
+        return c.density_status(p.n, p["pmass"], periodic_box=box, **kw), c
+    finally:
+        for k, _ in options:
+            c.set_option(k, 1 if k == "sym_from_rows" else 0)
+
+
+LISTS = (("graph_list_store", 200),)   # a variant of the list-based loop: the solve runs over it
+
+
+def test_an_unconverged_solve_keeps_the_last_iterations_rho():
+    """The rows of the gradient sweep are not built, nor the sweep run, for a solve whose
+    iterations ran out, whichever way its rows would be made."""
+    p = inputs.plummer(9000, hfact=1.2, lnsigma=0.8, seed=2)
+    out = []
+    for options in ((), (("sym_from_rows", 0),)):
+        st, c = _solve(p, options=options, max_iter=2)
+        assert st == 1
+        out.append((c.download(capi.HSML, p.n), c.download(capi.DENS_OUT, p.n), c.scalar("listTotal")))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
