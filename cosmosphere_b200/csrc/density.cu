@@ -13,6 +13,7 @@
  * still holds an unconverged particle appends the leaf to the next iteration's list.
  */
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 
@@ -167,9 +168,9 @@ gradient_row_kernel(int nAlive, const int* __restrict__ nbl, const int* __restri
                     const double4* __restrict__ acc4, double* __restrict__ rho, double* __restrict__ gradh,
                     double* __restrict__ divv, double* __restrict__ xiOut, double* __restrict__ ddivvdt,
                     double pmass, const DevBox* __restrict__ box, DevScalars* __restrict__ ds,
-                    const int* __restrict__ active)
+                    const NearLoop* __restrict__ L, double halfBox)
 {
-    if (active != nullptr && *active > 0) return;   // the Newton loop did not converge
+    if (near_failed(L, ds, halfBox)) return;
     nAlive = min(nAlive, ds->nAlive);
     double lx = 0, ly = 0, lz = 0;
     if (Periodic) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
@@ -214,12 +215,12 @@ gradient_warp_kernel(const __grid_constant__ NearTree t, const NearLoop* __restr
                      const int* __restrict__ over, const int* __restrict__ nbl, const int* __restrict__ nblCount,
                      const double4* __restrict__ vel4, const double4* __restrict__ acc4, double* __restrict__ rho,
                      double* __restrict__ gradh, double* __restrict__ divv, double* __restrict__ xiOut,
-                     double* __restrict__ ddivvdt, double pmass, DevScalars* __restrict__ ds)
+                     double* __restrict__ ddivvdt, double pmass, DevScalars* __restrict__ ds, double halfBox)
 {
     __shared__ NearScratch sScr[Rows ? 1 : kWarpsPerBlock];
     __shared__ double sTerm[kWarpsPerBlock][32 * kGradTerms];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (L != nullptr && L->active > 0) return;   // the Newton loop did not converge
+    if (near_failed(L, ds, halfBox)) return;
     const int n = Rows ? min(nAlive, ds->nAlive) : L->over;
     if (n == 0) return;
     if (!Rows && blockIdx.x == 0 && threadIdx.x == 0) ds->rowOverflow = 1;
@@ -1447,6 +1448,11 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             return res;
         }
     }
+    // half the box's shortest side: no support may reach it
+    double halfBox = NAN;   // open: nothing compares true
+    if (s.periodic)
+        halfBox = 0.5 * std::min({periodicBox[1] - periodicBox[0], periodicBox[3] - periodicBox[2],
+                                  periodicBox[5] - periodicBox[4]});
     if (!near && s.periodic && s.nAlive > 0)
     {
         const int nb = std::min(iceil(s.nAlive, 256), 2 * s.numSMs);
@@ -1458,9 +1464,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         COSMO_CUDA(cudaStreamSynchronize(s.st));
         double hm = 0.0;
         for (double v : part) hm = std::max(hm, v);
-        const double lmin = std::min({periodicBox[1] - periodicBox[0], periodicBox[3] - periodicBox[2],
-                                      periodicBox[5] - periodicBox[4]});
-        if (kRadKernel * hm >= 0.5 * lmin)
+        if (kRadKernel * hm >= halfBox)
         {
             res.status = 2;
             return res;
@@ -1479,12 +1483,10 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         res.unconverged = int(nActiveParticles);
         s.hscal->unconverged = res.unconverged;
         if (nActiveParticles > 0) return 1;
-        if (!s.periodic || s.nAlive == 0) return 0;
+        if (s.nAlive == 0) return 0;
         double hm;
         std::memcpy(&hm, &s.hscal->hmaxConv, sizeof hm);
-        const double lmin = std::min({periodicBox[1] - periodicBox[0], periodicBox[3] - periodicBox[2],
-                                      periodicBox[5] - periodicBox[4]});
-        return kRadKernel * hm >= 0.5 * lmin ? 2 : 0;
+        return kRadKernel * hm >= halfBox ? 2 : 0;
     };
     auto read_near = [&](NearLoop& nl) {
         COSMO_CUDA(cudaMemcpyAsync(&nl, s.nearLoop.get(), sizeof(NearLoop), cudaMemcpyDeviceToHost, s.st));
@@ -1513,7 +1515,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         }
         else
             fromRows = writeJ && s.nAlive > 0 && rowsBuilt && cover_rows(s, itemCap, cut, spreadG);
-        const int* active = near ? &s.nearLoop.get()->active : nullptr;
+        const NearLoop* loop = near ? s.nearLoop.get() : nullptr;
         if (fromRows)
             sym_rows_from_newton(s, near);
         else
@@ -1537,10 +1539,10 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         else
         {
             auto warps = [&](auto kern, int blocks) {
-                kern<<<blocks, kThreads, 0, s.st>>>(near_tree(s), near ? s.nearLoop.get() : nullptr, s.nAlive,
+                kern<<<blocks, kThreads, 0, s.st>>>(near_tree(s), loop, s.nAlive,
                                                     s.nearOver.get(), s.nbl.get(), s.nblCount.get(), s.vel4.get(),
                                                     s.acc4.get(), s.rho.get(), s.gradh.get(), s.divv.get(), s.xi.get(),
-                                                    s.ddivvdt.get(), pmass, ds);
+                                                    s.ddivvdt.get(), pmass, ds, halfBox);
                 COSMO_LAUNCHED();
             };
             if (s.nAlive <= kWarpPerParticle)
@@ -1551,7 +1553,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
                 auto gr = s.periodic ? gradient_row_kernel<true> : gradient_row_kernel<false>;
                 gr<<<iceil(s.nAlive, kThreads), kThreads, 0, s.st>>>(
                     s.nAlive, s.nbl.get(), s.nblCount.get(), s.xyzh.get(), s.vel4.get(), s.acc4.get(), s.rho.get(),
-                    s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), ds, active);
+                    s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), ds, loop, halfBox);
                 COSMO_LAUNCHED();
             }
             if (near && fromRows)

@@ -50,3 +50,18 @@ def test_an_unconverged_solve_keeps_the_last_iterations_rho():
         out.append((c.download(capi.HSML, p.n), c.download(capi.DENS_OUT, p.n), c.scalar("listTotal")))
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+# a warp per particle, and a lane
+@pytest.mark.parametrize("n,box", [(12, UNIT), (40000, [0.0, 1.0, 0.0, 1.0, 0.0, 0.02])])
+def test_a_support_of_half_the_box_keeps_the_last_iterations_rho(n, box):
+    p = _box(n)
+    p["z"] *= box[5]
+    p["h"] *= box[5] ** (1.0 / 3.0)
+    out = []
+    for gradients in (True, False):
+        st, c = _solve(p, box, with_gradients=gradients)
+        assert st == 2
+        out.append((c.download(capi.HSML, n), c.download(capi.DENS_OUT, n)))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
