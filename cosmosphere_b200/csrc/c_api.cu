@@ -857,6 +857,7 @@ double cosmo_x_scalar(const char* name)
     if (k == "nLeaves") return s.nLeaves;
     if (k == "numNodes") return s.numNodes;
     if (k == "itersRun") return s.itersRun;
+    if (k == "unconverged") return s.unconverged;
     if (k == "token") return double(s.token);
     if (k == "hfact") return s.hfact;
     if (k == "maxIter") return s.maxIter;
@@ -886,7 +887,6 @@ double cosmo_x_scalar(const char* name)
         if (k == "pairsForce") return double(s.hscal->pairs[2]);
         if (k == "rowOverflow") return double(s.hscal->rowOverflow);
         if (k == "candDensity") return double(s.hscal->pairs[3]);
-        if (k == "unconverged") return s.hscal->unconverged;
     }
     const Timings& t = s.t;
     if (k == "t_bbox") return t.bbox;

@@ -1292,8 +1292,10 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         rowsJ = s.nblJ.get();
     }
     s.rowsFromNewton = false;
-    s.hmaxNodeDone = true;
-    s.listsLoose = false;
+    // whatever way a block-tree solve ends, the lists and hmax per node held belong to an
+    // earlier tree: they are made when asked for
+    s.hmaxNodeDone = !near;
+    s.listsLoose = near;
     s.nearOverCount = 0;
     if (near) s.listsSym = false;
 
@@ -1441,7 +1443,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         check_dev_err(s, "solveDensH", listsWidened && !withGradients);
         tree_timings(s);
         res.itersRun = s.itersRun;
-        res.unconverged = int(nActiveParticles);
+        s.unconverged = res.unconverged = int(nActiveParticles);
         if (nActiveParticles > 0)
         {
             res.status = 1;
@@ -1481,7 +1483,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
         s.t.nrkern += elapsed_s(n0, e3);
         res.itersRun = s.itersRun;
         res.unconverged = int(nActiveParticles);
-        s.hscal->unconverged = res.unconverged;
+        s.unconverged = res.unconverged;
         if (nActiveParticles > 0) return 1;
         if (s.nAlive == 0) return 0;
         double hm;
@@ -1530,6 +1532,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
                 if (res.status != 0) return res;
             }
             build_symmetric(s);
+            s.hmaxNodeDone = true;
             symBuilt = true;
         }
         cudaEvent_t g1 = ev(s);

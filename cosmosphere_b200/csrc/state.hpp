@@ -182,6 +182,7 @@ struct State
     // node were not built, and are built only if asked for (hmaxNodeDone once done).
     bool rowsFromNewton = false, hmaxNodeDone = true;
     int itersRun = 0, maxIter = 100;
+    int unconverged = 0;                        // particles the last solve left unconverged
     long long settling0 = 0;                    // settling particles after the first Newton update
     int precision = 0;     // 0 plain FP64 (the drop-in form), 1 mixed FP32/FP64
     // Kernel variants (results are the same either way): staging = 1 stages the Newton

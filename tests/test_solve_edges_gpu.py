@@ -65,3 +65,27 @@ def test_a_support_of_half_the_box_keeps_the_last_iterations_rho(n, box):
         out.append((c.download(capi.HSML, n), c.download(capi.DENS_OUT, n)))
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+def test_what_an_unconverged_solve_leaves_to_read():
+    """The number of unconverged particles, hmax and lists that belong to the h held, not to
+    a set solved before."""
+    other, p = inputs.plummer(6000, hfact=1.2, lnsigma=0.9, seed=12), _box(6000, 3)
+    st, c = _solve(p, UNIT, LISTS, max_iter=2)
+    left = c.scalar("unconverged")
+    assert st == 1 and left > 0
+    st, c = _solve(other)
+    assert st == 0 and c.scalar("unconverged") == 0
+    c.array("hmax_node"), c.array("jlist")
+    st, c = _solve(p, UNIT, max_iter=2)
+    assert st == 1 and c.scalar("unconverged") == left
+    h, leaf = c.array("h"), c.array("particleLeaf")
+    assert c.array("hmax_node")[0] == h.max()
+    off, lists = c.array("jOffset").astype(np.int64), c.array("jlist")
+    assert off[0] == 0 and off[-1] == lists.size
+    pos = np.stack([c.array(k) for k in "xyz"])
+    for i in range(0, p.n, 500):
+        d = pos - pos[:, i:i + 1]
+        d -= np.round(d)
+        near = np.flatnonzero((d * d).sum(axis=0) < (2.0 * h[i]) ** 2)
+        assert np.isin(leaf[near], lists[off[leaf[i]]:off[leaf[i] + 1]]).all(), i
