@@ -537,6 +537,9 @@ void compute_forces(State& s, double pmass, double beta, double alphau, bool dis
         s.rowsToken == s.token && ((s.rowsFromNewton && !noRow) || (s.jlistToken == s.token && s.listsSym));
     if (!rowsReady)
     {
+        // positions may have been replaced in the sorted order since the tree was made
+        ensure_tree(s);
+        if (s.nLeaves > 0) leaf_boxes(s);
         build_symmetric(s);
         s.jlistToken = s.rowsToken = s.token;
         s.rowsFromNewton = false;

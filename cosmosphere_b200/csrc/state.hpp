@@ -323,6 +323,7 @@ void size_particle_arrays(State& s, int n);
 // tree.cu
 void build_order(State& s, const double* periodicBox, bool alsoSortVA, bool rowsJOn = false);
 void build_leaves(State& s);
+void leaf_boxes(State& s);    // of the tree held, over the particles' present positions
 void ensure_tree(State& s);   // the tree and hmax of its leaves, if the last solve made none
 void tree_timings(State& s);   // the last tree build's stage times, once its marks have passed
 // hmax of the leaves [0, nLeavesActive) of leaves, or of the first *countPtr of them when

@@ -985,6 +985,14 @@ void build_order(State& s, const double* periodicBox, bool alsoSortVA, bool rows
     std::copy(marks, marks + 5, s.treeEv);
 }
 
+// The leaves' bounding boxes over their particles where they are now.
+void leaf_boxes(State& s)
+{
+    s.leafBox.resize(2 * size_t(s.nLeaves), s.st);
+    leaf_box_kernel<<<iceil(s.nLeaves, 128), 128, 0, s.st>>>(s.layout.get(), s.nLeaves, s.xyzh.get(), s.leafBox.get());
+    COSMO_LAUNCHED();
+}
+
 // The leaf tree and the linked octree of the sorted particles.
 void build_leaves(State& s)
 {
@@ -1061,9 +1069,7 @@ void build_leaves(State& s)
     COSMO_LAUNCHED();
     particle_leaf_kernel<<<iceil(n, kBlk), kBlk, 0, s.st>>>(s.layout.get(), nL, n, ds, s.particleLeaf.get());
     COSMO_LAUNCHED();
-    s.leafBox.resize(2 * size_t(nL), s.st);
-    leaf_box_kernel<<<iceil(nL, 128), 128, 0, s.st>>>(s.layout.get(), nL, s.xyzh.get(), s.leafBox.get());
-    COSMO_LAUNCHED();
+    leaf_boxes(s);
     s.hmaxLeaf.resize(nL, s.st);
     s.hmaxNode.resize(numNodes, s.st);
     s.hmaxPre.resize(numNodes, s.st);

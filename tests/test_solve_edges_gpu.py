@@ -89,3 +89,31 @@ def test_what_an_unconverged_solve_leaves_to_read():
         d -= np.round(d)
         near = np.flatnonzero((d * d).sum(axis=0) < (2.0 * h[i]) ** 2)
         assert np.isin(leaf[near], lists[off[leaf[i]]:off[leaf[i] + 1]]).all(), i
+
+
+@pytest.mark.parametrize("gradients", [False, True])
+def test_symmetric_rows_of_moved_particles(gradients):
+    """Positions replaced in the sorted order, each particle somewhere in its leaf's cell: the
+    lists, which are cell by cell, still hold every pair, so the force pass finds all of
+    them."""
+    p = _box(5000, 5)
+    st, c = _solve(p, UNIT, LISTS, with_gradients=gradients)
+    assert st == 0
+    n, order, leaf = p.n, c.array("order"), c.array("particleLeaf")
+    node = c.array("leafToInternal")[leaf]
+    centre, half = c.array("centers").reshape(-1, 3)[node], c.array("sizes").reshape(-1, 3)[node]
+    pos = np.empty((3, n))
+    pos[:, order] = (centre + half * np.random.default_rng(6).uniform(-0.999, 0.999, (n, 3))).T
+    c.upload(capi.POS, pos, sorted_=True)
+    if gradients:
+        c.refresh_h()
+    c.upload(capi.THERMO, np.ones((4, n)), sorted_=True)
+    c.force(n, p["pmass"])
+    h = c.download(capi.HSML, n)[0]
+    pairs = 0
+    for a in range(0, n, 500):
+        d = pos[:, a:a + 500, None] - pos[:, None, :]
+        d -= np.round(d)
+        r2 = (d * d).sum(axis=0)
+        pairs += int(((r2 > 0) & (r2 < 4.0 * np.maximum(h[a:a + 500, None], h[None, :]) ** 2)).sum())
+    assert c.scalar("pairsForce") == pairs
