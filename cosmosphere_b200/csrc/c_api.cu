@@ -213,6 +213,8 @@ void size_particle_arrays(State& s, int n)
 {
     ensure_init(s);
     if (s.sizedFor == n) return;
+    // growing loses the keys: the last solve's tree, if it is still to be made, is made first
+    if (size_t(n) > s.keysA.cap) ensure_tree(s);
     for (auto* b : {&s.ux, &s.uy, &s.uz, &s.uh, &s.uvx, &s.uvy, &s.uvz, &s.uax, &s.uay, &s.uaz, &s.rho, &s.gradh,
                     &s.divv, &s.xi, &s.ddivvdt, &s.fx, &s.fy, &s.fz, &s.f4, &s.vsigmax, &s.divvF})
         b->resize(n, s.st);

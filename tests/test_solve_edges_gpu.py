@@ -117,3 +117,19 @@ def test_symmetric_rows_of_moved_particles(gradients):
         r2 = (d * d).sum(axis=0)
         pairs += int(((r2 > 0) & (r2 < 4.0 * np.maximum(h[a:a + 500, None], h[None, :]) ** 2)).sum())
     assert c.scalar("pairsForce") == pairs
+
+
+def test_the_tree_of_a_set_is_held_while_the_arrays_grow():
+    """The counts and arrays of the last solve's tree can be read after the arrays were sized
+    for a larger set, as before it."""
+    p = _box(5000, 7)
+    held = {}
+    for grown in (False, True):
+        st, c = _solve(p, UNIT)
+        assert st == 0
+        if grown:
+            c.arrays_init(40 * p.n)
+        for k in ("nLeaves", "numNodes"):
+            assert held.setdefault(k, c.scalar(k)) == c.scalar(k)
+        for k in ("layout", "csTree", "hmax_leaf", "centers"):
+            np.testing.assert_array_equal(held.setdefault(k, c.array(k)), c.array(k), err_msg=k)
