@@ -277,8 +277,9 @@ gradient_warp_kernel(const __grid_constant__ NearTree t, const NearLoop* __restr
         }
         else
         {
-            const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
-            const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
+            const float3 a = f.at(pi);
+            const float x = a.x, y = a.y, z = a.z;
+            const float r = f.length(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
             near_blocks<0, Periodic, false>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
                 near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, pair);
                 return r;
@@ -330,8 +331,9 @@ over_extras_kernel(const __grid_constant__ NearTree t, const NearLoop* __restric
         const int i = over[w];
         const double4 pi = t.xyzh[i];
         const double bi = kRadK2 * (pi.w * pi.w) * (1.0 + 1e-10);
-        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
-        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
+        const float3 a = f.at(pi);
+        const float x = a.x, y = a.y, z = a.z;
+        const float r = f.length(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
         near_blocks<0, Periodic, false>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
             near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, [&](const double4& pj, int j, bool valid) {
                 double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;

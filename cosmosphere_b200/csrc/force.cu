@@ -460,9 +460,10 @@ force_warp_kernel(const __grid_constant__ NearTree t, int n, const int* __restri
         }
         else
         {
-            const float x = float(A.p.x - f.cx), y = float(A.p.y - f.cy), z = float(A.p.z - f.cz);
+            const float3 a = f.at(A.p);
+            const float x = a.x, y = a.y, z = a.z;
             const float slack = f.slack(x, y, z);
-            const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * A.p.w) + slack;
+            const float r = f.length(kRadKernel * (1.0 + 1e-6) * A.p.w) + slack;
             near_blocks<0, Periodic, true>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
                 near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, pair);
                 return r;

@@ -109,11 +109,11 @@ near_leaf_levels_kernel(const __grid_constant__ NearTree t, NearNode* __restrict
         if (i < v.n)
         {
             const double4 p = t.xyzh[v.p0 + i];
-            const double x = p.x - f.cx, y = p.y - f.cy, z = p.z - f.cz;
+            const double x = (p.x - f.cx) * f.scale, y = (p.y - f.cy) * f.scale, z = (p.z - f.cz) * f.scale;
             lx = __double2float_rd(x); hx = __double2float_ru(x);
             ly = __double2float_rd(y); hy = __double2float_ru(y);
             lz = __double2float_rd(z); hz = __double2float_ru(z);
-            hm = __double2float_ru(p.w);
+            hm = f.length(p.w);
         }
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1)
@@ -175,7 +175,9 @@ __global__ void near_sets_kernel(int nsets, const int* __restrict__ offs, const 
     const bool per = b.periodic != 0;
     const float inf = INFINITY;
     const double dinf = double(inf);
-    sets[s] = NearSet{offs[s], nAlive[s], per ? f.lx : inf, per ? f.ly : inf, per ? f.lz : inf, f.len, f.cx, f.cy, f.cz,
+    sets[s] = NearSet{offs[s], nAlive[s],
+                      per ? f.lx : inf, per ? f.ly : inf, per ? f.lz : inf, f.len,
+                      f.cx, f.cy, f.cz, f.scale,
                       per ? b.len[0] : dinf, per ? b.len[1] : dinf, per ? b.len[2] : dinf, pmass[s]};
 }
 
@@ -423,7 +425,7 @@ near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
     const int* list = cover ? lists.cover : (L->all ? nullptr : lists.build[cur]);
     const double margin = cover ? kCoverMargin : kNearMargin;
     const double wide2 = kRadK2 * (margin * margin);
-    const NearFrame f(t.box);
+    NearFrame f(t.box);
     NearView v = Forest ? NearView{0, 0, 0, 0.0f, 0.0f, 0.0f} : near_view(t, f);
     double lx = 0, ly = 0, lz = 0;
     if (Periodic && !Forest) { lx = t.box->len[0]; ly = t.box->len[1]; lz = t.box->len[2]; }
@@ -439,19 +441,10 @@ near_rows_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
         const int i = mine ? (list ? list[at] : at) : 0;
         const int set = Forest ? setOf[i] : 0;
         const double4 pi = t.xyzh[i];
-        float x, y, z, slack;
-        if constexpr (Forest)
-        {
-            const NearFrame fs(sets[set]);
-            x = float(pi.x - fs.cx); y = float(pi.y - fs.cy); z = float(pi.z - fs.cz);
-            slack = fs.slack(x, y, z);
-        }
-        else
-        {
-            x = float(pi.x - f.cx); y = float(pi.y - f.cy); z = float(pi.z - f.cz);
-            slack = f.slack(x, y, z);
-        }
-        const float r = mine ? __double2float_ru(kRadKernel * margin * (1.0 + 1e-6) * pi.w) + slack : -1.0f;
+        if constexpr (Forest) f = NearFrame(sets[set]);
+        const float3 rel = f.at(pi);
+        const float x = rel.x, y = rel.y, z = rel.z;
+        const float r = mine ? f.length(kRadKernel * margin * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z) : -1.0f;
         scr.P[lane] = make_double4(pi.x, pi.y, pi.z, 1.0 / (pi.w * pi.w));
         scr.Q[lane] = make_float4(x, y, z, r * r * 1.000001f);
         // a member much wider than the others (a scattered h) searches by itself, after them
@@ -962,8 +955,9 @@ near_sum_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__ 
         }
         const double4* at0 = t.xyzh + v.p0;
         const double hi = pi.w, hinv2 = 1.0 / (hi * hi);
-        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
-        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * hi) + f.slack(x, y, z);
+        const float3 a = f.at(pi);
+        const float x = a.x, y = a.y, z = a.z;
+        const float r = f.length(kRadKernel * (1.0 + 1e-6) * hi) + f.slack(x, y, z);
         double2 sums = make_double2(0.0, 0.0);
         int nrec = 0;
         unsigned int got = 0;
@@ -1067,8 +1061,9 @@ near_huge_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
         }
         const double4* at0 = t.xyzh + v.p0;
         const double hi = pi.w, hinv2 = 1.0 / (hi * hi);
-        const float x = float(pi.x - f.cx), y = float(pi.y - f.cy), z = float(pi.z - f.cz);
-        const float r = __double2float_ru(kRadKernel * (1.0 + 1e-6) * hi) + f.slack(x, y, z);
+        const float3 a = f.at(pi);
+        const float x = a.x, y = a.y, z = a.z;
+        const float r = f.length(kRadKernel * (1.0 + 1e-6) * hi) + f.slack(x, y, z);
         const float r2max = r * r * 1.000001f;
         unsigned int got = 0;   // of this warp
         // the whole block over the 64-particle nodes scr.blk[0 .. cnt)

@@ -11,7 +11,9 @@
  * touches: on a lattice (58 neighbours) about 180 candidates per particle instead of 440,
  * and no list, no work items and no per-leaf bookkeeping between iterations.
  *
- * Boxes are FP32 relative to the root box's centre, rounded outward, and every radius
+ * Boxes are FP32 relative to the root box's centre, in units of a power of two near its
+ * largest side (so that squares stay in FP32's range whatever the caller's units), rounded
+ * outward, and every radius
  * carries a slack above the rounding of the tests, so a block is never left out that
  * holds a pair the exact FP64 test accepts.  Blocks come out in ascending order and the
  * lanes of a step hold 32 consecutive candidates of one particle, so what is accepted is
@@ -66,8 +68,8 @@ struct NearTree
 struct NearSet
 {
     int p0, n;                 // first particle of the sorted order, live particles
-    float lx, ly, lz, len;     // periods, largest side
-    double cx, cy, cz;         // box centre
+    float lx, ly, lz, len;     // periods, largest side (scaled)
+    double cx, cy, cz, scale;  // box centre, the search frame's scale
     double dlx, dly, dlz;      // periods
     double pmass;
 };
@@ -85,7 +87,7 @@ __host__ __device__ inline int near_count(int n, int level) { return (n + (8 << 
 struct NearScratch
 {
     double4 P[32];                 // the members: position and one test value
-    float4 Q[32];                  // position relative to the box centre, squared reach
+    float4 Q[32];                  // position and squared reach in the search frame
     int front[kNearLevels][32];    // accepted nodes of each level, not yet expanded
     int blk[kNearBlocks];          // accepted blocks, ascending
     int sel[kNearBlocks + 8];      // those one member reaches, then kNearNone
@@ -127,13 +129,23 @@ __device__ __forceinline__ void st_shared_if(bool p, int* a, int v)
                  :: "r"(int(p)), "r"(smem_u32(a)), "r"(v) : "memory");
 }
 
-// The search frame: box centre and periods, and the slack of a radius.  A relative
-// coordinate a is rounded by at most 2^-24 |a|, and a gap's two subtractions (and the fold
-// at the period) by as much again of terms no larger than the box, so the gap of a point
-// errs by less than 2^-22 (len + |a|) per axis; 4e-7 (len + |a|_1) covers three axes.
+// The power of two that brings a length into [1, 2) (1 for one that is 0 or beyond any use).
+__device__ __forceinline__ double near_scale(double len)
+{
+    const int e = int(__double_as_longlong(len) >> 52);   // the exponent's bits (len >= 0)
+    return e > 0 && e <= 2045 ? __longlong_as_double((long long)(2046 - e) << 52) : 1.0;
+}
+
+// The search frame: box centre, scale and periods, and the slack of a radius.  Lengths in it
+// are the caller's times the scale, which is exact: a reach of 2^64 or 2^-75 in the caller's
+// units would have a square of infinity or 0 in FP32, and every block would pass its test or
+// some of those it needs would not.  A relative coordinate a is rounded by at most 2^-24 |a|,
+// and a gap's two subtractions (and the fold at the period) by as much again of terms no
+// larger than the box, so the gap of a point errs by less than 2^-22 (len + |a|) per axis;
+// 4e-7 (len + |a|_1) covers three axes.
 struct NearFrame
 {
-    double cx, cy, cz;
+    double cx, cy, cz, scale;
     float lx, ly, lz, len;
 
     __device__ __forceinline__ explicit NearFrame(const DevBox* b)
@@ -141,15 +153,22 @@ struct NearFrame
         cx = b->lo[0] + 0.5 * b->len[0];
         cy = b->lo[1] + 0.5 * b->len[1];
         cz = b->lo[2] + 0.5 * b->len[2];
-        lx = float(b->len[0]);
-        ly = float(b->len[1]);
-        lz = float(b->len[2]);
+        scale = near_scale(fmax(b->len[0], fmax(b->len[1], b->len[2])));
+        lx = float(b->len[0] * scale);
+        ly = float(b->len[1] * scale);
+        lz = float(b->len[2] * scale);
         len = fmaxf(lx, fmaxf(ly, lz));
     }
     __device__ __forceinline__ explicit NearFrame(const NearSet& s)
-        : cx(s.cx), cy(s.cy), cz(s.cz), lx(s.lx), ly(s.ly), lz(s.lz), len(s.len)
+        : cx(s.cx), cy(s.cy), cz(s.cz), scale(s.scale), lx(s.lx), ly(s.ly), lz(s.lz), len(s.len)
     {
     }
+    // a position, and a length rounded up, in the frame
+    __device__ __forceinline__ float3 at(const double4& p) const
+    {
+        return make_float3(float((p.x - cx) * scale), float((p.y - cy) * scale), float((p.z - cz) * scale));
+    }
+    __device__ __forceinline__ float length(double r) const { return __double2float_ru(r * scale); }
     __device__ __forceinline__ float slack(float x, float y, float z) const
     {
         return 4e-7f * (len + fabsf(x) + fabsf(y) + fabsf(z));

@@ -133,3 +133,38 @@ def test_the_tree_of_a_set_is_held_while_the_arrays_grow():
             assert held.setdefault(k, c.scalar(k)) == c.scalar(k)
         for k in ("layout", "csTree", "hmax_leaf", "centers"):
             np.testing.assert_array_equal(held.setdefault(k, c.array(k)), c.array(k), err_msg=k)
+
+
+@pytest.mark.parametrize("power", [-200, -75, -70, 62, 70, 120, 200])
+@pytest.mark.parametrize("case", ["box", "plummer"])
+def test_units_change_nothing(case, power):
+    """Lengths times a power of two are the same solve: h times that power, rho over its cube,
+    in as many iterations, bit for bit.  (Beyond 2^62 and below 2^-70 the square of a
+    length leaves FP32's range.)"""
+    quantum = 2.0 ** power
+    p = _box(20000, 8) if case == "box" else inputs.plummer(20000, hfact=1.2, lnsigma=0.5, seed=9)
+    q = inputs.Particles(**{k: p[k] * quantum for k in "xyzh"}, pmass=p["pmass"])
+    out = []
+    for s, unit in ((p, 1.0), (q, quantum)):
+        box = None if case == "plummer" else [v * unit for v in UNIT]
+        st, c = _solve(s, box)
+        assert st == 0
+        out.append((c.download(capi.HSML, s.n)[0] / unit, c.download(capi.DENS_OUT, s.n)[0] * unit * unit * unit,
+                    c.array("activePerIter"), c.scalar("pairsGrad"), c.scalar("extraCount")))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_large_units_cost_no_more():
+    """A reach whose square overflows FP32 is not a search of everything: 300,000 particles in
+    a box 2^90 wide take about the time of the unit box (all pairs: a hundred times that)."""
+    p, best = _box(300000, 10), []
+    for unit in (1.0, 2.0 ** 90):
+        s = inputs.Particles(**{k: p[k] * unit for k in "xyzh"}, pmass=p["pmass"])
+        times = []
+        for _ in range(3):
+            st, c = _solve(s, [v * unit for v in UNIT])
+            assert st == 0
+            times.append(c.scalar("t_nrkern"))
+        best.append(min(times))
+    assert best[1] <= 2.0 * best[0]
