@@ -280,10 +280,18 @@ gradient_warp_kernel(const __grid_constant__ NearTree t, const NearLoop* __restr
             const float3 a = f.at(pi);
             const float x = a.x, y = a.y, z = a.z;
             const float r = f.length(kRadKernel * (1.0 + 1e-6) * pi.w) + f.slack(x, y, z);
+            auto inside = [&](const double4& pj) {
+                double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+                return pair_r2(dx, dy, dz) * hinv2 < kRadK2;
+            };
+            auto pairs32 = [&](int j, int count) { pair(ldg4(t.xyzh + j), j, lane < count); };
+            int held = 0;
             near_blocks<0, Periodic, false>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, 0.0f, [&](int nb) -> float {
-                near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, pair);
+                near_packed(sScr[wib], nb, v.n, t.xyzh, held, inside, pairs32);
                 return r;
             });
+            near_packed_end(sScr[wib], held, pairs32);
         }
         GradSums g;
 #pragma unroll
@@ -1199,7 +1207,7 @@ static void sym_rows_from_newton(State& s, bool near)
     if (near)
     {
         auto ov = s.periodic ? over_extras_kernel<true> : over_extras_kernel<false>;
-        ov<<<2 * s.numSMs, kThreads, 0, s.st>>>(near_tree(s), s.nearLoop.get(), s.nearOver.get(), s.hs.get(),
+        ov<<<std::min(iceil(nA, kWarpsPerBlock), persistent_blocks(s, ov, kThreads)), kThreads, 0, s.st>>>(near_tree(s), s.nearLoop.get(), s.nearOver.get(), s.hs.get(),
                                                 s.nblH.get(), s.extras.get(), s.extraCnt.get(), ds);
         COSMO_LAUNCHED();
     }
@@ -1561,8 +1569,11 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
                     s.gradh.get(), s.divv.get(), s.xi.get(), s.ddivvdt.get(), pmass, s.box.get(), ds, loop, halfBox);
                 COSMO_LAUNCHED();
             }
-            if (near && fromRows)
-                warps(s.periodic ? gradient_warp_kernel<true, false> : gradient_warp_kernel<false, false>, 2 * s.numSMs);
+            if (near && fromRows && s.nAlive > 0)
+            {
+                auto over = s.periodic ? gradient_warp_kernel<true, false> : gradient_warp_kernel<false, false>;
+                warps(over, std::min(iceil(s.nAlive, kWarpsPerBlock), persistent_blocks(s, over, kThreads)));
+            }
             // the group sweep of the rows that overflowed (none: it returns at once)
             auto gk = s.periodic ? gradient_kernel<true> : gradient_kernel<false>;
             if (!(near && fromRows)) gk<<<grid, kThreads, 0, s.st>>>(s.nLeaves, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),

@@ -464,10 +464,20 @@ force_warp_kernel(const __grid_constant__ NearTree t, int n, const int* __restri
             const float x = a.x, y = a.y, z = a.z;
             const float slack = f.slack(x, y, z);
             const float r = f.length(kRadKernel * (1.0 + 1e-6) * A.p.w) + slack;
+            // the exact tests terms() starts with
+            auto inside = [&](const double4& pj) {
+                double dx = A.p.x - pj.x, dy = A.p.y - pj.y, dz = A.p.z - pj.z;
+                nearest_image<Periodic>(dx, dy, dz, lx, ly, lz);
+                const double dr2 = pair_r2(dx, dy, dz);
+                return dr2 > 0.0 && !(dr2 >= kRadK2 * fmax(A.p.w * A.p.w, pj.w * pj.w) * (1.0 + 1e-10));
+            };
+            auto pairs32 = [&](int j, int count) { pair(ldg4(t.xyzh + j), j, lane < count); };
+            int held = 0;
             near_blocks<0, Periodic, true>(t, v, sScr[wib], x, y, z, 0.0f, 0.0f, 0.0f, r, slack, [&](int nb) -> float {
-                near_candidates(sScr[wib].blk, nb, v.n, t.xyzh, pair);
+                near_packed(sScr[wib], nb, v.n, t.xyzh, held, inside, pairs32);
                 return r;
             });
+            near_packed_end(sScr[wib], held, pairs32);
         }
         A.itx = __shfl_sync(0xffffffffu, sum, 0); A.ity = __shfl_sync(0xffffffffu, sum, 1);
         A.itz = __shfl_sync(0xffffffffu, sum, 2); A.jtx = __shfl_sync(0xffffffffu, sum, 3);

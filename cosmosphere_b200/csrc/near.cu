@@ -879,8 +879,8 @@ __device__ __noinline__ double2 near_add_records(double2* rec, int m, double2 s)
 // one warp's work, or a block's.
 __device__ __forceinline__ void sum_finish(int i, double hi, double2 sums, unsigned int got, NearLoop* L,
                                            const NearLists& lists, int nxt, double4* xyzh, double* rho, double* gradh,
-                                           int* converged, double* hs, double pmass, double tolh, double hfact,
-                                           unsigned long long& seen, unsigned long long& hconv)
+                                           int* converged, double* hs, double* rowH, double pmass, double tolh,
+                                           double hfact, unsigned long long& seen, unsigned long long& hconv)
 {
     double ro, go, ho;
     int conv;
@@ -896,7 +896,15 @@ __device__ __forceinline__ void sum_finish(int i, double hi, double2 sums, unsig
         converged[i] = 1;
         hs[i] = ho;
         hconv = ob > hconv ? ob : hconv;
-        lists.cover[atomicAdd(&L->cover, 1)] = i;
+        if (got > kNbl)
+        {
+            // no row would hold them: it is among those without one at once (near_rows_kernel,
+            // which counted kNbl + 1 for it, would find that out by another search)
+            rowH[i] = double(INFINITY);
+            lists.over[atomicAdd(&L->over, 1)] = i;
+        }
+        else
+            lists.cover[atomicAdd(&L->cover, 1)] = i;
         return;
     }
     const double ratio = ho / hi, expect = double(got) * ratio * ratio * ratio;
@@ -917,7 +925,8 @@ near_sum_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__ 
                 const int* __restrict__ setOf, NearLoop* __restrict__ L,
                 const __grid_constant__ NearLists lists, double4* __restrict__ xyzh,
                 double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
-                double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
+                double* __restrict__ hs, double* __restrict__ rowH, double pmass, double tolh, double hfact,
+                DevScalars* __restrict__ ds)
 {
     __shared__ NearScratch sScr[kNearWarps];
     __shared__ double2 sRec[kNearWarps][kNearRec];
@@ -996,8 +1005,8 @@ near_sum_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__ 
             pairs += got;
             if constexpr (Eval) eval_store(i, hi, sums.x, sums.y, pmass, rho, gradh);
             else
-                sum_finish(i, hi, sums, got, L, lists, nxt, xyzh, rho, gradh, converged, hs, pmass, tolh, hfact, seen,
-                           hconv);
+                sum_finish(i, hi, sums, got, L, lists, nxt, xyzh, rho, gradh, converged, hs, rowH, pmass, tolh, hfact,
+                           seen, hconv);
         }
         __syncwarp();
     }
@@ -1017,7 +1026,8 @@ near_huge_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
                 const int* __restrict__ setOf, NearLoop* __restrict__ L,
                  const __grid_constant__ NearLists lists, double4* __restrict__ xyzh,
                  double* __restrict__ rho, double* __restrict__ gradh, int* __restrict__ converged,
-                 double* __restrict__ hs, double pmass, double tolh, double hfact, DevScalars* __restrict__ ds)
+                 double* __restrict__ hs, double* __restrict__ rowH, double pmass, double tolh, double hfact,
+                 DevScalars* __restrict__ ds)
 {
     __shared__ NearScratch scr;
     __shared__ double2 sRec[kHugeWarps][kNearRec];
@@ -1147,8 +1157,8 @@ near_huge_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
             unsigned int all = 0;
             for (int k = 0; k < kHugeWarps; ++k) all += unsigned(sCount[k]);
             pairs += all;
-            sum_finish(i, hi, sSums, all, L, lists, nxt, xyzh, rho, gradh, converged, hs, pmass, tolh, hfact, seen,
-                       hconv);
+            sum_finish(i, hi, sSums, all, L, lists, nxt, xyzh, rho, gradh, converged, hs, rowH, pmass, tolh, hfact,
+                       seen, hconv);
         }
     }
     note_h(seen, hconv, ds, shH);
@@ -1267,13 +1277,13 @@ static void near_iteration(State& s, const NearJob& j, cudaGraphConditionalHandl
     COSMO_LAUNCHED();
     auto sum = NEAR_PICK(near_sum_kernel, j, NEAR_COMMA false);
     sum<<<persistent_blocks(s, sum, kThreads), kThreads, 0, s.st>>>(j.tree, j.sets, j.setOf, L, lists, j.xyzh, j.rho,
-                                                                    j.gradh, j.converged, s.hs.get(), j.pmass, j.tolh,
-                                                                    j.hfact, ds);
+                                                                    j.gradh, j.converged, s.hs.get(), s.nblH.get(), j.pmass,
+                                                                    j.tolh, j.hfact, ds);
     COSMO_LAUNCHED();
     // few particles have that many neighbours, if any: a block a multiprocessor
     auto huge = NEAR_PICK(near_huge_kernel, j);
     huge<<<s.numSMs, 32 * kHugeWarps, 0, s.st>>>(j.tree, j.sets, j.setOf, L, lists, j.xyzh, j.rho, j.gradh, j.converged,
-                                                 s.hs.get(), j.pmass, j.tolh, j.hfact, ds);
+                                                 s.hs.get(), s.nblH.get(), j.pmass, j.tolh, j.hfact, ds);
     COSMO_LAUNCHED();
     near_epilogue_kernel<<<1, kNearQueues, 0, s.st>>>(L, more, setCondition);
     COSMO_LAUNCHED();
@@ -1492,8 +1502,8 @@ void near_forest_eval(State& s, const NearForest& b)
     COSMO_LAUNCHED();
     auto sum = near_sum_kernel<true, true, true>;
     sum<<<persistent_blocks(s, sum, kThreads), kThreads, 0, s.st>>>(t, s.nearSets.get(), b.setOf, L, lists, b.xyzh,
-                                                                    b.rho, b.gradh, b.converged, s.hs.get(), 0.0, 0.0,
-                                                                    0.0, s.dscal.get());
+                                                                    b.rho, b.gradh, b.converged, s.hs.get(), nullptr, 0.0,
+                                                                    0.0, 0.0, s.dscal.get());
     COSMO_LAUNCHED();
 }
 

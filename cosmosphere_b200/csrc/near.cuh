@@ -411,4 +411,40 @@ __device__ __forceinline__ void near_candidates(const int* ids, int ns, int nLiv
     }
 }
 
+// The same, the candidates that pass test(pj) packed: use(j, count) for up to 32 of them at a time,
+// lane k < count the k-th, in ascending j (scr.sel holds those not handed out yet, held of
+// them).  A search of one particle's support tests two to three candidates for each pair it
+// accepts: evaluated where they were loaded, most lanes would wait for the others.  Call
+// near_packed_end after the last blocks.
+template<class Test, class Use>
+__device__ __forceinline__ void near_packed(NearScratch& scr, int nb, int nLive, const double4* __restrict__ xyzh,
+                                            int& held, Test&& test, Use&& use)
+{
+    const int lane = threadIdx.x & 31;
+    near_candidates(scr.blk, nb, nLive, xyzh, [&](const double4& pj, int j, bool valid) {
+        const bool ok = valid && test(pj);
+        const uint32_t m = __ballot_sync(0xffffffffu, ok);
+        if (ok) scr.sel[held + __popc(m & ((1u << lane) - 1u))] = j;
+        held += __popc(m);
+        __syncwarp();
+        if (held < 32) return true;
+        use(scr.sel[lane], 32);
+        const int beyond = scr.sel[32 + lane];
+        __syncwarp();
+        held -= 32;
+        if (lane < held) scr.sel[lane] = beyond;
+        __syncwarp();
+        return true;
+    });
+}
+
+template<class Use>
+__device__ __forceinline__ void near_packed_end(NearScratch& scr, int& held, Use&& use)
+{
+    const int lane = threadIdx.x & 31;
+    if (held > 0) use(scr.sel[min(lane, held - 1)], held);
+    held = 0;
+    __syncwarp();
+}
+
 } // namespace cosmo

@@ -168,3 +168,36 @@ def test_large_units_cost_no_more():
             times.append(c.scalar("t_nrkern"))
         best.append(min(times))
     assert best[1] <= 2.0 * best[0]
+
+
+def _whole(p, hfact, quintic, box, options):
+    """A solve and force pass: every result, and the seconds both took on the device."""
+    c = capi.Cosmo(quintic)
+    best = np.inf
+    for _ in range(3):
+        st, c = _solve(p, box, options, c, hfact=hfact)
+        assert st == 0
+        c.upload(capi.THERMO, np.ones((4, p.n)), sorted_=True)
+        c.force(p.n, p["pmass"], alphau=0.5)
+        best = min(best, sum(c.scalar("t_" + k) for k in ("bbox", "keysort", "tree", "nodes", "jbuild", "nrkern",
+                                                          "gjbuild", "gradkern", "fjbuild", "prep", "fkern")))
+    return [c.download(s, p.n) for s in (capi.HSML, capi.DENS_OUT, capi.GRAD_OUT, capi.FORCE_OUT)], best
+
+
+@pytest.mark.parametrize("case,hfact,quintic", [("box", 1.7, False), ("open", 2.0, False), ("plummer", 1.6, False),
+                                                ("box", 1.4, True)])
+def test_more_neighbours_than_a_row_holds(case, hfact, quintic):
+    """Sets of which every particle has more neighbours than a row holds: the searches of the
+    sweeps find the pairs that the lists' groups do, in the same order."""
+    p = _box(30000, 15, hfact) if case != "plummer" else inputs.plummer(20000, hfact=hfact, lnsigma=0.3, seed=16)
+    box = UNIT if case == "box" else None
+    near, lists = _whole(p, hfact, quintic, box, ()), _whole(p, hfact, quintic, box, LISTS)
+    for a, b in zip(near[0], lists[0]):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("hfact,quintic", [(1.6, False), (2.0, False), (1.4, True)])
+def test_more_neighbours_than_a_row_holds_cost_no_more_than_over_lists(hfact, quintic):
+    """Such sets took up to twice the list-based solve's time; 1.2 is the room for noise."""
+    p = _box(150000, 17, hfact)
+    assert _whole(p, hfact, quintic, UNIT, ())[1] <= 1.2 * _whole(p, hfact, quintic, UNIT, LISTS)[1]
