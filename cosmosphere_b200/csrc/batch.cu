@@ -567,7 +567,7 @@ __device__ __forceinline__ bool nr_step_b(double rhoi, double gradhi, double hi,
 // set's mass, periodicity and box.  A cut item scans its set's tree for its own box
 // instead of streaming the leaf's whole list.
 template<bool Mixed, bool EvalAll, bool Staged>
-__global__ void __launch_bounds__(kThreads, Mixed ? 4 : 5)   // measured best of 4, 5, 6
+__global__ void __launch_bounds__(kThreads, 4)   // at five and six blocks a multiprocessor its registers spill
 density_batch_kernel(const int4* __restrict__ items, int cap, const int* __restrict__ leafSet,
                      const uint2* __restrict__ range, const uint32_t* __restrict__ jOffset,
                      const uint32_t* __restrict__ jcount, const int* __restrict__ jlist, double4* __restrict__ xyzh,

@@ -39,11 +39,13 @@ constexpr double kSettle = 0.15;
 // iteration (once per leaf), and flags the lists stale when an updated h outgrows the
 // radius its leaf's list covers.  Staged: the group's j-stream is staged into shared
 // memory by bulk copies (the WarpStage of its warp) instead of loaded directly.
-// Four blocks a multiprocessor in the mixed form: at six its registers spill (the loop of a
-// 30,000-particle Plummer sphere 15.6 ms against 12.9; of a 300,000-particle box 3.10 against
-// 3.15).
+// Four blocks a multiprocessor: at five (plain) and six (mixed) its registers spill, which a
+// warp alone on its scheduler -- a small or concentrated set's longest group -- waits out at
+// every step (mixed, the loop of a 30,000-particle Plummer sphere 15.6 ms against 12.9, of a
+// 300,000-particle box 3.10 against 3.15; plain, a density solve of 3,000 Plummer particles
+// 4.37 against 3.28, 150,000 22.8 against 17.1, a box of 150,000 2.43 against 2.32).
 template<bool Periodic, bool Mixed, bool Staged>
-__global__ void __launch_bounds__(kThreads, Mixed ? 4 : 5)
+__global__ void __launch_bounds__(kThreads, 4)
 density_nr_kernel(const int4* __restrict__ items, int cap, const uint32_t* __restrict__ layout,
                   const uint32_t* __restrict__ jOffset, const uint32_t* __restrict__ jcount,
                   const int* __restrict__ jlist, double4* __restrict__ xyzh, double* __restrict__ rho,
