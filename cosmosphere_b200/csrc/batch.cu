@@ -1005,7 +1005,9 @@ static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int fla
     // the group engine's groups; the staged feed is a variant of that engine).  Its rows take
     // 1 KB a particle: very large batches keep the lists, which take less.  A batch with a
     // particle outside its set's box is solved over the lists (solve_density).
-    if (!lists && s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost)
+    // So does a large one of very many neighbours (near_crowded).
+    s.blockTree = !lists && s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost && !near_crowded(B.n, hfact);
+    if (s.blockTree)
     {
         const int st = batch_solve_near(B, tolh, hfact, maxIter, flags, t0);
         return s.hscal->outside ? batch_solve(B, tolh, hfact, maxIter, flags, 0, true) : st;
@@ -1290,6 +1292,7 @@ double cosmo_batch_scalar(const char* name)
     if (k == "t_total") return B.tTotal;
     if (k == "t_nr") return B.tNR;
     if (k == "graph") return B.graphUsed ? 1.0 : 0.0;
+    if (k == "blockTree") return B.core.blockTree ? 1.0 : 0.0;
     if (k == "t_nr") return B.tNR;
     if (k == "t_list") return B.tList;
     return NAN;

@@ -864,6 +864,7 @@ double cosmo_x_scalar(const char* name)
     if (k == "hfact") return s.hfact;
     if (k == "maxIter") return s.maxIter;
     if (k == "settling0") return double(s.settling0);
+    if (k == "blockTree") return s.blockTree ? 1.0 : 0.0;
     if (k == "loopGraph") return double(s.lastLoopGraph);
     if (k == "hmaxSeen" && s.hscal)
     {

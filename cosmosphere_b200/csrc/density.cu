@@ -1219,11 +1219,11 @@ static void sym_rows_from_newton(State& s, bool near)
 
 // Whether a solve's Newton loop runs over the block tree (near.cu): the plain form with the
 // gradient sweep.  The mixed form keeps the group engine (its rounding is defined by the
-// groups), a solve without gradients the lists it must leave behind, and so does one asked
-// for a variant of the list-based loop.
-static bool near_solve(const State& s, bool withGradients)
+// groups), a solve without gradients the lists it must leave behind, and so do a large set of
+// very many neighbours (near_crowded) and a solve asked for a variant of the list-based loop.
+static bool near_solve(const State& s, int n, double hfact, bool withGradients)
 {
-    return withGradients && s.precision == 0 && s.staging == 0 && s.splitStream == 0 && s.splitWork == 0 &&
+    return withGradients && !near_crowded(n, hfact) && s.precision == 0 && s.staging == 0 && s.splitStream == 0 && s.splitWork == 0 &&
            s.spreadGroups == 0 && s.graphListStorePct == 0;
 }
 
@@ -1248,7 +1248,8 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     // next few solves do not write them.
     const bool tryRows = s.symRowsSkip == 0;
     if (s.symRowsSkip > 0) --s.symRowsSkip;
-    const bool near = !lists && near_solve(s, withGradients);
+    const bool near = !lists && near_solve(s, n, hfact, withGradients);
+    s.blockTree = near;
     const bool writeJ = near ? s.symFromRows != 0
                              : withGradients && s.symFromRows && s.frozenFor != n && tryRows;
 

@@ -43,6 +43,21 @@ constexpr int kNearWarps  = 4;     // warps per block of the search kernels
 constexpr int kWarpPerParticle = 32768;
 constexpr int kWarpPerParticleForce = 12288;
 
+// Whether a solve over the block tree loses to one over lists: a large set of which every
+// particle has more neighbours than a row holds -- 4/3 pi (R hfact)^3 of them at its converged
+// h -- is all searches of single particles, where a leaf's groups share theirs.  Device times
+// of the whole step, block tree and lists: box of 1,000,000 at hfact 1.5 (113 neighbours)
+// 28.1 and 32.0 ms, 1.53 (120) 35.0 and 35.9, 1.55 (125) 41.2 and 37.9, 1.6 56.0 and 45.6,
+// 2.2 102 and 83; at 1.6 450,000 25.4 and 24.8, 340,000 19.4 and 22.7, 150,000 8.9 and 9.3
+// (a Plummer sphere 10.8 and 26.0).  Batches (whole solve): 10 boxes of 10,000 at 1.6 3.0
+// and 3.5, 6 of 100,000 15.5 and 11.4, 24 of 100,000 60.0 and 40.4.
+constexpr int kNearCrowded = 400000;
+inline bool near_crowded(int n, double hfact)
+{
+    const double reach = kRadKernel * hfact;
+    return n > kNearCrowded && 4.18879 * reach * reach * reach > 0.95 * kNbl;
+}
+
 // A node's box: centre, half extents (empty: negative infinity) and its largest h.
 struct alignas(32) NearNode
 {

@@ -75,3 +75,16 @@ def test_final_rho_of_unconverged_particles(max_iter, graph, quintic):
         r, g, size = _direct(s, h[k], quintic)
         assert np.max(np.abs(rho[k] / r - 1.0)) <= 1e-11, k
         assert np.max(np.abs(gradh[k] - g) / size) <= 1e-11, k
+
+
+@pytest.mark.parametrize("sizes,hfact,near", [((200000, 200000), 1.6, 1), ((200000, 200001), 1.6, 0),
+                                              ((200000, 200001), 1.5, 1)])
+def test_large_crowded_batches_are_solved_over_lists(sizes, hfact, near):
+    sets = [_box(n, 20 + k, hfact) for k, n in enumerate(sizes)]
+    st, b, got = _batch(sets, hfact=hfact, final_rho=True)
+    assert st == 0 and b.scalar("blockTree") == near
+    if not near:
+        _, _, ref = _batch(sets, staging=True, hfact=hfact, final_rho=True)
+        for a, r in zip(got, ref):
+            for x, y in zip(a, r):
+                np.testing.assert_array_equal(x, y)

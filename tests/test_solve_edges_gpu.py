@@ -223,3 +223,9 @@ def test_the_list_loop_of_a_small_concentrated_set(n):
             times.append(c.scalar("t_nrkern"))
         best.append(min(times))
     assert best[0] <= 1.4 * best[1]
+
+
+@pytest.mark.parametrize("n,hfact,near", [(400000, 1.6, 1), (400001, 1.6, 0), (400001, 1.5, 1)])
+def test_large_crowded_sets_are_solved_over_lists(n, hfact, near):
+    st, c = _solve(_box(n, 19, hfact), UNIT, hfact=hfact)
+    assert st == 0 and c.scalar("blockTree") == near
