@@ -988,7 +988,7 @@ static int batch_solve_near(Batch& B, double tolh, double hfact, int maxIter, in
     return B.unconverged > 0 ? 1 : 0;
 }
 
-static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int flags, int attempt = 0, bool lists = false)
+static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int flags, int attempt = 0)
 {
     State& s = B.core;
     if (!(hfact > 0.0)) hfact = kHfactDefault;
@@ -1003,15 +1003,17 @@ static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int fla
     batch_sort(B);
     // The plain form runs over the sets' block trees (the mixed form's rounding is defined by
     // the group engine's groups; the staged feed is a variant of that engine).  Its rows take
-    // 1 KB a particle: very large batches keep the lists, which take less.  A batch with a
-    // particle outside its set's box is solved over the lists (solve_density).
-    // So does a large one of very many neighbours (near_crowded).
-    s.blockTree = !lists && s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost && !near_crowded(B.n, hfact);
+    // 1 KB a particle: very large batches keep the lists, which take less.  So does a large one
+    // of very many neighbours (near_crowded), and one with a particle outside its set's box
+    // (solve_density; reading that flag first takes 12 us, solving every set twice for it
+    // would take a solve).
+    s.blockTree = s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost && !near_crowded(B.n, hfact);
     if (s.blockTree)
     {
-        const int st = batch_solve_near(B, tolh, hfact, maxIter, flags, t0);
-        return s.hscal->outside ? batch_solve(B, tolh, hfact, maxIter, flags, 0, true) : st;
+        read_scalars(s);
+        s.blockTree = s.hscal->outside == 0;
     }
+    if (s.blockTree) return batch_solve_near(B, tolh, hfact, maxIter, flags, t0);
     batch_forest(B);
     const int L = B.nLeaves;
     long long nAliveTotal = 0;
@@ -1092,7 +1094,7 @@ static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int fla
     if ((s.hscal->err & kErrListFull) && attempt < 6)
     {
         COSMO_CUDA(cudaMemsetAsync(&ds->err, 0, sizeof(int), s.st));
-        return batch_solve(B, tolh, hfact, maxIter, flags, attempt + 1, lists);
+        return batch_solve(B, tolh, hfact, maxIter, flags, attempt + 1);
     }
     LoopState fin{};
     COSMO_CUDA(cudaMemcpyAsync(&fin, B.loop.get(), sizeof(LoopState), cudaMemcpyDeviceToHost, s.st));

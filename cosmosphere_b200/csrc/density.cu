@@ -538,8 +538,10 @@ __global__ void __launch_bounds__(kThreads)
 sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restrict__ rowsR2,
                      int* __restrict__ nblCount, const double* __restrict__ hs, const double* __restrict__ rowH,
                      const double4* __restrict__ xyzh, const DevBox* __restrict__ box, int* __restrict__ nbl,
-                     int* __restrict__ extras, int* __restrict__ extraCnt, DevScalars* __restrict__ ds)
+                     int* __restrict__ extras, int* __restrict__ extraCnt, DevScalars* __restrict__ ds,
+                     const int* __restrict__ skip)
 {
+    if (skip != nullptr && *skip) return;
     constexpr bool kExact = std::is_same<T, double>::value;
     using R4 = typename std::conditional<kExact, double4, float4>::type;
     double lx = 0, ly = 0, lz = 0;
@@ -615,8 +617,10 @@ __global__ void __launch_bounds__(kThreads)
 sym_from_rows_warp_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restrict__ rowsR2,
                           int* __restrict__ nblCount, const double* __restrict__ hs, const double* __restrict__ rowH,
                           const double4* __restrict__ xyzh, const DevBox* __restrict__ box, int* __restrict__ nbl,
-                          int* __restrict__ extras, int* __restrict__ extraCnt, DevScalars* __restrict__ ds)
+                          int* __restrict__ extras, int* __restrict__ extraCnt, DevScalars* __restrict__ ds,
+                          const int* __restrict__ skip)
 {
+    if (skip != nullptr && *skip) return;
     constexpr bool kExact = std::is_same<T, double>::value;
     double lx = 0, ly = 0, lz = 0;
     if (Periodic && !kExact) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
@@ -1192,7 +1196,8 @@ static void sym_rows_from_newton(State& s, bool near)
     const int grid = std::max(1, iceil(nA, warp ? kWarpsPerBlock : kThreads));
     auto compact = [&](auto kern, const auto* rows) {
         kern<<<grid, kThreads, 0, s.st>>>(nA, s.nblJ.get(), rows, s.nblCount.get(), s.hs.get(), s.nblH.get(),
-                                          s.xyzh.get(), s.box.get(), s.nbl.get(), s.extras.get(), s.extraCnt.get(), ds);
+                                          s.xyzh.get(), s.box.get(), s.nbl.get(), s.extras.get(), s.extraCnt.get(), ds,
+                                          near ? &ds->outside : nullptr);   // a loop that was not run made no rows
     };
     // the mixed form's Newton rows hold FP32 r^2 in the same buffer
     const float* rowsF = reinterpret_cast<const float*>(s.nblR2.get());
@@ -1255,8 +1260,11 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
 
     // A particle outside the box lies in no cell of the leaf tree that its key puts it in, and
     // the lists (as the reference's do) may miss its pairs, which the block tree, whose boxes
-    // are the particles' own, finds: such a solve is made over the lists.
+    // are the particles' own, finds: such a solve is made over the lists.  The block-tree loop
+    // and the passes after it then do nothing, and a state that met such a set reads the flag
+    // before them at its next solve.
     auto onLists = [&]() {
+        s.metOutside = true;
         return solve_density(s, n, pmass, periodicBox, tolh, hfact, maxIter, withGradients, allowGraph, true);
     };
 
@@ -1274,12 +1282,13 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     if (near)
     {
         s.nAlive = n;
-        if (n > kReadAlive)
+        if (n > kReadAlive || s.metOutside)
         {
             read_scalars(s);
-            s.nAlive = s.hscal->nAlive;
+            if (n > kReadAlive) s.nAlive = s.hscal->nAlive;
             if (s.hscal->outside) return onLists();
         }
+        s.metOutside = false;
     }
     const int itemCap = std::max(s.nAlive, 1);
     if (!near)

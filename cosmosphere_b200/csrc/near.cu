@@ -253,13 +253,14 @@ __device__ __forceinline__ void note_h(unsigned long long seen, unsigned long lo
     }
 }
 
-// All live particles are searched first (the identity list); the counters of the row passes
+// All live particles are searched first (the identity list), or none where one lies outside
+// the box of its key (the set is solved over lists instead); the counters of the row passes
 // after the loop start from zero too.
 __global__ void near_init_kernel(NearLoop* L, DevScalars* ds, int maxIter, int frozen)
 {
     L->queue[threadIdx.x] = 0;
     if (threadIdx.x != 0) return;
-    const int n = ds->nAlive;
+    const int n = ds->outside ? 0 : ds->nAlive;
     L->iter = 0;
     L->maxIter = maxIter;
     L->active = n;
@@ -282,6 +283,7 @@ near_frozen_kernel(NearLoop* L, const int* __restrict__ order, const int* __rest
 {
     __shared__ int sh[3 * (kNearWarps + 1)];
     __shared__ unsigned long long shH[2];
+    if (ds->outside) return;
     const int n = *nLive;
     unsigned long long hconv = 0;
     for (int b = blockIdx.x * kThreads; b < n; b += gridDim.x * kThreads)

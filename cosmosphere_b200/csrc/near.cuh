@@ -377,12 +377,13 @@ void near_forest_newton(State& s, const NearForest& b, double tolh, double hfact
 void near_forest_eval(State& s, const NearForest& b);
 
 // Whether the block-tree loop L ended without a result, so that the passes after it have
-// nothing to do: some h did not converge, or the largest support reaches half the box
-// (halfBox; not a number for an open set).  L null: the list-based loop, which has told the host.
+// nothing to do: it was not run (a particle outside the box of its key), some h did not
+// converge, or the largest support reaches half the box (halfBox; not a number for an open
+// set).  L null: the list-based loop, which has told the host.
 __device__ __forceinline__ bool near_failed(const NearLoop* L, const DevScalars* ds, double halfBox)
 {
     return L != nullptr &&
-           (L->active > 0 || kRadKernel * __longlong_as_double((long long)ds->hmaxConv) >= halfBox);
+           (ds->outside || L->active > 0 || kRadKernel * __longlong_as_double((long long)ds->hmaxConv) >= halfBox);
 }
 
 // As many blocks of a kernel as the device holds at once.

@@ -228,6 +228,7 @@ struct State
     int frozenFor = 0;   // the particle count the mask was given for (0: none)
     bool keyExtentSet = false;
     double keyExtent[6] = {0, 0, 0, 0, 0, 0};   // xmin, xmax, ymin, ymax, zmin, zmax
+    bool metOutside = false;                    // the last solve's set had a particle outside its box
     bool blockTree = false; // the last solve's Newton loop ran over the block tree
     int lastLoopGraph = 0;  // the last solve's Newton loop ran as a graph (1) or on the host (0)
     // The graph-run loop's instantiated graph, kept while the parameters it was captured

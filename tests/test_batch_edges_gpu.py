@@ -88,3 +88,31 @@ def test_large_crowded_batches_are_solved_over_lists(sizes, hfact, near):
         for a, r in zip(got, ref):
             for x, y in zip(a, r):
                 np.testing.assert_array_equal(x, y)
+
+
+def test_a_set_outside_its_box_sends_the_batch_over_lists_once():
+    """One set of a batch has a particle beyond its periodic box: all are solved over lists, as
+    each alone, and nothing is solved twice (launches are a staged batch's, which runs over
+    lists by itself)."""
+    sets = [_box(5000, 30), _box(3000, 31), _plummer(4000, 32, 0.3), _box(900, 33)]
+    sets[1]["x"] = sets[1]["x"].copy()
+    sets[1]["x"][7] += 1.7
+    c = capi.Cosmo()
+    n0 = c.launches()
+    st, b, got = _batch(sets, graph=False)
+    n1 = c.launches()
+    st2, _, ref = _batch(sets, graph=False, staging=True)
+    n2 = c.launches()
+    assert st == 0 and st2 == 0 and b.scalar("blockTree") == 0
+    assert n1 - n0 <= n2 - n1 + 2
+    for a, r in zip(got, ref):
+        for x, y in zip(a, r):
+            np.testing.assert_array_equal(x, y)
+    for k, s in enumerate(sets):
+        n = s["x"].size
+        c.arrays_init(n)
+        c.upload(capi.POS, np.stack([s["x"], s["y"], s["z"]]))
+        c.upload(capi.HSML, s["h"])
+        assert c.density_status(n, s["pmass"], periodic_box=s.get("box"), with_gradients=False) == 0
+        np.testing.assert_array_equal(got[0][k], c.download(capi.HSML, n)[0])
+        np.testing.assert_array_equal(got[1][k], c.download(capi.DENS_OUT, n)[0])

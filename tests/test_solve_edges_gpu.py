@@ -229,3 +229,31 @@ def test_the_list_loop_of_a_small_concentrated_set(n):
 def test_large_crowded_sets_are_solved_over_lists(n, hfact, near):
     st, c = _solve(_box(n, 19, hfact), UNIT, hfact=hfact)
     assert st == 0 and c.scalar("blockTree") == near
+
+
+def test_a_set_outside_its_box_is_solved_once():
+    """A set with particles beyond the box of their keys is solved over the lists: the
+    block-tree loop before it does nothing, and is left out when the last solve met such a
+    set already.  Launches count the work: the first solve adds the order and one empty
+    iteration and sweep, the next ones at most the order."""
+    p = _box(20000, 11)
+    p["x"] += 0.3
+    p["y"][::5] -= 0.7
+    st, c = _solve(_box(20000, 12), UNIT)
+    assert st == 0
+
+    def run(options):
+        n0 = c.launches()
+        st, _ = _solve(p, UNIT, options, c=c)
+        return st, c.download(capi.HSML, p.n), c.download(capi.DENS_OUT, p.n), c.launches() - n0
+
+    c.set_option("newton_graph", 0)
+    try:
+        lists, first, again = run(LISTS), run(()), run(())
+    finally:
+        c.set_option("newton_graph", 1)
+    for got in (first, again):
+        for a, b in zip(got[:3], lists[:3]):
+            np.testing.assert_array_equal(a, b)
+    assert first[3] <= lists[3] + 24
+    assert again[3] <= lists[3] + 8
