@@ -961,6 +961,29 @@ static void final_rho(Batch& B)
 
 constexpr int kNearBatchMost = 48 << 20;   // particles
 
+// Whether the rows of a block-tree loop over B's particles (1 KB a particle, 2 KB of the
+// quintic kernel, which is nearly all it takes beyond the lists' buffers) fit the device: they
+// are held already, or growing them takes at most half of what is free, so that a batch which
+// the lists would have solved does not run out of memory.
+static bool near_rows_fit(Batch& B)
+{
+    State& s = B.core;
+    const size_t entries = size_t(B.n) * kNbl;
+    if (entries <= s.nblR2.cap) return true;
+    size_t avail = s.batchRoomMB >= 0 ? size_t(s.batchRoomMB) << 20 : 0;
+    if (s.batchRoomMB < 0)
+    {
+        // free on the device, and what the library's pool holds unused
+        size_t fr = 0, total = 0;
+        uint64_t reserved = 0, used = 0;
+        COSMO_CUDA(cudaMemGetInfo(&fr, &total));
+        COSMO_CUDA(cudaMemPoolGetAttribute(device_pool(), cudaMemPoolAttrReservedMemCurrent, &reserved));
+        COSMO_CUDA(cudaMemPoolGetAttribute(device_pool(), cudaMemPoolAttrUsedMemCurrent, &used));
+        avail = fr + size_t(reserved - used);
+    }
+    return (entries + entries / 8) * sizeof(double) <= avail / 2;   // DBuf grows by an eighth more
+}
+
 // A batched solve over the sets' block trees (near.cu).
 static int batch_solve_near(Batch& B, double tolh, double hfact, int maxIter, int flags, cudaEvent_t t0)
 {
@@ -1002,12 +1025,13 @@ static int batch_solve(Batch& B, double tolh, double hfact, int maxIter, int fla
     cudaEvent_t t0 = ev(s);
     batch_sort(B);
     // The plain form runs over the sets' block trees (the mixed form's rounding is defined by
-    // the group engine's groups; the staged feed is a variant of that engine).  Its rows take
-    // 1 KB a particle: very large batches keep the lists, which take less.  So does a large one
-    // of very many neighbours (near_crowded), and one with a particle outside its set's box
-    // (solve_density; reading that flag first takes 12 us, solving every set twice for it
-    // would take a solve).
-    s.blockTree = s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost && !near_crowded(B.n, hfact);
+    // the group engine's groups; the staged feed is a variant of that engine).  Very large
+    // batches, and those whose rows the device has no room for, keep the lists, which take
+    // less memory.  So does a large one of very many neighbours (near_crowded), and one with
+    // a particle outside its set's box (solve_density; reading that flag first takes 12 us,
+    // solving every set twice for it would take a solve).
+    s.blockTree = s.precision == 0 && s.staging == 0 && B.n <= kNearBatchMost && !near_crowded(B.n, hfact) &&
+                  near_rows_fit(B);
     if (s.blockTree)
     {
         read_scalars(s);
@@ -1251,6 +1275,7 @@ int cosmo_batch_density(double tolh, double hfact, int maxIter, int flags)
     Batch& B = batch();
     if (B.n < 1) return -1;
     B.core.precision = state().precision;
+    B.core.batchRoomMB = state().batchRoomMB;
     return batch_solve(B, tolh, hfact, maxIter > 0 ? maxIter : 100, flags);
 }
 

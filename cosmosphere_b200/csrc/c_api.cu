@@ -759,6 +759,12 @@ int cosmo_x_set_option(const char* name, int value)
         s.graphListStorePct = value;
         return 0;
     }
+    if (k == "batch_room_mb")
+    {
+        if (value < -1) return -1;
+        s.batchRoomMB = value;
+        return 0;
+    }
     if (k == "spread_groups")
     {
         if (value < 0 || value > 32) return -1;

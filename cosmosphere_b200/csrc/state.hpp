@@ -218,6 +218,9 @@ struct State
     // rebuild outgrow it, so the fallback to the host loop can be exercised
     // (cosmo_x_set_option "graph_list_store")
     int graphListStorePct = 0;
+    // megabytes a batch takes the device to have room for (-1: what is free; cosmo_x_set_option
+    // "batch_room_mb", a test of the batches the rows do not fit)
+    int batchRoomMB = -1;
     size_t listStore = 0;   // list entries a fill may write (0: all jlist holds)
     // Open boundaries: the particle extents the bounding box is made from, when the caller
     // gives them (a rank of a decomposed set uses the whole set's, so its keys and order

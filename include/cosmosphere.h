@@ -234,7 +234,9 @@ void cosmo_x_sync(void);
  * COSMO_SYM_FROM_ROWS); "sym_extra_cap" k > 0 holds at most k of the pairs other
  * particles' supports add to those rows (0: the built-in, one per live particle), so that
  * a solve that finds more hands the force pass to the list-built rows (a test of that
- * fallback).
+ * fallback); "batch_room_mb" k >= 0 has a plain batch take k megabytes as what the device has
+ * room for (-1, the default: what is free), over half of which its rows send it to the lists
+ * (a test of that choice).
  * Returns 0, or -1 for an unknown name or a value out of range. */
 int cosmo_x_set_option(const char* name, int value);
 

@@ -116,3 +116,26 @@ def test_a_set_outside_its_box_sends_the_batch_over_lists_once():
         assert c.density_status(n, s["pmass"], periodic_box=s.get("box"), with_gradients=False) == 0
         np.testing.assert_array_equal(got[0][k], c.download(capi.HSML, n)[0])
         np.testing.assert_array_equal(got[1][k], c.download(capi.DENS_OUT, n)[0])
+
+
+def test_a_batch_whose_rows_do_not_fit_is_solved_over_lists():
+    """Rows take 1 KB a particle: a batch they have no room for takes the lists, which do not
+    need it, and gives the same results."""
+    sets = [_box(300000, 40), _box(300001, 41)]
+    L, c = capi.load(), capi.Cosmo()
+    out = []
+    assert c.set_option("batch_room_mb", -2) == -1
+    for room in (500, -1):
+        held = L.cosmo_serve_stat(b"device_bytes")
+        assert c.set_option("batch_room_mb", room) == 0
+        try:
+            st, b, got = _batch(sets)
+        finally:
+            c.set_option("batch_room_mb", -1)
+        assert st == 0 and b.scalar("blockTree") == (room < 0)
+        if room >= 0:     # no rows (a batch solved before may hold some already)
+            assert L.cosmo_serve_stat(b"device_bytes") - held < 600001 * 128 * 8 // 2
+        out.append(got)
+    for a, r in zip(*out):
+        for x, y in zip(a, r):
+            np.testing.assert_array_equal(x, y)
