@@ -305,12 +305,8 @@ gradient_warp_kernel(const __grid_constant__ NearTree t, const NearLoop* __restr
     if (lane == 0 && pairs) atomicAdd(&ds->pairs[1], pairs);
 }
 
-// Extras: the pairs a row must gain from another particle's support, kExtra places a
-// particle.  (Once appended to one list through one counter, then counted, scanned and placed:
-// where h scatters there are ten a particle, and the counter's atomics took 5 ms of a
-// 2-million-particle step.)  extraCnt counts them all, so a particle with more than fit shows.
-constexpr int kExtra = kQuintic ? 64 : 32;   // of 2 M quintic Plummer particles 1% gain more than 32
-
+// A pair j must gain from i's support, among j's extras (near.cuh); extraCnt counts them all, so
+// a particle with more than fit shows.
 __device__ __forceinline__ void add_extra(int* __restrict__ extras, int* __restrict__ extraCnt, int j, int i)
 {
     const int k = atomicAdd(extraCnt + j, 1);

@@ -43,6 +43,12 @@ constexpr int kNearWarps  = 4;     // warps per block of the search kernels
 constexpr int kWarpPerParticle = 32768;
 constexpr int kWarpPerParticleForce = 12288;
 
+// Extras: the pairs a row must gain from another particle's support, kExtra places a
+// particle.  (Once appended to one list through one counter, then counted, scanned and placed:
+// where h scatters there are ten a particle, and the counter's atomics took 5 ms of a
+// 2-million-particle step.)
+constexpr int kExtra = kQuintic ? 64 : 32;   // of 2 M quintic Plummer particles 1% gain more than 32
+
 // Whether a solve over the block tree loses to one over lists: a large set of which every
 // particle has more neighbours than a row holds -- 4/3 pi (R hfact)^3 of them at its converged
 // h -- is all searches of single particles, where a leaf's groups share theirs.  Device times

@@ -31,6 +31,7 @@
 #include <thread>
 #include <vector>
 
+#include "near.cuh"
 #include "state.hpp"
 #include "../../include/cosmosphere.h"
 
@@ -117,11 +118,15 @@ double now_s()
 }
 
 // Device bytes a new set of n particles is charged at admission, until its real footprint
-// is known: ≈ 1 KB of particle arrays, FP32 copies, tree and lists, plus the neighbour
-// rows -- 4 bytes (symmetric, j) and 8 bytes (Newton, r^2) per row entry, 128 entries
-// per particle for the cubic kernel and 256 for the quintic one.
-constexpr long long kBytesPerParticle = 1024 + 12 * (kQuintic ? 256 : 128);
-constexpr long long kBytesFixed = 1ll << 20;
+// is known.  Per particle: 21 result and caller-order arrays, 6 records, 12 n of transfers,
+// keys, order, flags and thermo (536 bytes with the row counts and h), the block tree and its
+// loop's lists (48), FP32 copies of the mixed form (48), the leaf tree and lists of the solves
+// that make them (about 5 KB a leaf of some 20 particles; lists are longer where h scatters
+// by more than a factor of two); the rows, 16 bytes an entry (r^2,
+// its j, the symmetric row's j), and the places of their extras.  Buffers take an eighth more
+// than was asked for.  Fixed: the grid a leaf tree starts from.
+constexpr long long kBytesPerParticle = 9 * (536 + 48 + 48 + 256 + 16 * kNbl + 4 * kExtra) / 8;
+constexpr long long kBytesFixed = 4ll << 20;
 
 struct Request
 {
