@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "near.cuh"
 #include "state.hpp"
 #include "tma.cuh"
 #include "../../include/cosmosphere.h"
@@ -138,12 +139,14 @@ size_t state_device_bytes(const State& s)
                     &s.preToBfs, &s.childOffsets, &s.internalToLeaf, &s.levelRange, &s.leafToInternal, &s.jlist,
                     &s.activeA, &s.activeB, &s.allLeaves, &s.nodeValsTmp, &s.leafNext, &s.nbl, &s.nblCount,
                     &s.rowItems, &s.jlistPrev, &s.walked, &s.walkScratch, &s.coverFlag, &s.coverLeaves, &s.extraCnt,
-                    &s.extras, &s.nblJ, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1],
-                    &s.nearSum[0], &s.nearSum[1], &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
+                    &s.extras, &s.nblJ, &s.frozen, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0],
+                    &s.nearBuild[1], &s.nearSum[0], &s.nearSum[1], &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
         add(*d);
     add(s.leafBox);
     add(s.nearNode);
     add(s.nearLoop);
+    add(s.nearSets);
+    add(s.nloop);
     add(s.items);
     for (auto* d : {&s.counts, &s.ops, &s.opsScan, &s.layout, &s.startBounds, &s.nodeCount, &s.leafPreStart, &s.jcount,
                     &s.jstream, &s.jOffset, &s.scanTmp, &s.sortHist, &s.sortBase, &s.sortLookback, &s.jOffsetPrev})
@@ -168,12 +171,13 @@ void release_state(State& s)
                     &s.preToBfs, &s.childOffsets, &s.internalToLeaf, &s.levelRange, &s.leafToInternal, &s.jlist,
                     &s.activeA, &s.activeB, &s.allLeaves, &s.nodeValsTmp, &s.leafNext, &s.nbl, &s.nblCount,
                     &s.rowItems, &s.jlistPrev, &s.walked, &s.walkScratch, &s.coverFlag, &s.coverLeaves, &s.extraCnt,
-                    &s.extras, &s.nblJ, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0], &s.nearBuild[1],
-                    &s.nearSum[0], &s.nearSum[1], &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
+                    &s.extras, &s.nblJ, &s.frozen, &s.nearRow[0], &s.nearRow[1], &s.nearBuild[0],
+                    &s.nearBuild[1], &s.nearSum[0], &s.nearSum[1], &s.nearHuge[0], &s.nearHuge[1], &s.nearCover, &s.nearOver})
         b->release(s.st);
     s.leafBox.release(s.st);
     s.nearNode.release(s.st);
     s.nearLoop.release(s.st);
+    s.nearSets.release(s.st);
     s.items.release(s.st);
     for (auto* b : {&s.counts, &s.ops, &s.opsScan, &s.layout, &s.startBounds, &s.nodeCount, &s.leafPreStart, &s.jcount,
                     &s.jstream, &s.jOffset, &s.scanTmp, &s.sortHist, &s.sortBase, &s.sortLookback, &s.jOffsetPrev})

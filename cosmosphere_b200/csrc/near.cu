@@ -268,7 +268,7 @@ __global__ void near_init_kernel(NearLoop* L, DevScalars* ds, int maxIter, int f
     L->cover = L->over = 0;
     L->cnt[0] = NearCounts{0, frozen ? 0 : n, 0, 0};
     L->cnt[1] = NearCounts{0, 0, 0, 0};
-    L->ticket[0] = L->ticket[1] = L->ticket[2] = L->ticket[3] = 0;
+    L->ticket[0] = L->ticket[1] = 0;
     ds->extraCount = 0;
     ds->mergeOverflow = 0;
     ds->rowOverflow = 0;
@@ -322,7 +322,7 @@ __global__ void near_forest_zero_kernel(NearLoop* L, int maxIter)
     L->all = 0;
     L->cover = L->over = 0;
     L->cnt[0] = L->cnt[1] = NearCounts{0, 0, 0, 0};
-    L->ticket[0] = L->ticket[1] = L->ticket[2] = L->ticket[3] = 0;
+    L->ticket[0] = L->ticket[1] = 0;
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -950,7 +950,7 @@ near_sum_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__ 
     for (;;)
     {
         int w = 0;
-        if (lane == 0) w = atomicAdd(&L->ticket[1], 1);
+        if (lane == 0) w = atomicAdd(&L->ticket[0], 1);
         w = __shfl_sync(0xffffffffu, w, 0);
         if (w >= n) break;
         const int i = list[w];
@@ -1055,7 +1055,7 @@ near_huge_kernel(const __grid_constant__ NearTree t, const NearSet* __restrict__
         __syncthreads();
         if (threadIdx.x == 0)
         {
-            sItem = atomicAdd(&L->ticket[3], 1);
+            sItem = atomicAdd(&L->ticket[1], 1);
             sSums = make_double2(0.0, 0.0);
         }
         __syncthreads();
@@ -1176,7 +1176,7 @@ __global__ void near_epilogue_kernel(NearLoop* L, cudaGraphConditionalHandle mor
     const int it = L->iter, cur = it & 1, nxt = cur ^ 1;
     if (it < kLoopIters) L->activePerIter[it] = L->active;
     L->cnt[cur] = NearCounts{};
-    L->ticket[0] = L->ticket[1] = L->ticket[3] = 0;
+    L->ticket[0] = L->ticket[1] = 0;
     L->all = 0;
     L->active = L->cnt[nxt].row + L->cnt[nxt].build + L->cnt[nxt].sum + L->cnt[nxt].huge;
     L->iter = it + 1;

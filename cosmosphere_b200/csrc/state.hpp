@@ -137,7 +137,7 @@ struct NearLoop
     int iter, maxIter, active;   // active: particles the next iteration updates
     int all;                     // the search list is every live particle
     int cover, over;             // rows still to be made at the converged h; those that do not fit one
-    int ticket[4];               // work tickets: row search, direct sums, cover search, direct sums by blocks
+    int ticket[2];               // work tickets: direct sums by warps, by blocks
     NearCounts cnt[2];
     long long activePerIter[kLoopIters];
     int queue[kNearQueues];      // the row search's work, one queue a multiprocessor
