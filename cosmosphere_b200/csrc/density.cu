@@ -1314,7 +1314,15 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
     s.hmaxNodeDone = !near;
     s.listsLoose = near;
     s.nearOverCount = 0;
-    if (near) s.listsSym = false;
+    if (near)
+    {
+        // nor does it count what only the list-based loop does
+        s.listsSym = false;
+        s.listTotal = 0;
+        s.settling0 = 0;
+        s.lastLoopRebuilds = s.lastLoopRowBuilds = 0;
+        s.loopListEntries.clear();
+    }
 
     // the host loop swaps the two active-leaf buffers every iteration: put them back in
     // one order, so that a graph captured with them serves the next solve too

@@ -272,6 +272,7 @@ __global__ void near_init_kernel(NearLoop* L, DevScalars* ds, int maxIter, int f
     ds->extraCount = 0;
     ds->mergeOverflow = 0;
     ds->rowOverflow = 0;
+    ds->coverNeed = 0;
 }
 
 // The initial search list with fixed particles (the caller's mask through the sort order;
@@ -1383,6 +1384,7 @@ static bool near_graph(State& s, const NearJob& j, int maxIter, bool defer)
 static void near_run(State& s, const NearJob& j, int maxIter, bool graph, bool defer)
 {
     s.lastLoopGraph = 0;
+    s.nearLate.clear();
     if (graph && maxIter > 0 && maxIter <= kLoopIters && near_graph(s, j, maxIter, defer))
     {
         s.lastLoopGraph = 1;
@@ -1394,6 +1396,7 @@ static void near_run(State& s, const NearJob& j, int maxIter, bool graph, bool d
         COSMO_CUDA(cudaMemcpyAsync(s.hsmall, s.nearLoop.get(), 4 * sizeof(int), cudaMemcpyDeviceToHost, s.st));
         COSMO_CUDA(cudaStreamSynchronize(s.st));
         if (s.hsmall[2] == 0) break;
+        if (it + 1 >= kLoopIters && it + 1 < maxIter) s.nearLate.push_back(s.hsmall[2]);
     }
 }
 
@@ -1439,6 +1442,7 @@ long long near_results(State& s, const NearLoop& h)
     if (s.lastLoopGraph) g_launches += (unsigned long long)h.iter * s.nearKernels;
     s.itersRun = h.iter;
     s.activePerIter.assign(h.activePerIter, h.activePerIter + std::min(h.iter, kLoopIters));
+    s.activePerIter.insert(s.activePerIter.end(), s.nearLate.begin(), s.nearLate.end());
     return h.active;
 }
 

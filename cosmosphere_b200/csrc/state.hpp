@@ -247,6 +247,7 @@ struct State
     cudaGraphExec_t nearGraphExec = nullptr;
     std::vector<unsigned char> nearGraphKey, nearKeyPending;
     unsigned long long nearKernels = 0;              // kernels of one iteration
+    std::vector<int> nearLate;                       // active particles of its iterations beyond kLoopIters
     int nearOverCount = 0;                           // particles the last solve left without a row
     unsigned long long loopKernels[3] = {0, 0, 0};   // kernels of the body, the list branch, the rows branch
     int loopGraphBuilds = 0, loopGraphUpdates = 0;

@@ -257,3 +257,21 @@ def test_a_set_outside_its_box_is_solved_once():
             np.testing.assert_array_equal(a, b)
     assert first[3] <= lists[3] + 24
     assert again[3] <= lists[3] + 8
+
+
+def test_counts_of_every_iteration():
+    """activePerIter has an entry an iteration, however many there are."""
+    st, c = _solve(_box(3000, 13), UNIT, tolh=1e-18, max_iter=150)
+    assert st == 1 and c.scalar("itersRun") == 150
+    assert c.array("activePerIter").size == 150
+
+
+def test_list_loop_counts_belong_to_the_last_solve():
+    """What only the list-based loop counts is not left from an earlier solve of it."""
+    st, c = _solve(inputs.plummer(6000, hfact=1.2, lnsigma=0.9, seed=12), options=LISTS)
+    assert st == 0 and c.scalar("listTotal") > 0 and c.scalar("settling0") > 0
+    st, c = _solve(_box(6000, 14), UNIT)
+    assert st == 0
+    for k in ("listTotal", "settling0", "loopRebuilds", "loopRowBuilds", "coverNeed"):
+        assert c.scalar(k) == 0, k
+    assert c.array("loopListEntries").size == 0
