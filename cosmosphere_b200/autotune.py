@@ -20,6 +20,11 @@ particle's sums run over its accepted pairs in ascending j whatever the tree, th
 or the cut, so a tuned solve returns the same h, rho and d(rho)/dh bit for bit.  In the
 mixed form they change only how FP32 partial sums are grouped.
 
+They act on the batches that are solved over lists: mixed and staged ones, and of the plain
+ones those that the block tree does not serve (very large, very many neighbours, a particle
+outside its set's box).  For a class whose first timed solve ran over the block tree there is
+nothing to tune, and the table holds the defaults.
+
 Host-only logic; the timed solves go through `capi.Batch`.
 """
 from __future__ import annotations
@@ -202,6 +207,12 @@ def confirm(sets, table: "Table", repeats: int = 2, timer: Callable = batch_time
     return best, t_tuned, t_default
 
 
+def settings_act() -> bool:
+    """Whether the last batched solve ran over lists, so that these parameters act on it."""
+    from . import capi
+    return float(capi.load().cosmo_batch_scalar(b"blockTree")) == 0.0
+
+
 def tune(sets, max_particles: float = 2.0e6, repeats: int = 2, sweeps: int = 1,
          candidates: Dict[str, tuple] = CANDIDATES, timer: Callable = solve_time,
          classes: Iterable[int] | None = None) -> Table:
@@ -212,12 +223,19 @@ def tune(sets, max_particles: float = 2.0e6, repeats: int = 2, sweeps: int = 1,
     by_class: Dict[int, List[int]] = {}
     for k, n in enumerate(sizes):
         by_class.setdefault(size_class(n), []).append(k)
+    acts = settings_act if timer is solve_time else (lambda: True)
     wanted = set(by_class) if classes is None else set(classes) & set(by_class)
     table = Table()
     for c in sorted(wanted):
         idx = sample_sets(sizes, by_class[c], max_particles)
         sample = [sets[k] for k in idx]
-        best, cost, tried = coordinate_descent(lambda t: timer(sample, t, repeats), DEFAULT, candidates, sweeps)
+        first = timer(sample, DEFAULT, repeats)
+        if acts():
+            known = {DEFAULT: first}
+            best, cost, tried = coordinate_descent(
+                lambda t: known.pop(t) if t in known else timer(sample, t, repeats), DEFAULT, candidates, sweeps)
+        else:
+            best, cost, tried = DEFAULT, first, [(DEFAULT, first)]
         table.entries[c] = best
         table.times[c] = {"sets": len(idx), "particles": int(sum(sizes[k] for k in idx)),
                           "default_s": next(v for t, v in tried if t == DEFAULT), "tuned_s": cost,

@@ -1,8 +1,10 @@
-"""The batched form where it leaves the common path: iterations running out before every h
-has converged."""
+"""The batched form where it leaves the common path: iterations running out before every h has
+converged, and the batches that are solved over lists (many neighbours, rows that do not
+fit, a set outside its box, the settings of that loop)."""
 import numpy as np
 import pytest
 
+from cosmosphere_b200 import autotune as at
 from cosmosphere_b200 import capi, inputs
 
 pytestmark = pytest.mark.gpu
@@ -139,3 +141,53 @@ def test_a_batch_whose_rows_do_not_fit_is_solved_over_lists():
     for a, r in zip(*out):
         for x, y in zip(a, r):
             np.testing.assert_array_equal(x, y)
+
+
+SETTINGS = [dict(bucket=16), dict(bucket=128), dict(bucket=512), dict(list_margin=1.0), dict(list_margin=1.3),
+            dict(split_stream=32, split_work=32),
+            dict(bucket=[16, 128, 32, 64], list_margin=[1.0, 1.3, 1.05, 1.15],
+                 split_stream=[2048, 32, 4096, 8192], split_work=[65536, 64, 262144, 131072])]
+
+
+@pytest.fixture(scope="module")
+def mixture():
+    return [_box(4000, 50), _plummer(9000, 51, 0.2), _box(700, 52), _plummer(3000, 53, 0.6)]
+
+
+@pytest.fixture(scope="module")
+def near_results(mixture):
+    st, b, got = _batch(mixture, final_rho=True)
+    assert st == 0 and b.scalar("blockTree") == 1
+    return got
+
+
+# a staged batch and one with a particle outside its box run over lists, where the settings act
+@pytest.mark.parametrize("setting", [{}] + SETTINGS)
+@pytest.mark.parametrize("staging", [True, False])
+def test_settings_of_the_list_loop_keep_the_plain_results(mixture, near_results, setting, staging):
+    sets = mixture
+    if not staging:
+        out = _box(40, 54)
+        out["x"] = out["x"].copy()
+        out["x"][3] -= 1.2
+        sets = mixture + [out]
+        setting = {k: list(v) + [v[0]] if isinstance(v, list) else v for k, v in setting.items()}
+    st, b, got = _batch(sets, staging=staging, tuning=setting or None, final_rho=True)
+    assert st == 0 and b.scalar("blockTree") == 0
+    for a, r in zip(got, near_results):
+        for x, y in zip(a, r):
+            np.testing.assert_array_equal(x, y)
+
+
+def test_a_plain_batch_has_nothing_to_tune(mixture):
+    """The tuner times a plain class once and keeps the defaults; a mixed one it tunes."""
+    cands = {"bucket": (32, 64), "list_margin": (1.05, 1.15), "split_stream": (4096,), "split_work": (131072,)}
+    for mixed in (False, True):
+        capi.Cosmo().set_precision(mixed)
+        try:
+            table = at.tune(mixture, repeats=1, candidates=cands)
+        finally:
+            capi.Cosmo().set_precision(False)
+        for c, t in table.entries.items():
+            assert table.times[c]["evaluated"] == (3 if mixed else 1)
+            assert mixed or t == at.DEFAULT
