@@ -928,12 +928,12 @@ def run_particles(args, rank, world, local, dist, p, quintic, metric, label):
                      "algorithmic_bytes_per_iteration": BYTES_PER_DENSITY_UPDATE * head["nr_upd"]
                                                         / max(1, head["nr_launches"]),
                      "traffic": (ncu_traffic("newton_stage_per_iteration")
-                                 if args.workload == "lattice100" and args.npartx == 100 and not quintic
-                                 and not args.periodic else None),
-                     "traffic_note": "DRAM bytes per Newton iteration assembled from one-kernel ncu captures "
-                                     "(profiles/traffic.json, method in its note); above the algorithmic bytes "
-                                     "because the Newton rows (r^2 per pair) are written once and streamed by the "
-                                     "later iterations",
+                                 if plain is not None and args.workload == "lattice100" and args.npartx == 100
+                                 and not quintic and not args.periodic else None),
+                     "traffic_note": "DRAM bytes per Newton iteration, every launch of one step's loop captured by "
+                                     "ncu (profiles/traffic.json, method in its note); above the algorithmic bytes "
+                                     "because the rows (r^2 and j per pair) are written once and their r^2 streamed "
+                                     "by every iteration",
                      "fp64": {"achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved / fp64_peak,
                               "flop_convention": "30 FLOP per accepted pair + 30 per Newton update",
                               "peak_source": "FP64 FMA microkernel run in this bench "

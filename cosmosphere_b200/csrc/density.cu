@@ -1208,7 +1208,7 @@ static void sym_rows_from_newton(State& s, bool near)
     if (near)
     {
         auto ov = s.periodic ? over_extras_kernel<true> : over_extras_kernel<false>;
-        ov<<<std::min(iceil(nA, kWarpsPerBlock), 4 * s.numSMs), kThreads, 0, s.st>>>(
+        ov<<<std::min(iceil(nA, kWarpsPerBlock), near_over_blocks(s.hfact) * s.numSMs), kThreads, 0, s.st>>>(
             near_tree(s), s.nearLoop.get(), s.nearOver.get(), s.hs.get(), s.nblH.get(), s.extras.get(),
             s.extraCnt.get(), ds);
         COSMO_LAUNCHED();
@@ -1586,7 +1586,7 @@ DensResult solve_density(State& s, int n, double pmass, const double* periodicBo
             }
             if (near && fromRows && s.nAlive > 0)
                 warps(s.periodic ? gradient_warp_kernel<true, false> : gradient_warp_kernel<false, false>,
-                      std::min(iceil(s.nAlive, kWarpsPerBlock), 4 * s.numSMs));
+                      std::min(iceil(s.nAlive, kWarpsPerBlock), near_over_blocks(hfact) * s.numSMs));
             // the group sweep of the rows that overflowed (none: it returns at once)
             auto gk = s.periodic ? gradient_kernel<true> : gradient_kernel<false>;
             if (!(near && fromRows)) gk<<<grid, kThreads, 0, s.st>>>(s.nLeaves, s.layout.get(), s.jOffset.get(), s.jcount.get(), s.jlist.get(),

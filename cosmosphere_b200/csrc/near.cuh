@@ -36,10 +36,16 @@ constexpr int kNearBlocks = 128;   // blocks a warp holds at once
 constexpr int kNearWarps  = 4;     // warps per block of the search kernels
 
 // Up to this many particles a pass over rows gives each particle a warp: one lane each would
-// leave most of the chip idle and last as long as the longest row.  648 particles: Newton step
-// 33 -> 9 us an iteration, gradient 54 -> 16, force 66 -> 17; 20,000: gradient 82 -> 65, force
-// 93 -> 115 (its energy sum is four dependent additions a pair), so its line lies lower;
-// 120,000: gradient 181 -> 337.
+// leave most of the chip idle and last as long as the longest row.  Device us with a lane and
+// with a warp a particle, lattice and periodic box of random particles:
+//   particles       4,000              16,000             24,000             32,000
+//   Newton loop     135  92, 372 224   162 145, 436 330   174 180, 486 410   176 204, 514 470
+//   symmetric rows   34  25, 118  75    34  32, 136  98    38  36, 115  87    38  40, 130  99
+//   gradient         58  30,  74  31    62  58,  84  62    66  83,  89  81    67 105,  87 103
+//   force            60  30,  85  32    64  84,  91  94    69 126,  96 133    71 162, 101 175
+// (48,000: the Newton loop 209 269, 597 623.)  The three passes of a solve together draw level
+// between 24,000 (lattice) and above 32,000 (box, with more iterations); the force pass, whose
+// energy sum is four dependent additions a pair, at 12,000 (65 70, 88 73).
 constexpr int kWarpPerParticle = 32768;
 constexpr int kWarpPerParticleForce = 12288;
 
@@ -58,11 +64,20 @@ constexpr int kExtra = kQuintic ? 64 : 32;   // of 2 M quintic Plummer particles
 // (a Plummer sphere 10.8 and 26.0).  Batches (whole solve): 10 boxes of 10,000 at 1.6 3.0
 // and 3.5, 6 of 100,000 15.5 and 11.4, 24 of 100,000 60.0 and 40.4.
 constexpr int kNearCrowded = 400000;
-inline bool near_crowded(int n, double hfact)
+
+// The neighbours of a converged particle, over what a row holds.
+inline double near_fill(double hfact)
 {
     const double reach = kRadKernel * hfact;
-    return n > kNearCrowded && 4.18879 * reach * reach * reach > 0.95 * kNbl;
+    return 4.18879 * reach * reach * reach / kNbl;
 }
+inline bool near_crowded(int n, double hfact) { return n > kNearCrowded && near_fill(hfact) > 0.95; }
+
+// Blocks a multiprocessor for the sweeps of the particles without a row, whose number is on
+// the device: four where an average particle comes near not fitting one (150,000 in a box at
+// hfact 1.6, nearly all of them: gradient 2.3 -> 1.3 ms with the packed pairs), else
+// two: there are few or none.
+inline int near_over_blocks(double hfact) { return near_fill(hfact) > 0.6 ? 4 : 2; }
 
 // A node's box: centre, half extents (empty: negative infinity) and its largest h.
 struct alignas(32) NearNode

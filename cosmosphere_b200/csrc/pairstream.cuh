@@ -3,7 +3,7 @@
  *
  * A warp owns one group of up to 32 i-particles of one leaf (one per lane).  It walks
  * the leaf's j-leaf list in ascending order, loading 32 consecutive j particles per
- * batch with coalesced 128-bit loads.  Each j is tested ONCE, by the lane that loaded
+ * batch with coalesced 256-bit loads.  Each j is tested ONCE, by the lane that loaded
  * it, against a conservative box around the whole group (the "group filter"); the
  * survivors are compacted with a ballot, in order, into a per-warp shared-memory ring,
  * and every lane then evaluates them one by one (broadcast reads).  A j rejected by the
