@@ -44,12 +44,15 @@ constexpr int kTest = 8;     // mixed: candidates a lane tests in one turn of it
 // thousands of candidates) is tested with a candidate a lane, and its kept pairs are evaluated
 // by all lanes and only added by their owners: with a particle a lane most lanes had nothing
 // to test or evaluate (the loop of a 30,000-particle Plummer sphere 16.9 -> 12.9 ms, 9 sets of
-// 6,000 to 18,000 8.5 -> 7.1, 40 sets of 10,000 to 300,000 48.1 -> 46.4; lines at 12 and 16
-// instead measured no better).  Its columns lie one after the other, with as much room again
-// for the second term: 126 pairs of two terms for each of eight particles fit in the columns'
-// 2048 words beside the particles' own data, and 252 words a particle keep the owners'
-// accesses on different banks.
-constexpr int kFew = 8;
+// 6,000 to 18,000 8.5 -> 7.1, 40 sets of 10,000 to 300,000 48.1 -> 46.4).  Lines at 8, 12 and
+// 16: a quintic Plummer sphere of 14,000, whose cut groups hold nine, 13.0, 10.2 and 10.5 ms
+// (with the plain form's records 12.3), of 8,000 (sixteen) 7.7, 7.7 and 7.0 (7.9), cubic ones
+// 8.8, 8.2, 8.6 (10.3) and 5.6, 5.5, 5.8 (6.3).  Its columns
+// lie one after the other, with as much room again for the second term: 118 pairs of two
+// terms for each of eight particles, or 82 for each of twelve, fit in the columns' 2048 words
+// beside the particles' own data; 236 words a particle keep the owners' accesses on
+// different banks, 164 all but four of them.
+constexpr int kFew = 12;
 constexpr int kColumn = 64;   // mixed: accepted pairs a lane keeps before they are evaluated
 
 template<bool Mixed>
@@ -226,7 +229,7 @@ __device__ __forceinline__ void density_group(unsigned char* scr, bool mine, int
         // particles, one after the other with as much room again for the second term
         const bool few = ng <= kFew;
         float* columns = rx + 3 * kRing;
-        const int room = few ? 126 : kColumn;
+        const int room = few ? (ng <= 8 ? 118 : 82) : kColumn;
         float* column = columns + (few ? 2 * room * lane : lane);
         float* member = columns + kColumn * 32 - 4 * kFew;   // few: x, y, z, 1/h^2 of kFew each
         // relative coordinates at the centre's nearest image are every accepted pair's
