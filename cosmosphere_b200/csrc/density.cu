@@ -1225,8 +1225,8 @@ static void sym_rows_from_newton(State& s, bool near)
 // very many neighbours (near_crowded) and a solve asked for a variant of the list-based loop.
 static bool near_solve(const State& s, int n, double hfact, bool withGradients)
 {
-    return withGradients && !near_crowded(n, hfact) && s.precision == 0 && s.staging == 0 && s.splitStream == 0 && s.splitWork == 0 &&
-           s.spreadGroups == 0 && s.graphListStorePct == 0;
+    return withGradients && !near_crowded(n, hfact) && s.precision == 0 && s.staging == 0 && s.splitStream == 0 &&
+           s.splitWork == 0 && s.spreadGroups == 0 && s.graphListStorePct == 0;
 }
 
 DensResult solve_density(State& s, int n, double pmass, const double* periodicBox, double tolh, double hfact,
