@@ -170,8 +170,9 @@ gradient_row_kernel(int nAlive, const int* __restrict__ nbl, const int* __restri
                     double pmass, const DevBox* __restrict__ box, DevScalars* __restrict__ ds,
                     const NearLoop* __restrict__ L, double halfBox)
 {
+    const int live = ds->nAlive;
     if (near_failed(L, ds, halfBox)) return;
-    nAlive = min(nAlive, ds->nAlive);
+    nAlive = min(nAlive, live);
     double lx = 0, ly = 0, lz = 0;
     if (Periodic) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
     unsigned long long pairs = 0;
@@ -220,9 +221,8 @@ gradient_warp_kernel(const __grid_constant__ NearTree t, const NearLoop* __restr
     __shared__ NearScratch sScr[Rows ? 1 : kWarpsPerBlock];
     __shared__ double sTerm[kWarpsPerBlock][32 * kGradTerms];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (near_failed(L, ds, halfBox)) return;
     const int n = Rows ? min(nAlive, ds->nAlive) : L->over;
-    if (n == 0) return;
+    if (near_failed(L, ds, halfBox) || n == 0) return;
     if (!Rows && blockIdx.x == 0 && threadIdx.x == 0) ds->rowOverflow = 1;
     const NearFrame f(t.box);
     const NearView v = near_view(t, f);
@@ -523,27 +523,28 @@ struct SymTest
 // double as the force pass's dr^2) that the force pass takes,
 // dr^2 < R^2 max(h_i^2, h_j^2) (1 + 1e-10) -- sym_rows_kernel's test -- written in the
 // same order into the interleaved rows of the gradient and force passes (hs: h in the
-// sorted order, 8 bytes a particle).  A pair the force pass takes because of this
-// particle's support (dr^2 < R^2 h_i^2 (1 + 1e-10)) is in j's Newton row too unless dr^2
-// reaches the radius j's row covers (R rowH, with 1e-9 to spare; only a pair beyond j's
-// own support can); such a pair puts i among j's extras, to be merged into j's row.  The mixed form's rows hold that double rounded to float (within 2^-24 of
-// it): where it lies within 1e-6 of a bound the test uses, dr^2 is taken again from the
-// positions, so every test decides as on the double and the rows are the same.
+// sorted order, 8 bytes a particle; live: how many have rows -- a warp per particle waits
+// for each word it asks for first, 4 us of a 20,000-particle pass for a second one).  A pair
+// the force pass takes because of this particle's support (dr^2 < R^2 h_i^2 (1 + 1e-10)) is
+// in j's Newton row too unless dr^2 reaches the radius j's row covers (R rowH, with 1e-9 to
+// spare; only a pair beyond j's own support can); such a pair puts i among j's extras, to be
+// merged into j's row.  The mixed form's rows hold that double rounded to float (within
+// 2^-24 of it): where it lies within 1e-6 of a bound the test uses, dr^2 is taken again from
+// the positions, so every test decides as on the double and the rows are the same.
 template<class T, bool Periodic>
 __global__ void __launch_bounds__(kThreads)
 sym_from_rows_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __restrict__ rowsR2,
                      int* __restrict__ nblCount, const double* __restrict__ hs, const double* __restrict__ rowH,
                      const double4* __restrict__ xyzh, const DevBox* __restrict__ box, int* __restrict__ nbl,
                      int* __restrict__ extras, int* __restrict__ extraCnt, DevScalars* __restrict__ ds,
-                     const int* __restrict__ skip)
+                     const int* __restrict__ live)
 {
-    if (skip != nullptr && *skip) return;
     constexpr bool kExact = std::is_same<T, double>::value;
     using R4 = typename std::conditional<kExact, double4, float4>::type;
     double lx = 0, ly = 0, lz = 0;
     if (Periodic && !kExact) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
     int added = 0;
-    nAlive = min(nAlive, ds->nAlive);
+    nAlive = min(nAlive, *live);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nAlive; i += gridDim.x * blockDim.x)
     {
         const int cnt = nblCount[i];
@@ -614,15 +615,14 @@ sym_from_rows_warp_kernel(int nAlive, const int* __restrict__ rowsJ, const T* __
                           int* __restrict__ nblCount, const double* __restrict__ hs, const double* __restrict__ rowH,
                           const double4* __restrict__ xyzh, const DevBox* __restrict__ box, int* __restrict__ nbl,
                           int* __restrict__ extras, int* __restrict__ extraCnt, DevScalars* __restrict__ ds,
-                          const int* __restrict__ skip)
+                          const int* __restrict__ live)
 {
-    if (skip != nullptr && *skip) return;
     constexpr bool kExact = std::is_same<T, double>::value;
     double lx = 0, ly = 0, lz = 0;
     if (Periodic && !kExact) { lx = box->len[0]; ly = box->len[1]; lz = box->len[2]; }
     const int lane = threadIdx.x & 31;
     int added = 0;
-    nAlive = min(nAlive, ds->nAlive);
+    nAlive = min(nAlive, *live);
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nAlive; i += (gridDim.x * blockDim.x) >> 5)
     {
         const int cnt = nblCount[i];
@@ -1193,7 +1193,7 @@ static void sym_rows_from_newton(State& s, bool near)
     auto compact = [&](auto kern, const auto* rows) {
         kern<<<grid, kThreads, 0, s.st>>>(nA, s.nblJ.get(), rows, s.nblCount.get(), s.hs.get(), s.nblH.get(),
                                           s.xyzh.get(), s.box.get(), s.nbl.get(), s.extras.get(), s.extraCnt.get(), ds,
-                                          near ? &ds->outside : nullptr);   // a loop that was not run made no rows
+                                          near ? &ds->rowsLive : &ds->nAlive);
     };
     // the mixed form's Newton rows hold FP32 r^2 in the same buffer
     const float* rowsF = reinterpret_cast<const float*>(s.nblR2.get());

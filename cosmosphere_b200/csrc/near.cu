@@ -260,7 +260,8 @@ __global__ void near_init_kernel(NearLoop* L, DevScalars* ds, int maxIter, int f
 {
     L->queue[threadIdx.x] = 0;
     if (threadIdx.x != 0) return;
-    const int n = ds->outside ? 0 : ds->nAlive;
+    const int live = ds->nAlive, outside = ds->outside;
+    const int n = outside ? 0 : live;
     L->iter = 0;
     L->maxIter = maxIter;
     L->active = n;
@@ -273,6 +274,7 @@ __global__ void near_init_kernel(NearLoop* L, DevScalars* ds, int maxIter, int f
     ds->mergeOverflow = 0;
     ds->rowOverflow = 0;
     ds->coverNeed = 0;
+    ds->rowsLive = n;
 }
 
 // The initial search list with fixed particles (the caller's mask through the sort order;

@@ -108,6 +108,7 @@ struct DevScalars
     int leafStart;               // leaves of the grid the leaf tree's refinement starts from
     int leafDone;                // that grid is the leaf tree (no node of it holds more than kBucket)
     unsigned long long hmaxConv; // bits of the largest converged h (the block-tree loop)
+    int rowsLive;                // live particles of the block-tree loop (0: it was not run)
     int outside;                 // some live particle lies outside the box its key is taken in (box_left)
 };
 
